@@ -158,7 +158,10 @@ extern "C" parsec_context_t *dplasma_b200_init(int device)
     ctx->stream_cb = getenv_int("DPLASMA_B200_STREAM_CB", 8);
     ctx->no_stream = getenv_int("DPLASMA_B200_NO_STREAM", 0) != 0;
     ctx->stream_trace = getenv_int("DPLASMA_B200_STREAM_TRACE", 0) != 0;
-    ctx->potrf_delay = getenv_int("DPLASMA_B200_DELAY", 3 * ctx->potrf_grid);
+    ctx->potrf_delay = getenv_int("DPLASMA_B200_DELAY", ctx->potrf_grid);
+    ctx->f64_chunk = std::min(15, std::max(0, getenv_int("DPLASMA_B200_F64_CHUNK", 0)));
+    // blocks of 16 x 16 keep the operands of neighbouring tasks in L2 (N = 32768: 0.1 %)
+    ctx->f64_block = getenv_int("DPLASMA_B200_F64_BLOCK", 16);
     ctx->mx_delay = getenv_int("DPLASMA_B200_MX_DELAY", 6 * ctx->potrf_grid);
     ctx->wave_occ = getenv_int("DPLASMA_B200_NO_WAVE", 0) ? 0 : wave_max_blocks_per_sm();
     int occs = sweep_max_blocks_per_sm();

@@ -77,7 +77,9 @@ struct Context {
     void *bufs[BUF_COUNT] = {};
     size_t bufsz[BUF_COUNT] = {};
     int task_mt = -1, task_nbs = -1, task_delay = -1, ntasks = 0;
-    int task_mixed = 0;                      // chunk size of the cached mixed task list (0: FP64 list)
+    int task_mixed = 0;                      // chunk size of the cached task list (> 0 mixed, < 0 FP64 blocks)
+    int f64_chunk = 0;                       // 128-wide panels per FP64 update task (0: by size)
+    int f64_block = 0;                       // blocked order of the FP64 update tasks (block columns and rows; 0: by columns)
     int mx_chunk = 0;                        // panels per mixed-precision update task (0: by operand form)
     int mx_block_w = 0, mx_block_h = 0;      // blocked order of the mixed update tasks (tile columns x rows; 0: by columns)
     int stream_cb = 0;                       // tile columns per phase of the streamed factorization (0: 16)

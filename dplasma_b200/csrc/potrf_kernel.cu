@@ -46,6 +46,7 @@ template <bool MIXED>
 __device__ __forceinline__ int all_updates(const PotrfArgs &a, int m, int n)
 {
     if (MIXED) return (n + a.mx_chunk - 1) / a.mx_chunk;
+    if (a.fchunk) return block_updates(n, a.fchunk);
     return n * step_blocks<MIXED>(a, m, n);
 }
 
@@ -86,6 +87,15 @@ __device__ bool wait_deps(const PotrfArgs &a, uint64_t t)
                    wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
                    wait_geq(a.upd_done + (int64_t)m * a.mt + n, k, a.abort_flag, a.status, a.dep_limit_ns);
         }
+        if (a.fchunk) {
+            // block order: panels [k, kl]; as above the last panel's strips
+            // imply the earlier ones, and a block's updates run in order
+            const int kl = k + task_bi(t) - 1;
+            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, 1, a.abort_flag, a.status, a.dep_limit_ns) &&
+                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, 1, a.abort_flag, a.status, a.dep_limit_ns) &&
+                   wait_geq(a.upd_done + (int64_t)m * a.mt + n, block_update_index(k, n, a.fchunk), a.abort_flag,
+                            a.status, a.dep_limit_ns);
+        }
         return wait_geq(a.trsm_done + (int64_t)m * a.mt + k, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
                wait_geq(a.trsm_done + (int64_t)n * a.mt + k, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
                wait_geq(a.upd_done + (int64_t)m * a.mt + n, k * step_blocks<MIXED>(a, m, n), a.abort_flag, a.status,
@@ -106,6 +116,53 @@ __device__ __forceinline__ unsigned char *ring16_of(double *ring)
 }
 
 // ---------------------------------------------------------------------------
+// ticket selection.  With potrf_pos set, one CTA (the first to start) runs
+// every POTRF: its code then stays in that SM's instruction caches, where a
+// POTRF on a CTA that had not run one for a while spent a third of its time on
+// instruction fetch (123 against about 80 us for a 128-wide tile).  That CTA
+// takes its tasks in ticket order too, so every task it runs depends on tasks
+// earlier in the order only; it draws other tickets while its next POTRF is
+// more than a grid's width ahead, or when tickets before it stay undrawn (no
+// other CTA may be resident).  The others pass over POTRF tickets.  One lane.
+// ---------------------------------------------------------------------------
+struct ChainState {
+    int next;      // next POTRF
+    int carry;     // a drawn ticket beyond potrf_pos[next], or -1
+};
+__device__ __forceinline__ int draw_ticket(const PotrfArgs &a)
+{
+    int t;
+    do t = atomicAdd(a.ticket, 1);
+    while (a.potrf_pos && t < a.ntasks && task_type(a.tasks[t]) == T_POTRF);
+    return t;
+}
+template <bool MIXED>
+__device__ int chain_ticket(const PotrfArgs &a, ChainState &cs)
+{
+    const int pp = cs.next < a.mt ? a.potrf_pos[cs.next] : 0x7fffffff;
+    if (cs.carry < 0) {
+        const int margin = gridDim.x > 1 ? (int)gridDim.x : 0;
+        bool draw = ld_volatile(a.ticket) < pp - margin;
+        if (!draw) {
+            const uint64_t t0 = globaltimer_ns();
+            while (!draw && ld_volatile(a.ticket) < pp && !ld_volatile(a.abort_flag) &&
+                   ld_acquire(a.upd_done + (int64_t)cs.next * a.mt + cs.next) < all_updates<MIXED>(a, cs.next, cs.next)) {
+                draw = globaltimer_ns() - t0 > 20000;
+                __nanosleep(64);
+            }
+        }
+        if (draw) cs.carry = draw_ticket(a);
+    }
+    if (cs.carry >= 0 && cs.carry < pp) {
+        const int t = cs.carry;
+        cs.carry = -1;
+        return t;
+    }
+    cs.next++;
+    return pp;
+}
+
+// ---------------------------------------------------------------------------
 // producer warp
 // ---------------------------------------------------------------------------
 template <bool MIXED>
@@ -121,10 +178,12 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
         if (a.tc_trsm) tma_prefetch_desc(lmap);
     }
     bool pipe_ok = true;
+    const bool chain = ctl->chain != 0;
+    ChainState cs = {0, -1};
     int prev_mode = -1;      // MIXED: 0 FP64 ring, 1 16-bit ring (same shared memory)
     while (true) {
         int tk = -1;
-        if (lane == 0) tk = ld_volatile(a.abort_flag) ? -1 : atomicAdd(a.ticket, 1);
+        if (lane == 0 && !ld_volatile(a.abort_flag)) tk = chain ? chain_ticket<MIXED>(a, cs) : draw_ticket(a);
         tk = __shfl_sync(0xffffffffu, tk, 0);
         bool end = (tk < 0 || tk >= a.ntasks);
         uint64_t t = end ? 0 : a.tasks[tk];
@@ -290,7 +349,15 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
                 epi_it++;
                 fence_proxy_async();
             }
+            // block order: the operands change with each panel of 128
+            const bool panels = !MIXED && a.fchunk && ty == T_GEMM;
+            const double *Aop = jb.A, *Bop = jb.B;
             for (int k0 = 0; k0 < jb.K; k0 += BK) {
+                if (panels && (k0 & (BLK - 1)) == 0) {
+                    const int j = task_k(t) + k0 / BLK;
+                    Aop = tile_ptr(a, task_m(t), j) - (int64_t)k0 * jb.lda;
+                    Bop = tile_ptr(a, task_n(t), j) - (int64_t)k0 * jb.ldb;
+                }
                 const uint32_t s = stage_it % NST, r = stage_it / NST;
                 if (r > 0 && !warp_mbar_wait(&ctl->empty[s], (r - 1) & 1, a.pipe_limit_ns)) {
                     if (lane == 0) report(a, ST_MBAR_TIMEOUT, 4, stage_it, tk);
@@ -302,10 +369,10 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
                 if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * BK * BLK * (uint32_t)sizeof(double));
                 __syncwarp();
                 if (lane < BK)
-                    bulk_g2s(As + lane * SP, jb.A + (int64_t)(k0 + lane) * jb.lda, BLK * sizeof(double),
+                    bulk_g2s(As + lane * SP, Aop + (int64_t)(k0 + lane) * jb.lda, BLK * sizeof(double),
                              &ctl->full[s]);
                 else
-                    bulk_g2s(Bs + (lane - BK) * SP, jb.B + (int64_t)(k0 + lane - BK) * jb.ldb,
+                    bulk_g2s(Bs + (lane - BK) * SP, Bop + (int64_t)(k0 + lane - BK) * jb.ldb,
                              BLK * sizeof(double), &ctl->full[s]);
                 stage_it++;
             }
@@ -337,7 +404,12 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
     constexpr uint32_t NST = MIXED ? NSTAGE_MIXED : NSTAGE;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int wm = warp & 1, wn = warp >> 1;
+    // the two warps of a sub-partition (w and w + 4) get column groups 0 and 3
+    // or 1 and 2, so a triangular operand loads all four alike
+    const int wm = warp & 1, wn = warp < 4 ? warp >> 1 : 5 - (warp >> 1);
+    // columns this warp forms end at K = klim (triangular B), and a block on
+    // the diagonal needs nothing right of column 64 in its upper rows
+    const int klim = jb.tri ? 32 * (wn + 1) : (jb.mode == J_SUB_LOWER && wm == 0 && wn >= 2) ? 0 : jb.K;
     double acc[4][4][4];
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
@@ -355,6 +427,7 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
         }
         const double *As = ring + s * STAGE_DOUBLES + wm * 64 + g;
         const double *Bs = ring + s * STAGE_DOUBLES + BK * SP + wn * 32 + g;
+        if (k0 < klim) {
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 4) {
             double af[4][2], bf[4];
@@ -370,6 +443,7 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
             for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
+        }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl->empty[s]);
@@ -562,21 +636,9 @@ template <bool MIXED>
 __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int nbi = a.nbi;
+    const int nbi = a.ld;
     double *T = tile_ptr(a, k, k);
     double *Wk = wblk_ptr(a, k, 0);
-    double *Ls = ring;               // 32 x 33, row-major
-    double *Dv = Ls + 32 * 33;       // 32 x 33, row-major: inverse of the 32x32 diagonal block
-    double *colb = Dv + 32 * 33;     // 32 (+pad)
-    double *Xs = colb + 64;          // panel X, [c][r] with pitch XP
-    double *Sw = colb + 64;          // W assembly staging (aliases Xs, used afterwards)
-    const int XP = nbi + 4;
-    double *Lb = Xs + 32 * XP;       // [8][32][4]: blocked copy of the 32x32 factor
-
-    for (int e = tid; e < a.nbs * BLK * BLK; e += NCONS) Wk[e] = 0.0;
-    if (tid == 0) ctl->fail = 0;
-    named_bar_sync(1, NCONS);
     unsigned long long tp = (a.ptrace && tid == 0) ? globaltimer_ns() : 0;
     auto phase = [&](int i) {
         if (a.ptrace && tid == 0) {
@@ -585,181 +647,44 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
             tp = now;
         }
     };
-
-    // (a) 32x32 diagonal block at column p0 by warp 0: unblocked Cholesky,
-    // lane i owns row i, then its inverse (Dv) and its place in W
-    auto diag_block = [&](int p0) {
-        unsigned long long ts = (a.ptrace && lane == 0) ? globaltimer_ns() : 0;
-        auto sub = [&](int i) {
-            if (a.ptrace && lane == 0) {
-                const unsigned long long now = globaltimer_ns();
-                a.ptrace[PTRACE_W * k + 4 + i] += now - ts;
-                ts = now;
-            }
-        };
-        double d[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) d[c] = (c <= lane) ? __ldcg(T + (int64_t)(p0 + c) * nbi + p0 + lane) : 0.0;
-        // phase trace only: a use of the loaded values, so they have arrived at the timestamp
-        if (a.ptrace) { double z = 0; for (int c = 0; c < 32; ++c) z += d[c]; if (z == 12345.0) colb[0] = z; }
-        sub(0);
-        double rdiag = 0.0;      // lane j: 1 / L(j,j)
-        const int failcol = chol32_blk<double>(d, lane, rdiag, Lb);
-        __syncwarp();
-        sub(1);
-        if (failcol >= 0) {
-            if (lane == 0) {
-                ctl->fail = 1;
-                const int col = p0 + failcol;   // tile-local column; padding follows the valid part
-                if (col < a.nb_user && k * a.nb_user + col < a.n_user) atomicCAS(a.info, 0, k * a.nb_user + col + 1);
+#pragma unroll 1
+    for (int b = 0; b < a.nbs; ++b) {
+        double *Tb = T + (int64_t)b * BLK * nbi + b * BLK;
+        p128_load(ring, Tb, nbi, false, tid);
+        named_bar_sync(1, NCONS);
+        const int f = potrf128_smem(ring, &ctl->fail, Tb, nbi, Wk + (int64_t)b * BLK * BLK, warp, lane, 1);
+        phase(0);
+        if (f >= 0) {
+            if (tid == 0) {
+                // column within the caller's tile; padding follows the valid part
+                const int col = ((k % a.tbs) * a.nbs + b) * BLK + f, tile = k / a.tbs;
+                if (col < a.nb_user && tile * a.nb_user + col < a.n_user) atomicCAS(a.info, 0, tile * a.nb_user + col + 1);
                 atomicExch(a.abort_flag, 1);
             }
-        } else {
-#pragma unroll 8
-            for (int c = 0; c < 32; ++c)
-                if (c <= lane) T[(int64_t)(p0 + c) * nbi + p0 + lane] = Lb[(c >> 2) * 128 + lane * 4 + (c & 3)];
-            sub(2);
-            // inverse of the 32x32 lower block (Dv row-major: Dv[i*33 + c] =
-            // Dinv(i, c)) and its place in the 128-block inverse W
-            const int b = p0 / BLK, q0 = p0 % BLK;
-            double *Wb = Wk + (int64_t)b * BLK * BLK;
-            inv32_blk<double>(Lb, lane, rdiag, [&](int i, int c, double x) {
-                Dv[i * 33 + c] = x;
-                Wb[(int64_t)(q0 + c) * BLK + q0 + i] = x;
-            });
-            // phase trace only: the inverse is complete at the timestamp
-            if (a.ptrace) { __syncwarp(); if (Dv[lane * 33] == 12345.0) colb[1] = 0; }
-            sub(3);
+            return;
         }
-    };
-    // (c) one 32x32 block (bi, bj) of the trailing update of step p0:
-    // T22 -= X X^T (DMMA from the panel copy Xs)
-    auto update_item = [&](int it, int p0) {
-        int bi = (int)((sqrtf(8.0f * it + 1.0f) - 1.0f) * 0.5f);
-        while ((bi + 1) * (bi + 2) / 2 <= it) ++bi;
-        while (bi * (bi + 1) / 2 > it) --bi;
-        const int bj = it - bi * (bi + 1) / 2;
-        double acc[2][4][4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-#pragma unroll
-        for (int kk = 0; kk < 32; kk += 4) {
-            const double *xr = Xs + (kk + t) * XP;
-            double af[2][2], bf[4];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi) {
-                af[mi][0] = xr[bi * 32 + mi * 16 + g];
-                af[mi][1] = xr[bi * 32 + mi * 16 + g + 8];
-            }
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) bf[ni] = xr[bj * 32 + ni * 8 + g];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
-        }
-        // all loads first, then the stores: interleaved, every load would
-        // wait for the previous store (the compiler cannot tell the
-        // addresses apart) and the update would take one L2 round trip
-        // per element
-        double old[2][4][4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = p0 + 32 + bi * 32 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                    const int c = p0 + 32 + bj * 32 + ni * 8 + 2 * t + (q & 1);
-                    old[mi][ni][q] = (r >= c) ? __ldcg(T + (int64_t)c * nbi + r) : 0.0;
-                }
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = p0 + 32 + bi * 32 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                    const int c = p0 + 32 + bj * 32 + ni * 8 + 2 * t + (q & 1);
-                    if (r >= c) T[(int64_t)c * nbi + r] = old[mi][ni][q] - acc[mi][ni][q];
-                }
-    };
-
-    // Look-ahead: after the panel of step p0, warp 0 updates the next
-    // diagonal block (item 0) and factors it while warps 1-7 update the rest
-    // of the trailing part, so the 32x32 factorization and inverse (the
-    // serial part of the task) overlap the update instead of following it.
-    if (warp == 0) diag_block(0);
-    named_bar_sync(1, NCONS);
-    phase(0);
-    if (ctl->fail) return;
-    for (int p0 = 0; p0 < nbi; p0 += 32) {
-        // (b) panel below the block: X = P * Dinv^T (P = T[p0+32:, p0:p0+32])
-        // on the FP64 tensor cores, one 32-row block of X per warp and turn
-        const int R = nbi - p0 - 32;
-        for (int rb = warp; rb < R / 32; rb += NCONS / 32) {
-            const int rr0 = rb * 32, r0 = p0 + 32 + rr0;
-            double af[8][2][2];
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
-                    const double *col = T + (int64_t)(p0 + ks * 4 + t) * nbi + r0 + mi * 16 + g;
-                    af[ks][mi][0] = __ldcg(col);
-                    af[ks][mi][1] = __ldcg(col + 8);
-                }
-            double acc[2][4][4];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) {
-                    const double bf = Dv[(ni * 8 + g) * 33 + ks * 4 + t];   // Dinv^T(l, c) = Dinv(c, l)
-#pragma unroll
-                    for (int mi = 0; mi < 2; ++mi) dmma_16x8x4(acc[mi][ni], af[ks][mi][0], af[ks][mi][1], bf);
-                }
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int rr = rr0 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                        const int c = ni * 8 + 2 * t + (q & 1);
-                        T[(int64_t)(p0 + c) * nbi + p0 + 32 + rr] = acc[mi][ni][q];
-                        Xs[c * XP + rr] = acc[mi][ni][q];
-                    }
+        if (b + 1 == a.nbs) break;
+        // the rest of the tile: strips X_i = A_ib W_b^T, then C_ij -= X_i X_j^T
+        // with X_j in shared memory
+#pragma unroll 1
+        for (int i = b + 1; i < a.nbs; ++i) {
+            double *Ai = T + (int64_t)b * BLK * nbi + i * BLK;
+            p128_rows(true, false, ring, Ai, Ai, nbi, warp, lane);
         }
         named_bar_sync(1, NCONS);
         phase(1);
-
-        if (p0 + 32 < nbi) {
-            const int nb32 = R / 32;
-            const int nitems = nb32 * (nb32 + 1) / 2;
-            if (warp == 0) {
-                update_item(0, p0);
-                __syncwarp();          // the block's new values, written by every lane, before the reload
-                diag_block(p0 + 32);
-            } else {
-                for (int it = warp; it < nitems; it += NCONS / 32 - 1) update_item(it, p0);
-            }
+#pragma unroll 1
+        for (int j = b + 1; j < a.nbs; ++j) {
+            p128_load(ring, T + (int64_t)b * BLK * nbi + j * BLK, nbi, true, tid);
             named_bar_sync(1, NCONS);
-            phase(2);
-            if (ctl->fail) return;
+#pragma unroll 1
+            for (int i = j; i < a.nbs; ++i)
+                p128_rows(false, i == j, ring, T + (int64_t)b * BLK * nbi + i * BLK, T + (int64_t)j * BLK * nbi + i * BLK,
+                          nbi, warp, lane);
+            named_bar_sync(1, NCONS);
         }
+        phase(2);
     }
-
-    // Inverses of the 128x128 diagonal blocks from the 32x32 ones.
-    assemble_w128(T, nbi, Wk, a.nbs, Sw, warp, lane, NCONS / 32, 1, NCONS);
     if (MIXED && a.tc_trsm) {
         // the factor and W are complete: the first release of POTRF(k) lets
         // the FP64 strip of the next tile row (the one on the critical path)
@@ -768,7 +693,6 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
         named_bar_sync(1, NCONS);
         if (tid == 0) red_release_add(a.potrf_done + k, 1);
     }
-    phase(3);
     if (a.nbs == 2 && a.Wx) {
         // the off-diagonal block of the tile's inverse, Linv10 = -W1 (L10 W0),
         // so the TRSM strips are two independent products; P = L10 W0 is kept
@@ -1154,7 +1078,7 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
         if (ty == T_POTRF) {
             if (MIXED && a.A0) stream_add_rows(a, k, k, 0, a.nbi);   // potrf_task's first barrier orders it
             potrf_task<MIXED>(a, ctl, ring, k);
-            if (!ctl->fail) release = a.potrf_done + k;
+            if (ctl->fail < 0) release = a.potrf_done + k;
         } else if (ty == T_TRSM && tc_strip<MIXED>(a, k, m)) {
             ok = tc_trsm(a, ctl, ring16, t, st16, mx_it, tcuse);
             release = a.trsm_done + (int64_t)m * a.mt + k;
@@ -1241,7 +1165,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_init(&ctl->tmem_full, 1);
         mbar_init(&ctl->epi, 1);
         mbar_init(&ctl->prep, NCONS / 32);
-        ctl->fail = 0;
+        ctl->fail = -1;
+        ctl->chain = a.potrf_pos && atomicAdd(a.chain, 1) == 0;
     }
     if (MIXED && threadIdx.x < 32) {
         tmem_alloc(&ctl->tmem_base, MX_TMEM_COLS);
@@ -1274,6 +1199,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 size_t potrf_smem_bytes(bool mixed)
 {
     const size_t ctl = ((sizeof(SmemCtl) + 127) / 128) * 128;
+    static_assert(NSTAGE * STAGE_DOUBLES >= P128_DOUBLES && MX_NST * MX_STAGE_BYTES >= P128_DOUBLES * 8,
+                  "the ring holds POTRF's scratch");
     if (!mixed) return ctl + (size_t)NSTAGE * STAGE_DOUBLES * sizeof(double);
     // FP64 ring, then the 16-bit ring aligned to 1024 B (worst-case padding)
     // one region for the FP64 ring, POTRF scratch and the 1024-aligned 16-bit ring
@@ -1286,44 +1213,18 @@ size_t potrf_smem_bytes() { return potrf_smem_bytes(false); }
 // ---------------------------------------------------------------------------
 // host: ticket order
 // ---------------------------------------------------------------------------
-// POTRF(0), TRSM(*,0); then for each step k: the update of column k+1
-// (critical path), POTRF(k+1), `delay` tasks of the remaining step-k update,
-// TRSM(*,k+1), the rest of the step-k update by increasing column.  Every
-// task's dependencies precede it, so CTAs that take tickets in order always
-// make progress (no co-residency assumption).
-std::vector<uint64_t> build_potrf_tasks(int mt, int nbs, int delay)
+// Tile order (task-insertion pools, the allocation-free entry; the self check
+// reports in its tasks): POTRF(0), TRSM(*,0); then for each step k: the update
+// of column k+1 (critical path), POTRF(k+1), `delay` tasks of the remaining
+// step-k update, TRSM(*,k+1), the rest of the step-k update by increasing
+// column.  Every task's dependencies precede it, so CTAs that take tickets in
+// order always make progress (no co-residency assumption).
+size_t build_potrf_tasks_into(uint64_t *out, size_t cap, int mt, int nbs, int delay);
+static std::vector<uint64_t> build_potrf_tasks(int mt, int nbs, int delay)
 {
-    std::vector<uint64_t> v;
-    auto push_update_tile = [&](int m, int n, int k) {
-        for (int bi = 0; bi < nbs; ++bi)
-            for (int bj = 0; bj < nbs; ++bj) {
-                if (m == n && bj > bi) continue;
-                v.push_back(make_task(T_GEMM, k, m, n, bi, bj));
-            }
-    };
-    auto push_trsm = [&](int k) {
-        for (int m = k + 1; m < mt; ++m)
-            for (int bi = 0; bi < nbs; ++bi) v.push_back(make_task(T_TRSM, k, m, k, bi, 0));
-    };
-    v.push_back(make_task(T_POTRF, 0, 0, 0, 0, 0));
-    push_trsm(0);
-    std::vector<uint64_t> rest;
-    for (int k = 0; k + 1 < mt; ++k) {
-        for (int m = k + 1; m < mt; ++m) push_update_tile(m, k + 1, k);
-        v.push_back(make_task(T_POTRF, k + 1, k + 1, k + 1, 0, 0));
-        rest.clear();
-        for (int n = k + 2; n < mt; ++n)
-            for (int m = n; m < mt; ++m)
-                for (int bi = 0; bi < nbs; ++bi)
-                    for (int bj = 0; bj < nbs; ++bj) {
-                        if (m == n && bj > bi) continue;
-                        rest.push_back(make_task(T_GEMM, k, m, n, bi, bj));
-                    }
-        const size_t d = std::min<size_t>(rest.size(), (size_t)std::max(delay, 0));
-        v.insert(v.end(), rest.begin(), rest.begin() + d);
-        push_trsm(k + 1);
-        v.insert(v.end(), rest.begin() + d, rest.end());
-    }
+    uint64_t none;
+    std::vector<uint64_t> v(build_potrf_tasks_into(&none, 0, mt, nbs, delay));
+    build_potrf_tasks_into(v.data(), v.size(), mt, nbs, delay);
     return v;
 }
 
@@ -1412,9 +1313,175 @@ std::vector<uint64_t> build_potrf_tasks_mixed(int mt, int nbs, int delay, int S,
     return v;
 }
 
+// Block order of the FP64 factorization, on the P x P grid of 128x128 blocks
+// whatever the tile edge.  An update task applies S panels (128 S columns) to
+// one block, so the large factorizations keep the long inner products of wide
+// tiles; the last panel of each column is a task of its own, so that the chain
+// POTRF(k) -> TRSM(k+1,k) -> update of (k+1,k+1) -> POTRF(k+1) has one
+// 128-deep product per link.  The update task of block (m,n) with the panels
+// j0 .. j0+cnt-1 carries k = j0 and bi = cnt.  Full chunks are spread over the
+// S steps after their last panel as in the mixed order below.  Step k: panel k
+// on column k+1, POTRF(k+1), the open chunk up to panel k on column k+2 (it
+// runs beside POTRF(k+1)), `delay` tasks of the step's share, TRSM(*,k+1), the
+// rest of the share.
+static void block_share(std::vector<uint64_t> &v, int bw, int bh);
+std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, int bh)
+{
+    std::vector<uint64_t> v;
+    auto push_trsm = [&](int k) {
+        for (int m = k + 1; m < P; ++m) v.push_back(make_task(T_TRSM, k, m, k, 0, 0));
+    };
+    // share[k]: the full chunks issued in step k.  Chunk c closes with panel
+    // k = c S + S - 1; column n >= k + 2 takes it before its open chunk, which
+    // step n - 2 issues (in step k itself when n = k + 2: no open chunk then)
+    std::vector<std::vector<uint64_t>> share(P > 0 ? P : 1);
+    for (int k = S - 1; k + 2 < P; k += S) {
+        long long work = 0, done = 0;
+        for (int n = k + 2; n < P; ++n) work += P - n;
+        for (int n = k + 2; n < P; ++n) {
+            int part = (int)((done * S) / (work > 0 ? work : 1));
+            part = std::min(part, std::min(S - 1, std::max(n - 3 - k, 0)));
+            for (int m = n; m < P; ++m) share[k + part].push_back(make_task(T_GEMM, k - S + 1, m, n, S, 0));
+            done += P - n;
+        }
+    }
+    for (auto &sh : share) block_share(sh, bw, bh);
+    v.push_back(make_task(T_POTRF, 0, 0, 0, 0, 0));
+    push_trsm(0);
+    for (int k = 0; k + 1 < P; ++k) {
+        for (int m = k + 1; m < P; ++m) v.push_back(make_task(T_GEMM, k, m, k + 1, 1, 0));
+        v.push_back(make_task(T_POTRF, k + 1, k + 1, k + 1, 0, 0));
+        const int open = (k + 1) % S;                 // panels of column k+2's open chunk
+        if (open != 0 && k + 2 < P)
+            for (int m = k + 2; m < P; ++m) v.push_back(make_task(T_GEMM, k + 1 - open, m, k + 2, open, 0));
+        const std::vector<uint64_t> &rest = share[k];
+        const size_t d = std::min<size_t>(rest.size(), (size_t)std::max(delay, 0));
+        v.insert(v.end(), rest.begin(), rest.begin() + d);
+        push_trsm(k + 1);
+        v.insert(v.end(), rest.begin() + d, rest.end());
+    }
+    return v;
+}
+
 // ---------------------------------------------------------------------------
 // host: run one factorization of the device tiles
 // ---------------------------------------------------------------------------
+// The ticket order of a shape on the device (kept until another shape is
+// factored), with the tickets of the POTRFs behind it.  chunk > 0: mixed, this
+// many panels per update task; chunk < 0: FP64 on blocks, -chunk panels.
+static int prepare_tasks(Context *ctx, PotrfArgs &a, int mt, int nbs, int chunk)
+{
+    const bool mixed = chunk > 0;
+    const int delay = mixed ? ctx->mx_delay : ctx->potrf_delay;
+    if (ctx->task_mt != mt || ctx->task_nbs != nbs || ctx->task_delay != delay || ctx->task_mixed != chunk) {
+        std::vector<uint64_t> tasks =
+            mixed ? build_potrf_tasks_mixed(mt, nbs, delay, chunk, ctx->mx_block_w, ctx->mx_block_h)
+                  : build_potrf_tasks_blocks(mt * nbs, -chunk, delay, ctx->f64_block, ctx->f64_block);
+        const size_t nt = tasks.size();
+        int np = 0;
+        std::vector<int> pos;
+        for (size_t i = 0; i < nt; ++i)
+            if (task_type(tasks[i]) == T_POTRF) pos.push_back((int)i);
+        np = (int)pos.size();
+        unsigned char *dt = (unsigned char *)ctx->buffer(BUF_TASKS, nt * sizeof(uint64_t) + np * sizeof(int));
+        ctx->task_mt = -1;
+        if (!dt) return DPLASMA_ERR_OUT_OF_RESOURCES;
+        CK(cudaMemcpyAsync(dt, tasks.data(), nt * sizeof(uint64_t), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(dt + nt * sizeof(uint64_t), pos.data(), np * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+        ctx->task_mt = mt;
+        ctx->task_nbs = nbs;
+        ctx->task_delay = delay;
+        ctx->task_mixed = chunk;
+        ctx->ntasks = (int)nt;
+    }
+    a.tasks = (const uint64_t *)ctx->buffer(BUF_TASKS, 0);
+    a.ntasks = ctx->ntasks;
+    a.potrf_pos = (const int *)(a.tasks + a.ntasks);
+    return 0;
+}
+
+// Panels per FP64 update task on a grid of P blocks.  Every task pays one pass of
+// L2 reductions over its block (about 10 us beside 17 us of products per
+// panel), so the large grids take many (N = 32768, P = 256: 4 panels 391 ms, 8
+// 367, 12 362.6, 15 360.6; P = 128: 8 48.6, 12 48.4, 15 48.8); on a small grid
+// the open chunk of the next column would take longer than a step of the chain
+// it runs beside (P = 64: 4 8.30 ms, 6 8.19, 8 8.31; P = 32: 2 2.744, 4 2.741, 6
+// 2.864, 8 3.038).
+static int f64_panels(const Context *ctx, int P)
+{
+    if (ctx->f64_chunk > 0) return ctx->f64_chunk;
+    return P <= 48 ? 4 : P <= 96 ? 6 : P <= 192 ? 12 : 15;
+}
+
+// The counters of a launch in one zeroed array: 16 words (ticket, INFO, abort,
+// status, diag[4], chain claim), POTRF, TRSM and update counts on a P x P grid,
+// task counts per CTA.
+constexpr int CTR_HEAD = 16;
+static size_t ctr_ints(int P, int grid) { return CTR_HEAD + (size_t)P + 2 * (size_t)P * P + grid; }
+static void set_counters(PotrfArgs &a, int *ctr, int P)
+{
+    a.ticket = ctr + 0;
+    a.info = ctr + 1;
+    a.abort_flag = ctr + 2;
+    a.status = ctr + 3;
+    a.diag = ctr + 4;
+    a.chain = ctr + 8;
+    a.potrf_done = ctr + CTR_HEAD;
+    a.trsm_done = a.potrf_done + P;
+    a.upd_done = a.trsm_done + (size_t)P * P;
+    a.task_count = a.upd_done + (size_t)P * P;
+}
+
+// Self check of the FP64 block order in tasks of the tile order: every part (a
+// block and panel) of every tile task must have been run once.  tot = task runs
+// of whole tile tasks, bad = tile tasks with a part not run exactly once.
+static void selfcheck_tiles(const std::vector<uint64_t> &tl, const std::vector<int> &ran, int mt, int nbs,
+                            long long &tickets, long long &tot, long long &bad)
+{
+    const int P = mt * nbs;
+    // runs of panel j on block (m, n): [-1] is the block's own POTRF or TRSM
+    auto at = [&](int m, int n, int j) { return ((size_t)m * (m + 1) / 2 + n) * (P + 1) + (j + 1); };
+    std::vector<unsigned char> cnt((size_t)P * (P + 1) / 2 * (P + 1), 0);
+    for (size_t i = 0; i < tl.size(); ++i) {
+        const uint64_t t = tl[i];
+        const int c = std::min(ran[i], 100);
+        if (task_type(t) == T_POTRF) cnt[at(task_k(t), task_k(t), -1)] += c;
+        else if (task_type(t) == T_TRSM) cnt[at(task_m(t), task_k(t), -1)] += c;
+        else
+            for (int j = task_k(t); j < task_k(t) + task_bi(t); ++j) cnt[at(task_m(t), task_n(t), j)] += c;
+    }
+    tickets = tot = bad = 0;
+    auto tally = [&](int lo, int hi) {
+        ++tickets;
+        tot += lo;
+        bad += lo != 1 || hi != 1;
+    };
+    auto part = [&](int m, int n, int j, int &lo, int &hi) {
+        lo = std::min<int>(lo, cnt[at(m, n, j)]);
+        hi = std::max<int>(hi, cnt[at(m, n, j)]);
+    };
+    for (int k = 0; k < mt; ++k) {
+        const int b0 = k * nbs, b1 = b0 + nbs;
+        int lo = 255, hi = 0;                              // POTRF(k): all parts inside the tile
+        for (int m = b0; m < b1; ++m)
+            for (int n = b0; n <= m; ++n)
+                for (int j = b0 - 1; j < n; ++j) part(m, n, j < b0 ? -1 : j, lo, hi);
+        tally(lo, hi);
+        for (int m = b1; m < P; ++m) {                     // TRSM strips: block row m of tile column k
+            lo = 255, hi = 0;
+            for (int n = b0; n < b1; ++n)
+                for (int j = b0 - 1; j < n; ++j) part(m, n, j < b0 ? -1 : j, lo, hi);
+            tally(lo, hi);
+        }
+        for (int n = b1; n < P; ++n)                       // step k's update of block (m, n)
+            for (int m = n; m < P; ++m) {
+                lo = 255, hi = 0;
+                for (int j = b0; j < b1; ++j) part(m, n, j, lo, hi);
+                tally(lo, hi);
+            }
+    }
+}
+
 // Tensor map of the 16-bit panel copies: rows of nbi elements (K-major), one
 // row per matrix row of every lower tile, boxes of 64 x 128 with 128-byte
 // swizzle (the canonical K-major UMMA operand layout).
@@ -1496,68 +1563,50 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
         ctx->set_error("persistent kernel does not fit on an SM");
         return DPLASMA_ERR_UNEXPECTED;
     }
-    // task list (cached per shape)
     // panels accumulated per update task: the FP32 accumulation in tensor
     // memory runs over chunk*256 products, which sets the factor's accuracy
     // in the split form (8: 6 refinement steps at kappa 1e6 and N=65536, 12:
     // 7, 16: 8); single 16-bit operands are limited by their own rounding
-    // and take 16 (same refinement steps as 8, 15% faster factorization)
-    const int chunk = !mixed ? 0 : (ctx->mx_chunk > 0 ? ctx->mx_chunk : (p16_fmt == 2 ? 8 : 16));
-    const int delay = mixed ? ctx->mx_delay : ctx->potrf_delay;
-    if (ctx->task_mt != mt || ctx->task_nbs != nbs || ctx->task_delay != delay || ctx->task_mixed != chunk) {
-        std::vector<uint64_t> tasks = mixed ? build_potrf_tasks_mixed(mt, nbs, delay, chunk, ctx->mx_block_w,
-                                                                      ctx->mx_block_h)
-                                            : build_potrf_tasks(mt, nbs, ctx->potrf_delay);
-        uint64_t *dt = (uint64_t *)ctx->buffer(BUF_TASKS, tasks.size() * sizeof(uint64_t));
-        if (!dt) return DPLASMA_ERR_OUT_OF_RESOURCES;
-        CK(cudaMemcpyAsync(dt, tasks.data(), tasks.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-        ctx->task_mt = mt;
-        ctx->task_nbs = nbs;
-        ctx->task_delay = delay;
-        ctx->task_mixed = chunk;
-        ctx->ntasks = (int)tasks.size();
-    }
+    // and take 16 (same refinement steps as 8, 15% faster factorization).
+    // FP64 runs on 128x128 blocks, f64_panels(P) panels per task
+    const int chunk = !mixed ? -f64_panels(ctx, mt * nbs) : (ctx->mx_chunk > 0 ? ctx->mx_chunk : (p16_fmt == 2 ? 8 : 16));
+    const int P = mixed ? mt : mt * nbs;               // the scheduler's grid
+    PotrfArgs a;
+    int erc = prepare_tasks(ctx, a, mt, nbs, chunk);
+    if (erc) return erc;
     double *W = (double *)ctx->buffer(BUF_W, (size_t)mt * nbs * BLK * BLK * sizeof(double));
-    // opt-in: TRSM strips of 256-wide tiles as two independent products on the
+    // opt-in (mixed): TRSM strips of 256-wide tiles as two independent products on the
     // tile's whole inverse (strips 84 -> 70 us, but POTRF +55 us on the
     // critical path: no net gain at N = 32768 .. 65536)
     // opt-in: mixed split FP16 TRSM strips on the tensor cores (the inverse's
     // second block row is then needed as well)
     const bool tc = mixed && nbs == 2 && p16_fmt == 2 && ctx->trsm_tc;
-    double *Wx = nbs == 2 && (ctx->trsm_inv || tc)
+    double *Wx = mixed && nbs == 2 && (ctx->trsm_inv || tc)
                      ? (double *)ctx->buffer(BUF_WX, (size_t)mt * 2 * BLK * BLK * sizeof(double))
                      : nullptr;
-    if (nbs == 2 && (ctx->trsm_inv || tc) && !Wx) return DPLASMA_ERR_OUT_OF_RESOURCES;
-    const size_t nctr = 8 + (size_t)mt + 2 * (size_t)mt * mt + grid;
+    if (mixed && nbs == 2 && (ctx->trsm_inv || tc) && !Wx) return DPLASMA_ERR_OUT_OF_RESOURCES;
+    const size_t nctr = ctr_ints(P, grid);
     int *ctr = (int *)ctx->buffer(BUF_COUNTERS, nctr * sizeof(int));
     if (!W || !ctr) return DPLASMA_ERR_OUT_OF_RESOURCES;
     CK(cudaMemsetAsync(ctr, 0, nctr * sizeof(int), st));
 
-    PotrfArgs a;
     a.A = dA;
     a.W = W;
     a.Wx = Wx;
-    a.tasks = (const uint64_t *)ctx->buffer(BUF_TASKS, 0);
-    a.ntasks = ctx->ntasks;
-    a.mt = mt;
-    a.nbi = nbi;
-    a.nbs = nbs;
+    a.mt = P;
+    a.nbi = mixed ? nbi : BLK;
+    a.nbs = mixed ? nbs : 1;
+    a.ld = nbi;
+    a.tbs = mixed ? 1 : nbs;
+    a.fchunk = mixed ? 0 : -chunk;
     a.nb_user = nb_user;
     a.n_user = n_user;
-    a.ticket = ctr + 0;
-    a.info = ctr + 1;
-    a.abort_flag = ctr + 2;
-    a.status = ctr + 3;
-    a.potrf_done = ctr + 8;
-    a.trsm_done = a.potrf_done + mt;
-    a.upd_done = a.trsm_done + (size_t)mt * mt;
-    a.task_count = a.upd_done + (size_t)mt * mt;
-    a.diag = ctr + 4;
+    set_counters(a, ctr, P);
     a.trace = nullptr;
     a.ptrace = nullptr;
     a.ran = nullptr;
     // one-shot fault injection of this call (host side only)
-    a.fail_potrf = ctx->inject_kind == INJECT_TASK_FAILED ? ctx->inject_arg : -1;
+    a.fail_potrf = ctx->inject_kind == INJECT_TASK_FAILED ? ctx->inject_arg * a.tbs : -1;
     a.skip_ticket = ctx->inject_kind == INJECT_WITHHOLD ? ctx->inject_arg : -1;
     ctx->inject_kind = 0;
     if (ctx->self_check) {
@@ -1572,9 +1621,9 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
         a.trace_exit = a.trace + (size_t)a.ntasks * 4;
         a.trace_cta = (int *)(a.trace_exit + 8 * (size_t)grid);
         CK(cudaMemsetAsync(a.trace, 0, tbytes, st));
-        a.ptrace = (unsigned long long *)ctx->buffer(BUF_PTRACE, (size_t)mt * PTRACE_W * sizeof(unsigned long long));
+        a.ptrace = (unsigned long long *)ctx->buffer(BUF_PTRACE, (size_t)P * PTRACE_W * sizeof(unsigned long long));
         if (!a.ptrace) return DPLASMA_ERR_OUT_OF_RESOURCES;
-        CK(cudaMemsetAsync(a.ptrace, 0, (size_t)mt * PTRACE_W * sizeof(unsigned long long), st));
+        CK(cudaMemsetAsync(a.ptrace, 0, (size_t)P * PTRACE_W * sizeof(unsigned long long), st));
     }
     a.dep_limit_ns = ctx->dep_limit_ns;
     a.pipe_limit_ns = ctx->pipe_limit_ns;
@@ -1659,14 +1708,20 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
         ctx->last_tasks_executed = tot;
         ctx->last_tickets = a.ntasks;
         ctx->last_tickets_bad = bad;
-        if (hs[1] == 0 && (bad != 0 || tot != a.ntasks)) {
+        if (a.fchunk) {
+            std::vector<uint64_t> tl(a.ntasks);
+            CK(cudaMemcpy(tl.data(), a.tasks, tl.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost));
+            selfcheck_tiles(tl, ran, mt, nbs, ctx->last_tickets, ctx->last_tasks_executed, ctx->last_tickets_bad);
+        }
+        if (hs[1] == 0 && (bad != 0 || tot != a.ntasks || ctx->last_tickets_bad != 0)) {
             ctx->set_error("potrf self check: %lld of %d tickets did not run exactly once (%lld task runs)", bad,
                            a.ntasks, tot);
             return DPLASMA_ERR_UNEXPECTED;
         }
     }
     if (a.trace) {
-        // one line per ticket: type k m n bi bj fetched deps_met started finished cta (ns, relative)
+        // one line per ticket (FP64: 128-blocks; an update has its first panel in k and
+        // their number in bi): type k m n bi bj fetched deps_met started finished cta (ns, relative)
         std::vector<unsigned long long> tr((size_t)a.ntasks * 4), tx(8 * (size_t)grid);
         std::vector<int> tc(a.ntasks);
         std::vector<uint64_t> tl(a.ntasks);
@@ -1687,14 +1742,13 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
                         task_n(t), task_bi(t), task_bj(t), rel(tr[4 * i]), rel(tr[4 * i + 1]), rel(tr[4 * i + 2]),
                         rel(tr[4 * i + 3]), tc[i]);
             }
-            std::vector<unsigned long long> pt((size_t)mt * PTRACE_W);
+            std::vector<unsigned long long> pt((size_t)P * PTRACE_W);
             cudaMemcpy(pt.data(), a.ptrace, pt.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
-            for (int k = 0; k < mt; ++k) {
+            for (int k = 0; k < P; ++k) {
                 const unsigned long long *q = pt.data() + (size_t)PTRACE_W * k;
-                fprintf(f, "# potrf %d diag_ns %llu panel_ns %llu update_ns %llu inverse_ns %llu load_ns %llu chol_ns %llu "
-                           "store_ns %llu inv32_ns %llu l10w0_ns %llu linv10_ns %llu w1copy_ns %llu linv16_ns %llu "
-                           "tc_strips %llu tc_stage_ns %llu tc_epilogue_ns %llu\n",
-                        k, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13], q[14]);
+                fprintf(f, "# potrf %d block_ns %llu strip_ns %llu update_ns %llu l10w0_ns %llu linv10_ns %llu w1copy_ns %llu "
+                           "linv16_ns %llu tc_strips %llu tc_stage_ns %llu tc_epilogue_ns %llu\n",
+                        k, q[0], q[1], q[2], q[8], q[9], q[10], q[11], q[12], q[13], q[14]);
             }
             for (int c = 0; c < grid; ++c)
                 fprintf(f, "# cta %d producer_exit %lld consumer_exit %lld potrf_wait_done %lld end_pushed %lld end_seen %lld "
@@ -1734,23 +1788,9 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     }
     const int chunk = ctx->mx_chunk > 0 ? ctx->mx_chunk : (p16_fmt == 2 ? 8 : 16);
     const int cb = ctx->stream_cb > 0 ? ctx->stream_cb : 8;        // tile columns per copy phase
-    // the ticket order of the mixed factorization (the same as for a matrix
-    // already on the device, and the same cache)
-    if (ctx->task_mt != mt || ctx->task_nbs != nbs || ctx->task_delay != ctx->mx_delay || ctx->task_mixed != chunk) {
-        std::vector<uint64_t> tasks =
-            build_potrf_tasks_mixed(mt, nbs, ctx->mx_delay, chunk, ctx->mx_block_w, ctx->mx_block_h);
-        uint64_t *dt = (uint64_t *)ctx->buffer(BUF_TASKS, tasks.size() * sizeof(uint64_t));
-        if (!dt) return DPLASMA_ERR_OUT_OF_RESOURCES;
-        CK(cudaMemcpyAsync(dt, tasks.data(), tasks.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-        ctx->task_mt = mt;
-        ctx->task_nbs = nbs;
-        ctx->task_delay = ctx->mx_delay;
-        ctx->task_mixed = chunk;
-        ctx->ntasks = (int)tasks.size();
-    }
     const int nph = (mt + cb - 1) / cb;
     double *W = (double *)ctx->buffer(BUF_W, (size_t)mt * nbs * BLK * BLK * sizeof(double));
-    const size_t nctr = 8 + (size_t)mt + 2 * (size_t)mt * mt + grid;
+    const size_t nctr = ctr_ints(mt, grid);
     int *ctr = (int *)ctx->buffer(BUF_COUNTERS, nctr * sizeof(int));
     if (!W || !ctr) return DPLASMA_ERR_OUT_OF_RESOURCES;
 
@@ -1768,15 +1808,12 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     a.nbs = nbs;
     a.nb_user = nb_user;
     a.n_user = n_user;
-    a.ticket = ctr + 0;
-    a.info = ctr + 1;
-    a.abort_flag = ctr + 2;
-    a.status = ctr + 3;
-    a.diag = ctr + 4;
-    a.potrf_done = ctr + 8;
-    a.trsm_done = a.potrf_done + mt;
-    a.upd_done = a.trsm_done + (size_t)mt * mt;
-    a.task_count = a.upd_done + (size_t)mt * mt;
+    a.ld = nbi;
+    a.tbs = 1;
+    set_counters(a, ctr, mt);
+    // the ticket order of a matrix already on the device
+    int e = prepare_tasks(ctx, a, mt, nbs, chunk);
+    if (e) return e;
     a.fail_potrf = -1;
     a.skip_ticket = -1;
     a.dep_limit_ns = ctx->dep_limit_ns;
@@ -1796,7 +1833,7 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     a.p16_target = p16_fmt == 1 ? 1.0f : 16384.0f;
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));
-    int e = make_p16_map(ctx, &tmap, pb, (split ? 2 : 1) * rows, nbi, a.p16_fmt, split);
+    e = make_p16_map(ctx, &tmap, pb, (split ? 2 : 1) * rows, nbi, a.p16_fmt, split);
     if (e) return e;
     CUtensorMap lmap;
     memset(&lmap, 0, sizeof(lmap));
@@ -1852,8 +1889,6 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     // One launch in the ordinary ticket order: the updates never wait for
     // data, POTRF(k) and the strips of column k wait for column k's phase.
     // The columns of phase p are one contiguous run of tiles.
-    a.tasks = (const uint64_t *)ctx->buffer(BUF_TASKS, 0);
-    a.ntasks = ctx->ntasks;
     potrf_persistent_kernel<true><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
     CK(cudaGetLastError());
     ctx->launches += 1;
@@ -1916,8 +1951,8 @@ int potrf_max_blocks_per_sm() { return max_blocks_per_sm<false>(); }
 // ---------------------------------------------------------------------------
 namespace db2 {
 
-// Same ticket order as build_potrf_tasks, written into a caller buffer
-// without heap use; returns the count, or 0 if it does not fit in `cap`.
+// The tile order written into a caller buffer without heap use; returns the
+// count, or 0 if it does not fit in `cap` (cap 0: the count alone).
 size_t build_potrf_tasks_into(uint64_t *out, size_t cap, int mt, int nbs, int delay)
 {
     size_t n = 0;
@@ -1959,7 +1994,7 @@ size_t build_potrf_tasks_into(uint64_t *out, size_t cap, int mt, int nbs, int de
         put_trsm(k + 1);
         put_rest_range(k, d, total);
     }
-    return fits ? n : 0;
+    return fits || cap == 0 ? n : 0;
 }
 
 int potrf_launch_prealloc(cudaStream_t st, double *dA, int mt, int nbi, int nb_user, int n_user, double *W,
@@ -1975,6 +2010,11 @@ int potrf_launch_prealloc(cudaStream_t st, double *dA, int mt, int nbi, int nb_u
     a.mt = mt;
     a.nbi = nbi;
     a.nbs = nbi / BLK;
+    a.ld = nbi;
+    a.tbs = 1;
+    a.fchunk = 0;
+    a.potrf_pos = nullptr;
+    a.chain = nullptr;
     a.nb_user = nb_user;
     a.n_user = n_user;
     a.ticket = ctr + 0;
@@ -2040,6 +2080,14 @@ extern "C" int dplasma_b200_debug_task_list_blocked(int mixed_chunk, int mt, int
     return (int)v.size();
 }
 
+
+// the FP64 block order (P blocks per side, S panels per update task)
+extern "C" int dplasma_b200_debug_task_list_blocks(int P, int S, int delay, int block, unsigned long long *out, int cap)
+{
+    const std::vector<uint64_t> v = db2::build_potrf_tasks_blocks(P, S, delay, block, block);
+    for (size_t i = 0; i < v.size() && (int)i < cap; ++i) out[i] = v[i];
+    return (int)v.size();
+}
 
 extern "C" int dplasma_b200_debug_task_list(int mixed_chunk, int mt, int nbs, int delay, unsigned long long *out,
                                             int cap)

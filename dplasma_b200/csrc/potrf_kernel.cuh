@@ -26,13 +26,14 @@
 // 32x32 diagonal factorizations.
 #pragma once
 #include "dev_common.cuh"
+#include "dev_potrf128.cuh"
 
 namespace db2 {
 
 constexpr int BLK = 128;         // output block edge handled by one CTA job
 constexpr int BK = 16;           // K depth of one pipeline stage
 constexpr int SP = BLK + 4;      // shared pitch (doubles) of an operand row, = 4 mod 16
-constexpr int NSTAGE = 5;        // pipeline stages
+constexpr int NSTAGE = 6;        // pipeline stages (the ring is also POTRF's scratch, dev_potrf128.cuh)
 constexpr int NCONS = 256;       // consumer threads (2 warpgroups)
 constexpr int NTHREADS = NCONS + 128;   // + producer warpgroup (one active warp)
 constexpr int PRODUCER_REGS = 48;
@@ -67,11 +68,10 @@ constexpr int TC_A_BYTES = BLK * MX_KC_SPLIT * 2;   // 8 KB, written by the cons
 constexpr int TC_B_OFF = 2 * TC_A_BYTES;            // B by TMA (Linv in split FP16)
 constexpr int TC_BLO_OFF = TC_B_OFF + 2 * TC_A_BYTES;
 constexpr int TC_B_BYTES = 4 * TC_A_BYTES;          // 32 KB per stage
-// Trace slots per step k (ptrace): POTRF(k) diagonal blocks, panels, updates,
-// 128-block inverses, and inside the diagonal blocks load, factor, store,
-// 32-block inverse; then the tile inverse's parts (L10 W0, -W1 (L10 W0), W1
-// copy, split FP16 copy) and the tensor-core TRSM strips of step k (count, ns
-// until the accumulator was ready, ns of the epilogue).
+// Trace slots per step k (ptrace): POTRF(k) 128-blocks (factor and inverse),
+// strips and updates inside the tile; from slot 8 the tile inverse's parts (L10
+// W0, -W1 (L10 W0), W1 copy, split FP16 copy) and the tensor-core TRSM strips of
+// step k (count, ns until the accumulator was ready, ns of the epilogue).
 constexpr int PTRACE_W = 16;
 
 // Task encoding (64 bits): type[0:4) k[4:20) m[20:36) n[36:52) bi[52:56) bj[56:60)
@@ -88,6 +88,16 @@ __host__ __device__ __forceinline__ int task_n(uint64_t t) { return (int)((t >> 
 __host__ __device__ __forceinline__ int task_bi(uint64_t t) { return (int)((t >> 52) & 0xF); }
 __host__ __device__ __forceinline__ int task_bj(uint64_t t) { return (int)((t >> 56) & 0xF); }
 
+// FP64 block order: column n's updates are the panels 0 .. n-2 in chunks of S
+// (the last one may be short), then panel n-1 alone, which is the one the
+// chain waits for.  How many there are, and the place of the one that starts at
+// panel j0.
+__host__ __device__ __forceinline__ int block_updates(int n, int S) { return n == 0 ? 0 : (n - 1 + S - 1) / S + 1; }
+__host__ __device__ __forceinline__ int block_update_index(int j0, int n, int S)
+{
+    return j0 == n - 1 ? (n - 1 + S - 1) / S : j0 / S;
+}
+
 struct PotrfArgs {
     double *A;             // device tiles (lower, packed)
     double *W;             // mt * nbs blocks of 128x128: inverses of diagonal blocks
@@ -97,6 +107,13 @@ struct PotrfArgs {
     const uint64_t *tasks; // ticket order
     int ntasks;
     int mt, nbi, nbs;      // tiles per side, tile edge, 128-blocks per tile edge
+    // where tile (m, n) lies: the FP64 factorization runs on 128x128 blocks
+    // (nbi = 128, nbs = 1, mt counts blocks) of physical tiles of edge ld =
+    // 128 tbs, mt / tbs per side; otherwise tbs = 1 and ld = nbi
+    int ld, tbs;
+    int fchunk;            // FP64 block order: panels per update task (0: tile order, one panel per task)
+    const int *potrf_pos;  // [mt] tickets of POTRF(0..mt-1), all run by one CTA (null: by whoever draws them)
+    int *chain;            // claimed by the first CTA to start, which runs the POTRFs of potrf_pos
     int nb_user;           // caller's tile size (INFO numbering)
     int n_user;            // caller's matrix order
     int *ticket;           // next ticket
@@ -146,7 +163,10 @@ struct PotrfArgs {
 
 __device__ __forceinline__ double *tile_ptr(const PotrfArgs &a, int m, int n)
 {
-    return a.A + lower_tile_index(m, n, a.mt) * (int64_t)a.nbi * a.nbi;
+    if (a.tbs == 1) return a.A + lower_tile_index(m, n, a.mt) * (int64_t)a.nbi * a.nbi;
+    const int tm = m / a.tbs, tn = n / a.tbs;
+    return a.A + lower_tile_index(tm, tn, a.mt / a.tbs) * (int64_t)a.ld * a.ld +
+           (int64_t)(n - tn * a.tbs) * BLK * a.ld + (m - tm * a.tbs) * BLK;
 }
 __device__ __forceinline__ double *wblk_ptr(const PotrfArgs &a, int k, int b)
 {
@@ -164,6 +184,7 @@ struct Job {
     int lda, ldb, ldc;
     int K;
     int mode;
+    bool tri;      // B is lower triangular (row c is zero beyond column c)
     bool signal;   // the next job of the same task reads this job's output
     // mixed precision, TRSM store jobs: the 16-bit copy of the block is
     // written by the same epilogue (K-major rows of pitch nbi; null otherwise)
@@ -182,16 +203,22 @@ __device__ __forceinline__ int task_njobs(const PotrfArgs &a, uint64_t t)
 __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
 {
     Job jb;
-    const int nbi = a.nbi;
+    jb.tri = false;
+    const int nbi = a.ld;
     const int k = task_k(t), m = task_m(t), n = task_n(t), bi = task_bi(t), bj = task_bj(t);
     if (task_type(t) == T_GEMM) {
         // C(m,n)[bi,bj] -= A(m,k)[bi,:] * A(n,k)[bj,:]^T     (src/zpotrf_L.jdf:619-623, :453-456)
         jb.A = tile_ptr(a, m, k) + bi * BLK;
         jb.B = tile_ptr(a, n, k) + bj * BLK;
         jb.C = tile_ptr(a, m, n) + (int64_t)bj * BLK * nbi + bi * BLK;
+        if (a.fchunk) {
+            // block order: panels k .. k + bi - 1 of block (m, n)
+            jb.A = jb.B = nullptr;                     // panel by panel (producer_warp)
+            jb.C = tile_ptr(a, m, n);
+        }
         jb.lda = nbi; jb.ldb = nbi; jb.ldc = nbi;
-        jb.K = nbi;
-        jb.mode = (m == n && bi == bj) ? J_SUB_LOWER : J_SUB;
+        jb.K = a.fchunk ? bi * BLK : nbi;
+        jb.mode = (m == n && (bi == bj || a.fchunk)) ? J_SUB_LOWER : J_SUB;
         jb.signal = false;
         jb.p16 = nullptr;
         jb.p16_scale = 1.f;
@@ -212,6 +239,7 @@ __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
         } else {
             jb.B = wblk_ptr(a, k, 0);
             jb.K = BLK;
+            jb.tri = true;
         }
         jb.mode = J_STORE;
         jb.signal = false;
@@ -234,6 +262,7 @@ __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
             jb.B = wblk_ptr(a, k, p); jb.ldb = BLK;
             jb.K = BLK;
             jb.mode = J_STORE;
+            jb.tri = true;
             jb.signal = (p < a.nbs - 1);
         } else {
             jb.A = Amk + bi * BLK; jb.lda = nbi;                    // X_0..X_{p-1}
@@ -268,9 +297,10 @@ struct __align__(16) SmemCtl {
     uint64_t astage[MX_NST];   // tensor-core TRSM: the consumer warps staged the A operand
     uint64_t tmem_full;
     int tick[TASKQ];
-    int fail;
+    int fail;          // POTRF: the failing column within the block, or -1
     uint32_t tmem_base;
-    int pad[2];
+    int chain;         // this CTA runs the POTRF tickets
+    int pad[1];
 };
 
 }  // namespace db2

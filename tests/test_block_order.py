@@ -1,0 +1,54 @@
+"""CPU test of the FP64 factorization's block order: on the P x P grid of
+128x128 blocks every task's dependencies (the rules the kernel waits on) are
+produced by tasks earlier in the order, and every block receives every panel
+once, in increasing order."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import dplasma_b200 as db
+
+T_POTRF, T_TRSM, T_GEMM = 1, 2, 3
+
+
+def tasks(P, S, delay, block):
+    f = db.lib().dplasma_b200_debug_task_list_blocks
+    f.argtypes = [ctypes.c_int] * 4 + [ctypes.c_void_p, ctypes.c_int]
+    n = f(P, S, delay, block, None, 0)
+    out = np.zeros(n, dtype=np.uint64)
+    assert f(P, S, delay, block, out.ctypes.data, n) == n
+    return [(int(t) & 0xF, (int(t) >> 4) & 0xFFFF, (int(t) >> 20) & 0xFFFF, (int(t) >> 36) & 0xFFFF,
+             (int(t) >> 52) & 0xF) for t in out]
+
+
+@pytest.mark.parametrize("P,S,delay,block", [(1, 4, 0, 0), (2, 4, 3, 0), (3, 4, 444, 0), (5, 1, 0, 0), (6, 4, 2, 0),
+                                             (16, 4, 148, 0), (33, 4, 148, 8), (40, 3, 10, 5), (24, 8, 444, 0),
+                                             (31, 15, 30, 4)])
+def test_block_order(P, S, delay, block):
+    potrf = np.zeros(P, int)
+    trsm = np.zeros((P, P), int)
+    upd = np.zeros((P, P), int)        # update tasks done
+    panels = np.zeros((P, P), int)     # panels applied, in order
+
+    def count(n):
+        return 0 if n == 0 else -(-(n - 1) // S) + 1
+
+    for i, (ty, k, m, n, cnt) in enumerate(tasks(P, S, delay, block)):
+        if ty == T_POTRF:
+            assert panels[k, k] == k and upd[k, k] == count(k), (i, k)
+            potrf[k] += 1
+        elif ty == T_TRSM:
+            assert potrf[k] == 1 and upd[m, k] == count(k) and panels[m, k] == k, (i, k, m)
+            trsm[m, k] += 1
+        else:
+            assert ty == T_GEMM and 1 <= cnt <= S and k + cnt <= n <= m
+            # every panel it reads is solved; the kernel waits for the last one
+            assert (trsm[m, k:k + cnt] == 1).all() and (trsm[n, k:k + cnt] == 1).all(), (i, k, m, n)
+            assert panels[m, n] == k
+            assert upd[m, n] == (-(-(n - 1) // S) if k == n - 1 else k // S), (i, k, m, n)
+            panels[m, n] += cnt
+            upd[m, n] += 1
+    assert (potrf == 1).all()
+    for m in range(P):
+        assert (trsm[m, :m] == 1).all() and (panels[m, :m + 1] == np.arange(m + 1)).all()
