@@ -29,7 +29,7 @@
 #include <vector>
 
 #include "dev_common.cuh"
-#include "dev_trtri.cuh"
+#include "dev_potrf128.cuh"
 #include "internal.h"
 
 namespace db2 {
@@ -288,29 +288,19 @@ __global__ void ag_sym(double *X, int ld, int n)
 }
 
 // inverses of the 128x128 diagonal blocks of a dense lower factor, written
-// into the diagonal blocks of W (ld = ldw); W's other blocks untouched
+// into the diagonal blocks of W (ld = ldw); W's other blocks untouched.
+// 76 -> 14 us at 32 blocks with the blocks in shared memory
 __global__ void __launch_bounds__(256) ag_trtri_diag(const double *L, int ld, double *W, int ldw, double *scratch,
                                                      int unit_diag)
 {
     extern __shared__ __align__(16) double tsm[];
     const int b = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x;
     const double *T = L + (int64_t)(b * AG_T) * ld + b * AG_T;
     double *Wk = scratch + (int64_t)b * AG_T * AG_T;   // 128x128, ld 128
-    for (int e = tid; e < AG_T * AG_T; e += 256) Wk[e] = 0.0;
+    p128_load(tsm, T, ld, false, tid);
     __syncthreads();
-    double *Ls = tsm + warp * (32 * 33);
-    for (int d = warp; d < 4; d += 8) {
-        const int p0 = d * 32;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) Ls[lane * 33 + c] = (c <= lane) ? T[(int64_t)(p0 + c) * ld + p0 + lane] : 0.0;
-        __syncwarp();
-        invert32_lower(Ls, lane, unit_diag, [&](int i, int c, double v) { Wk[(int64_t)(p0 + c) * AG_T + p0 + i] = v; });
-        __syncwarp();
-    }
-    __syncthreads();
-    assemble_w128(T, ld, Wk, 1, tsm + 8 * 32 * 33, warp, lane, 8, 1, 256);
-    __syncthreads();
+    p128_invert(tsm, tsm + P128_S + P128_D, unit_diag, Wk, tid >> 5, tid & 31, 1);
     double *Wb = W + (int64_t)(b * AG_T) * ldw + b * AG_T;
     for (int e = tid; e < AG_T * AG_T; e += 256) {
         const int r = e % AG_T, c = e / AG_T;
@@ -327,7 +317,7 @@ static int ag_inverse(Context *ctx, const double *L, double *W, double *Y, doubl
     cudaStream_t st = ctx->stream;
     int rc;
     CK(cudaMemsetAsync(W, 0, (size_t)ld * ld * sizeof(double), st));
-    const size_t tsmem = (8 * 32 * 33 + 8 * 32 * 36) * sizeof(double);
+    const size_t tsmem = P128_INV_DOUBLES * sizeof(double);
     CK(cudaFuncSetAttribute(ag_trtri_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
     ag_trtri_diag<<<P, 256, tsmem, st>>>(L, ld, W, ld, scr, unit);
     CK(cudaGetLastError());

@@ -14,12 +14,13 @@
 //     on the chain but the last block's;
 //   - while warp 0 updates and factors the next diagonal block the others update
 //     the rest, assemble the finished rows of the inverse and store what is done.
-// Measured on one SM: 49,000 cycles (25 us) with load and stores; the form it
-// replaces (block in L2, inverse on the chain, a panel per barrier) took 123 us
-// where its code was cold and about 75 us warm.
+// Measured in place: 33 us with load and stores; the form it replaces (block in
+// L2, inverse on the chain, a panel per barrier) took 123 us where its code was
+// cold and about 75 us warm.
 #pragma once
 #include "dev_common.cuh"
 #include "dev_chol32.cuh"
+#include "dev_frag.cuh"
 
 namespace db2 {
 
@@ -27,198 +28,8 @@ constexpr int P128_SP = 132;                              // pitch of the block'
 constexpr int P128_DP = 36;                               // pitch of the 32x32 inverses (= 4 mod 16)
 constexpr int P128_S = 128 * P128_SP;                     // the block; W's off-diagonal blocks in its upper part
 constexpr int P128_D = 4 * 32 * P128_DP;                  // inverses of the 32x32 diagonal blocks, row-major
-constexpr int P128_LB = 1024 + 32;                        // blocked copy of the current 32x32 factor, 1/diagonal
+constexpr int P128_LB = C32_LB;                           // blocked copy of the current 32x32 factor, 1/diagonal
 constexpr int P128_DOUBLES = P128_S + P128_D + P128_LB;   // shared scratch in doubles
-
-// 1 / sqrt(x) without a branch, x within the range the caller checks: the
-// hardware's approximation and two Newton steps y += y (1/2 - x/2 y^2).
-__device__ __forceinline__ double rsqrt_newton(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double h = 0.5 * x;
-    y = fma(y, fma(-h * y, y, 0.5), y);
-    y = fma(y, fma(-h * y, y, 0.5), y);
-    return y;
-}
-
-// Columns J0 .. J0+15 of the 32x32 factorization (frame: d[k] = A(i, j + k) at
-// column j); LIVE columns of the frame are kept up to date.
-template <int LIVE>
-__device__ __forceinline__ void chol32_half(double (&d)[32], int J0, int lane, double &dg, double &lp, double &piv,
-                                            double &rdiag, bool &ok, double *Sd, int sp, double *Lb)
-{
-#pragma unroll
-    for (int jj = 0; jj < 16; ++jj) {
-        const int j = J0 + jj;
-        // what the next pivot needs from lane j + 1, before the pivot's root is known
-        const double dn = __shfl_sync(0xffffffffu, dg, j + 1);       // its diagonal entry
-        const double an = __shfl_sync(0xffffffffu, d[0], j + 1);     // A(j+1, j)
-        ok = ok && piv > 1e-280 && piv < 1e280;
-        const double r = rsqrt_newton(piv);
-        // column j - 1 applied to the columns beyond j
-        if (j > 0) {
-            // (16-byte pairs where row j + k is even)
-            const double *Lp = Sd + (j - 1) * sp + j;
-            if (jj & 1) {
-#pragma unroll
-                for (int k = 1; k < LIVE; k += 2) {
-                    const double2 v = *reinterpret_cast<const double2 *>(Lp + k);
-                    d[k] = fma(-lp, v.x, d[k]);
-                    if (k + 1 < LIVE) d[k + 1] = fma(-lp, v.y, d[k + 1]);
-                }
-            } else {
-                d[1] = fma(-lp, Lp[1], d[1]);
-#pragma unroll
-                for (int k = 2; k < LIVE; k += 2) {
-                    const double2 v = *reinterpret_cast<const double2 *>(Lp + k);
-                    d[k] = fma(-lp, v.x, d[k]);
-                    if (k + 1 < LIVE) d[k + 1] = fma(-lp, v.y, d[k + 1]);
-                }
-            }
-        }
-        const double ln = an * r;                                     // L(j+1, j)
-        const double pn = fma(-ln, ln, dn);
-        double l = d[0] * r;
-        const double s = fma(fma(-l, l, piv), 0.5 * r, l);            // lane j: sqrt, corrected
-        dg = fma(-l, l, dg);
-        const double d0 = fma(-l, ln, d[1]);
-        if (lane == j) {
-            l = s;
-            rdiag = r;
-        }
-        if (lane >= j) Sd[j * sp + lane] = l;
-        Lb[(j >> 2) * 128 + lane * 4 + (j & 3)] = lane >= j ? l : 0.0;
-        __syncwarp();
-        lp = l;
-        piv = pn;
-#pragma unroll
-        for (int k = 1; k < LIVE - 1; ++k) d[k] = d[k + 1];
-        d[0] = d0;
-    }
-}
-
-// Cholesky factor of the 32x32 block at Sd (column c, row r at c * sp + r) in
-// place by one warp, lane i owning row i.  Also the blocked copy Lb
-// ([8][32][4]) and rd[c] = 1 / L(c,c).  Returns false when a pivot leaves the
-// range in which the branch-free root is good (or is not positive): the block
-// is then spoilt below the diagonal.
-__device__ __forceinline__ bool chol32_col(double (&d)[32], int lane, double *Sd, int sp, double *Lb, double *rd)
-{
-    double dg = 0.0, lp = 0.0, rdiag = 0.0;
-#pragma unroll
-    for (int c = 0; c < 32; ++c)
-        if (lane == c) dg = d[c];
-    double piv = __shfl_sync(0xffffffffu, dg, 0);
-    bool ok = true;
-    chol32_half<32>(d, 0, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
-    chol32_half<16>(d, 16, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
-    rd[lane] = rdiag;
-    __syncwarp();
-    return ok;
-}
-
-// Solve L x = b for one right-hand side per lane (b[c], c = 0..31), L in the
-// blocked copy Lb and rd[c] = 1 / L(c,c): steps of four columns in a rotating
-// frame, out(c, x) receives x_c.
-template <class Out>
-__device__ __forceinline__ void sweep32(const double *Lb, const double *rd, double (&b)[32], Out out)
-{
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-        const double *Lk = Lb + (j >> 2) * 128;
-        double r4[4];
-        c32_load4(rd + j, r4);
-        const double l10 = Lk[(j + 1) * 4], l20 = Lk[(j + 2) * 4], l21 = Lk[(j + 2) * 4 + 1];
-        const double l30 = Lk[(j + 3) * 4], l31 = Lk[(j + 3) * 4 + 1], l32 = Lk[(j + 3) * 4 + 2];
-        double x[4];
-        x[0] = b[0] * r4[0];
-        x[1] = (b[1] - l10 * x[0]) * r4[1];
-        b[2] -= l20 * x[0];
-        b[3] -= l30 * x[0];
-        x[2] = (b[2] - l21 * x[1]) * r4[2];
-        b[3] -= l31 * x[1];
-        x[3] = (b[3] - l32 * x[2]) * r4[3];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) out(j + r, x[r]);
-#pragma unroll
-        for (int c = 4; c < 32; ++c) {
-            if (j + c < 32) {
-                double v[4];
-                c32_load4(Lk + (j + c) * 4, v);
-                b[c] -= v[0] * x[0];
-                b[c] -= v[1] * x[1];
-                b[c] -= v[2] * x[2];
-                b[c] -= v[3] * x[3];
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 28; ++q) b[q] = b[q + 4];
-    }
-}
-
-// acc (MI*16 x NI*8 fragments of one warp) += (-) A B over one 32-deep block:
-// A(m, k) at Ap[k * ak + m * am], B(k, n) at Bp[k * bk + n * bn].
-template <int MI, int NI>
-__device__ __forceinline__ void mma32(double (&acc)[MI][NI][4], const double *Ap, int ak, int am, const double *Bp,
-                                      int bk, int bn, bool neg, int lane)
-{
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int kk = 0; kk < 32; kk += 4) {
-        double af[MI][2], bf[NI];
-#pragma unroll
-        for (int mi = 0; mi < MI; ++mi) {
-            af[mi][0] = Ap[(kk + t) * ak + (mi * 16 + g) * am];
-            af[mi][1] = Ap[(kk + t) * ak + (mi * 16 + g + 8) * am];
-            if (neg) {
-                af[mi][0] = -af[mi][0];
-                af[mi][1] = -af[mi][1];
-            }
-        }
-#pragma unroll
-        for (int ni = 0; ni < NI; ++ni) bf[ni] = Bp[(kk + t) * bk + (ni * 8 + g) * bn];
-#pragma unroll
-        for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < NI; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
-    }
-}
-// fragments <-> memory, element (r, c) at p[r * rs + c * cs]
-template <int MI, int NI>
-__device__ __forceinline__ void frag_load(double (&acc)[MI][NI][4], const double *p, int rs, int cs, int lane)
-{
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NI; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                acc[mi][ni][q] = p[(mi * 16 + g + ((q & 2) ? 8 : 0)) * rs + (ni * 8 + 2 * t + (q & 1)) * cs];
-}
-template <int MI, int NI>
-__device__ __forceinline__ void frag_store(const double (&acc)[MI][NI][4], double *p, int rs, int cs, int lane)
-{
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NI; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                p[(mi * 16 + g + ((q & 2) ? 8 : 0)) * rs + (ni * 8 + 2 * t + (q & 1)) * cs] = acc[mi][ni][q];
-}
-template <int MI, int NI>
-__device__ __forceinline__ void frag_zero(double (&acc)[MI][NI][4])
-{
-#pragma unroll
-    for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NI; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-}
 
 __device__ __forceinline__ void named_bar_arrive(int id, int nthreads)
 {
@@ -232,7 +43,7 @@ __device__ __forceinline__ void named_bar_arrive(int id, int nthreads)
 // P128_UNITS[phase][warp] lists up to two units per warp; phase 2 j is the one
 // in which warp 0 factors diagonal block j, 2 j + 1 the sweeps of that step,
 // 8 the last products.  Row i needs D_i (phase 2 i + 1) and the rows above.
-constexpr uint16_t p128_unit(int i, int c, int h, int l0, int l1, int first, int dg)
+__host__ __device__ constexpr uint16_t p128_unit(int i, int c, int h, int l0, int l1, int first, int dg)
 {
     return (uint16_t)(1 | i << 1 | c << 3 | h << 5 | l0 << 6 | l1 << 8 | first << 10 | dg << 11);
 }
@@ -349,7 +160,7 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
                                              int bar)
 {
     constexpr int SP = P128_SP, DP = P128_DP;
-    double *D = S + P128_S, *Lb = D + P128_D, *rd = Lb + 1024;
+    double *D = S + P128_S, *Lb = D + P128_D, *rd = Lb + C32_RD;
     const int w = warp < 4 ? warp - 1 : warp - 2;       // 0..5 for the helpers
     const bool helper = warp != 0 && warp != 4;         // warp 4 shares warp 0's sub-partition
 #pragma unroll 1
@@ -441,6 +252,45 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
     }
     return -1;
 }
+
+// Inverse of the lower triangular block in S (unit: diagonal taken as 1) to
+// the 128x128 block Wb, zero above the diagonal, by the 256 threads of barrier
+// `bar`; LB4 is scratch of 4 P128_LB doubles, S keeps the layout above.
+__device__ __forceinline__ void p128_invert(double *S, double *LB4, int unit, double *Wb, int warp, int lane, int bar)
+{
+    constexpr int SP = P128_SP, DP = P128_DP;
+    double *D = S + P128_S;
+    if (warp < 4) {
+        // the four diagonal blocks: blocked copy, then the unit vectors
+        double *Lb = LB4 + warp * P128_LB, *rd = Lb + C32_RD;
+        const double *Sd = S + warp * 32 * SP + warp * 32 + lane;
+#pragma unroll 8
+        for (int c = 0; c < 32; ++c) Lb[(c >> 2) * 128 + lane * 4 + (c & 3)] = c <= lane ? Sd[c * SP] : 0.0;
+        rd[lane] = unit ? 1.0 : 1.0 / Sd[lane * SP];
+        __syncwarp();
+        double b[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) b[c] = c == lane ? 1.0 : 0.0;
+        double *o = D + warp * 32 * DP + lane;
+        sweep32(Lb, rd, b, [&](int c, double x) { o[c * DP] = x; });
+    } else {
+        // W is zero above its diagonal blocks
+#pragma unroll 1
+        for (int c = 32 + (warp - 4); c < 128; c += 4)
+#pragma unroll
+            for (int r0 = 0; r0 < 96; r0 += 32)
+                if (r0 + 32 <= (c & ~31)) Wb[c * 128 + r0 + lane] = 0.0;
+    }
+    named_bar_sync(bar, 256);
+    // block row i: W_ic = -D_i sum_{l=c}^{i-1} L_il W_lc, a column half per warp
+#pragma unroll 1
+    for (int i = 1; i < 4; ++i) {
+        if (warp < 2 * i) p128_run_unit(p128_unit(i, warp >> 1, warp & 1, warp >> 1, i, 1, 1), S, D, Wb, lane);
+        if (warp >= 6 && i < 3) p128_put_d(D, 2 * (i - 1) + (warp - 6), Wb, lane);
+        named_bar_sync(bar, 256);
+    }
+}
+constexpr int P128_INV_DOUBLES = P128_S + P128_D + 4 * P128_LB;
 
 // Load the lower 32-blocks (whole: all) of the 128x128 block at T (leading
 // dimension ld), 256 threads.

@@ -39,6 +39,7 @@ enum BufferId : int {
     BUF_ADJ,          // adjoint: dense L, W = L^-1 and two products
     BUF_BATCH_SCR,    // batched: per-CTA inverses of the diagonal blocks
     BUF_BATCH_W,      // batched inverse: per-CTA padded factor and L^-1
+    BUF_WX_EXCH,      // triangular sweeps: solved blocks on their way along the chain
     BUF_SELFCHECK,    // per-ticket run counters (self check)
     BUF_WX,           // second block row [Linv10 | W1] of the inverses of 256-wide diagonal tiles
     BUF_LINV16,       // inverses of the diagonal tiles in split FP16 (tensor-core TRSM strips)

@@ -9,7 +9,10 @@
 //     known (acc_nq then holds every term but q's), waits for Y_q and forms
 //     Y_nq = Z - M_nq Y_q with M_nq = W_nq^{op} op(L)_{nq,q} (prepared for
 //     every block before the sweep, wave_prep_kernel), stores it and raises
-//     nq's flag;
+//     nq's flag.  The solved block travels to that CTA and the next block's
+//     through an exchange buffer whose words say by themselves whether they have arrived (it starts
+//     as all-ones NaNs, which no result is), so the chain has one store and the
+//     polling load on it and no fence, flag and separate read;
 //   * otherwise: waits for q's flag and stages Y_q in shared memory;
 //   * applies acc_p -= op(L)_pq Y_q to each owned block p still to solve.
 // Each owned accumulator is updated in increasing q by one CTA, so the result
@@ -17,7 +20,8 @@
 // ring of bulk copies ahead of the flags (they do not depend on Y), so the
 // critical path per block is one flag and one 128x128 product, while the bulk
 // of L streams from HBM on all SMs at once.  CTAs wait on one another, hence
-// the cooperative launch.
+// the cooperative launch.  When the blocks leave SMs idle, several groups of
+// CTAs sweep a share of the right-hand-side columns each (sweep_shape).
 //
 // L and W arrive by TMA tensor loads with the 128-byte swizzle (a stage of
 // 32 KB takes 8 or 2 loads).  The stage holds 16-row slabs of 128-byte lines
@@ -35,10 +39,11 @@
 
 #include "dev_common.cuh"
 #include "dev_tcgen05.cuh"
-#include "dev_trtri.cuh"
+#include "dev_frag.cuh"
 #include "internal.h"
 
 #include <stdio.h>
+#include <algorithm>
 #include <vector>
 
 namespace db2 {
@@ -61,8 +66,10 @@ struct WaveArgs {
     int ldy;
     int mt, nbi, nbs, nblk;
     int c0;
+    int gsub;              // CTAs per column group
     double alpha;
-    int *flags;
+    double *X;             // exchange buffer: [group][block][column][row]
+    int *flags;            // [group][block]
     int *status;
     uint64_t limit_ns;
     uint32_t smem_bytes;   // dynamic shared memory of the launch
@@ -110,6 +117,22 @@ __device__ __forceinline__ int wv_block(int qi, int P) { return TRANS ? P - 1 - 
 template <bool TRANS>
 __device__ __forceinline__ int wv_pos(int p, int P) { return TRANS ? P - 1 - p : p; }
 
+// A word of the exchange buffer that has not arrived: all ones, a NaN that no
+// arithmetic returns and that wv_send replaces by another NaN.
+constexpr unsigned long long WV_EMPTY = ~0ull;
+__device__ __forceinline__ void wv_send(double *p, double v)
+{
+    unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    if (u == WV_EMPTY) u = 0x7ff8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+}
+__device__ __forceinline__ unsigned long long wv_peek(const double *p)
+{
+    unsigned long long u;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
+    return u;
+}
+
 template <int NC, bool TRANS>
 __global__ void __launch_bounds__(WV_THREADS, 1)
     trsm_wave_kernel(WaveArgs a, const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap wmap,
@@ -128,7 +151,12 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
         if (tid == 0) atomicCAS(a.status, ST_OK, ST_BAD_TASK);
         return;
     }
-    const int c = blockIdx.x, G = gridDim.x, P = a.nblk;
+    const int group = blockIdx.x / a.gsub;
+    const int c = blockIdx.x - group * a.gsub, G = a.gsub, P = a.nblk;
+    a.c0 += group * NC;
+    a.flags += group * P;
+    a.X += (int64_t)group * P * (NC * 128);
+    if (group > 0) a.trace = nullptr;
     if (tid == 0) {
         for (int s = 0; s < WV_NST; ++s) {
             mbar_init(&ctl->full[s], 1);
@@ -326,6 +354,13 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
     // the solved block to global memory, then its flag; its copy in shared
     // memory (for this CTA's own updates) is written afterwards by own_stage,
     // once the deferred products no longer read that buffer
+    auto send = [&](const double (&y)[NT][4], int q) {
+        double *Xq = a.X + (int64_t)q * (NC * 128);
+#pragma unroll
+        for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) wv_send(Xq + (ni * 8 + 2 * t + (e & 1)) * 128 + ((e & 2) ? rb : ra), y[ni][e]);
+    };
     auto publish = [&](const double (&y)[NT][4], int q) {
         double *Yq = a.Y + (int64_t)a.c0 * a.ldy + (int64_t)q * 128;
 #pragma unroll
@@ -391,6 +426,7 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
             if (lane == 0) mbar_arrive(&ctl->empty[s]);
             ++it;
         }
+        send(res, q);
         named_bar_sync(1, 256);
         double *Yq = a.Y + (int64_t)a.c0 * a.ldy + (int64_t)q * 128;
 #pragma unroll
@@ -458,7 +494,44 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
         tmark(5);
         if (tr && tid == 0) tr[6] += 1;
         const bool own_nq = nq >= 0 && nq % G == c, own_nnq = nnq >= 0 && nnq % G == c;
-        if (q % G != c) {
+        if (q % G != c && (own_nq || own_nnq)) {
+            // critical path (of the next block, or of the Z of the one after): Y_q
+            // word by word from the exchange buffer
+            constexpr int NV = NC * 128 / 256;
+            const double *Xq = a.X + (int64_t)q * (NC * 128) + tid;
+            unsigned long long v[NV];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] = wv_peek(Xq + 256 * i);
+            bool good = true;
+            uint64_t t0 = 0;
+            for (int spins = 0;; ++spins) {
+                bool all = true;
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (v[i] == WV_EMPTY) {
+                        v[i] = wv_peek(Xq + 256 * i);
+                        all = false;
+                    }
+                if (all) break;
+                if ((spins & 255) == 255) {
+                    const uint64_t t1 = globaltimer_ns();
+                    if (t0 == 0) t0 = t1;
+                    if (ld_volatile(a.status) != ST_OK || t1 - t0 > a.limit_ns) {
+                        atomicCAS(a.status, ST_OK, ST_DEP_TIMEOUT);
+                        good = false;
+                        break;
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const int e = tid + 256 * i;
+                Yq[(e >> 7) * WV_YP + (e & 127)] = -__longlong_as_double((long long)v[i]);
+            }
+            // one decision for all consumer warps; the barrier also ends the staging
+            if (named_bar_or(1, 256, !good)) break;
+            tmark(0);
+        } else if (q % G != c) {
             // Y_q from its owner
             int good = 1;
             if (tid == 0) {
@@ -489,6 +562,7 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
             for (int i = 0; i < WV_RMAX; ++i) {
                 if (c + i * G != nq) continue;
                 update(acc[i], Yq);
+                if (ok) send(acc[i], nq);
                 if (named_bar_or(1, 256, !ok))
                     ok = false;
                 else
@@ -541,20 +615,32 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
 //   forward:  M_b = W_b L_{b,b-1},  b = 1 .. P-1;
 //   backward: M_b = L_{b+1,b} W_b,  b = 0 .. P-2 (the backward ring reads the
 //             transpose, W_b^T L_{b+1,b}^T).
+// Four CTAs of 32 rows per block (the block of one warp is 32 x 16), so a short
+// sweep's preparation takes one 32-row product's time: 33 us (one CTA per block)
+// before at 31 blocks, 8 us now.
 __global__ void __launch_bounds__(256) wave_prep_kernel(const double *A, const double *W, int mt, int nbi, int nbs,
                                                         int transposed, double *M)
 {
-    const int b = transposed ? (int)blockIdx.x : (int)blockIdx.x + 1;
+    const int b = transposed ? (int)blockIdx.x : (int)blockIdx.x + 1, s = blockIdx.y;
     const int p = transposed ? b + 1 : b, q = transposed ? b : b - 1;     // the sub-diagonal block L_{p,q}
     const double *Lpq = A + lower_tile_index(p / nbs, q / nbs, mt) * (int64_t)nbi * nbi +
                         (int64_t)(q % nbs) * 128 * nbi + (p % nbs) * 128;
     const double *Wb = W + (int64_t)b * 128 * 128;
-    double *Mb = M + (int64_t)b * 128 * 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (!transposed)
-        gemm128_tri(Wb, 128, true, Lpq, nbi, false, false, Mb, 128, 1.0, warp, lane, 8);
-    else
-        gemm128_tri(Lpq, nbi, false, Wb, 128, true, false, Mb, 128, 1.0, warp, lane, 8);
+    double acc[2][2][4];
+    frag_zero(acc);
+    if (!transposed) {
+        // rows 32 s .. of W reach K block s
+#pragma unroll 1
+        for (int l = 0; l <= s; ++l)
+            mma32(acc, Wb + l * 32 * 128 + 32 * s, 128, 1, Lpq + (int64_t)(16 * warp) * nbi + 32 * l, 1, nbi, false, lane);
+    } else {
+        // columns 16 w .. of W start in K block w / 2
+#pragma unroll 1
+        for (int l = warp >> 1; l < 4; ++l)
+            mma32(acc, Lpq + (int64_t)(32 * l) * nbi + 32 * s, nbi, 1, Wb + 16 * warp * 128 + 32 * l, 1, 128, false, lane);
+    }
+    frag_store(acc, M + (int64_t)b * 128 * 128 + 16 * warp * 128 + 32 * s, 1, 128, lane);
 }
 
 static size_t wave_smem_bytes(int nc)
@@ -596,6 +682,25 @@ int wave_max_blocks_per_sm()
     return best;
 }
 
+// Columns per group (a multiple of 8), groups and CTAs per group of a launch.
+// The chain's step grows with the columns (one 128 x 128 x nc product), so a
+// sweep with SMs to spare takes the narrowest groups whose CTAs own at most two
+// blocks each; where one group needs the grid, up to 32 columns go through it
+// at a time (WV_RMAX blocks per CTA).  Every group reads L.
+struct SweepShape {
+    int nc, groups, gsub;
+};
+static SweepShape sweep_shape(int nblk, int nrhs, int grid)
+{
+    for (int nc = 8; nc <= 32; nc += 8) {
+        const int ng = (nrhs + nc - 1) / nc;
+        if (2 * ng > grid || (ng > 1 && nrhs % nc != 0)) continue;   // groups are all alike
+        const int gsub = std::max(2, std::min(nblk, grid / ng));
+        if (ng == 1 || (nblk + gsub - 1) / gsub <= 2) return {nc, ng, gsub};
+    }
+    return {std::min(32, nrhs), 1, std::max(2, std::min(nblk, grid))};
+}
+
 // Returns 1 when the shape does not fit the wavefront kernel (more than
 // WV_RMAX blocks per CTA), 0 on success, a negative dplasma error otherwise.
 int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, double *dB, int ldb, int nrhs,
@@ -606,11 +711,16 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
     // which the schedule's deferral relies on
     const int grid = ctx->sms * (ctx->wave_occ > 0 ? 1 : 0);
     if (grid < 2 || nblk > WV_RMAX * grid) return 1;
-    const int nchunks = (nrhs + 31) / 32;
-    const size_t per = (size_t)nblk + 4;
-    int *ctr = (int *)ctx->buffer(BUF_SOLVE_CTR, per * nchunks * sizeof(int));
-    if (!ctr) return DPLASMA_ERR_OUT_OF_RESOURCES;
-    CK(cudaMemsetAsync(ctr, 0, per * nchunks * sizeof(int), ctx->stream));
+    const SweepShape sh = sweep_shape(nblk, nrhs, grid);
+    const int per_launch = sh.nc * sh.groups, nlaunch = (nrhs + per_launch - 1) / per_launch;
+    // status, then one flag per block and group, for each launch
+    const size_t per = 4 + (size_t)nblk * sh.groups;
+    int *ctr = (int *)ctx->buffer(BUF_SOLVE_CTR, per * nlaunch * sizeof(int));
+    const size_t xbytes = (size_t)nblk * 128 * per_launch * sizeof(double);
+    double *X = (double *)ctx->buffer(BUF_WX_EXCH, xbytes * nlaunch);
+    if (!ctr || !X) return DPLASMA_ERR_OUT_OF_RESOURCES;
+    CK(cudaMemsetAsync(ctr, 0, per * nlaunch * sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(X, 0xff, xbytes * nlaunch, ctx->stream));      // WV_EMPTY
     // L: rows of the tiles contiguous (nbi), one line per tile column;
     // W: 128x128 column-major blocks.  Boxes of 16 doubles (128 bytes, the
     // swizzle span) by 32 (forward: k columns) or 128 (backward: columns).
@@ -618,7 +728,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
     double *M = (double *)ctx->buffer(BUF_WM, (size_t)nblk * 128 * 128 * sizeof(double));
     if (!M) return DPLASMA_ERR_OUT_OF_RESOURCES;
     if (nblk > 1) {
-        wave_prep_kernel<<<nblk - 1, 256, 0, ctx->stream>>>(dA, W, g.mt, g.nbi, g.nbi / 128, transposed, M);
+        wave_prep_kernel<<<dim3(nblk - 1, 4), 256, 0, ctx->stream>>>(dA, W, g.mt, g.nbi, g.nbi / 128, transposed, M);
         CK(cudaGetLastError());
         ctx->launches++;
     }
@@ -634,7 +744,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         rc0 = encode_map_2d(ctx, &mmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void *)M, 128, (uint64_t)nblk * 128,
                             128 * sizeof(double), 16, box1, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc0) return rc0;
-    for (int ch = 0; ch < nchunks; ++ch) {
+    for (int ch = 0; ch < nlaunch; ++ch) {
         WaveArgs a;
         a.A = dA;
         a.W = W;
@@ -644,46 +754,53 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         a.nbi = g.nbi;
         a.nbs = g.nbi / 128;
         a.nblk = nblk;
-        a.c0 = ch * 32;
+        a.c0 = ch * per_launch;
+        a.gsub = sh.gsub;
+        a.X = X + (size_t)ch * (xbytes / sizeof(double));
         a.alpha = alpha;
         a.status = ctr + per * ch;
         a.flags = ctr + per * ch + 4;
         a.limit_ns = ctx->dep_limit_ns;
         a.trace = nullptr;
         if (ctx->wave_trace_path[0]) {
-            const size_t tb = ((size_t)grid * WV_TR_SLOTS + nblk) * sizeof(unsigned long long);
+            const size_t tb = ((size_t)sh.gsub * WV_TR_SLOTS + nblk) * sizeof(unsigned long long);
             a.trace = (unsigned long long *)ctx->buffer(BUF_WTRACE, tb);
             if (!a.trace) return DPLASMA_ERR_OUT_OF_RESOURCES;
             CK(cudaMemsetAsync(a.trace, 0, tb, ctx->stream));
         }
-        const int nc = (nrhs - a.c0) < 32 ? (nrhs - a.c0) : 32;   // nrhs is a multiple of 8
+        // nrhs and nc are multiples of 8; the last launch may have fewer groups,
+        // and narrower ones where a single group remains
+        const int left = nrhs - a.c0;
+        const int ng = std::min(sh.groups, (left + sh.nc - 1) / sh.nc);
+        const int nc = ng == 1 ? std::min(left, sh.nc) : sh.nc;
+        const int cta = ng * sh.gsub;
         int rc;
         if (transposed)
-            rc = nc <= 8    ? launch_wave<8, true>(ctx, a, grid, lmap, wmap, mmap)
-                 : nc <= 16 ? launch_wave<16, true>(ctx, a, grid, lmap, wmap, mmap)
-                 : nc <= 24 ? launch_wave<24, true>(ctx, a, grid, lmap, wmap, mmap)
-                            : launch_wave<32, true>(ctx, a, grid, lmap, wmap, mmap);
+            rc = nc <= 8    ? launch_wave<8, true>(ctx, a, cta, lmap, wmap, mmap)
+                 : nc <= 16 ? launch_wave<16, true>(ctx, a, cta, lmap, wmap, mmap)
+                 : nc <= 24 ? launch_wave<24, true>(ctx, a, cta, lmap, wmap, mmap)
+                            : launch_wave<32, true>(ctx, a, cta, lmap, wmap, mmap);
         else
-            rc = nc <= 8    ? launch_wave<8, false>(ctx, a, grid, lmap, wmap, mmap)
-                 : nc <= 16 ? launch_wave<16, false>(ctx, a, grid, lmap, wmap, mmap)
-                 : nc <= 24 ? launch_wave<24, false>(ctx, a, grid, lmap, wmap, mmap)
-                            : launch_wave<32, false>(ctx, a, grid, lmap, wmap, mmap);
+            rc = nc <= 8    ? launch_wave<8, false>(ctx, a, cta, lmap, wmap, mmap)
+                 : nc <= 16 ? launch_wave<16, false>(ctx, a, cta, lmap, wmap, mmap)
+                 : nc <= 24 ? launch_wave<24, false>(ctx, a, cta, lmap, wmap, mmap)
+                            : launch_wave<32, false>(ctx, a, cta, lmap, wmap, mmap);
         if (rc) return rc;
         if (a.trace) {
             // one line per sweep: CTA-summed ns per part, and the mean step of
             // the wavefront (ns between consecutive publishes) per eighth of the blocks
-            std::vector<unsigned long long> h((size_t)grid * WV_TR_SLOTS + nblk);
+            std::vector<unsigned long long> h((size_t)sh.gsub * WV_TR_SLOTS + nblk);
             CK(cudaMemcpyAsync(h.data(), a.trace, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                                ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
             unsigned long long sum[WV_TR_SLOTS] = {0};
-            for (int b = 0; b < grid; ++b)
+            for (int b = 0; b < sh.gsub; ++b)
                 for (int k = 0; k < WV_TR_SLOTS; ++k) sum[k] += h[(size_t)b * WV_TR_SLOTS + k];
             if (FILE *f = fopen(ctx->wave_trace_path, "a")) {
                 fprintf(f, "sweep trans %d nblk %d nc %d cta_ns wait %llu stage %llu crit %llu deferred %llu znext %llu "
                            "rest %llu positions %llu steps_ns",
                         transposed, nblk, nc, sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6]);
-                const unsigned long long *pt = h.data() + (size_t)grid * WV_TR_SLOTS;
+                const unsigned long long *pt = h.data() + (size_t)sh.gsub * WV_TR_SLOTS;
                 for (int e = 0; e < 8; ++e) {
                     const int q0 = e * nblk / 8, q1 = (e + 1) * nblk / 8;
                     const int b0 = transposed ? nblk - 1 - q0 : q0, b1 = transposed ? nblk - q1 : q1 - 1;
@@ -696,7 +813,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         }
     }
     int st = 0;
-    for (int ch = 0; ch < nchunks; ++ch) {
+    for (int ch = 0; ch < nlaunch; ++ch) {
         CK(cudaMemcpyAsync(&st, ctr + per * ch, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         if (st != ST_OK) {
