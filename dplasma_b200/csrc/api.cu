@@ -250,11 +250,13 @@ static int potrf_impl(Context *ctx, dplasma_enum_t uplo, parsec_tiled_matrix_t *
 {
     // nb_tasks: tile edge of the task DAG when it differs from the caller's
     // tiles (the recursive variant's sub-tiles); 0 = the caller's
-    Geom g = make_geom(A->m, nb_tasks > 0 ? nb_tasks : A->mb);
+    const int nbt = nb_tasks > 0 ? nb_tasks : A->mb;
+    const Geom gc = make_geom(A->m, nbt);
+    Geom g = work_geom(A->m, nbt);
     if (gout) *gout = g;
     if (A->m == 0) return 0;
-    if (g.mt > 65535 || g.nbi > 512) {
-        ctx->set_error("unsupported geometry (mt=%d, nb=%d): at most 65535 tile rows and nb <= 512", g.mt, g.nb);
+    if (gc.mt > 65535 || gc.nbi > 512) {
+        ctx->set_error("unsupported geometry (mt=%d, nb=%d): at most 65535 tile rows and nb <= 512", gc.mt, gc.nb);
         return DPLASMA_ERR_INTERNAL_LIMIT;
     }
     const bool inplace = in_place_ok(A, uplo, g);
@@ -408,7 +410,7 @@ extern "C" int dplasma_dpotrs(parsec_context_t *parsec, dplasma_enum_t uplo, con
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
     if (A->m == 0) return 0;
-    Geom g = make_geom(A->m, A->mb);
+    Geom g = work_geom(A->m, A->mb);
     const double *dA;
     double *W;
     if ((rc = load_factor(ctx, uplo, A, g, 0, &dA, &W))) return rc;
@@ -480,7 +482,7 @@ extern "C" int dplasma_dtrsm(parsec_context_t *parsec, dplasma_enum_t side, dpla
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
     if (A->m == 0) return 0;
-    Geom g = make_geom(A->m, A->mb);
+    Geom g = work_geom(A->m, A->mb);
     const double *dA;
     double *W;
     if ((rc = load_factor(ctx, uplo, A, g, diag == dplasmaUnit, &dA, &W))) return rc;
@@ -696,6 +698,7 @@ extern "C" int dplasma_b200_dsposv_ex(parsec_context_t *parsec, dplasma_enum_t u
         ctx->set_error("mixed-precision solve needs a tile size nb with 128 < nb <= 256 (got %d)", g.nb);
         return DPLASMA_ERR_NOT_SUPPORTED;
     }
+    g = make_geom(A->m, 256);       // whole tiles whatever the caller's edge (work_geom)
     const bool inplace = in_place_ok(A, uplo, g);
     double *A0 = inplace ? (double *)A->mat : (double *)ctx->buffer(BUF_A0, g.elems() * sizeof(double));
     double *L = (double *)ctx->buffer(BUF_A, g.elems() * sizeof(double));
@@ -705,7 +708,7 @@ extern "C" int dplasma_b200_dsposv_ex(parsec_context_t *parsec, dplasma_enum_t u
     const double *stream_src = nullptr;
     if (!inplace && !ctx->no_stream && o.shift == 0.0 && A->location == DPLASMA_B200_HOST &&
         A->storage == PARSEC_MATRIX_TILE &&
-        A->uplo == dplasmaLower && uplo == dplasmaLower && A->mb == A->nb && g.nbi == g.nb && g.n % g.nb == 0 &&
+        A->uplo == dplasmaLower && uplo == dplasmaLower && A->mb == A->nb && g.nbi == g.nb && g.nb == A->mb && g.n % g.nb == 0 &&
         A->lmt == g.mt) {
         cudaPointerAttributes pa;
         if (cudaPointerGetAttributes(&pa, A->mat) == cudaSuccess && pa.type == cudaMemoryTypeHost)
@@ -853,8 +856,8 @@ extern "C" int dplasma_dpotrf_adjoint(parsec_context_t *parsec, dplasma_enum_t u
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
     if (L->m == 0) return 0;
-    Geom g = make_geom(L->m, L->mb);
-    if (g.mt > 65535 || g.nbi > 512) return DPLASMA_ERR_INTERNAL_LIMIT;
+    const Geom gc = make_geom(L->m, L->mb), g = work_geom(L->m, L->mb);
+    if (gc.mt > 65535 || gc.nbi > 512) return DPLASMA_ERR_INTERNAL_LIMIT;
     double *Lt = (double *)ctx->buffer(BUF_A, g.elems() * sizeof(double));
     double *Lbt = (double *)ctx->buffer(BUF_A0, g.elems() * sizeof(double));
     if (!Lt || !Lbt) return DPLASMA_ERR_OUT_OF_RESOURCES;
@@ -885,8 +888,8 @@ static int inverse_api(parsec_context_t *parsec, const char *name, dplasma_enum_
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
     if (A->m == 0) return 0;
-    Geom g = make_geom(A->m, A->mb);
-    if (g.mt > 65535 || g.nbi > 512) return DPLASMA_ERR_INTERNAL_LIMIT;
+    const Geom gc = make_geom(A->m, A->mb), g = work_geom(A->m, A->mb);
+    if (gc.mt > 65535 || gc.nbi > 512) return DPLASMA_ERR_INTERNAL_LIMIT;
     double *Lt = (double *)ctx->buffer(BUF_A, g.elems() * sizeof(double));
     if (!Lt) return DPLASMA_ERR_OUT_OF_RESOURCES;
     if ((rc = upload_sym(ctx, A, uplo, g, Lt))) return rc;

@@ -143,6 +143,7 @@ struct Geom {
     size_t elems() const { return ntiles() * tile_elems(); }
 };
 Geom make_geom(int n, int nb);
+Geom work_geom(int n, int nb);
 
 // potrf_kernel.cu
 int potrf_device(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user, int *info);

@@ -19,6 +19,13 @@ Geom make_geom(int n, int nb)
     return g;
 }
 
+// Tiles of 128 where the caller's edge is no multiple of it (the matrix is
+// copied anyway): padded tile by tile, an edge of 93 costs (128/93)^3 = 2.6 times
+// the flops and 1.4 times the steps of the chain, 320 (384/320)^3 = 1.7 times
+// (N = 378 in 93-wide tiles: 5 steps, 0.37 ms; now 3, 0.23 ms; N = 7000 in
+// 320-wide ones: 9.0 ms, now 5.6 ms).
+Geom work_geom(int n, int nb) { return make_geom(n, nb % 128 == 0 ? nb : 128); }
+
 // ---------------------------------------------------------------------------
 // caller layout description, usable on the device
 // ---------------------------------------------------------------------------
@@ -89,106 +96,84 @@ __device__ __forceinline__ void tile_of_index(int64_t idx, int mt, int &m, int &
     m = nn + (int)rem;
 }
 
-__global__ void to_internal_kernel(DescView src, int uplo_upper, int n_user, int nb, int nbi, int mt, double *dA)
+// Caller's storage <-> device tiles, TO the tiles or back.  Internal tile (m,n)
+// element (r,c) is matrix element (i,j) = (m nb + r, n nb + c), whatever the
+// caller's own tile edge; only i >= j is moved (the stored triangle; upper
+// storage holds its mirror (j,i)).  The rest of a diagonal tile is zero and the
+// padding the identity.  One CTA per 64x64 piece, sixteen elements a thread;
+// an upper matrix is transposed through shared memory so that both sides are
+// read and written in runs of 64.  (One CTA per tile with an index division per
+// element took 137 us for N = 4096 in 256-wide tiles, 378 for the strided side
+// of an upper N = 7000.)
+constexpr int LM = 64;
+__device__ __forceinline__ int64_t view_elem(const DescView &v, int a, int b)
 {
+    if (v.storage == PARSEC_MATRIX_LAPACK) return (int64_t)b * v.lda + a;
+    const int ta = a / v.mb, tb = b / v.nb;
+    return view_tile_offset(v, ta, tb) + (a - ta * v.mb) + (int64_t)(b - tb * v.nb) * v.mb;
+}
+
+template <bool TO>
+__global__ void __launch_bounds__(256) sym_move_kernel(DescView v, int upper, int n_user, int nb, int nbi, int mt,
+                                                       double *dA)
+{
+    __shared__ double sm[LM][LM + 1];
     int m, n;
     tile_of_index(blockIdx.x, mt, m, n);
-    double *T = dA + (int64_t)blockIdx.x * nbi * nbi;
+    const int per = nbi / LM, r0 = (blockIdx.y % per) * LM, c0 = (blockIdx.y / per) * LM;
     const int tm = (m == mt - 1) ? n_user - m * nb : nb;
     const int tn = (n == mt - 1) ? n_user - n * nb : nb;
-    const int ld = view_ld(src);
-    const int64_t off = uplo_upper ? view_tile_offset(src, n, m) : view_tile_offset(src, m, n);
-    const double *S = src.mat + off;
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        double v;
-        if (r < tm && c < tn)
-            v = uplo_upper ? S[(int64_t)r * ld + c] : S[(int64_t)c * ld + r];
-        else
-            v = (m == n && r == c) ? 1.0 : 0.0;
-        T[e] = v;
+    double *T = dA + (int64_t)blockIdx.x * nbi * nbi + (int64_t)c0 * nbi + r0;
+    const int x = threadIdx.x & (LM - 1), y = threadIdx.x / LM;
+    constexpr int NY = 256 / LM;
+    // element (r, c) of the piece: moved, or what the tile holds instead
+    auto moved = [&](int r, int c) { return r0 + r < tm && c0 + c < tn && m * nb + r0 + r >= n * nb + c0 + c; };
+    auto filler = [&](int r, int c) {
+        return m == n && r0 + r == c0 + c && !(r0 + r < tm && c0 + c < tn) ? 1.0 : 0.0;
+    };
+    if (!upper) {
+        const int i = m * nb + r0 + x;
+#pragma unroll 8
+        for (int c = y; c < LM; c += NY) {
+            const int j = n * nb + c0 + c;
+            if (TO) T[(int64_t)c * nbi + x] = moved(x, c) ? v.mat[view_elem(v, i, j)] : filler(x, c);
+            else if (moved(x, c)) v.mat[view_elem(v, i, j)] = T[(int64_t)c * nbi + x];
+        }
+        return;
+    }
+    // caller's side: runs along c (rows of its column i)
+    if (TO) {
+#pragma unroll 8
+        for (int r = y; r < LM; r += NY)
+            sm[x][r] = moved(r, x) ? v.mat[view_elem(v, n * nb + c0 + x, m * nb + r0 + r)] : filler(r, x);
+        __syncthreads();
+#pragma unroll 8
+        for (int c = y; c < LM; c += NY) T[(int64_t)c * nbi + x] = sm[c][x];
+    } else {
+#pragma unroll 8
+        for (int c = y; c < LM; c += NY) sm[c][x] = T[(int64_t)c * nbi + x];
+        __syncthreads();
+#pragma unroll 8
+        for (int r = y; r < LM; r += NY)
+            if (moved(r, x)) v.mat[view_elem(v, n * nb + c0 + x, m * nb + r0 + r)] = sm[x][r];
     }
 }
 
-__global__ void from_internal_kernel(DescView dst, int uplo_upper, int n_user, int nb, int nbi, int mt, const double *dA)
+template <bool TO>
+static int sym_move(Context *ctx, const DescView &v, dplasma_enum_t uplo, const Geom &g, double *dA)
 {
-    int m, n;
-    tile_of_index(blockIdx.x, mt, m, n);
-    const double *T = dA + (int64_t)blockIdx.x * nbi * nbi;
-    const int tm = (m == mt - 1) ? n_user - m * nb : nb;
-    const int tn = (n == mt - 1) ? n_user - n * nb : nb;
-    const int ld = view_ld(dst);
-    const int64_t off = uplo_upper ? view_tile_offset(dst, n, m) : view_tile_offset(dst, m, n);
-    double *D = dst.mat + off;
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        if (r < tm && c < tn) {
-            if (uplo_upper)
-                D[(int64_t)r * ld + c] = T[e];
-            else
-                D[(int64_t)c * ld + r] = T[e];
-        }
-    }
-}
-
-// Internal tiles of a different edge than the caller's (the recursive
-// variant's sub-tiles): element by element.  Internal tile (m,n) element
-// (r,c) is matrix element (i,j) = (m nb + r, n nb + c); only i >= j is moved
-// (the stored triangle), the rest of a diagonal tile is zero and the padding
-// the identity.
-__global__ void to_internal_retile_kernel(DescView src, int uplo_upper, int n_user, int nb, int nbi, int mt,
-                                          double *dA)
-{
-    int m, n;
-    tile_of_index(blockIdx.x, mt, m, n);
-    double *T = dA + (int64_t)blockIdx.x * nbi * nbi;
-    const int tm = (m == mt - 1) ? n_user - m * nb : nb;
-    const int tn = (n == mt - 1) ? n_user - n * nb : nb;
-    const int ld = view_ld(src);
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        const int64_t i = (int64_t)m * nb + r, j = (int64_t)n * nb + c;
-        double v;
-        if (r < tm && c < tn) {
-            if (i < j) {
-                v = 0.0;
-            } else {
-                // lower storage holds (i, j); upper storage its mirror (j, i)
-                const int64_t a = uplo_upper ? j : i, b = uplo_upper ? i : j;
-                v = src.mat[view_tile_offset(src, (int)(a / src.mb), (int)(b / src.nb)) + (a % src.mb) +
-                            (b % src.nb) * ld];
-            }
-        } else {
-            v = (m == n && r == c) ? 1.0 : 0.0;
-        }
-        T[e] = v;
-    }
-}
-
-__global__ void from_internal_retile_kernel(DescView dst, int uplo_upper, int n_user, int nb, int nbi, int mt,
-                                            const double *dA)
-{
-    int m, n;
-    tile_of_index(blockIdx.x, mt, m, n);
-    const double *T = dA + (int64_t)blockIdx.x * nbi * nbi;
-    const int tm = (m == mt - 1) ? n_user - m * nb : nb;
-    const int tn = (n == mt - 1) ? n_user - n * nb : nb;
-    const int ld = view_ld(dst);
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        const int64_t i = (int64_t)m * nb + r, j = (int64_t)n * nb + c;
-        if (r < tm && c < tn && i >= j) {
-            const int64_t a = uplo_upper ? j : i, b = uplo_upper ? i : j;
-            dst.mat[view_tile_offset(dst, (int)(a / dst.mb), (int)(b / dst.nb)) + (a % dst.mb) + (b % dst.nb) * ld] =
-                T[e];
-        }
-    }
+    const int per = g.nbi / LM;
+    sym_move_kernel<TO><<<dim3((unsigned)g.ntiles(), per * per), 256, 0, ctx->stream>>>(v, uplo == dplasmaUpper, g.n,
+                                                                                       g.nb, g.nbi, g.mt, dA);
+    CK(cudaGetLastError());
+    ctx->launches++;
+    return 0;
 }
 
 static bool fast_path(const parsec_tiled_matrix_t *A, dplasma_enum_t uplo, const Geom &g)
 {
     return A->storage == PARSEC_MATRIX_TILE && A->uplo == dplasmaLower && uplo == dplasmaLower &&
-           g.nbi == g.nb && (g.n % g.nb) == 0 && A->lmt == g.mt && A->mb == A->nb;
+           g.nbi == g.nb && g.nb == A->mb && (g.n % g.nb) == 0 && A->lmt == g.mt && A->mb == A->nb;
 }
 
 int upload_sym(Context *ctx, const parsec_tiled_matrix_t *A, dplasma_enum_t uplo, const Geom &g, double *dA)
@@ -206,15 +191,7 @@ int upload_sym(Context *ctx, const parsec_tiled_matrix_t *A, dplasma_enum_t uplo
         if (!src) return DPLASMA_ERR_OUT_OF_RESOURCES;
         CK(cudaMemcpyAsync(src, A->mat, bytes, cudaMemcpyHostToDevice, st));
     }
-    DescView v = view_of(A, src);
-    if (g.nb != A->mb)
-        to_internal_retile_kernel<<<(unsigned)g.ntiles(), 256, 0, st>>>(v, uplo == dplasmaUpper, g.n, g.nb, g.nbi,
-                                                                        g.mt, dA);
-    else
-        to_internal_kernel<<<(unsigned)g.ntiles(), 256, 0, st>>>(v, uplo == dplasmaUpper, g.n, g.nb, g.nbi, g.mt, dA);
-    CK(cudaGetLastError());
-    ctx->launches++;
-    return 0;
+    return sym_move<true>(ctx, view_of(A, src), uplo, g, dA);
 }
 
 int download_sym(Context *ctx, parsec_tiled_matrix_t *A, dplasma_enum_t uplo, const Geom &g, const double *dA)
@@ -229,15 +206,8 @@ int download_sym(Context *ctx, parsec_tiled_matrix_t *A, dplasma_enum_t uplo, co
     }
     double *dst = (double *)A->mat;
     if (A->location != DPLASMA_B200_DEVICE) dst = (double *)ctx->buffer(BUF_STAGE, 0);   // filled by upload_sym
-    DescView v = view_of(A, dst);
-    if (g.nb != A->mb)
-        from_internal_retile_kernel<<<(unsigned)g.ntiles(), 256, 0, st>>>(v, uplo == dplasmaUpper, g.n, g.nb, g.nbi,
-                                                                          g.mt, dA);
-    else
-        from_internal_kernel<<<(unsigned)g.ntiles(), 256, 0, st>>>(v, uplo == dplasmaUpper, g.n, g.nb, g.nbi, g.mt,
-                                                                   dA);
-    CK(cudaGetLastError());
-    ctx->launches++;
+    const int rc = sym_move<false>(ctx, view_of(A, dst), uplo, g, const_cast<double *>(dA));
+    if (rc) return rc;
     if (A->location != DPLASMA_B200_DEVICE) CK(cudaMemcpyAsync(A->mat, dst, bytes, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return 0;
