@@ -46,7 +46,7 @@ template <bool MIXED>
 __device__ __forceinline__ int all_updates(const PotrfArgs &a, int m, int n)
 {
     if (MIXED) return (n + a.mx_chunk - 1) / a.mx_chunk;
-    if (a.fchunk) return block_updates(n, a.fchunk);
+    if (a.fchunk) return block_all_updates(m, n, a.fchunk);
     return n * step_blocks<MIXED>(a, m, n);
 }
 
@@ -91,8 +91,9 @@ __device__ bool wait_deps(const PotrfArgs &a, uint64_t t)
             // block order: panels [k, kl]; as above the last panel's strips
             // imply the earlier ones, and a block's updates run in order
             const int kl = k + task_bi(t) - 1;
-            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, 1, a.abort_flag, a.status, a.dep_limit_ns) &&
-                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, 1, a.abort_flag, a.status, a.dep_limit_ns) &&
+            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, block_strips(m, kl), a.abort_flag, a.status,
+                            a.dep_limit_ns) &&
+                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, block_strips(n, kl), a.abort_flag, a.status, a.dep_limit_ns) &&
                    wait_geq(a.upd_done + (int64_t)m * a.mt + n, block_update_index(k, n, a.fchunk), a.abort_flag,
                             a.status, a.dep_limit_ns);
         }
@@ -352,6 +353,10 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
             // block order: the operands change with each panel of 128
             const bool panels = !MIXED && a.fchunk && ty == T_GEMM;
             const double *Aop = jb.A, *Bop = jb.B;
+            // a slab: 32 rows of A (and of B, for a diagonal block, what lies below the slab's last column)
+            const int a0 = jb.slab >= 0 ? jb.slab * SLAB_ROWS : 0;
+            const uint32_t arows = jb.slab >= 0 ? SLAB_ROWS : BLK;
+            const uint32_t brows = jb.slab >= 0 && jb.mode == J_SUB_LOWER ? (jb.slab + 1) * SLAB_ROWS : BLK;
             for (int k0 = 0; k0 < jb.K; k0 += BK) {
                 if (panels && (k0 & (BLK - 1)) == 0) {
                     const int j = task_k(t) + k0 / BLK;
@@ -366,14 +371,14 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
                 }
                 double *As = ring + s * STAGE_DOUBLES;
                 double *Bs = As + BK * SP;
-                if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], 2 * BK * BLK * (uint32_t)sizeof(double));
+                if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], BK * (arows + brows) * (uint32_t)sizeof(double));
                 __syncwarp();
                 if (lane < BK)
-                    bulk_g2s(As + lane * SP, Aop + (int64_t)(k0 + lane) * jb.lda, BLK * sizeof(double),
+                    bulk_g2s(As + lane * SP, Aop + (int64_t)(k0 + lane) * jb.lda + a0, arows * sizeof(double),
                              &ctl->full[s]);
                 else
                     bulk_g2s(Bs + (lane - BK) * SP, Bop + (int64_t)(k0 + lane - BK) * jb.ldb,
-                             BLK * sizeof(double), &ctl->full[s]);
+                             brows * sizeof(double), &ctl->full[s]);
                 stage_it++;
             }
             prev_signal = jb.signal;
@@ -505,6 +510,70 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
                 }
     }
     __threadfence();   // this thread's reductions are performed before any later release
+    return true;
+}
+
+// ---------------------------------------------------------------------------
+// consumers: a 32-row slab of a 128x128 job (the chain's links), 16 columns per
+// warp.  A link of 32 x 128 x 128 took 7 us where the whole block took 20
+// (strip) and 26 us (update of the diagonal block).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool consume_slab(const PotrfArgs &a, SmemCtl *ctl, const double *ring, const Job &jb,
+                                             uint32_t &stage_it)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;
+    // column group: the two warps of a sub-partition share a triangular load evenly
+    const int cg = warp < 4 ? warp : 11 - warp;
+    const bool lower = jb.mode == J_SUB_LOWER;
+    const int klim = jb.tri ? 16 * (cg + 1) : (lower && cg > 2 * jb.slab + 1) ? 0 : jb.K;
+    double acc[2][2][4];
+    frag_zero(acc);
+    for (int k0 = 0; k0 < jb.K; k0 += BK) {
+        const uint32_t s = stage_it % NSTAGE, r = stage_it / NSTAGE;
+        if (!warp_mbar_wait(&ctl->full[s], r & 1, a.pipe_limit_ns)) {
+            if (lane == 0) report(a, ST_MBAR_TIMEOUT, 18, stage_it, warp);
+            stage_it += (jb.K - k0) / BK;
+            return false;
+        }
+        if (k0 < klim) {
+            const double *As = ring + s * STAGE_DOUBLES + g;
+            const double *Bs = ring + s * STAGE_DOUBLES + BK * SP + cg * 16 + g;
+#pragma unroll
+            for (int kk = 0; kk < BK; kk += 4) {
+                const int row = (kk + t) * SP;
+                double af[2][2], bf[2];
+#pragma unroll
+                for (int mi = 0; mi < 2; ++mi) {
+                    af[mi][0] = As[row + mi * 16];
+                    af[mi][1] = As[row + mi * 16 + 8];
+                }
+#pragma unroll
+                for (int ni = 0; ni < 2; ++ni) bf[ni] = Bs[row + ni * 8];
+#pragma unroll
+                for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                    for (int ni = 0; ni < 2; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->empty[s]);
+        stage_it++;
+    }
+    const int r0 = jb.slab * SLAB_ROWS;
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + mi * 16 + g + ((q & 2) ? 8 : 0);
+                const int c = cg * 16 + ni * 8 + 2 * t + (q & 1);
+                double *p = jb.C + (int64_t)c * jb.ldc + r;
+                if (jb.mode == J_STORE) *p = acc[mi][ni][q];
+                else if (!lower || r >= c) red_add_f64(p, -acc[mi][ni][q]);
+            }
+    __threadfence();
     return true;
 }
 
@@ -1097,7 +1166,8 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             const int nj = task_njobs(a, t);
             for (int j = 0; j < nj; ++j) {
                 const Job jb = task_job(a, t, j);
-                ok = consume_job<MIXED>(a, ctl, ring, jb, stage_it) && ok;
+                ok = (!MIXED && jb.slab >= 0 ? consume_slab(a, ctl, ring, jb, stage_it)
+                                             : consume_job<MIXED>(a, ctl, ring, jb, stage_it)) && ok;
                 if (jb.signal) {
                     fence_proxy_async();
                     if (named_bar_or(1, NCONS, !ok)) {
@@ -1318,7 +1388,7 @@ std::vector<uint64_t> build_potrf_tasks_mixed(int mt, int nbs, int delay, int S,
 // one block, so the large factorizations keep the long inner products of wide
 // tiles; the last panel of each column is a task of its own, so that the chain
 // POTRF(k) -> TRSM(k+1,k) -> update of (k+1,k+1) -> POTRF(k+1) has one
-// 128-deep product per link.  The update task of block (m,n) with the panels
+// 128-deep product per link, which four tasks share (slabs).  The update task of block (m,n) with the panels
 // j0 .. j0+cnt-1 carries k = j0 and bi = cnt.  Full chunks are spread over the
 // S steps after their last panel as in the mixed order below.  Step k: panel k
 // on column k+1, POTRF(k+1), the open chunk up to panel k on column k+2 (it
@@ -1329,7 +1399,8 @@ std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, 
 {
     std::vector<uint64_t> v;
     auto push_trsm = [&](int k) {
-        for (int m = k + 1; m < P; ++m) v.push_back(make_task(T_TRSM, k, m, k, 0, 0));
+        for (int s = 0; s < SLABS && k + 1 < P; ++s) v.push_back(make_task(T_TRSM, k, k + 1, k, 0, 1 + s));
+        for (int m = k + 2; m < P; ++m) v.push_back(make_task(T_TRSM, k, m, k, 0, 0));
     };
     // share[k]: the full chunks issued in step k.  Chunk c closes with panel
     // k = c S + S - 1; column n >= k + 2 takes it before its open chunk, which
@@ -1349,7 +1420,8 @@ std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, 
     v.push_back(make_task(T_POTRF, 0, 0, 0, 0, 0));
     push_trsm(0);
     for (int k = 0; k + 1 < P; ++k) {
-        for (int m = k + 1; m < P; ++m) v.push_back(make_task(T_GEMM, k, m, k + 1, 1, 0));
+        for (int s = 0; s < SLABS; ++s) v.push_back(make_task(T_GEMM, k, k + 1, k + 1, 1, 1 + s));
+        for (int m = k + 2; m < P; ++m) v.push_back(make_task(T_GEMM, k, m, k + 1, 1, 0));
         v.push_back(make_task(T_POTRF, k + 1, k + 1, k + 1, 0, 0));
         const int open = (k + 1) % S;                 // panels of column k+2's open chunk
         if (open != 0 && k + 2 < P)
@@ -1441,15 +1513,19 @@ static void selfcheck_tiles(const std::vector<uint64_t> &tl, const std::vector<i
     const int P = mt * nbs;
     // runs of panel j on block (m, n): [-1] is the block's own POTRF or TRSM
     auto at = [&](int m, int n, int j) { return ((size_t)m * (m + 1) / 2 + n) * (P + 1) + (j + 1); };
-    std::vector<unsigned char> cnt((size_t)P * (P + 1) / 2 * (P + 1), 0);
+    constexpr int SLAB_SUM = 1 + 8 + 64 + 512;
+    std::vector<int> cnt((size_t)P * (P + 1) / 2 * (P + 1), 0);
     for (size_t i = 0; i < tl.size(); ++i) {
         const uint64_t t = tl[i];
-        const int c = std::min(ran[i], 100);
-        if (task_type(t) == T_POTRF) cnt[at(task_k(t), task_k(t), -1)] += c;
-        else if (task_type(t) == T_TRSM) cnt[at(task_m(t), task_k(t), -1)] += c;
+        const int c = std::min(ran[i], 7);
+        // a slab counts once when all SLABS ran once: its runs weigh 1, 8, 64, 512
+        const int s = task_bj(t) - 1, w = s < 0 ? SLAB_SUM : 1 << (3 * s);
+        if (task_type(t) == T_POTRF) cnt[at(task_k(t), task_k(t), -1)] += c * w;
+        else if (task_type(t) == T_TRSM) cnt[at(task_m(t), task_k(t), -1)] += c * w;
         else
-            for (int j = task_k(t); j < task_k(t) + task_bi(t); ++j) cnt[at(task_m(t), task_n(t), j)] += c;
+            for (int j = task_k(t); j < task_k(t) + task_bi(t); ++j) cnt[at(task_m(t), task_n(t), j)] += c * w;
     }
+    for (auto &q : cnt) q = q == SLAB_SUM ? 1 : q == 0 ? 0 : 2;
     tickets = tot = bad = 0;
     auto tally = [&](int lo, int hi) {
         ++tickets;

@@ -98,6 +98,18 @@ __host__ __device__ __forceinline__ int block_update_index(int j0, int n, int S)
     return j0 == n - 1 ? (n - 1 + S - 1) / S : j0 / S;
 }
 
+// The links of the chain, L(k+1,k) and panel k on block (k+1,k+1), are split
+// into SLABS tasks of 32 rows on as many CTAs (bj = 1 + slab), so a link takes a
+// quarter of the products' time.  Tasks that complete a strip or a block's last
+// panel:
+constexpr int SLABS = 4;
+constexpr int SLAB_ROWS = BLK / SLABS;
+__host__ __device__ __forceinline__ int block_strips(int m, int k) { return m == k + 1 ? SLABS : 1; }
+__host__ __device__ __forceinline__ int block_all_updates(int m, int n, int S)
+{
+    return block_updates(n, S) + (m == n && n > 0 ? SLABS - 1 : 0);
+}
+
 struct PotrfArgs {
     double *A;             // device tiles (lower, packed)
     double *W;             // mt * nbs blocks of 128x128: inverses of diagonal blocks
@@ -184,6 +196,7 @@ struct Job {
     int lda, ldb, ldc;
     int K;
     int mode;
+    int slab;      // 32-row slab of the block, or -1: all 128 rows
     bool tri;      // B is lower triangular (row c is zero beyond column c)
     bool signal;   // the next job of the same task reads this job's output
     // mixed precision, TRSM store jobs: the 16-bit copy of the block is
@@ -203,9 +216,10 @@ __device__ __forceinline__ int task_njobs(const PotrfArgs &a, uint64_t t)
 __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
 {
     Job jb;
-    jb.tri = false;
     const int nbi = a.ld;
     const int k = task_k(t), m = task_m(t), n = task_n(t), bi = task_bi(t), bj = task_bj(t);
+    jb.tri = false;
+    jb.slab = a.fchunk ? bj - 1 : -1;
     if (task_type(t) == T_GEMM) {
         // C(m,n)[bi,bj] -= A(m,k)[bi,:] * A(n,k)[bj,:]^T     (src/zpotrf_L.jdf:619-623, :453-456)
         jb.A = tile_ptr(a, m, k) + bi * BLK;
