@@ -611,18 +611,21 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
 }
 
 // The products of the critical path, formed before a sweep (128x128,
-// column-major, block b at M + b * 128^2):
-//   forward:  M_b = W_b L_{b,b-1},  b = 1 .. P-1;
-//   backward: M_b = L_{b+1,b} W_b,  b = 0 .. P-2 (the backward ring reads the
-//             transpose, W_b^T L_{b+1,b}^T).
+// column-major, block b of distance d at M + ((d - 1) * nblk + b) * 128^2):
+//   forward:  M_b = W_b L_{b,b-d},  b = d .. P-1;
+//   backward: M_b = L_{b+d,b} W_b,  b = 0 .. P-1-d (the backward ring reads the
+//             transpose, W_b^T L_{b+d,b}^T);
+// d = 1, and 2 for the one-block sweep (blockIdx.z).
 // Four CTAs of 32 rows per block (the block of one warp is 32 x 16), so a short
 // sweep's preparation takes one 32-row product's time: 33 us (one CTA per block)
-// before at 31 blocks, 8 us now.
+// before at 31 blocks, 13 us now.
 __global__ void __launch_bounds__(256) wave_prep_kernel(const double *A, const double *W, int mt, int nbi, int nbs,
-                                                        int transposed, double *M)
+                                                        int nblk, int transposed, double *M)
 {
-    const int b = transposed ? (int)blockIdx.x : (int)blockIdx.x + 1, s = blockIdx.y;
-    const int p = transposed ? b + 1 : b, q = transposed ? b : b - 1;     // the sub-diagonal block L_{p,q}
+    const int d = 1 + blockIdx.z, s = blockIdx.y;
+    const int b = transposed ? (int)blockIdx.x : (int)blockIdx.x + d;
+    if (b + (transposed ? d : 0) >= nblk) return;
+    const int p = transposed ? b + d : b, q = transposed ? b : b - d;     // the sub-diagonal block L_{p,q}
     const double *Lpq = A + lower_tile_index(p / nbs, q / nbs, mt) * (int64_t)nbi * nbi +
                         (int64_t)(q % nbs) * 128 * nbi + (p % nbs) * 128;
     const double *Wb = W + (int64_t)b * 128 * 128;
@@ -640,7 +643,227 @@ __global__ void __launch_bounds__(256) wave_prep_kernel(const double *A, const d
         for (int l = warp >> 1; l < 4; ++l)
             mma32(acc, Lpq + (int64_t)(32 * l) * nbi + 32 * s, nbi, 1, Wb + 16 * warp * 128 + 32 * l, 1, 128, false, lane);
     }
-    frag_store(acc, M + (int64_t)b * 128 * 128 + 16 * warp * 128 + 32 * s, 1, 128, lane);
+    frag_store(acc, M + ((int64_t)(d - 1) * nblk + b) * 128 * 128 + 16 * warp * 128 + 32 * s, 1, 128, lane);
+}
+
+// ---------------------------------------------------------------------------
+// The sweep with one block per CTA (the blocks of a column group all resident,
+// up to N = 18944 on 148 SMs).  It is bound by the chain from one solved block to
+// the next, so all else is taken off it:
+//     Y_p = Z_p - M2_p Y_{p-2} - M1_p Y_{p-1},  Z_p = W_p (B_p - sum_{q<p-2} L_pq Y_q),
+//     M1_p = W_p L_{p,p-1},  M2_p = W_p L_{p,p-2}  (wave_prep_kernel),
+// (in solve order): Z is formed one step before it is needed, and what follows
+// the arrival of a block is one 128 x 128 product.  Blocks travel through the
+// exchange buffer only, to every CTA (the chain's next two poll without pause,
+// the others back off); there are no flags.  A step took 5 us with Z formed from
+// Y_{p-2} on and the block handed on by flag, fence and a separate read.
+// ---------------------------------------------------------------------------
+template <int NC, bool TRANS>
+__global__ void __launch_bounds__(WV_THREADS, 1)
+    trsm_chain_kernel(WaveArgs a, const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap wmap,
+                      const __grid_constant__ CUtensorMap mmap)
+{
+    constexpr int WV_NST = wv_nst(NC);
+    extern __shared__ __align__(1024) unsigned char smraw[];
+    WaveCtl *ctl = reinterpret_cast<WaveCtl *>(smraw);
+    const uint32_t sbase = smem_u32(smraw);
+    double *ring = reinterpret_cast<double *>(smraw + ((((sbase + 128 + 1023u) & ~1023u)) - sbase));
+    double *Ybuf = ring + WV_NST * WV_A_DOUBLES;   // two Y stages of NC x WV_YP
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if ((size_t)(reinterpret_cast<unsigned char *>(Ybuf + 2 * NC * WV_YP) - smraw) > a.smem_bytes) {
+        if (tid == 0) atomicCAS(a.status, ST_OK, ST_BAD_TASK);
+        return;
+    }
+    const int P = a.nblk, group = blockIdx.x / P, pos = blockIdx.x - group * P;
+    const int p = wv_block<TRANS>(pos, P), c0 = a.c0 + group * NC;
+    const double *X = a.X + (int64_t)group * P * (NC * 128);
+    if (tid == 0) {
+        for (int s = 0; s < WV_NST; ++s) {
+            mbar_init(&ctl->full[s], 1);
+            mbar_init(&ctl->empty[s], 8);
+        }
+    }
+    __syncthreads();
+    if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
+        if (warp != 8) return;
+        // producer: L(p, q) of the positions before pos - 2, then W, M2, M1
+        uint32_t it = 0;
+        bool ok = true;
+        if (lane == 0) {
+            tma_prefetch_desc(&lmap);
+            tma_prefetch_desc(&wmap);
+            tma_prefetch_desc(&mmap);
+        }
+        auto issue = [&](const CUtensorMap *map, int x0, int y0) {
+            for (int s0 = 0; s0 < 128 && ok; s0 += WV_KS) {
+                const uint32_t s = it % WV_NST, r = it / WV_NST;
+                if (r > 0 && !warp_mbar_wait(&ctl->empty[s], (r - 1) & 1, a.limit_ns)) {
+                    if (lane == 0) atomicCAS(a.status, ST_OK, ST_MBAR_TIMEOUT);
+                    ok = false;
+                    break;
+                }
+                double *As = ring + s * WV_A_DOUBLES;
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&ctl->full[s], 128 * WV_KS * (uint32_t)sizeof(double));
+                    if (!TRANS) {
+#pragma unroll
+                        for (int slab = 0; slab < 8; ++slab)     // 16 rows x 32 columns each
+                            tma_load_2d(As + slab * 512, map, x0 + slab * 16, y0 + s0, &ctl->full[s]);
+                    } else {
+#pragma unroll
+                        for (int slab = 0; slab < 2; ++slab)     // 16 k x 128 columns each
+                            tma_load_2d(As + slab * 2048, map, x0 + s0 + slab * 16, y0, &ctl->full[s]);
+                    }
+                }
+                __syncwarp();
+                ++it;
+            }
+        };
+        for (int qi = 0; qi + 2 < pos && ok; ++qi) {
+            const int q = wv_block<TRANS>(qi, P);
+            int x, y;
+            if (TRANS) wv_lcoord(a, q, p, x, y);
+            else wv_lcoord(a, p, q, x, y);
+            issue(&lmap, x, y);
+        }
+        issue(&wmap, 0, p * 128);
+        if (pos >= 2) issue(&mmap, 0, (P + p) * 128);
+        if (pos >= 1) issue(&mmap, 0, p * 128);
+        const uint32_t fst = it > WV_NST ? it - WV_NST : 0;
+        for (uint32_t k = fst; k < it; ++k) warp_mbar_wait(&ctl->full[k % WV_NST], (k / WV_NST) & 1, a.limit_ns);
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;\n");
+    constexpr int NT = NC / 8;
+    const int g = lane >> 2, t = lane & 3;
+    const int ra = warp * 16 + wv_perm<TRANS>(g), rb = warp * 16 + wv_perm<TRANS>(g + 8);   // fragment rows
+    double *Yp = a.Y + (int64_t)c0 * a.ldy + (int64_t)p * 128;
+    double acc[NT][4];
+#pragma unroll
+    for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            acc[ni][e] = a.alpha * __ldcg(Yp + (int64_t)(ni * 8 + 2 * t + (e & 1)) * a.ldy + ((e & 2) ? rb : ra));
+    uint32_t it = 0;
+    bool ok = true;
+    // ac += (next 128x128 block of the ring) Yst; independent partial sums for few columns
+    constexpr int NPART = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+    auto product = [&](double (&ac)[NT][4], const double *Yst) {
+        double part[NPART][NT][4];
+#pragma unroll
+        for (int h = 0; h < NPART; ++h)
+#pragma unroll
+            for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[h][ni][e] = 0.0;
+        for (int s0 = 0; s0 < 128 && ok; s0 += WV_KS) {
+            const uint32_t s = it % WV_NST, r = it / WV_NST;
+            if (!warp_mbar_wait(&ctl->full[s], r & 1, a.limit_ns)) {
+                if (lane == 0) atomicCAS(a.status, ST_OK, ST_MBAR_TIMEOUT);
+                ok = false;
+                break;
+            }
+            const double *As = ring + s * WV_A_DOUBLES;
+#pragma unroll
+            for (int kk = 0; kk < WV_KS; kk += 4) {
+                const double a0 = As[wv_aidx<TRANS>(ra, kk + t)];
+                const double a1 = As[wv_aidx<TRANS>(rb, kk + t)];
+#pragma unroll
+                for (int ni = 0; ni < NT; ++ni)
+                    dmma_16x8x4(part[(kk >> 2) % NPART][ni], a0, a1, Yst[(ni * 8 + g) * WV_YP + s0 + kk + t]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl->empty[s]);
+            ++it;
+        }
+#pragma unroll
+        for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                double v = part[0][ni][e];
+#pragma unroll
+                for (int h = 1; h < NPART; ++h) v += part[h][ni][e];
+                ac[ni][e] += v;
+            }
+    };
+    // acc = op(W) acc, staged in Yst
+    auto wmul = [&](double *Yst) {
+#pragma unroll
+        for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                Yst[(ni * 8 + 2 * t + (e & 1)) * WV_YP + ((e & 2) ? rb : ra)] = acc[ni][e];
+                acc[ni][e] = 0.0;
+            }
+        named_bar_sync(1, 256);
+        product(acc, Yst);
+    };
+    if (pos < 3) wmul(Ybuf + NC * WV_YP);         // position 0 stages in the other buffer
+    for (int qi = 0; qi < pos; ++qi) {
+        const int q = wv_block<TRANS>(qi, P), ahead = pos - qi;
+        double *Yst = Ybuf + (qi & 1) * (NC * WV_YP);
+        // Y_q word by word from the exchange buffer
+        constexpr int NV = NC * 128 / 256;
+        const double *Xq = X + (int64_t)q * (NC * 128) + tid;
+        unsigned long long v[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = wv_peek(Xq + 256 * i);
+        bool good = true;
+        uint64_t t0 = 0;
+        const bool far = ahead > 3;               // not next on the chain: one word, with pauses
+        for (int spins = 1;; ++spins) {
+            bool all = true;
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (v[i] == WV_EMPTY) all = false;
+            if (all) break;
+            if (far) __nanosleep(ahead > 8 ? 300 : 100);
+            if (far && v[0] == WV_EMPTY) {
+                v[0] = wv_peek(Xq);
+            } else {
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (v[i] == WV_EMPTY) v[i] = wv_peek(Xq + 256 * i);
+            }
+            if ((spins & 255) == 0) {
+                const uint64_t t1 = globaltimer_ns();
+                if (t0 == 0) t0 = t1;
+                if (ld_volatile(a.status) != ST_OK || t1 - t0 > a.limit_ns) {
+                    atomicCAS(a.status, ST_OK, ST_DEP_TIMEOUT);
+                    good = false;
+                    break;
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int e = tid + 256 * i;
+            Yst[(e >> 7) * WV_YP + (e & 127)] = -__longlong_as_double((long long)v[i]);
+        }
+        // one decision for all consumer warps; the barrier also ends the staging
+        // (this buffer's readers of two positions ago passed the last one)
+        if (named_bar_or(1, 256, !good || !ok)) return;
+        product(acc, Yst);                        // L(p, q), or M2 / M1 at the end
+        if (ahead == 3) {
+            // every product but the last two: Z, staged in the other buffer,
+            // whose last readers are one position back
+            wmul(Ybuf + ((qi + 1) & 1) * (NC * WV_YP));
+            named_bar_sync(1, 256);               // the next position stages there again
+        }
+    }
+    if (!ok) return;                              // a lost wait: the status stops the others
+    double *Xp = a.X + ((int64_t)group * P + p) * (NC * 128);
+#pragma unroll
+    for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            wv_send(Xp + (ni * 8 + 2 * t + (e & 1)) * 128 + ((e & 2) ? rb : ra), acc[ni][e]);
+#pragma unroll
+    for (int ni = 0; ni < NT; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            Yp[(int64_t)(ni * 8 + 2 * t + (e & 1)) * a.ldy + ((e & 2) ? rb : ra)] = acc[ni][e];
 }
 
 static size_t wave_smem_bytes(int nc)
@@ -650,14 +873,15 @@ static size_t wave_smem_bytes(int nc)
 }
 
 template <int NC, bool TRANS>
-static int launch_wave(Context *ctx, WaveArgs &a, int grid, CUtensorMap &lmap, CUtensorMap &wmap, CUtensorMap &mmap)
+static int launch_wave(Context *ctx, WaveArgs &a, int grid, bool chain, CUtensorMap &lmap, CUtensorMap &wmap,
+                       CUtensorMap &mmap)
 {
     const size_t smem = wave_smem_bytes(NC);
     a.smem_bytes = (uint32_t)smem;
-    CK(cudaFuncSetAttribute(trsm_wave_kernel<NC, TRANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const void *fn = chain ? (const void *)trsm_chain_kernel<NC, TRANS> : (const void *)trsm_wave_kernel<NC, TRANS>;
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *args[] = {&a, &lmap, &wmap, &mmap};
-    CK(cudaLaunchCooperativeKernel((const void *)trsm_wave_kernel<NC, TRANS>, dim3(grid), dim3(WV_THREADS), args, smem,
-                                   ctx->stream));
+    CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(WV_THREADS), args, smem, ctx->stream));
     ctx->launches++;
     return 0;
 }
@@ -668,9 +892,13 @@ int wave_max_blocks_per_sm()
     const void *fns[] = {(const void *)trsm_wave_kernel<8, false>,  (const void *)trsm_wave_kernel<8, true>,
                          (const void *)trsm_wave_kernel<16, false>, (const void *)trsm_wave_kernel<16, true>,
                          (const void *)trsm_wave_kernel<24, false>, (const void *)trsm_wave_kernel<24, true>,
-                         (const void *)trsm_wave_kernel<32, false>, (const void *)trsm_wave_kernel<32, true>};
-    const int ncs[] = {8, 8, 16, 16, 24, 24, 32, 32};
-    for (int i = 0; i < 8; ++i) {
+                         (const void *)trsm_wave_kernel<32, false>, (const void *)trsm_wave_kernel<32, true>,
+                         (const void *)trsm_chain_kernel<8, false>,  (const void *)trsm_chain_kernel<8, true>,
+                         (const void *)trsm_chain_kernel<16, false>, (const void *)trsm_chain_kernel<16, true>,
+                         (const void *)trsm_chain_kernel<24, false>, (const void *)trsm_chain_kernel<24, true>,
+                         (const void *)trsm_chain_kernel<32, false>, (const void *)trsm_chain_kernel<32, true>};
+    const int ncs[] = {8, 8, 16, 16, 24, 24, 32, 32, 8, 8, 16, 16, 24, 24, 32, 32};
+    for (int i = 0; i < 16; ++i) {
         const void *fn = fns[i];
         const size_t smem = wave_smem_bytes(ncs[i]);
         int n = 0;
@@ -684,21 +912,20 @@ int wave_max_blocks_per_sm()
 
 // Columns per group (a multiple of 8), groups and CTAs per group of a launch.
 // The chain's step grows with the columns (one 128 x 128 x nc product), so a
-// sweep with SMs to spare takes the narrowest groups whose CTAs own at most two
-// blocks each; where one group needs the grid, up to 32 columns go through it
-// at a time (WV_RMAX blocks per CTA).  Every group reads L.
+// sweep with SMs to spare takes the narrowest groups whose blocks have a CTA
+// each; where one group needs the grid, up to 32 columns go through it at a time
+// (up to WV_RMAX blocks per CTA).  Every group reads L.
 struct SweepShape {
     int nc, groups, gsub;
 };
 static SweepShape sweep_shape(int nblk, int nrhs, int grid)
 {
-    for (int nc = 8; nc <= 32; nc += 8) {
+    for (int nc = 8; nc <= 32 && nblk <= grid; nc += 8) {
         const int ng = (nrhs + nc - 1) / nc;
-        if (2 * ng > grid || (ng > 1 && nrhs % nc != 0)) continue;   // groups are all alike
-        const int gsub = std::max(2, std::min(nblk, grid / ng));
-        if (ng == 1 || (nblk + gsub - 1) / gsub <= 2) return {nc, ng, gsub};
+        if (ng > 1 && nrhs % nc != 0) continue;            // groups are all alike
+        if (ng * nblk <= grid) return {nc, ng, nblk};
     }
-    return {std::min(32, nrhs), 1, std::max(2, std::min(nblk, grid))};
+    return {std::min(32, nrhs), 1, nblk <= grid ? nblk : std::max(2, grid)};
 }
 
 // Returns 1 when the shape does not fit the wavefront kernel (more than
@@ -725,10 +952,13 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
     // W: 128x128 column-major blocks.  Boxes of 16 doubles (128 bytes, the
     // swizzle span) by 32 (forward: k columns) or 128 (backward: columns).
     // the critical path's products W_b L_{b,b-1} (or L_{b+1,b} W_b)
-    double *M = (double *)ctx->buffer(BUF_WM, (size_t)nblk * 128 * 128 * sizeof(double));
+    // (one block per CTA: also W_b L_{b,b-2})
+    const bool chain = sh.gsub == nblk && !ctx->wave_trace_path[0];
+    const int nd = chain ? 2 : 1;
+    double *M = (double *)ctx->buffer(BUF_WM, (size_t)nd * nblk * 128 * 128 * sizeof(double));
     if (!M) return DPLASMA_ERR_OUT_OF_RESOURCES;
     if (nblk > 1) {
-        wave_prep_kernel<<<dim3(nblk - 1, 4), 256, 0, ctx->stream>>>(dA, W, g.mt, g.nbi, g.nbi / 128, transposed, M);
+        wave_prep_kernel<<<dim3(nblk - 1, 4, nd), 256, 0, ctx->stream>>>(dA, W, g.mt, g.nbi, g.nbi / 128, nblk, transposed, M);
         CK(cudaGetLastError());
         ctx->launches++;
     }
@@ -741,7 +971,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         rc0 = encode_map_2d(ctx, &wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void *)W, 128, (uint64_t)nblk * 128,
                             128 * sizeof(double), 16, box1, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!rc0)
-        rc0 = encode_map_2d(ctx, &mmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void *)M, 128, (uint64_t)nblk * 128,
+        rc0 = encode_map_2d(ctx, &mmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void *)M, 128, (uint64_t)nd * nblk * 128,
                             128 * sizeof(double), 16, box1, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc0) return rc0;
     for (int ch = 0; ch < nlaunch; ++ch) {
@@ -776,15 +1006,15 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         const int cta = ng * sh.gsub;
         int rc;
         if (transposed)
-            rc = nc <= 8    ? launch_wave<8, true>(ctx, a, cta, lmap, wmap, mmap)
-                 : nc <= 16 ? launch_wave<16, true>(ctx, a, cta, lmap, wmap, mmap)
-                 : nc <= 24 ? launch_wave<24, true>(ctx, a, cta, lmap, wmap, mmap)
-                            : launch_wave<32, true>(ctx, a, cta, lmap, wmap, mmap);
+            rc = nc <= 8    ? launch_wave<8, true>(ctx, a, cta, chain, lmap, wmap, mmap)
+                 : nc <= 16 ? launch_wave<16, true>(ctx, a, cta, chain, lmap, wmap, mmap)
+                 : nc <= 24 ? launch_wave<24, true>(ctx, a, cta, chain, lmap, wmap, mmap)
+                            : launch_wave<32, true>(ctx, a, cta, chain, lmap, wmap, mmap);
         else
-            rc = nc <= 8    ? launch_wave<8, false>(ctx, a, cta, lmap, wmap, mmap)
-                 : nc <= 16 ? launch_wave<16, false>(ctx, a, cta, lmap, wmap, mmap)
-                 : nc <= 24 ? launch_wave<24, false>(ctx, a, cta, lmap, wmap, mmap)
-                            : launch_wave<32, false>(ctx, a, cta, lmap, wmap, mmap);
+            rc = nc <= 8    ? launch_wave<8, false>(ctx, a, cta, chain, lmap, wmap, mmap)
+                 : nc <= 16 ? launch_wave<16, false>(ctx, a, cta, chain, lmap, wmap, mmap)
+                 : nc <= 24 ? launch_wave<24, false>(ctx, a, cta, chain, lmap, wmap, mmap)
+                            : launch_wave<32, false>(ctx, a, cta, chain, lmap, wmap, mmap);
         if (rc) return rc;
         if (a.trace) {
             // one line per sweep: CTA-summed ns per part, and the mean step of
