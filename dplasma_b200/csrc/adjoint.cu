@@ -10,7 +10,7 @@
 //                       W_ij = -W_ii sum_{k=j}^{i-1} L_ik W_kj, block row by row
 //     Y = Phi(L^T Lbar) lower tiles, k >= i
 //     Z = Y W           lower tiles, j <= k <= i
-//     Abar = sym(W^T Z) all tiles, k >= max(i, j)
+//     Abar = sym(W^T Z) lower tiles: (W^T Z + Z^T W) / 2, k >= i
 // on dense column-major copies in the padded index space of the device
 // tiles (padding rows: identity in L, zero in Lbar, hence zero in Abar).
 // Every product runs on one FP64 tensor-core GEMM kernel over 128x128 output
@@ -41,17 +41,19 @@ constexpr int AG_P = 132;     // shared pitch
 // Tile sets and K ranges (block indices):
 //   LOWER_KGE_I   tiles i >= j                 k in [i, P-1]
 //   LOWER_JKI     tiles i >= j                 k in [j, i]
-//   FULL_KGE_MAX  all tiles                    k in [max(i,j), P-1]
+//   SYM_KGE_I     tiles i >= j                 k in [i, P-1], A^T B + B^T A
 //   LVL_T, LVL_W  one level of the recursive triangular inverse: for every
 //                 diagonal block [o, o+2h) of 2h tiles, with W11 = the inverse
 //                 of its first half and W22 of its second (previous level),
 //                   LVL_T: Y21 = L21 W11     tiles (o+h+i, o+j), k in [o+j, o+h)
 //                   LVL_W: W21 = -W22 Y21    tiles (o+h+i, o+j), k in [o+h, o+h+i]
 //                 (h = rowblk; the last block's second half may be short)
-enum : int { AG_LOWER_KGE_I = 1, AG_LOWER_JKI = 2, AG_FULL_KGE_MAX = 3, AG_LVL_T = 5, AG_LVL_W = 6 };
+// Blocks run in order, so every mode starts with its longest K ranges: the last
+// wave is then made of short ones (N = 4096: JKI 1224 us in row order).
+enum : int { AG_LOWER_KGE_I = 1, AG_LOWER_JKI = 2, AG_SYM_KGE_I = 3, AG_LVL_T = 5, AG_LVL_W = 6 };
 
 struct AgArgs {
-    int mode, P, rowblk;
+    int mode, P, rowblk, nblk;
     const double *A;
     int lda, transA;
     const double *B;
@@ -77,9 +79,16 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
     const int tix = blockIdx.x;
     if (a.mode == AG_LVL_T || a.mode == AG_LVL_W) {
         const int h = a.rowblk;
-        const int b = tix / (h * h), rem = tix % (h * h);
-        const int jj = rem / h, ii = rem % h;
+        const int b = tix % a.nblk, rem = tix / a.nblk;
         const int o = b * 2 * h;
+        int ii, jj;
+        if (a.mode == AG_LVL_T) {
+            ii = rem % h;
+            jj = rem / h;
+        } else {
+            ii = h - 1 - rem / h;
+            jj = rem % h;
+        }
         if (ii >= min(h, a.P - o - h)) return;   // beyond a short last block
         i = o + h + ii;
         j = o + jj;
@@ -92,24 +101,23 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             k0 = 0;
             k1 = ii;
         }
-    } else if (a.mode == AG_FULL_KGE_MAX) {
-        i = tix % a.P;
-        j = tix / a.P;
-        k0 = max(i, j);
-        k1 = a.P - 1;
+    } else if (a.mode == AG_LOWER_JKI) {
+        // by diagonals i - j = P-1, P-2, ..: the d-th from the corner holds d + 1 tiles
+        int d = (int)((sqrtf(8.0f * tix + 1.0f) - 1.0f) * 0.5f);
+        while ((d + 1) * (d + 2) / 2 <= tix) ++d;
+        while (d * (d + 1) / 2 > tix) --d;
+        j = tix - d * (d + 1) / 2;
+        i = j + a.P - 1 - d;
+        k0 = j;
+        k1 = i;
     } else {
         int bi = (int)((sqrtf(8.0f * tix + 1.0f) - 1.0f) * 0.5f);
         while ((bi + 1) * (bi + 2) / 2 <= tix) ++bi;
         while (bi * (bi + 1) / 2 > tix) --bi;
         i = bi;
         j = tix - bi * (bi + 1) / 2;
-        if (a.mode == AG_LOWER_KGE_I) {
-            k0 = i;
-            k1 = a.P - 1;
-        } else {
-            k0 = j;
-            k1 = i;
-        }
+        k0 = i;
+        k1 = a.P - 1;
     }
     double acc[4][4][4];
 #pragma unroll
@@ -121,19 +129,20 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
 
     const int kbeg = k0 * AG_T, kend = (k1 + 1) * AG_T;
     double ra[8], rb[8];
+    const double *Aop = a.A, *Bop = a.B;
     auto load = [&](int kc) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int e = tid + 256 * q;
             if (!a.transA) {
                 const int r = e & 127, kk = e >> 7;
-                ra[q] = a.A[(int64_t)(ako * AG_T + kc + kk) * a.lda + i * AG_T + r];
+                ra[q] = Aop[(int64_t)(ako * AG_T + kc + kk) * a.lda + i * AG_T + r];
             } else {
                 const int kk = e & 15, r = e >> 4;
-                ra[q] = a.A[(int64_t)(i * AG_T + r) * a.lda + ako * AG_T + kc + kk];
+                ra[q] = Aop[(int64_t)(i * AG_T + r) * a.lda + ako * AG_T + kc + kk];
             }
             const int kk = e & 15, c = e >> 4;
-            rb[q] = a.B[(int64_t)(j * AG_T + c) * a.ldb + bko * AG_T + kc + kk];
+            rb[q] = Bop[(int64_t)(j * AG_T + c) * a.ldb + bko * AG_T + kc + kk];
         }
     };
     auto store = [&](int buf) {
@@ -151,14 +160,23 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             Bs[buf][kk * AG_P + c] = rb[q];
         }
     };
-    if (kbeg < kend) {
-        load(kbeg);
+    // one pass over K, or two with the operands exchanged (SYM)
+    const int len = kend - kbeg, total = a.mode == AG_SYM_KGE_I ? 2 * len : len;
+    auto stage = [&](int at) {
+        if (at >= len) {
+            Aop = a.B;
+            Bop = a.A;
+        }
+        load(kbeg + (at >= len ? at - len : at));
+    };
+    if (total > 0) {
+        stage(0);
         store(0);
         __syncthreads();
         int buf = 0;
-        for (int kc = kbeg; kc < kend; kc += AG_K) {
-            const bool more = kc + AG_K < kend;
-            if (more) load(kc + AG_K);
+        for (int at = 0; at < total; at += AG_K) {
+            const bool more = at + AG_K < total;
+            if (more) stage(at + AG_K);
             const double *Ab = As[buf] + wm * 64 + g;
             const double *Bb = Bs[buf] + wn * 32 + g;
 #pragma unroll
@@ -214,6 +232,7 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
     a.mode = mode;
     a.P = P;
     a.rowblk = rowblk;
+    a.nblk = rowblk > 0 ? (P + 2 * rowblk - 1) / (2 * rowblk) : 0;
     a.A = A;
     a.lda = lda;
     a.transA = transA;
@@ -224,8 +243,7 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
     a.alpha = alpha;
     a.beta = beta;
     int ntile;
-    if (mode == AG_LVL_T || mode == AG_LVL_W) ntile = ((P + 2 * rowblk - 1) / (2 * rowblk)) * rowblk * rowblk;
-    else if (mode == AG_FULL_KGE_MAX) ntile = P * P;
+    if (mode == AG_LVL_T || mode == AG_LVL_W) ntile = a.nblk * rowblk * rowblk;
     else ntile = P * (P + 1) / 2;
     if (ntile <= 0) return 0;
     CK(cudaFuncSetAttribute(ag_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AG_SMEM));
@@ -238,25 +256,23 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
 // ---------------------------------------------------------------------------
 // layout helpers (padded index space of the device tiles, ld = Np)
 // ---------------------------------------------------------------------------
-__global__ void ag_tiles_to_dense(const double *T, int mt, int nbi, double *D, int ld)
-{
-    const int m = blockIdx.x, n = blockIdx.y;
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        double v = 0.0;
-        if (m > n || (m == n && r >= c)) v = T[lower_tile_index(m >= n ? m : n, m >= n ? n : m, mt) * (int64_t)nbi * nbi + e];
-        D[(int64_t)(n * nbi + c) * ld + m * nbi + r] = v;
-    }
-}
-
-__global__ void ag_dense_to_tiles(const double *D, int ld, int mt, int nbi, double *T)
+// Lower tiles <-> the dense lower part, one CTA per 64x64 piece; the part above
+// the diagonal of a diagonal tile is zero in the dense form, the tiles above it
+// are never read.
+constexpr int AG_M = 64;
+template <bool TO_DENSE>
+__global__ void __launch_bounds__(256) ag_move(double *T, int mt, int nbi, double *D, int ld)
 {
     const int m = blockIdx.x, n = blockIdx.y;
     if (m < n) return;
-    double *Tt = T + lower_tile_index(m, n, mt) * (int64_t)nbi * nbi;
-    for (int e = threadIdx.x; e < nbi * nbi; e += blockDim.x) {
-        const int r = e % nbi, c = e / nbi;
-        Tt[e] = D[(int64_t)(n * nbi + c) * ld + m * nbi + r];
+    const int per = nbi / AG_M, r = (blockIdx.z % per) * AG_M + (threadIdx.x & (AG_M - 1));
+    const int c0 = (blockIdx.z / per) * AG_M + threadIdx.x / AG_M;
+    double *Tt = T + lower_tile_index(m, n, mt) * (int64_t)nbi * nbi + r;
+    double *Dt = D + (int64_t)(n * nbi) * ld + m * nbi + r;
+#pragma unroll 8
+    for (int c = c0; c < c0 + AG_M; c += 256 / AG_M) {
+        if (TO_DENSE) Dt[(int64_t)c * ld] = (m == n && r < c) ? 0.0 : Tt[(int64_t)c * nbi];
+        else if (m != n || r >= c) Tt[(int64_t)c * nbi] = Dt[(int64_t)c * ld];
     }
 }
 
@@ -271,19 +287,6 @@ __global__ void ag_phi(double *Y, int ld, int P)
         double &v = Yb[(int64_t)c * ld + r];
         if (r < c) v = 0.0;
         else if (r == c) v *= 0.5;
-    }
-}
-
-// lower part of sym(X) = (X + X^T)/2 into S (may be X itself: each pair
-// (r,c), r > c, is read and written by one thread)
-__global__ void ag_sym(double *X, int ld, int n)
-{
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n; e += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(e % n), c = (int)(e / n);
-        if (r < c) continue;
-        const double v = 0.5 * (X[(int64_t)c * ld + r] + X[(int64_t)r * ld + c]);
-        X[(int64_t)c * ld + r] = v;
-        X[(int64_t)r * ld + c] = v;
     }
 }
 
@@ -316,7 +319,6 @@ static int ag_inverse(Context *ctx, const double *L, double *W, double *Y, doubl
 {
     cudaStream_t st = ctx->stream;
     int rc;
-    CK(cudaMemsetAsync(W, 0, (size_t)ld * ld * sizeof(double), st));
     const size_t tsmem = P128_INV_DOUBLES * sizeof(double);
     CK(cudaFuncSetAttribute(ag_trtri_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
     ag_trtri_diag<<<P, 256, tsmem, st>>>(L, ld, W, ld, scr, unit);
@@ -341,10 +343,10 @@ int potrf_adjoint_tiles(Context *ctx, const double *Lt, double *Lbt, const Geom 
     double *L = D, *W = D + nn, *Y = D + 2 * nn, *Z = D + 3 * nn, *scr = D + 4 * nn;
     cudaStream_t st = ctx->stream;
     int rc;
-    const dim3 tg(g.mt, g.mt);
-    ag_tiles_to_dense<<<tg, 256, 0, st>>>(Lt, g.mt, g.nbi, L, ld);
+    const dim3 tg(g.mt, g.mt, (g.nbi / AG_M) * (g.nbi / AG_M));
+    ag_move<true><<<tg, 256, 0, st>>>(const_cast<double *>(Lt), g.mt, g.nbi, L, ld);
     CK(cudaGetLastError());
-    ag_tiles_to_dense<<<tg, 256, 0, st>>>(Lbt, g.mt, g.nbi, Z, ld);   // Lbar (lower) into Z for now
+    ag_move<true><<<tg, 256, 0, st>>>(Lbt, g.mt, g.nbi, Z, ld);   // Lbar (lower) into Z for now
     CK(cudaGetLastError());
     ctx->launches += 2;
     // W = L^-1
@@ -356,13 +358,11 @@ int potrf_adjoint_tiles(Context *ctx, const double *Lt, double *Lbt, const Geom 
     ctx->launches++;
     // Z = Y W, lower tiles, j <= k <= i
     if ((rc = ag_gemm(ctx, AG_LOWER_JKI, P, 0, Y, ld, 0, W, ld, Z, ld, 1.0, 0.0))) return rc;
-    // Abar = sym(W^T Z), all tiles
-    if ((rc = ag_gemm(ctx, AG_FULL_KGE_MAX, P, 0, W, ld, 1, Z, ld, Y, ld, 1.0, 0.0))) return rc;
-    ag_sym<<<ctx->sms * 8, 256, 0, st>>>(Y, ld, Np);
+    // Abar = sym(W^T Z), lower tiles
+    if ((rc = ag_gemm(ctx, AG_SYM_KGE_I, P, 0, W, ld, 1, Z, ld, Y, ld, 0.5, 0.0))) return rc;
+    ag_move<false><<<tg, 256, 0, st>>>(Lbt, g.mt, g.nbi, Y, ld);
     CK(cudaGetLastError());
-    ag_dense_to_tiles<<<tg, 256, 0, st>>>(Y, ld, g.mt, g.nbi, Lbt);
-    CK(cudaGetLastError());
-    ctx->launches += 2;
+    ctx->launches++;
     CK(cudaStreamSynchronize(st));
     return 0;
 }
@@ -390,8 +390,8 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
     double *L = D, *W = D + nn, *Y = D + 2 * nn, *scr = D + 4 * nn;
     cudaStream_t st = ctx->stream;
     int rc;
-    const dim3 tg(g.mt, g.mt);
-    ag_tiles_to_dense<<<tg, 256, 0, st>>>(Lt, g.mt, g.nbi, L, ld);
+    const dim3 tg(g.mt, g.mt, (g.nbi / AG_M) * (g.nbi / AG_M));
+    ag_move<true><<<tg, 256, 0, st>>>(Lt, g.mt, g.nbi, L, ld);
     CK(cudaGetLastError());
     ctx->launches++;
     *info = 0;
@@ -430,7 +430,7 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
         if ((rc = ag_gemm(ctx, AG_LOWER_KGE_I, P, 0, src, ld, 1, src, ld, Y, ld, 1.0, 0.0))) return rc;
         out = Y;
     }
-    ag_dense_to_tiles<<<tg, 256, 0, st>>>(out, ld, g.mt, g.nbi, Lt);
+    ag_move<false><<<tg, 256, 0, st>>>(Lt, g.mt, g.nbi, out, ld);
     CK(cudaGetLastError());
     ctx->launches++;
     CK(cudaStreamSynchronize(st));
