@@ -61,15 +61,16 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
 }
 // Poll for the phase of `bar` with the given parity to complete, giving up
 // after `limit_ns` nanoseconds.  Returns false on timeout.  Called by one
-// lane; see warp_mbar_wait for the whole-warp form.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns)
+// lane; see warp_mbar_wait for the whole-warp form.  The first `eager` polls
+// follow one another, the others pause.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns, int eager = 64)
 {
     if (mbar_test(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     int spins = 0;
     while (true) {
         if (mbar_test(bar, parity)) return true;
-        if (++spins > 64) {
+        if (++spins > eager) {
             if (globaltimer_ns() - t0 > limit_ns) return false;
             __nanosleep(20);
         }
@@ -78,10 +79,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
 // Lane 0 of the calling warp polls; the result is broadcast and the warp
 // reconverges (__shfl_sync orders the lanes' later accesses after lane 0's
 // acquire).  All 32 lanes must call it.
-__device__ __forceinline__ bool warp_mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns)
+__device__ __forceinline__ bool warp_mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns, int eager = 64)
 {
     int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, limit_ns) ? 1 : 0;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, limit_ns, eager) ? 1 : 0;
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
@@ -123,6 +124,9 @@ __device__ __forceinline__ void red_release_add(int *p, int v)
 {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// Order this thread's earlier accesses before its later ones for other SMs
+// (lighter than __threadfence, which is sequentially consistent).
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 // Fire-and-forget FP64 add performed at L2 (no value returned, so the issuing
 // thread never waits for the line).
 __device__ __forceinline__ void red_add_f64(double *p, double v)
@@ -147,7 +151,9 @@ __device__ __forceinline__ int ld_acquire_sys(const int *p)
 __device__ __forceinline__ bool wait_geq(const int *ctr, int target, const int *abort_flag, int *status,
                                          uint64_t limit_ns)
 {
-    if (ld_acquire(ctr) >= target) return true;
+    // the chain's waits are short: poll without pause first
+    for (int i = 0; i < 64; ++i)
+        if (ld_acquire(ctr) >= target) return true;
     const uint64_t t0 = globaltimer_ns();
     unsigned ns = 32;
     while (true) {

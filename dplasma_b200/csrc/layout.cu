@@ -22,8 +22,8 @@ Geom make_geom(int n, int nb)
 // Tiles of 128 where the caller's edge is no multiple of it (the matrix is
 // copied anyway): padded tile by tile, an edge of 93 costs (128/93)^3 = 2.6 times
 // the flops and 1.4 times the steps of the chain, 320 (384/320)^3 = 1.7 times
-// (N = 378 in 93-wide tiles: 5 steps, 0.37 ms; now 3, 0.23 ms; N = 7000 in
-// 320-wide ones: 9.0 ms, now 5.6 ms).
+// (N = 378 in 93-wide tiles: 5 steps, 0.37 ms, now 3, 0.22 ms; N = 7000 in
+// 320-wide ones: 9.0 ms, now 5.8 ms).
 Geom work_geom(int n, int nb) { return make_geom(n, nb % 128 == 0 ? nb : 128); }
 
 // ---------------------------------------------------------------------------

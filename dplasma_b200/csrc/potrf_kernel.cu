@@ -83,8 +83,9 @@ __device__ bool wait_deps(const PotrfArgs &a, uint64_t t)
             // imply the earlier ones (TRSM(m,j+1) follows the update of (m,j+1)
             // by panel j, which read TRSM(m,j)); chunks of one tile in order
             const int kl = min(k * a.mx_chunk + a.mx_chunk, n) - 1;
-            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
-                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
+            auto strips = [&](int r) { return r == kl + 1 && a.crit_slabs ? nbs * SLABS : nbs; };
+            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, strips(m), a.abort_flag, a.status, a.dep_limit_ns) &&
+                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, strips(n), a.abort_flag, a.status, a.dep_limit_ns) &&
                    wait_geq(a.upd_done + (int64_t)m * a.mt + n, k, a.abort_flag, a.status, a.dep_limit_ns);
         }
         if (a.fchunk) {
@@ -399,6 +400,33 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
     }
 }
 
+// 16-bit copy of two adjacent values (row r, columns c and c + 1) of a solved
+// block for the tensor-core updates: the value times its row scale (a power of
+// two, exact) rounded to bf16 or fp16, in the split form hi = fp16(x) and lo =
+// fp16(x - hi); one 32-bit store each.
+template <bool MIXED>
+__device__ __forceinline__ void store_p16(const PotrfArgs &a, const Job &jb, double x0, double x1, int r, int c)
+{
+    const int pitch = a.nbi;
+    uint32_t hw = 0, lw = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const double xs = (e ? x1 : x0) * (double)jb.p16_scale;
+        unsigned short hv, lv = 0;
+        if (a.p16_fmt) {
+            hv = __bfloat16_as_ushort(__float2bfloat16_rn((float)xs));
+        } else {
+            const __half hh = __float2half_rn((float)xs);
+            hv = __half_as_ushort(hh);
+            if (a.mx_split) lv = __half_as_ushort(__float2half_rn((float)(xs - (double)__half2float(hh))));
+        }
+        hw |= (uint32_t)hv << (16 * e);
+        lw |= (uint32_t)lv << (16 * e);
+    }
+    *reinterpret_cast<uint32_t *>(jb.p16 + (int64_t)r * pitch + c) = hw;
+    if (a.mx_split) *reinterpret_cast<uint32_t *>(jb.p16 + ((int64_t)a.p16_rows + r) * pitch + c) = lw;
+}
+
 // ---------------------------------------------------------------------------
 // consumers: one 128x128 FP64 GEMM job.  Returns false if a wait gave up.
 // ---------------------------------------------------------------------------
@@ -476,40 +504,16 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
                 }
             }
     if (MIXED && jb.p16) {
-        // 16-bit copy of the solved block for the tensor-core updates: the
-        // value times its row scale (a power of two, exact) rounded to bf16 or
-        // fp16, in the split form hi = fp16(x) and lo = fp16(x - hi); two
-        // adjacent columns per 32-bit store
-        const int pitch = a.nbi;
-        unsigned short *Plo = jb.p16 + (int64_t)a.p16_rows * pitch;
 #pragma unroll
         for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int r = wm * 64 + mi * 16 + g + 8 * h;
-                    const int c = wn * 32 + ni * 8 + 2 * t;
-                    uint32_t hw = 0, lw = 0;
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const double xs = acc[mi][ni][2 * h + e] * (double)jb.p16_scale;
-                        unsigned short hv, lv = 0;
-                        if (a.p16_fmt) {
-                            hv = __bfloat16_as_ushort(__float2bfloat16_rn((float)xs));
-                        } else {
-                            const __half hh = __float2half_rn((float)xs);
-                            hv = __half_as_ushort(hh);
-                            if (a.mx_split) lv = __half_as_ushort(__float2half_rn((float)(xs - (double)__half2float(hh))));
-                        }
-                        hw |= (uint32_t)hv << (16 * e);
-                        lw |= (uint32_t)lv << (16 * e);
-                    }
-                    *reinterpret_cast<uint32_t *>(jb.p16 + (int64_t)r * pitch + c) = hw;
-                    if (a.mx_split) *reinterpret_cast<uint32_t *>(Plo + (int64_t)r * pitch + c) = lw;
-                }
+                for (int h = 0; h < 2; ++h)
+                    store_p16<MIXED>(a, jb, acc[mi][ni][2 * h], acc[mi][ni][2 * h + 1], wm * 64 + mi * 16 + g + 8 * h,
+                                     wn * 32 + ni * 8 + 2 * t);
     }
-    __threadfence();   // this thread's reductions are performed before any later release
+    if (jb.signal) fence_acq_rel_gpu();        // read back by this CTA's own copies
     return true;
 }
 
@@ -518,11 +522,13 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
 // warp.  A link of 32 x 128 x 128 took 7 us where the whole block took 20
 // (strip) and 26 us (update of the diagonal block).
 // ---------------------------------------------------------------------------
+template <bool MIXED>
 __device__ __forceinline__ bool consume_slab(const PotrfArgs &a, SmemCtl *ctl, const double *ring, const Job &jb,
                                              uint32_t &stage_it)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
+    constexpr uint32_t NST = MIXED ? NSTAGE_MIXED : NSTAGE;
     // column group: the two warps of a sub-partition share a triangular load evenly
     const int cg = warp < 4 ? warp : 11 - warp;
     const bool lower = jb.mode == J_SUB_LOWER;
@@ -530,7 +536,7 @@ __device__ __forceinline__ bool consume_slab(const PotrfArgs &a, SmemCtl *ctl, c
     double acc[2][2][4];
     frag_zero(acc);
     for (int k0 = 0; k0 < jb.K; k0 += BK) {
-        const uint32_t s = stage_it % NSTAGE, r = stage_it / NSTAGE;
+        const uint32_t s = stage_it % NST, r = stage_it / NST;
         if (!warp_mbar_wait(&ctl->full[s], r & 1, a.pipe_limit_ns)) {
             if (lane == 0) report(a, ST_MBAR_TIMEOUT, 18, stage_it, warp);
             stage_it += (jb.K - k0) / BK;
@@ -572,8 +578,9 @@ __device__ __forceinline__ bool consume_slab(const PotrfArgs &a, SmemCtl *ctl, c
                 double *p = jb.C + (int64_t)c * jb.ldc + r;
                 if (jb.mode == J_STORE) *p = acc[mi][ni][q];
                 else if (!lower || r >= c) red_add_f64(p, -acc[mi][ni][q]);
+                if (MIXED && jb.p16 && (q & 1)) store_p16<MIXED>(a, jb, acc[mi][ni][q - 1], acc[mi][ni][q], r, c - 1);
             }
-    __threadfence();
+    if (jb.signal) fence_acq_rel_gpu();
     return true;
 }
 
@@ -925,7 +932,6 @@ __device__ bool mixed_update(const PotrfArgs &a, SmemCtl *ctl, unsigned char *ri
                 }
             }
         }
-        __threadfence();
         if (a.trace && tid == 0) {
             // per CTA: ns until the accumulators were ready, ns of the epilogue, tasks
             const unsigned long long tq2 = globaltimer_ns();
@@ -1099,7 +1105,6 @@ __device__ bool tc_trsm(const PotrfArgs &a, SmemCtl *ctl, unsigned char *ring16,
             *reinterpret_cast<uint4 *>(Pl + col) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
     }
-    __threadfence();
     tc_fence_before();
     if (a.ptrace) {
         named_bar_sync(1, NCONS);
@@ -1127,7 +1132,7 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
     int executed = 0;
     while (true) {
         const uint32_t slot = task_it % TASKQ, round = task_it / TASKQ;
-        const bool got = warp_mbar_wait(&ctl->tfull[slot], round & 1, a.pipe_limit_ns);
+        const bool got = warp_mbar_wait(&ctl->tfull[slot], round & 1, a.pipe_limit_ns, 1024);
         if (named_bar_or(1, NCONS, !got)) {
             if (tid == 0) report(a, ST_MBAR_TIMEOUT, 5, task_it, stage_it);
             break;
@@ -1158,7 +1163,8 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             if (MIXED && a.A0 && ty == T_TRSM) {
                 // streamed matrix: the strip's rows = untouched copy + updates,
                 // in place, before the producer loads them
-                stream_add_rows(a, m, k, task_bi(t) * BLK, BLK);
+                const int s = a.crit_slabs ? task_bj(t) - 1 : -1;
+                stream_add_rows(a, m, k, task_bi(t) * BLK + (s >= 0 ? s * SLAB_ROWS : 0), s >= 0 ? SLAB_ROWS : BLK);
                 fence_proxy_async();
                 __syncwarp();
                 if ((tid & 31) == 0) mbar_arrive(&ctl->prep);
@@ -1166,8 +1172,8 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             const int nj = task_njobs(a, t);
             for (int j = 0; j < nj; ++j) {
                 const Job jb = task_job(a, t, j);
-                ok = (!MIXED && jb.slab >= 0 ? consume_slab(a, ctl, ring, jb, stage_it)
-                                             : consume_job<MIXED>(a, ctl, ring, jb, stage_it)) && ok;
+                ok = (jb.slab >= 0 ? consume_slab<MIXED>(a, ctl, ring, jb, stage_it)
+                                   : consume_job<MIXED>(a, ctl, ring, jb, stage_it)) && ok;
                 if (jb.signal) {
                     fence_proxy_async();
                     if (named_bar_or(1, NCONS, !ok)) {
@@ -1185,10 +1191,10 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             break;
         }
         if (tid == 0) {
-            if (release) {
-                __threadfence();
-                red_release_add(release, 1);
-            }
+            // one release for the CTA: the barrier above orders every thread's
+            // stores and reductions before it (a fence in each thread, and one
+            // more here, held every task up by about 2 us)
+            if (release) red_release_add(release, 1);
             if (a.ran) atomicAdd(a.ran + tk, 1);
             if (a.trace) {
                 a.trace[4 * (int64_t)tk + 3] = globaltimer_ns();
@@ -1438,6 +1444,24 @@ std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, 
 // ---------------------------------------------------------------------------
 // host: run one factorization of the device tiles
 // ---------------------------------------------------------------------------
+// Mixed order: the strips of the next tile row, the chain's link, as SLABS tasks
+// of 32 rows each on as many CTAs (70 us as two 128-row strips of three dependent
+// products, 20 us in slabs).
+static void split_critical_strips(std::vector<uint64_t> &v)
+{
+    std::vector<uint64_t> out;
+    out.reserve(v.size() + v.size() / 8);
+    for (uint64_t t : v) {
+        if (task_type(t) != T_TRSM || task_m(t) != task_k(t) + 1) {
+            out.push_back(t);
+            continue;
+        }
+        for (int s = 0; s < SLABS; ++s)
+            out.push_back(make_task(T_TRSM, task_k(t), task_m(t), task_n(t), task_bi(t), 1 + s));
+    }
+    v.swap(out);
+}
+
 // The ticket order of a shape on the device (kept until another shape is
 // factored), with the tickets of the POTRFs behind it.  chunk > 0: mixed, this
 // many panels per update task; chunk < 0: FP64 on blocks, -chunk panels.
@@ -1449,6 +1473,7 @@ static int prepare_tasks(Context *ctx, PotrfArgs &a, int mt, int nbs, int chunk)
         std::vector<uint64_t> tasks =
             mixed ? build_potrf_tasks_mixed(mt, nbs, delay, chunk, ctx->mx_block_w, ctx->mx_block_h)
                   : build_potrf_tasks_blocks(mt * nbs, -chunk, delay, ctx->f64_block, ctx->f64_block);
+        if (mixed) split_critical_strips(tasks);
         const size_t nt = tasks.size();
         int np = 0;
         std::vector<int> pos;
@@ -1675,6 +1700,7 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
     a.ld = nbi;
     a.tbs = mixed ? 1 : nbs;
     a.fchunk = mixed ? 0 : -chunk;
+    a.crit_slabs = mixed;
     a.nb_user = nb_user;
     a.n_user = n_user;
     set_counters(a, ctr, P);
@@ -1886,6 +1912,7 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     a.n_user = n_user;
     a.ld = nbi;
     a.tbs = 1;
+    a.crit_slabs = 1;
     set_counters(a, ctr, mt);
     // the ticket order of a matrix already on the device
     int e = prepare_tasks(ctx, a, mt, nbs, chunk);
@@ -2089,6 +2116,7 @@ int potrf_launch_prealloc(cudaStream_t st, double *dA, int mt, int nbi, int nb_u
     a.ld = nbi;
     a.tbs = 1;
     a.fchunk = 0;
+    a.crit_slabs = 0;
     a.potrf_pos = nullptr;
     a.chain = nullptr;
     a.nb_user = nb_user;

@@ -123,6 +123,7 @@ struct PotrfArgs {
     // (nbi = 128, nbs = 1, mt counts blocks) of physical tiles of edge ld =
     // 128 tbs, mt / tbs per side; otherwise tbs = 1 and ld = nbi
     int ld, tbs;
+    int crit_slabs;        // the strips of the next tile row come in SLABS tasks each (mixed order)
     int fchunk;            // FP64 block order: panels per update task (0: tile order, one panel per task)
     const int *potrf_pos;  // [mt] tickets of POTRF(0..mt-1), all run by one CTA (null: by whoever draws them)
     int *chain;            // claimed by the first CTA to start, which runs the POTRFs of potrf_pos
@@ -219,7 +220,7 @@ __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
     const int nbi = a.ld;
     const int k = task_k(t), m = task_m(t), n = task_n(t), bi = task_bi(t), bj = task_bj(t);
     jb.tri = false;
-    jb.slab = a.fchunk ? bj - 1 : -1;
+    jb.slab = (a.fchunk || a.crit_slabs) ? bj - 1 : -1;
     if (task_type(t) == T_GEMM) {
         // C(m,n)[bi,bj] -= A(m,k)[bi,:] * A(n,k)[bj,:]^T     (src/zpotrf_L.jdf:619-623, :453-456)
         jb.A = tile_ptr(a, m, k) + bi * BLK;
