@@ -22,7 +22,7 @@ accuracy (A and B stay resident in HBM; A is 17 GB, larger than L2).
           against the measured FP64 DMMA peak;
   kappa_sweep : kappa 1e2/1e4/1e6 x FP16/BF16/split-FP16 against FP64;
   batched : 4096 GP-kernel systems (n in [32, 512]) factored, solved and
-          log-det'ed in one graph-replayed launch, FP64 and FP32;
+          log-det'ed in one launch, FP64 and FP32;
   adjoint : GP log-marginal likelihood at N=16384, forward vs forward+backward;
   cpu_baseline : the reference's own CORE kernels (compiled from its sources)
           run as the tile DAG on all host cores, on a bounded N.
@@ -185,7 +185,7 @@ def measured_peaks():
 
 def bench_batched(ctx, db, torch, peak64):
     """4096 GP-kernel systems, n uniform in [32, 512] (seed 11), NRHS=1, FP64 and
-    FP32: Cholesky + solve + log-det in one graph-replayed persistent launch."""
+    FP32: Cholesky + solve + log-det in one persistent launch."""
     B = 4096
     rng = np.random.default_rng(11)
     sizes = [int(v) for v in rng.integers(32, 513, B)]
@@ -203,7 +203,7 @@ def bench_batched(ctx, db, torch, peak64):
         mats = [K.to(dt).clone() for K in base]
         rhs = [y.to(dt).clone() for y in ys]
         keep = []
-        info, _ = ctx.posv_batched(mats, rhs, keep=keep)       # autotunes, records the graph
+        info, _ = ctx.posv_batched(mats, rhs, keep=keep)       # warm-up
         times = []
         for _ in range(3):
             for m, K in zip(mats, base):

@@ -7,9 +7,9 @@
 * ``gp_log_marginal_likelihood_batched(Ks, ys)``: the same for a list of
   independent problems; forward is one batched launch
   (``dplasma_b200_dposv_batched``: factor, solve, log-det), backward one
-  batched inverse (``dplasma_b200_dpotri_batched``) for the K_i^-1, with all
-  problems in one flat buffer so that the rest is a fixed number of
-  whole-batch tensor operations; ``se_kernel_batched`` builds the K_i the
+  (``dplasma_b200_gp_gradient_batched``: the K_i^-1 and the gradients from
+  them), with all problems in one flat buffer so that the rest is a fixed
+  number of whole-batch tensor operations on vectors; ``se_kernel_batched`` builds the K_i the
   same way, and ``gp_log_marginal_likelihood_flat`` takes the batch as one
   flat tensor (one autograd node).
 * ``gp_log_marginal_likelihood(K, y)``: ``-1/2 y^T K^-1 y - 1/2 log det K
@@ -32,7 +32,7 @@ import math
 
 import torch
 
-from . import Context, desc_general, attach, Lower, STORAGE_LAPACK, torch_ready
+from . import Context, desc_general, attach, lib, Lower, STORAGE_LAPACK, torch_ready
 
 _ctx = {}
 
@@ -82,6 +82,18 @@ def _adjoint(Lrow: torch.Tensor, Lbar: torch.Tensor) -> torch.Tensor:
         raise RuntimeError(f"dplasma_dpotrf_adjoint: {rc} {ctx.last_error()}")
     up = torch.triu(Bc)                      # column-major lower part = row-major upper
     return up + torch.triu(Bc, 1).t()
+
+
+def _plain(g: torch.Tensor) -> bool:
+    """Whether a kernel may read g and nobody differentiates or batches what
+    comes of it (create_graph, is_grads_batched)."""
+    if g.requires_grad:
+        return False
+    try:
+        g.data_ptr()
+    except RuntimeError:
+        return False
+    return True
 
 
 def _inverse_from_factor(Lrow: torch.Tensor) -> torch.Tensor:
@@ -161,6 +173,26 @@ def gp_log_marginal_likelihood(K: torch.Tensor, y: torch.Tensor) -> torch.Tensor
 _layouts = {}
 
 
+class _Layout(dict):
+    """A batch's layout; mpad and vpad are made when a padded array is first
+    built (64-bit indices of every matrix entry: 0.2 s for 1024 problems)."""
+
+    def __missing__(self, key):
+        if key not in ("mpad", "vpad"):
+            raise KeyError(key)
+        import numpy as np
+        nmax, sz = self["nmax"], self["sizes"]
+        mpad = np.empty(sum(n * n for n in sz), np.int64)
+        vpad = np.empty(sum(sz), np.int64)
+        for b, (n, mo, vo) in enumerate(zip(sz, self["moff_h"], self["voff_h"])):
+            r = np.arange(n, dtype=np.int64)
+            mpad[mo:mo + n * n] = b * nmax * nmax + (r[:, None] * nmax + r[None, :]).ravel()
+            vpad[vo:vo + n] = b * nmax + r
+        dev = self["moff"].device
+        self["mpad"], self["vpad"] = torch.from_numpy(mpad).to(dev), torch.from_numpy(vpad).to(dev)
+        return self[key]
+
+
 def _batch_layout(sizes, device):
     """Flat and padded index maps of a batch of orders `sizes` (cached): every
     problem's matrix lives row-major at moff[b] in one flat buffer and at
@@ -175,21 +207,14 @@ def _batch_layout(sizes, device):
     B, nmax = len(sz), int(sz.max())
     moff = np.concatenate([[0], np.cumsum(sz * sz)[:-1]]).astype(np.int64)
     voff = np.concatenate([[0], np.cumsum(sz)[:-1]]).astype(np.int64)
-    mpad = np.empty(int((sz * sz).sum()), np.int64)
-    vpad = np.empty(int(sz.sum()), np.int64)
-    for b in range(B):
-        n = int(sz[b])
-        r = np.arange(n, dtype=np.int64)
-        mpad[moff[b]:moff[b] + n * n] = b * nmax * nmax + (r[:, None] * nmax + r[None, :]).ravel()
-        vpad[voff[b]:voff[b] + n] = b * nmax + r
 
     def dev(a):
         return torch.from_numpy(a).to(device)
 
-    lay = {"B": B, "nmax": nmax, "sizes": list(int(v) for v in sz), "n32": dev(sz.astype(np.int32)),
-           "moff": dev(moff), "voff": dev(voff), "mpad": dev(mpad), "vpad": dev(vpad),
+    lay = _Layout({"B": B, "nmax": nmax, "sizes": list(int(v) for v in sz), "n32": dev(sz.astype(np.int32)),
+           "moff": dev(moff), "voff": dev(voff),
            "pid": dev(np.repeat(np.arange(B, dtype=np.int64), sz)), "nf": dev(sz.astype(np.float64)),
-           "moff_h": moff.tolist(), "voff_h": voff.tolist()}
+           "moff_h": moff.tolist(), "voff_h": voff.tolist()})
     if len(_layouts) > 8:
         _layouts.clear()
     _layouts[key] = lay
@@ -227,28 +252,30 @@ def _gp_flat_backward(Lflat, alpha, g, lay):
     """(dK flat, dy flat) of the batch from the factors and alpha"""
     dev = Lflat.device
     ctx = context(dev)
-    B, nmax = lay["B"], lay["nmax"]
-    inv = Lflat.clone()
-    ptr = inv.data_ptr() + 8 * lay["moff"]
+    B = lay["B"]
+    if not _plain(g):
+        dK, _ = _gp_flat_backward(Lflat, alpha, torch.ones(B, dtype=Lflat.dtype, device=dev), lay)
+        n2 = lay["n32"].long() ** 2
+        return (g.index_select(0, torch.repeat_interleave(torch.arange(B, device=dev), n2)) * dK,
+                -g.index_select(0, lay["pid"]) * alpha)
+    g = g.contiguous()
+    dK = torch.empty_like(Lflat)
+    pL = Lflat.data_ptr() + 8 * lay["moff"]
+    pal = alpha.data_ptr() + 8 * lay["voff"]
+    pdK = dK.data_ptr() + 8 * lay["moff"]
     info = torch.empty(B, dtype=torch.int32, device=dev)
-    torch_ready(inv, ptr, lay["n32"])
-    from . import lib
-    rc = lib().dplasma_b200_dpotri_batched(ctx.h, B, lay["n32"].data_ptr(), lay["n32"].data_ptr(), ptr.data_ptr(),
-                                           info.data_ptr())
+    torch_ready(Lflat, alpha, g, pL, pal, pdK, lay["n32"])
+    n32 = lay["n32"].data_ptr()
+    rc = lib().dplasma_b200_gp_gradient_batched(ctx.h, B, n32, n32, pL.data_ptr(), pal.data_ptr(), g.data_ptr(),
+                                                pdK.data_ptr(), info.data_ptr())
     if rc != 0 or bool((info != 0).any()):
         raise RuntimeError(f"batched inverse failed: {rc} {ctx.last_error()}")
-    # K_i^-1 is the column-major lower = row-major upper triangle of each block
-    P = torch.zeros(B * nmax * nmax, dtype=torch.float64, device=dev).index_copy_(0, lay["mpad"], inv)
-    P = P.view(B, nmax, nmax)
-    Kinv = torch.triu(P) + torch.triu(P, 1).transpose(1, 2)
-    al = torch.zeros(B * nmax, dtype=torch.float64, device=dev).index_copy_(0, lay["vpad"], alpha).view(B, nmax)
-    dK = g.view(B, 1, 1) * (0.5 * al[:, :, None] * al[:, None, :] - 0.5 * Kinv)
-    return dK.reshape(-1).index_select(0, lay["mpad"]), -g.index_select(0, lay["pid"]) * alpha
+    return dK, -g.index_select(0, lay["pid"]) * alpha
 
 
 class _GPLogMLBatched(torch.autograd.Function):
     """List form: the problems are gathered into one flat buffer, then one
-    batched factor + solve + log-det launch forward and one batched inverse
+    batched factor + solve + log-det launch forward and one batched gradient
     launch backward, with a fixed number of whole-batch tensor operations
     around them."""
 

@@ -184,8 +184,6 @@ extern "C" void dplasma_b200_fini(parsec_context_t **pctx)
     Context *ctx = &(*pctx)->impl;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    for (auto &gr : ctx->bt_graph)
-        if (gr.exec) cudaGraphExecDestroy(gr.exec);
     for (int i = 0; i < BUF_COUNT; ++i)
         if (ctx->bufs[i]) cudaFree(ctx->bufs[i]);
     cudaEventDestroy(ctx->ev0);
@@ -812,7 +810,7 @@ static int posv_batched_api(parsec_context_t *parsec, int batch, const int *n, c
     cudaSetDevice(ctx->device);
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
-    return batched_posv<T>(ctx, batch, n, lda, A, B, B ? nrhs : 0, logdet, info, 0);
+    return batched_posv<T>(ctx, batch, n, lda, A, B, B ? nrhs : 0, logdet, info);
 }
 
 extern "C" int dplasma_b200_dposv_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
@@ -969,4 +967,18 @@ extern "C" int dplasma_b200_dpotri_batched(parsec_context_t *parsec, int batch, 
     ctx->launches = 0;
     ctx->errmsg[0] = 0;
     return batched_potri(ctx, batch, n, lda, A, info);
+}
+
+extern "C" int dplasma_b200_gp_gradient_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
+                                                const double *const *L, const double *const *alpha, const double *g,
+                                                double *const *dK, int *info)
+{
+    if (batch < 0) return -2;
+    if (!n || !lda || !L || !alpha || !g || !dK || !info) return DPLASMA_ERR_ILLEGAL_VALUE;
+    if (!parsec) return DPLASMA_ERR_NOT_INITIALIZED;
+    Context *ctx = &parsec->impl;
+    cudaSetDevice(ctx->device);
+    ctx->launches = 0;
+    ctx->errmsg[0] = 0;
+    return batched_potri(ctx, batch, n, lda, const_cast<double *const *>(L), info, alpha, g, dK);
 }

@@ -7,21 +7,19 @@
 // CTAs take problems from an atomic work queue in decreasing order of n
 // (longest first), so one launch balances sizes from 1 to 512.  A problem is
 // factored right-looking in 32-column panels:
-//   1. warp 0 factors the 32x32 diagonal block in registers, four columns
-//      per step (dev_chol32.cuh), and forms its inverse;
-//   2. the panel below becomes L = P D^-T (FP64: tensor cores, one 32-row
-//      block per warp; FP32: one row per thread), stored to global memory
-//      and to a shared panel;
+//   1. warp 0 factors the 32x32 diagonal block (chol32_col);
+//   2. the rows below are solved by substitution, one row per lane (sweep32), to
+//      global memory and to a shared panel; the right-hand sides are one more set
+//      of rows of the same solve, the inverse of the diagonal block (for the
+//      backward solve) one more sweep on the unit vectors, so neither is on the
+//      chain;
 //   3. the lower triangle of the trailing matrix is updated from the shared
 //      panel in 32x32 tiles, one warp per tile (FP64 tensor cores; FP32 on
-//      the FMA pipes), the next panel's columns first so that warp 0 factors
-//      the next diagonal block while the others finish the update.
-// The number of warps per problem is picked per size class by timing the variants on
-// the caller's own batch the first time (autotuning), and the launch is
-// recorded once as a CUDA graph and replayed while the arguments stay the
-// same.
-// The solve runs the two triangular sweeps on the factor in 32-row blocks,
-// and the log-determinant is 2 * sum log L(i,i).
+//      the FMA pipes), the next diagonal block first so that warp 0 factors
+//      it while the others finish the update.
+// What bounds a problem is the latency of these steps, so several problems
+// share an SM (bt_variants).  The solve ends with the backward sweep on the
+// factor in 32-row blocks; the log-determinant is 2 * sum log L(i,i).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -36,8 +34,8 @@
 namespace db2 {
 
 constexpr int BT_NB = 32;
-constexpr int BT_PP = 36;          // shared pitch of panel rows (== 4 mod 16: conflict-free FP64 fragments)
-constexpr int BT_NMAX = 4096;      // largest n of one problem (panel rows in shared memory)
+constexpr int BT_DP = 33;          // pitch of a diagonal block in shared memory
+constexpr int BT_NMAX = 4096;      // largest n of one problem
 constexpr int BT_MAXRHS = 16;      // right-hand sides per problem
 
 template <typename T>
@@ -52,265 +50,318 @@ struct BatchArgs {
     int *info;            // per problem
     const int *order;     // problems by decreasing n
     int *ticket;
-    T *dscr;              // per CTA: inverses of the 32x32 diagonal blocks of its current problem
+    T *dscr;              // per CTA (dstride): inverses of the 32x32 diagonal blocks of its current problem
+    int64_t dstride;
+    int prow;             // panel rows kept in shared memory
 };
 
-// Diagonal block j0 (jb <= 32 columns) of one problem by warp 0: factor in
-// registers, write L back, accumulate log det, form the inverse into Dinv.
-// Returns the failing column within the block or -1.
+// Diagonal block j0 (jb <= 32 columns) of one problem by one warp: factor,
+// write L back, accumulate log det; the blocked copy Lb and the reciprocal
+// diagonal rd serve the sweeps.  in_sm: the block lies in Lb's place already
+// (column c, row r at c * BT_DP + r; also in the matrix).  Returns the failing
+// column within the block or -1.
 template <typename T>
-__device__ int bt_diag(T *A, int lda, int j0, int jb, T *Dinv, T *Ls, double &ld_acc, int lane)
+__device__ __forceinline__ int bt_diag(T *A, int lda, int j0, int jb, bool in_sm, T *Lb, T *rd, double &ld_acc, int lane)
 {
     T d[32];
+    // padding rows are the identity (a running pointer: 32 addresses would take the registers)
+    auto load = [&](const T *p, int ld) {
+        p += lane;
 #pragma unroll
-    for (int c = 0; c < 32; ++c)
-        d[c] = (lane < jb && c < jb) ? ((c <= lane) ? A[(int64_t)(j0 + c) * lda + j0 + lane] : T(0))
-                                     : (c == lane ? T(1) : T(0));
-    T rdiag = T(0);
-    int failcol = chol32_blk<T>(d, lane, rdiag, Ls);     // Ls: blocked copy of L ([8][32][4])
-    if (failcol >= jb) failcol = -1;      // padding rows are the identity
-    if (failcol >= 0) return failcol;
+        for (int c = 0; c < 32; ++c) {
+            d[c] = (lane < jb && c < jb) ? ((c <= lane) ? *p : T(0)) : (c == lane ? T(1) : T(0));
+            p += ld;
+        }
+    };
+    T *Aj = A + (int64_t)j0 * lda + j0;
+    if (in_sm) load(Lb, BT_DP);
+    else load(Aj, lda);
     __syncwarp();
-    if (lane < jb) {
-#pragma unroll 8
-        for (int c = 0; c < 32; ++c)
-            if (c <= lane && c < jb) A[(int64_t)(j0 + c) * lda + j0 + lane] = Ls[(c >> 2) * 128 + lane * 4 + (c & 3)];
-        ld_acc -= 2.0 * log((double)rdiag);   // rdiag = 1 / L(i,i)
+    int f = -1;
+    if (!chol32_col<T>(d, lane, (T *)nullptr, 0, Lb, rd)) {
+        // a pivot outside the fast root's range, or not positive
+        load(Aj, lda);
+        T rdiag = T(0);
+        f = chol32_blk<T>(d, lane, rdiag, Lb);
+        rd[lane] = rdiag;
+        __syncwarp();
+        if (f >= jb) f = -1;
+        if (f >= 0) return f;
     }
-    inv32_blk<T>(Ls, lane, rdiag, [&](int i, int c, T x) { Dinv[i * BT_PP + c] = x; });   // Dinv[i][c], lower
-    __syncwarp();
+    if (lane < jb) {
+        T *p = Aj + lane;
+#pragma unroll 8
+        for (int c = 0; c < 32; ++c) {
+            if (c <= lane && c < jb) *p = Lb[(c >> 2) * 128 + lane * 4 + (c & 3)];
+            p += lda;
+        }
+        ld_acc -= 2.0 * log((double)rd[lane]);   // rd = 1 / L(i,i)
+    }
     return -1;
 }
 
-// One 32x32 tile (rb, cb), rb >= cb, of the trailing update C -= P P^T by one
-// warp; C is the trailing matrix (origin at A(o, o)), m its order.  The C
-// values are loaded before the products, so their latency overlaps them.
-__device__ __forceinline__ void bt_tile(double *A, int lda, int o, int m, const double *P, int rb, int cb, int lane)
+// The next diagonal block (tile (0,0) of the trailing matrix) before it is
+// factored, C -= P P^T in lower 16x16 quarters q = 0 (top), 1 (below), 2: to the
+// matrix and to shared memory at Sd (pitch BT_DP).
+__device__ __forceinline__ void bt_quarter(double *C, int lda, int m, const double *Pr, int sr, double *Sd, int q,
+                                           int lane)
 {
     const int g = lane >> 2, t = lane & 3;
-    double old[2][4][4];
+    const int qr = q == 0 ? 0 : 16, qc = q == 2 ? 16 : 0;
+    double acc[2][4];
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int e = 0; e < 4; ++e) {
+            const int r = qr + g + ((e & 2) ? 8 : 0), c = qc + ni * 8 + 2 * t + (e & 1);
+            acc[ni][e] = (r < m && c <= r) ? C[(int64_t)c * lda + r] : 0.0;
+        }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = rb * 32 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                const int c = cb * 32 + ni * 8 + 2 * t + (q & 1);
-                old[mi][ni][q] = (r < m && c < m && r >= c) ? A[(int64_t)(o + c) * lda + o + r] : 0.0;
-            }
+    for (int kk = 0; kk < 32; kk += 4) {
+        const double *pk = Pr + (int64_t)(kk + t) * sr + g;
+        const double a0 = qr + g < m ? -pk[qr] : 0.0, a1 = qr + g + 8 < m ? -pk[qr + 8] : 0.0;
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni)
+            dmma_16x8x4(acc[ni], a0, a1, qc + ni * 8 + g < m ? pk[qc + ni * 8] : 0.0);
+    }
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = qr + g + ((e & 2) ? 8 : 0), c = qc + ni * 8 + 2 * t + (e & 1);
+            Sd[c * BT_DP + r] = acc[ni][e];
+            if (r < m && c <= r) C[(int64_t)c * lda + r] = acc[ni][e];
+        }
+}
+__device__ __forceinline__ void bt_quarter(float *C, int lda, int m, const float *Pr, int sr, float *Sd, int q, int lane)
+{
+    // half the columns of a row per lane: quarter q has rows qr + (lane / 2), eight columns each
+    const int qr = q == 0 ? 0 : 16, qc = (q == 2 ? 16 : 0) + 8 * (lane & 1), r = qr + (lane >> 1);
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = (r < m && qc + j <= r) ? C[(int64_t)(qc + j) * lda + r] : 0.f;
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+        const float pr = -Pr[k * sr + r];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = fmaf(pr, Pr[k * sr + qc + j], acc[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        Sd[(qc + j) * BT_DP + r] = acc[j];
+        if (r < m && qc + j <= r) C[(int64_t)(qc + j) * lda + r] = acc[j];
+    }
+}
+
+// One 32x32 tile (rb, cb), rb >= cb, of the trailing update C -= P P^T by one
+// warp; C is the trailing matrix (origin at A(o, o)), m its order, P the panel
+// (rows beyond m zero) with k stride RP.  The C values are the accumulators'
+// start.
+// FULL: all 32 x 32 elements exist (below the diagonal block, inside m).
+template <bool FULL>
+__device__ __forceinline__ void bt_tile_f64(double *A, int lda, int o, int m, const double *P, int RP, int rb, int cb,
+                                            int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+    double *C = A + (int64_t)(o + cb * 32 + 2 * t) * lda + o + rb * 32 + g;
+    const int mr = m - rb * 32 - g, mc = m - cb * 32 - 2 * t, dd = rb == cb ? g - 2 * t : 1 << 20;
+    // element (row 16 mi + 8 h, column 8 ni + e) of this thread
+    auto in = [&](int r, int c) { return FULL || (r < mr && c < mc && r - c + dd >= 0); };
     double acc[2][4][4];
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int ni = 0; ni < 4; ++ni) {
+        const double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
+            for (int q = 0; q < 4; ++q) {
+                const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
+                acc[mi][ni][q] = in(r, c) ? ((q & 1) ? p1 : p0)[r] : 0.0;
+            }
+    }
+    const double *a0 = P + t * RP + rb * 32 + g, *b0 = P + t * RP + cb * 32 + g;
 #pragma unroll
     for (int kk = 0; kk < 32; kk += 4) {
         double af[2][2], bf[4];
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi) {
-            af[mi][0] = P[(rb * 32 + mi * 16 + g) * BT_PP + kk + t];
-            af[mi][1] = P[(rb * 32 + mi * 16 + g + 8) * BT_PP + kk + t];
+            af[mi][0] = -a0[mi * 16];
+            af[mi][1] = -a0[mi * 16 + 8];
         }
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) bf[ni] = P[(cb * 32 + ni * 8 + g) * BT_PP + kk + t];
+        for (int ni = 0; ni < 4; ++ni) bf[ni] = b0[ni * 8];
+        a0 += 4 * RP;
+        b0 += 4 * RP;
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
     }
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int ni = 0; ni < 4; ++ni) {
+        double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int r = rb * 32 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                const int c = cb * 32 + ni * 8 + 2 * t + (q & 1);
-                if (r < m && c < m && r >= c) A[(int64_t)(o + c) * lda + o + r] = old[mi][ni][q] - acc[mi][ni][q];
+                const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
+                if (in(r, c)) ((q & 1) ? p1 : p0)[r] = acc[mi][ni][q];
             }
+    }
+}
+__device__ __forceinline__ void bt_tile(double *A, int lda, int o, int m, const double *P, int RP, int rb, int cb,
+                                        int lane)
+{
+    if (rb > cb && rb * 32 + 32 <= m) bt_tile_f64<true>(A, lda, o, m, P, RP, rb, cb, lane);
+    else bt_tile_f64<false>(A, lda, o, m, P, RP, rb, cb, lane);
 }
 // FP32: lane = row of the tile, 32 columns per lane (the panel values of the
-// columns are shared-memory broadcasts)
-__device__ __forceinline__ void bt_tile(float *A, int lda, int o, int m, const float *P, int rb, int cb, int lane)
+// columns are broadcasts)
+__device__ __forceinline__ void bt_tile(float *A, int lda, int o, int m, const float *P, int RP, int rb, int cb,
+                                        int lane)
 {
     const int r = rb * 32 + lane;
-    float old[32], acc[32];
+    float acc[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         const int c = cb * 32 + j;
-        old[j] = (r < m && c < m && r >= c) ? A[(int64_t)(o + c) * lda + o + r] : 0.f;
-        acc[j] = 0.f;
+        acc[j] = (r < m && c < m && r >= c) ? A[(int64_t)(o + c) * lda + o + r] : 0.f;
     }
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
-        const float pr = P[r * BT_PP + k];
+        const float pr = -P[k * RP + r];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = fmaf(pr, P[(cb * 32 + j) * BT_PP + k], acc[j]);
+        for (int j = 0; j < 32; j += 4) {
+            float v[4];
+            c32_load4(P + k * RP + cb * 32 + j, v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[j + e] = fmaf(pr, v[e], acc[j + e]);
+        }
     }
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         const int c = cb * 32 + j;
-        if (r < m && c < m && r >= c) A[(int64_t)(o + c) * lda + o + r] = old[j] - acc[j];
+        if (r < m && c < m && r >= c) A[(int64_t)(o + c) * lda + o + r] = acc[j];
     }
 }
 
 // One problem, whole CTA.  Right-looking in 32-column panels with one step of
-// look-ahead: after the panel, the warps first update the next panel's
-// columns; then warp 0 factors the next diagonal block while the other warps
-// update the rest of the trailing matrix.  Returns INFO (0 or the 1-based
-// failing column).
-// Warp 0, after the diagonal block j0 was factored and inverted: keep the
-// inverse for the backward solve and apply it to the right-hand sides,
-// y_j = D^-1 b_j (forward substitution with the block inverse), y_j kept in
-// ybuf for the panel update of the rows below and stored in place in B.
-template <typename T>
-__device__ __forceinline__ void bt_diag_rhs(const T *Dinv, T *dscr, int j0, int jb, T *B, int ldb, int nrhs,
-                                            T *ybuf, int lane)
-{
-    T *Dk = dscr + (int64_t)(j0 / BT_NB) * 32 * 32;
-#pragma unroll 4
-    for (int i = 0; i < 32; ++i) Dk[i * 32 + lane] = Dinv[i * BT_PP + lane];
-    for (int col = 0; col < nrhs; ++col) {
-        T *b = B + (int64_t)col * ldb + j0;
-        const T bl = lane < jb ? b[lane] : T(0);
-        T y = T(0);
-#pragma unroll
-        for (int l = 0; l < 32; ++l) y = fma(Dinv[lane * BT_PP + l], __shfl_sync(0xffffffffu, bl, l), y);
-        if (lane < jb) b[lane] = y;
-        ybuf[col * 32 + lane] = lane < jb ? y : T(0);
-    }
-}
-
-template <typename T, int NT, int TILE>
-__device__ int bt_factor(T *A, int n, int lda, T *Dinv, T *Ls, T *P, int *sflag, double *logdet_out, T *B,
-                         int nrhs, T *dscr, T *ybuf)
+// look-ahead: after the panel, three warps update the next diagonal block; then
+// warp 0 factors it while the other warps update the rest of the trailing matrix.
+// P: the panel, RP its k stride.  Returns INFO (0 or the 1-based failing column).
+template <typename T, int NT>
+__device__ int bt_factor(T *A, int n, int lda, T *Lb, T *P, int RP, int *sflag, double *logdet_out,
+                         T *B, int nrhs, T *dscr, T *ybuf)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int NW = NT / 32;
+    T *rd = Lb + C32_RD;
     double ld_acc = 0.0;
-    int info = 0;
     if (warp == 0) {
-        const int f = bt_diag<T>(A, lda, 0, min(BT_NB, n), Dinv, Ls, ld_acc, lane);
+        const int f = bt_diag<T>(A, lda, 0, min(BT_NB, n), false, Lb, rd, ld_acc, lane);
         if (lane == 0) sflag[0] = f;
-        if (f < 0 && B) bt_diag_rhs<T>(Dinv, dscr, 0, min(BT_NB, n), B, n, nrhs, ybuf, lane);
     }
     __syncthreads();
-    if (sflag[0] >= 0) info = sflag[0] + 1;
+    int info = sflag[0] >= 0 ? sflag[0] + 1 : 0;
     for (int j0 = 0; j0 < n && info == 0; j0 += BT_NB) {
         const int jb = min(BT_NB, n - j0);
-        const int o = j0 + jb, m = n - o;
-        if (m <= 0) break;
-        // panel rows below: L = A D^-T, to global and to the shared panel
-        // (rows up to the next multiple of 32 are zero-filled)
-        const int m32 = (m + 31) & ~31;
-        if constexpr (sizeof(T) == 8) {
-            // FP64: X = P Dinv^T on the tensor cores, one 32-row block per warp
-            // and turn, then each lane forward-solves its row of B
-            for (int rb = warp; rb < m32 / 32; rb += NW) {
-                const int rr0 = rb * 32;
-                const int g = lane >> 2, t = lane & 3;
-                double af[8][2][2];
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks)
-#pragma unroll
-                    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int rr = rr0 + mi * 16 + g + 8 * h, c = ks * 4 + t;
-                            af[ks][mi][h] = (rr < m && c < jb) ? (double)A[(int64_t)(j0 + c) * lda + o + rr] : 0.0;
-                        }
-                double acc[2][4][4];
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) {
-                        const double bf = (double)Dinv[(ni * 8 + g) * BT_PP + ks * 4 + t];   // Dinv^T(l, c)
-#pragma unroll
-                        for (int mi = 0; mi < 2; ++mi) dmma_16x8x4(acc[mi][ni], af[ks][mi][0], af[ks][mi][1], bf);
-                    }
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const int rr = rr0 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                            const int c = ni * 8 + 2 * t + (q & 1);
-                            const bool in = rr < m && c < jb;
-                            if (in) A[(int64_t)(j0 + c) * lda + o + rr] = (T)acc[mi][ni][q];
-                            P[rr * BT_PP + c] = in ? (T)acc[mi][ni][q] : T(0);
-                        }
-                __syncwarp();
-                const int rr = rr0 + lane;
-                if (B && rr < m) {
-                    for (int col = 0; col < nrhs; ++col) {
-                        T acc1 = T(0);
-#pragma unroll 8
-                        for (int c = 0; c < 32; ++c) acc1 = fma(P[rr * BT_PP + c], ybuf[col * 32 + c], acc1);
-                        B[(int64_t)col * n + o + rr] -= acc1;
-                    }
-                }
+        const int o = j0 + jb, m = n - o, mb = (m + 31) / 32;
+        // (P) rows below, the right-hand sides and the inverse of the diagonal
+        // block, each 32 vectors of the same substitution (the inverse and the
+        // right-hand sides also after the last block)
+        const int nit = mb + (B ? 2 : 0);
+#pragma unroll 1
+        for (int it = NW > 1 ? NW - 1 - warp : 0; it < nit; it += NW) {
+            T b[32];
+            const int rr = it * 32 + lane;
+            const bool rows = it < mb, rhs = it == mb;
+            T *src = A + (int64_t)j0 * lda + o + rr;
+            int64_t stride = lda;
+            bool live = rows && rr < m;
+            if (rhs) {
+                src = B + (int64_t)lane * n + j0;
+                stride = 1;
+                live = lane < nrhs;
             }
-        } else
-        for (int rr = tid; rr < m32; rr += NT) {
-            if (rr >= m) {
-#pragma unroll
-                for (int c = 0; c < 32; ++c) P[rr * BT_PP + c] = T(0);
-                continue;
-            }
-            const int r = o + rr;
-            T a[32];
-#pragma unroll
-            for (int c = 0; c < 32; ++c) a[c] = (c < jb) ? A[(int64_t)(j0 + c) * lda + r] : T(0);
+            const T *q = src;
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
-                T x = T(0);
+                b[c] = (live && c < jb) ? *q : T(0);
+                q += stride;
+            }
+            if (!rows && !rhs) {
 #pragma unroll
-                for (int l = 0; l <= c; ++l) x = fma(a[l], Dinv[c * BT_PP + l], x);
-                if (c < jb) A[(int64_t)(j0 + c) * lda + r] = x;
-                P[rr * BT_PP + c] = (c < jb) ? x : T(0);
+                for (int c = 0; c < 32; ++c) b[c] = c == lane ? T(1) : T(0);
             }
-            // forward solve of the rows below: b_r -= L(r, panel) y_panel
-            if (B) {
-                for (int col = 0; col < nrhs; ++col) {
-                    T acc = T(0);
-#pragma unroll 8
-                    for (int c = 0; c < 32; ++c) acc = fma(P[rr * BT_PP + c], ybuf[col * 32 + c], acc);
-                    B[(int64_t)col * n + r] -= acc;
-                }
-            }
+            T *Dk = dscr + (int64_t)(j0 / BT_NB) * 32 * 32 + lane;
+            T *Pp = P + rr;
+            sweep32<T>(Lb, rd, b, [&](int c, T x) {               // in order of c
+                if (live && c < jb) *src = x;
+                src += stride;
+                if (rows) *Pp = x;
+                Pp += RP;
+                if (rhs && lane < nrhs) ybuf[lane * 32 + c] = c < jb ? x : T(0);
+                if (!rows && !rhs) Dk[c * 32] = x;            // D^-1(c, lane)
+            });
         }
         __syncthreads();
-        const int mb = m32 / 32;
-        // (a) the next panel's columns: tiles (rb, 0)
-        for (int rb = warp; rb < mb; rb += NW) bt_tile(A, lda, o, m, P, rb, 0, lane);
-        __syncthreads();
-        // (b) warp 0: next diagonal block; the others: tiles (rb, cb), cb >= 1
+        if (m <= 0) break;
+        // the next diagonal block, in quarters on three warps; then warp 0
+        // factors it while the others do all other tiles and the right-hand
+        // sides below, b_r -= L(r, panel) y_panel
+        T *C00 = A + (int64_t)o * lda + o;
+        if (NW >= 4 ? warp < 3 : warp == 0) {
+#pragma unroll 1
+            for (int q = NW >= 4 ? warp : 0; q < 3; q += NW >= 4 ? 3 : 1)
+                bt_quarter(C00, lda, m, P, RP, Lb, q, lane);
+            if (NW >= 4) {
+                if (warp > 0) asm volatile("bar.arrive 1, 96;" ::: "memory");
+                else asm volatile("bar.sync 1, 96;" ::: "memory");
+            } else {
+                __syncwarp();
+            }
+        }
         if (warp == 0) {
-            // the rows of B in this block were final after the panel above
-            __threadfence_block();
-            const int f = bt_diag<T>(A, lda, o, min(BT_NB, m), Dinv, Ls, ld_acc, lane);
+            const int f = bt_diag<T>(A, lda, o, min(BT_NB, m), true, Lb, rd, ld_acc, lane);
             if (lane == 0) sflag[0] = f;
-            if (f < 0 && B) bt_diag_rhs<T>(Dinv, dscr, o, min(BT_NB, m), B, n, nrhs, ybuf, lane);
-        } else {
-            const int nrest = mb * (mb + 1) / 2 - mb;   // tiles with cb >= 1
-            for (int it = warp - 1; it < nrest; it += NW - 1) {
-                // tiles with cb >= 1 enumerated column by column
-                int cb = 1, rem = it;
+        }
+        const int ntile = mb * (mb + 1) / 2;
+        // warp 4 shares warp 0's sub-partition (and its FP64 pipe): it helps only
+        // where the tiles outlast the diagonal block
+        const bool spare = NW == 8 && ntile < 24;
+        if ((warp > 0 && !(spare && warp == 4)) || NW == 1) {
+            const int w = NW == 1 ? 0 : warp - 1 - (spare && warp > 4);
+            const int NH = NW == 1 ? 1 : NW - 1 - spare;
+#pragma unroll 1
+            for (int it = 1 + w; it < ntile; it += NH) {
+                // tiles enumerated column by column
+                int cb = 0, rem = it;
                 while (rem >= mb - cb) {
                     rem -= mb - cb;
                     ++cb;
                 }
-                bt_tile(A, lda, o, m, P, cb + rem, cb, lane);
+                const int rb = cb + rem;
+                bt_tile(A, lda, o, m, P, RP, rb, cb, lane);
+            }
+            if (B) {
+#pragma unroll 1
+                for (int it = NH - 1 - w; it < mb; it += NH) {
+                    const int rr = it * 32 + lane;
+                    if (rr >= m) continue;
+                    const T *pr = P + rr;
+                    T pv[32];
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        pv[c] = *pr;
+                        pr += RP;
+                    }
+                    for (int col = 0; col < nrhs; ++col) {
+                        T s = T(0);
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) s = fma(pv[c], ybuf[col * 32 + c], s);
+                        B[(int64_t)col * n + o + rr] -= s;
+                    }
+                }
             }
         }
         __syncthreads();
@@ -327,56 +378,75 @@ __device__ int bt_factor(T *A, int n, int lda, T *Dinv, T *Ls, T *P, int *sflag,
 
 // Backward solve L^T X = Y in place (Y from the fused forward solve), whole
 // CTA, with the stored inverses of the diagonal blocks: for each block j from
-// the last, s = L(below, j)^T x_below (one warp per column, lanes over rows),
-// then x_j = D_j^-T (y_j - s).  No serial substitution chain.
+// the last, s = L(below, j)^T x_below (lanes over rows, four columns of a warp
+// at a time so that their loads overlap), then x_j = D_j^-T (y_j - s).  x
+// stays in shared memory (xs, n values); red holds 32.
 template <typename T, int NT>
-__device__ void bt_backward(const T *A, int n, int lda, T *B, int nrhs, const T *dscr, T *red)
+__device__ void bt_backward(const T *A, int n, int lda, T *B, int nrhs, const T *dscr, T *red, T *xs)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int NW = NT / 32;
     for (int col = 0; col < nrhs; ++col) {
         T *b = B + (int64_t)col * n;
+        __syncthreads();
+        for (int i = tid; i < n; i += NT) xs[i] = b[i];
+        __syncthreads();
         const int nblk = (n + BT_NB - 1) / BT_NB;
         for (int bk = nblk - 1; bk >= 0; --bk) {
-            const int j0 = bk * BT_NB, jb = min(BT_NB, n - j0);
-            for (int c = warp; c < jb; c += NW) {
-                T s0 = T(0), s1 = T(0);
-                const T *Lc = A + (int64_t)(j0 + c) * lda;
-                int r = j0 + jb + lane;
-                for (; r + 32 < n; r += 64) {
-                    s0 = fma(Lc[r], b[r], s0);
-                    s1 = fma(Lc[r + 32], b[r + 32], s1);
-                }
-                if (r < n) s0 = fma(Lc[r], b[r], s0);
-                T s = s0 + s1;
+            const int j0 = bk * BT_NB, jb = min(BT_NB, n - j0), o = j0 + jb;
+            T dk[32];
+            if (warp == 0) {
+                const T *Dk = dscr + (int64_t)bk * 32 * 32 + lane;   // Dk[i * 32 + c] = D^-1(i, c)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (lane == 0) red[c] = s;
+                for (int i = 0; i < 32; ++i) dk[i] = Dk[i * 32];
+            }
+            for (int c = 4 * warp; c < jb; c += 4 * NW) {
+                T s[4] = {T(0), T(0), T(0), T(0)};
+                const T *Lc[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) Lc[q] = A + (int64_t)(j0 + min(c + q, jb - 1)) * lda;
+#pragma unroll 2
+                for (int r = o + lane; r < n; r += 32) {
+                    const T x = xs[r];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) s[q] = fma(Lc[q][r], x, s[q]);
+                }
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], w);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (lane == q) red[c + q] = s[q];
             }
             __syncthreads();
             if (warp == 0) {
-                const T *Dk = dscr + (int64_t)bk * 32 * 32;   // Dk[i * 32 + c] = D^-1(i, c)
-                const T tl = lane < jb ? b[j0 + lane] - red[lane] : T(0);
-                T x = T(0);
+                const T tl = lane < jb ? xs[j0 + lane] - red[lane] : T(0);
+                T x0 = T(0), x1 = T(0);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) x = fma(Dk[i * 32 + lane], __shfl_sync(0xffffffffu, tl, i), x);
-                if (lane < jb) b[j0 + lane] = x;
+                for (int i = 0; i < 32; i += 2) {
+                    x0 = fma(dk[i], __shfl_sync(0xffffffffu, tl, i), x0);
+                    x1 = fma(dk[i + 1], __shfl_sync(0xffffffffu, tl, i + 1), x1);
+                }
+                if (lane < jb) {
+                    xs[j0 + lane] = x0 + x1;
+                    b[j0 + lane] = x0 + x1;
+                }
             }
             __syncthreads();
         }
     }
 }
 
-template <typename T, int NT, int TILE>
-__global__ void __launch_bounds__(NT) batched_posv_kernel(BatchArgs<T> a)
+template <typename T, int NT, int OCC>
+__global__ void __launch_bounds__(NT, OCC) batched_posv_kernel(BatchArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char bsm[];
-    T *Dinv = reinterpret_cast<T *>(bsm);
-    T *Ls = Dinv + 32 * BT_PP;                // diagonal-block staging
-    T *P = Ls + 32 * BT_PP;                   // panel rows, BT_PP pitch
+    T *Lb = reinterpret_cast<T *>(bsm);       // blocked copy of the diagonal factor, 1 / diagonal
+    T *P = Lb + C32_LB;                       // panel, k stride prow + 4
     __shared__ int sflag[2];
     __shared__ T ybuf[32 * BT_MAXRHS];
-    T *dscr = a.dscr + (int64_t)blockIdx.x * (BT_NMAX / BT_NB) * 32 * 32;
+    T *dscr = a.dscr + (int64_t)blockIdx.x * a.dstride;
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) sflag[1] = atomicAdd(a.ticket, 1);
@@ -388,9 +458,9 @@ __global__ void __launch_bounds__(NT) batched_posv_kernel(BatchArgs<T> a)
         int info = 0;
         if (n > 0) {
             T *Bi = (a.B && a.nrhs > 0) ? a.B[i] : nullptr;
-            info = bt_factor<T, NT, TILE>(a.A[i], n, lda, Dinv, Ls, P, sflag, a.logdet ? a.logdet + i : nullptr, Bi,
-                                          a.nrhs, dscr, ybuf);
-            if (info == 0 && Bi) bt_backward<T, NT>(a.A[i], n, lda, Bi, a.nrhs, dscr, P);
+            info = bt_factor<T, NT>(a.A[i], n, lda, Lb, P, a.prow + 4, sflag,
+                                    a.logdet ? a.logdet + i : nullptr, Bi, a.nrhs, dscr, ybuf);
+            if (info == 0 && Bi) bt_backward<T, NT>(a.A[i], n, lda, Bi, a.nrhs, dscr, Lb, P);
         } else if (threadIdx.x == 0 && a.logdet) {
             a.logdet[i] = 0.0;
         }
@@ -399,38 +469,32 @@ __global__ void __launch_bounds__(NT) batched_posv_kernel(BatchArgs<T> a)
 }
 
 // ---------------------------------------------------------------------------
-// host: variants, autotuning, graph
+// host: launch shapes
 // ---------------------------------------------------------------------------
-template <typename T, int NT, int TILE>
-static size_t bt_smem(int nmax)
-{
-    return (size_t)(64 * BT_PP + (size_t)((std::max(nmax, 32) + 31) & ~31) * BT_PP) * sizeof(T);
-}
-
-// prepare: shared-memory attribute and grid (not stream work, so it runs
-// before a capture); launch: the kernel alone (capturable)
 template <typename T>
-using BtLaunch = int (*)(Context *, const BatchArgs<T> &, int nmax, cudaStream_t, bool prepare);
+using BtLaunch = int (*)(Context *, BatchArgs<T> &, int nmax);
 
-template <typename T, int NT, int TILE>
-static int bt_launch(Context *ctx, const BatchArgs<T> &a, int nmax, cudaStream_t st, bool prepare)
+// OCC: CTAs of an SM the registers are limited for
+template <typename T, int NT, int OCC>
+static int bt_launch(Context *ctx, BatchArgs<T> &a, int nmax)
 {
-    const size_t smem = bt_smem<T, NT, TILE>(nmax);
-    static int grid_cache[BT_NMAX / 32 + 2] = {};
-    const int key = (nmax + 31) / 32;
-    if (prepare) {
-        CK(cudaFuncSetAttribute(batched_posv_kernel<T, NT, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
-        int occ = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_posv_kernel<T, NT, TILE>, NT, smem));
-        if (occ < 1) {
-            ctx->set_error("batched kernel does not fit (n max %d)", nmax);
-            return DPLASMA_ERR_INTERNAL_LIMIT;
-        }
-        grid_cache[key] = ctx->sms * std::min(occ, 4);   // the diagonal-inverse scratch holds 4 CTAs per SM
-        return 0;
+    // the panel's rows: those below the first block
+    a.prow = std::max(32, (nmax - 1) / 32 * 32);
+    const size_t smem = (C32_LB + 32 * (size_t)(a.prow + 4)) * sizeof(T);
+    CK(cudaFuncSetAttribute(batched_posv_kernel<T, NT, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int occ = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_posv_kernel<T, NT, OCC>, NT, smem));
+    if (occ < 1) {
+        ctx->set_error("batched kernel does not fit (n max %d)", nmax);
+        return DPLASMA_ERR_INTERNAL_LIMIT;
     }
-    batched_posv_kernel<T, NT, TILE><<<grid_cache[key], NT, smem, st>>>(a);
+    const int grid = std::min(a.batch, ctx->sms * occ);
+    // inverses of the diagonal blocks of the CTA's problem
+    a.dstride = (int64_t)((nmax + BT_NB - 1) / BT_NB) * 32 * 32;
+    a.dscr = (T *)ctx->buffer(BUF_BATCH_SCR, (size_t)grid * a.dstride * sizeof(T));
+    if (!a.dscr) return DPLASMA_ERR_OUT_OF_RESOURCES;
+    CK(cudaMemsetAsync(a.ticket, 0, sizeof(int), ctx->stream));
+    batched_posv_kernel<T, NT, OCC><<<grid, NT, smem, ctx->stream>>>(a);
     CK(cudaGetLastError());
     ctx->launches++;
     return 0;
@@ -445,28 +509,37 @@ template <typename T>
 static const BtVariant<T> *bt_variants(int &count)
 {
     static const BtVariant<T> v[] = {
-        {"4 warps per problem", bt_launch<T, 128, 32>},
-        {"8 warps per problem", bt_launch<T, 256, 32>},
+        {"1 warp per problem", bt_launch<T, 32, 8>},
+        {"4 warps per problem", bt_launch<T, 128, 3>},
+        {"8 warps per problem", bt_launch<T, 256, 1>},
+        {"8 warps per problem, two per SM", bt_launch<T, 256, 2>},
     };
     count = (int)(sizeof(v) / sizeof(v[0]));
     return v;
 }
 
-// Per-size-class choice of the autotuner, cached in the context: the class
-// is the largest n rounded up to a power of two (64 .. 4096).
-static int bt_class(int nmax)
+// Warps per problem: a problem's latency falls with its warps (large problems, and
+// batches that leave SMs idle), the work in flight on an SM rises with the
+// problems that share it (small ones).  Kernel times in ms on 148 SMs with 1 / 4 /
+// 8 / 8 warps two per SM:
+//   FP32, 8192 problems of 8 to 96:     0.338 / 0.432 / 0.955 / 0.570
+//   FP64, 1024 problems of 64 to 256:   0.614 / 0.391 / 0.482 / 0.520
+//   FP64, 4096 problems of 32 to 512:   22.4  / 9.6   / 5.45  / 7.7
+//   FP32, 2000 problems of 64 to 512:     -   / 2.60  / 2.60  / 2.26
+//   FP64, 2000 problems of 8 to 64:     0.081 / 0.130
+// (before, with the inverse of each diagonal block on the chain and the shapes timed
+// on the caller's batch: 0.78, 0.54, 7.6 for the first three).
+static int bt_choose(bool fp64, int batch, int nmax, int sms)
 {
-    int c = 0, v = 64;
-    while (v < nmax && c < 6) {
-        v <<= 1;
-        ++c;
-    }
-    return c;
+    if (batch <= 2 * sms) return 2;
+    if (nmax <= 96) return 0;
+    if (nmax <= 256) return 1;
+    return fp64 ? 2 : 3;
 }
 
 template <typename T>
 int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *const *d_A, T *const *d_B, int nrhs,
-                 double *d_logdet, int *d_info, int tune)
+                 double *d_logdet, int *d_info)
 {
     if (batch <= 0) return 0;
     cudaStream_t st = ctx->stream;
@@ -482,7 +555,7 @@ int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *c
         }
         nmax = std::max(nmax, v);
     }
-    if (nmax > BT_NMAX || (size_t)(nmax + 96) * BT_PP * sizeof(T) > 220 * 1024) {
+    if (nmax > BT_NMAX || (size_t)(nmax + 96) * 36 * sizeof(T) > 220 * 1024) {
         ctx->set_error("batched problems of order %d exceed the limit", nmax);
         return DPLASMA_ERR_INTERNAL_LIMIT;
     }
@@ -491,18 +564,13 @@ int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *c
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hn[x] > hn[y]; });
     int *dord = (int *)ctx->buffer(BUF_BATCH, ((size_t)batch + 64) * sizeof(int));
     if (!dord) return DPLASMA_ERR_OUT_OF_RESOURCES;
-    int *ticket = dord + batch + 32;
     CK(cudaMemcpyAsync(dord, order.data(), batch * sizeof(int), cudaMemcpyHostToDevice, st));
 
     if (nrhs > BT_MAXRHS) {
         ctx->set_error("batched solve takes at most %d right-hand sides (got %d)", BT_MAXRHS, nrhs);
         return DPLASMA_ERR_NOT_SUPPORTED;
     }
-    // per-CTA inverses of the diagonal blocks (at most 4 CTAs per SM)
-    T *dscr = (T *)ctx->buffer(BUF_BATCH_SCR, (size_t)ctx->sms * 4 * (BT_NMAX / BT_NB) * 32 * 32 * sizeof(T));
-    if (!dscr) return DPLASMA_ERR_OUT_OF_RESOURCES;
     BatchArgs<T> a;
-    a.dscr = dscr;
     a.batch = batch;
     a.n = d_n;
     a.lda = d_lda;
@@ -512,107 +580,19 @@ int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *c
     a.logdet = d_logdet;
     a.info = d_info;
     a.order = dord;
-    a.ticket = ticket;
-
+    a.ticket = dord + batch + 32;
     int nv = 0;
     const BtVariant<T> *vars = bt_variants<T>(nv);
-    const int cls = bt_class(nmax);
-    int &choice = ctx->bt_choice[sizeof(T) == 8 ? 0 : 1][cls];
-    if (tune || choice < 0) {
-        // autotune on a scratch copy of the batch: the variants run on the
-        // same problems, the inputs are restored from the copy in between
-        std::vector<int> hlda(batch);
-        std::vector<T *> hA(batch);
-        CK(cudaMemcpyAsync(hlda.data(), d_lda, batch * sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hA.data(), d_A, batch * sizeof(T *), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        size_t tot = 0;
-        std::vector<size_t> off(batch);
-        for (int i = 0; i < batch; ++i) {
-            off[i] = tot;
-            tot += (size_t)hlda[i] * hn[i];
-        }
-        T *save = (T *)ctx->buffer(BUF_BATCH_SAVE, std::max<size_t>(tot, 1) * sizeof(T));
-        if (!save) return DPLASMA_ERR_OUT_OF_RESOURCES;
-        for (int i = 0; i < batch; ++i)
-            if (hn[i] > 0)
-                CK(cudaMemcpyAsync(save + off[i], hA[i], (size_t)hlda[i] * hn[i] * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        BatchArgs<T> ta = a;
-        ta.B = nullptr;
-        float best = 1e30f;
-        int bestv = 0;
-        for (int v = 0; v < nv; ++v) {
-            for (int rep = 0; rep < 2; ++rep) {
-                for (int i = 0; i < batch; ++i)
-                    if (hn[i] > 0)
-                        CK(cudaMemcpyAsync(hA[i], save + off[i], (size_t)hlda[i] * hn[i] * sizeof(T),
-                                           cudaMemcpyDeviceToDevice, st));
-                CK(cudaMemsetAsync(ticket, 0, sizeof(int), st));
-                int rc = vars[v].fn(ctx, ta, nmax, st, true);
-                if (rc) return rc;
-                CK(cudaEventRecord(ctx->ev2, st));
-                rc = vars[v].fn(ctx, ta, nmax, st, false);
-                CK(cudaEventRecord(ctx->ev3, st));
-                CK(cudaEventSynchronize(ctx->ev3));
-                if (rc) break;
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, ctx->ev2, ctx->ev3);
-                if (rep == 1 && ms < best) {
-                    best = ms;
-                    bestv = v;
-                }
-            }
-        }
-        for (int i = 0; i < batch; ++i)
-            if (hn[i] > 0)
-                CK(cudaMemcpyAsync(hA[i], save + off[i], (size_t)hlda[i] * hn[i] * sizeof(T), cudaMemcpyDeviceToDevice, st));
-        choice = bestv;
-    }
-    ctx->bt_last_variant = choice;
-    // the launch itself: counter reset + kernel, replayed from a CUDA graph
-    // that is recorded once per argument set
-    BatchGraph &gr = ctx->bt_graph[sizeof(T) == 8 ? 0 : 1];
-    const bool same = gr.exec && gr.batch == batch && gr.n == (const void *)d_n && gr.lda == (const void *)d_lda &&
-                      gr.A == (const void *)d_A && gr.B == (const void *)d_B && gr.nrhs == nrhs &&
-                      gr.logdet == (const void *)d_logdet && gr.info == (const void *)d_info && gr.variant == choice &&
-                      gr.nmax == nmax && gr.order == dord;
-    if (!same) {
-        if (gr.exec) cudaGraphExecDestroy(gr.exec);
-        gr.exec = nullptr;
-        int rc = vars[choice].fn(ctx, a, nmax, st, true);
-        if (rc) return rc;
-        cudaGraph_t graph = nullptr;
-        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        if (cudaMemsetAsync(ticket, 0, sizeof(int), st) != cudaSuccess) rc = DPLASMA_ERR_UNEXPECTED;
-        if (!rc) rc = vars[choice].fn(ctx, a, nmax, st, false);
-        const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-        if (rc) {
-            if (graph) cudaGraphDestroy(graph);
-            return rc;
-        }
-        CK(ce);
-        CK(cudaGraphInstantiate(&gr.exec, graph, 0));
-        cudaGraphDestroy(graph);
-        gr.batch = batch;
-        gr.n = d_n;
-        gr.lda = d_lda;
-        gr.A = d_A;
-        gr.B = d_B;
-        gr.nrhs = nrhs;
-        gr.logdet = d_logdet;
-        gr.info = d_info;
-        gr.variant = choice;
-        gr.nmax = nmax;
-        gr.order = dord;
-    }
+    const int choice = bt_choose(sizeof(T) == 8, batch, nmax, ctx->sms);
     CK(cudaEventRecord(ctx->ev0, st));
-    CK(cudaGraphLaunch(gr.exec, st));
+    const int rc = vars[choice].fn(ctx, a, nmax);
+    if (rc) return rc;
+    ctx->bt_last_variant = choice;
     CK(cudaEventRecord(ctx->ev1, st));
     CK(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     ctx->last_factor_ms = ms;
-    ctx->launches++;
     return 0;
 }
 
@@ -677,6 +657,12 @@ struct BatchInvArgs {
     int *ticket;
     double *scr;      // per CTA: padded factor and W, each nmax32^2
     int nmax32;
+    // GP gradient (null: the inverse goes to A's lower triangle): the factor
+    // stays, out_i (both triangles, leading dimension lda_i) = g_i / 2 (alpha_i
+    // alpha_i^T - K_i^-1)
+    const double *const *alpha;
+    const double *g;
+    double *const *out;
 };
 
 __global__ void __launch_bounds__(256) batched_potri_kernel(BatchInvArgs a)
@@ -803,7 +789,13 @@ __global__ void __launch_bounds__(256) batched_potri_kernel(BatchInvArgs a)
             __syncthreads();
         }
         if (info == 0) {
-            // A^-1 = W^T W, lower tiles (i >= j), into A
+            // A^-1 = W^T W, lower tiles (i >= j), into A, or straight into the
+            // likelihood's gradient: the tile and its mirror, from registers
+            // (the inverse, its symmetric copy and the rank-1 term as whole-batch
+            // passes took 2.8 ms of the 1024-problem gradient's 4.7)
+            const double *al = a.alpha ? a.alpha[pi] : nullptr;
+            const double hg = a.alpha ? 0.5 * a.g[pi] : 0.0;
+            double *O = a.alpha ? a.out[pi] : nullptr;
             const int ntile = nb * (nb + 1) / 2;
             for (int it = warp; it < ntile; it += 8) {
                 int bi = (int)((sqrtf(8.0f * it + 1.0f) - 1.0f) * 0.5f);
@@ -828,7 +820,15 @@ __global__ void __launch_bounds__(256) batched_potri_kernel(BatchInvArgs a)
                         for (int q = 0; q < 4; ++q) {
                             const int r = 32 * bi + mi * 16 + g + ((q & 2) ? 8 : 0);
                             const int c = 32 * bj + ni * 8 + 2 * t + (q & 1);
-                            if (r < n && c < n && r >= c) A[(int64_t)c * lda + r] = acc[mi][ni][q];
+                            if (O) {
+                                if (r < n && c < n) {
+                                    const double v = hg * (__ldg(al + r) * __ldg(al + c) - acc[mi][ni][q]);
+                                    O[(int64_t)c * lda + r] = v;
+                                    if (bi != bj) O[(int64_t)r * lda + c] = v;
+                                }
+                            } else if (r < n && c < n && r >= c) {
+                                A[(int64_t)c * lda + r] = acc[mi][ni][q];
+                            }
                         }
             }
         }
@@ -837,7 +837,8 @@ __global__ void __launch_bounds__(256) batched_potri_kernel(BatchInvArgs a)
     }
 }
 
-int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, double *const *d_A, int *d_info)
+int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, double *const *d_A, int *d_info,
+                  const double *const *d_alpha, const double *d_g, double *const *d_out)
 {
     if (batch <= 0) return 0;
     cudaStream_t st = ctx->stream;
@@ -873,6 +874,9 @@ int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, dou
     a.ticket = ticket;
     a.scr = scr;
     a.nmax32 = nmax32;
+    a.alpha = d_alpha;
+    a.g = d_g;
+    a.out = d_out;
     CK(cudaEventRecord(ctx->ev0, st));
     batched_potri_kernel<<<grid, 256, smem, st>>>(a);
     CK(cudaGetLastError());
@@ -886,8 +890,8 @@ int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, dou
 }
 
 template int batched_posv<double>(Context *, int, const int *, const int *, double *const *, double *const *, int,
-                                  double *, int *, int);
+                                  double *, int *);
 template int batched_posv<float>(Context *, int, const int *, const int *, float *const *, float *const *, int,
-                                 double *, int *, int);
+                                 double *, int *);
 
 }  // namespace db2

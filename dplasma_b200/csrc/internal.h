@@ -35,7 +35,6 @@ enum BufferId : int {
     BUF_KRYLOV,       // GMRES basis
     BUF_PTRACE,       // per-POTRF phase times (opt-in trace)
     BUF_BATCH,        // batched: work order and queue counter
-    BUF_BATCH_SAVE,   // batched: copy of the inputs while autotuning
     BUF_ADJ,          // adjoint: dense L, W = L^-1 and two products
     BUF_BATCH_SCR,    // batched: per-CTA inverses of the diagonal blocks
     BUF_BATCH_W,      // batched inverse: per-CTA padded factor and L^-1
@@ -47,14 +46,6 @@ enum BufferId : int {
     BUF_ARRIVED,      // streamed factorization: per-phase arrival flags
     BUF_WM,           // triangular sweeps: the critical path's products W_b L_{b,b-1}
     BUF_COUNT
-};
-
-// A recorded launch of the batched kernel and the arguments it was made for.
-struct BatchGraph {
-    cudaGraphExec_t exec = nullptr;
-    int batch = 0, nrhs = 0, variant = -1, nmax = 0;
-    const void *n = nullptr, *lda = nullptr, *A = nullptr, *B = nullptr, *logdet = nullptr, *info = nullptr,
-               *order = nullptr;
 };
 
 struct Context {
@@ -91,9 +82,7 @@ struct Context {
     long long last_tasks_executed = 0;
     long long last_tickets = 0, last_tickets_bad = 0;   // self check of the last factorization
     int inject_kind = 0, inject_arg = -1;                // one-shot fault injection of the next factorization
-    int bt_choice[2][8] = {{-1, -1, -1, -1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1, -1, -1, -1}};   // autotuned variant
     int bt_last_variant = -1;
-    BatchGraph bt_graph[2];                  // FP64, FP32
     char errmsg[512] = {0};
     char trace_path[512] = {0};   // DPLASMA_B200_TRACE: per-task timestamps of the scheduler
     char wave_trace_path[512] = {0};   // DPLASMA_B200_WAVE_TRACE: per-sweep summary of the triangular sweeps
@@ -205,9 +194,11 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
 // batched.cu
 template <typename T>
 int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *const *d_A, T *const *d_B, int nrhs,
-                 double *d_logdet, int *d_info, int tune);
+                 double *d_logdet, int *d_info);
 const char *batched_variant_name(int fp64, int v);
-int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, double *const *d_A, int *d_info);
+// d_alpha (may be null), d_g, d_out: the GP gradient instead of the inverse
+int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, double *const *d_A, int *d_info,
+                  const double *const *d_alpha = nullptr, const double *d_g = nullptr, double *const *d_out = nullptr);
 
 // norms.cu
 int lansy_inf_device(Context *ctx, const double *dA, const Geom &g, double *out);

@@ -380,15 +380,14 @@ int dplasma_dpotrf_adjoint(parsec_context_t *parsec, dplasma_enum_t uplo, const 
 /* dplasma_b200_dposv_batched / _sposv_batched: no dplasma counterpart.  Factor
  * (Cholesky, lower), solve and log-determinant of `batch` independent SPD
  * systems A_i X_i = B_i of orders n[i] (0 <= n[i] <= 512 in FP64, 1024 in
- * FP32), in one persistent launch replayed from a CUDA graph.  Every array
+ * FP32), in one persistent launch.  Every array
  * argument is DEVICE memory: n, lda (int[batch]); A (pointers to the
  * column-major n[i] x n[i] matrices, lower triangle read, overwritten by
  * L_i); B (pointers to the n[i] x nrhs right-hand sides, leading dimension
  * n[i], overwritten by X_i; B itself or B[i] may be NULL to factor only);
  * logdet (double[batch], 2 sum log L_i(j,j); NaN when INFO > 0; may be
- * NULL); info (int[batch], LAPACK INFO of each problem).  The first call for
- * a size class (largest n up to the next power of two) times the kernel
- * variants on the caller's batch and keeps the fastest.  Returns 0 or a
+ * NULL); info (int[batch], LAPACK INFO of each problem).  The warps per
+ * problem follow from the largest order and the batch.  Returns 0 or a
  * negative code. */
 int dplasma_b200_dposv_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
                                double *const *A, double *const *B, int nrhs, double *logdet, int *info);
@@ -400,7 +399,15 @@ int dplasma_b200_sposv_batched(parsec_context_t *parsec, int batch, const int *n
  * dplasma_dpotri.  All arrays in device memory; one persistent launch. */
 int dplasma_b200_dpotri_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
                                 double *const *A, int *info);
-/* Name of the kernel variant the last batched call used (autotuner choice). */
+/* The gradients dK_i = g_i / 2 (alpha_i alpha_i^T - K_i^-1) of g_i times the
+ * Gaussian-process log marginal likelihoods of a batch, from the factors L_i as
+ * dposv_batched leaves them (column-major lower, leading dimension lda_i; not
+ * changed) and alpha_i = K_i^-1 y_i: n_i x n_i, both triangles, leading
+ * dimension lda_i, not overlapping L_i.  Arrays and INFO as above. */
+int dplasma_b200_gp_gradient_batched(parsec_context_t *ctx, int batch, const int *n, const int *lda,
+                                     const double *const *L, const double *const *alpha, const double *g,
+                                     double *const *dK, int *info);
+/* Name of the kernel variant the last batched call used. */
 const char *dplasma_b200_batched_variant(const parsec_context_t *parsec);
 
 /* ---- ScaLAPACK-compatible entry ------------------------------------------ */

@@ -1,0 +1,176 @@
+"""GPU tests of the launch shapes that follow from sizes: the block order and
+the shared-memory POTRF of the FP64 factorization at block and 32-column
+edges, re-tiled caller layouts, the one-block-per-CTA sweeps and their column
+groups, the batched kernel's warps per problem, and the Gaussian-process
+gradients.  Each is compared with numpy / torch in 64 bits; tolerances are
+the reference's residual ratio (< 10 in units of N eps) or stated beside."""
+import numpy as np
+import pytest
+
+import dplasma_b200 as db
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+
+
+def spd(n, seed, scale=1.0):
+    g = np.random.default_rng(seed)
+    a = g.uniform(-0.5, 0.5, (n, n))
+    a = np.tril(a) + np.tril(a, -1).T
+    a[np.diag_indices(n)] += n
+    return np.asfortranarray(a * scale)
+
+
+def dev_desc(dense, nb, uplo, lapack=False):
+    n = dense.shape[0]
+    d = db.desc_general(n, n, nb, nb, storage=db.STORAGE_LAPACK, lda=n) if lapack else db.desc_sym(n, nb, uplo)
+    buf = torch.from_numpy(db.pack(dense, d)).cuda()
+    torch.cuda.synchronize()
+    return db.attach(d, buf), buf
+
+
+def factor_ratio(L, A):
+    return np.abs(L @ L.T - A).sum(1).max() / (np.abs(A).sum(1).max() * A.shape[0] * EPS)
+
+
+@pytest.mark.parametrize("n,nb,uplo,lapack", [
+    (1, 1, "L", False), (31, 32, "L", False), (33, 128, "U", True), (127, 128, "L", True), (129, 93, "U", False),
+    (256, 200, "L", False),            # as many tiles of 128 as of 200: still two layouts
+    (257, 256, "L", True), (640, 128, "L", False), (1000, 320, "U", True), (1536, 512, "L", False),
+    (6400, 128, "L", False)])          # 50 blocks: six panels per update task
+def test_factor_shapes(gpu_ctx, n, nb, uplo, lapack):
+    A = spd(n, n)
+    up = db.Lower if uplo == "L" else db.Upper
+    d, buf = dev_desc(A, nb, up, lapack)
+    before = db.unpack(buf.cpu().numpy(), d)
+    assert gpu_ctx.dpotrf(up, d) == 0, gpu_ctx.last_error()
+    out = db.unpack(buf.cpu().numpy(), d)
+    L = np.tril(out) if uplo == "L" else np.triu(out).T
+    assert factor_ratio(L, A) < 10.0
+    # the other triangle of what is stored is not touched
+    other = np.triu if uplo == "L" else np.tril
+    assert np.array_equal(other(out, 1 if uplo == "L" else -1), other(before, 1 if uplo == "L" else -1))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -990, 2.0 ** 990])
+def test_factor_pivots_outside_the_fast_range(gpu_ctx, scale):
+    # powers of two: the factor is the scaled factor, to a last place of the
+    # root (both roots of a pivot are correct to that)
+    n = 300
+    A = spd(n, 7)
+    d, buf = dev_desc(A * scale, 256, db.Lower, True)
+    assert gpu_ctx.dpotrf(db.Lower, d) == 0, gpu_ctx.last_error()
+    L = np.tril(db.unpack(buf.cpu().numpy(), d)) / np.sqrt(scale)
+    assert factor_ratio(L, A) < 10.0
+
+
+@pytest.mark.parametrize("n,bad", [(300, 0), (300, 31), (300, 32), (300, 127), (300, 128), (300, 299), (1000, 700)])
+@pytest.mark.parametrize("value", [-1.0, 0.0, np.nan])
+def test_info_at_block_edges(gpu_ctx, n, bad, value):
+    A = spd(n, n)
+    A[bad, bad] = value if bad == 0 else A[bad, bad] * 0 + value
+    if bad > 0:
+        A[bad, :bad] = A[:bad, bad] = 0.0          # the pivot is A(bad, bad) itself
+    d, buf = dev_desc(A, 96, db.Lower, True)
+    assert gpu_ctx.dpotrf(db.Lower, d) == bad + 1
+
+
+@pytest.mark.parametrize("n,nrhs", [(100, 1), (200, 9), (300, 33), (385, 16), (512, 64), (700, 40), (2000, 24)])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+def test_sweep_shapes(gpu_ctx, n, nrhs, uplo):
+    g = np.random.default_rng(n + nrhs)
+    up = db.Lower if uplo == "L" else db.Upper
+    A = spd(n, n)
+    d, buf = dev_desc(A, 256, up, True)
+    B = g.uniform(-0.5, 0.5, (n, nrhs))
+    bB = torch.from_numpy(np.ascontiguousarray(B.T).reshape(-1)).cuda()
+    torch.cuda.synchronize()
+    dB = db.attach(db.desc_general(n, nrhs, 256, 256, storage=db.STORAGE_LAPACK, lda=n), bB)
+    assert gpu_ctx.dposv(up, d, dB) == 0, gpu_ctx.last_error()
+    X = bB.cpu().numpy().reshape(nrhs, n).T
+    r = np.abs(A @ X - B).sum(1).max()
+    assert r / ((np.abs(A).sum(1).max() * np.abs(X).sum(1).max() + np.abs(B).sum(1).max()) * n * EPS) < 10.0
+
+
+def test_sweep_passes_nans_on(gpu_ctx):
+    # every NaN payload travels through the sweep's exchange buffer, the one
+    # that marks an empty word included
+    n, nrhs = 700, 3
+    A = spd(n, 1)
+    d, buf = dev_desc(A, 256, db.Lower, True)
+    B = np.zeros((nrhs, n))
+    B[0, 5] = np.nan
+    B.view(np.uint64)[1, 300] = 0xFFFFFFFFFFFFFFFF
+    bB = torch.from_numpy(B.reshape(-1)).cuda()
+    torch.cuda.synchronize()
+    dB = db.attach(db.desc_general(n, nrhs, 256, 256, storage=db.STORAGE_LAPACK, lda=n), bB)
+    assert gpu_ctx.dposv(db.Lower, d, dB) == 0, gpu_ctx.last_error()
+    X = bB.cpu().numpy().reshape(nrhs, n)
+    assert np.isnan(X[0]).all() and np.isnan(X[1]).all() and (X[2] == 0).all()
+
+
+@pytest.mark.parametrize("count,lo,hi,dtype,nrhs", [
+    (700, 1, 96, "f64", 1), (700, 90, 96, "f32", 3), (600, 97, 256, "f64", 2), (600, 97, 256, "f32", 16),
+    (320, 257, 300, "f64", 1), (320, 257, 300, "f32", 1), (3, 500, 512, "f64", 1), (3, 1000, 1024, "f32", 1),
+    (40, 1, 70, "f64", 4)])
+def test_batched_shapes(gpu_ctx, count, lo, hi, dtype, nrhs):
+    # kernels with nugget 1: condition <= n + 1, so solutions agree to about n eps times that
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator().manual_seed(count + hi)
+    sizes = torch.randint(lo, hi + 1, (count,), generator=g).tolist()
+    sizes[0], sizes[-1] = hi, lo
+    Ks, ys = [], []
+    for n in sizes:
+        x = torch.rand(n, 3, generator=g, dtype=torch.float64)
+        Ks.append((torch.exp(-12.5 * torch.cdist(x, x) ** 2) + torch.eye(n, dtype=torch.float64)).to(dt).double())
+        ys.append(torch.randn(nrhs, n, generator=g, dtype=torch.float64).to(dt).double())
+    mats = [K.to(dt).cuda() for K in Ks]
+    rhs = [y.to(dt).cuda() for y in ys]
+    info, logdet = gpu_ctx.posv_batched(mats, rhs)
+    assert (info == 0).all()
+    u = EPS if dtype == "f64" else 2.0 ** -24
+    for n, K, y, m, r, ld in zip(sizes, Ks, ys, mats, rhs, logdet):
+        L = torch.linalg.cholesky(K)
+        F = torch.triu(m.double().cpu()).t()
+        assert (F - L).norm() <= 10 * n * u * L.norm()
+        X = torch.cholesky_solve(y.t(), L).t()
+        assert (r.double().cpu() - X).norm() <= 10 * n * (n + 1) * u * X.norm()
+        assert abs(ld - 2 * torch.log(torch.diagonal(L)).sum()) <= 10 * n * n * u
+
+
+@pytest.mark.parametrize("n,scale", [(70, 2.0 ** -990), (300, 2.0 ** 990)])
+def test_batched_pivots_outside_the_fast_range(gpu_ctx, n, scale):
+    A = spd(n, 3)
+    m = torch.from_numpy(np.ascontiguousarray(A * scale)).cuda()
+    info, _ = gpu_ctx.posv_batched([m])
+    assert int(info[0]) == 0
+    assert factor_ratio(np.triu(m.cpu().numpy()).T / np.sqrt(scale), A) < 10.0
+
+
+def test_gp_gradients_differentiate_and_batch_over_the_outer_gradient():
+    # the gradients are linear in the incoming one for whoever differentiates
+    # (create_graph) or batches it (is_grads_batched) as for the plain kernel call
+    from dplasma_b200 import autograd as dag
+    g = torch.Generator().manual_seed(5)
+    Ks, ys = [], []
+    for n in (65, 40):
+        x = torch.rand(n, 3, generator=g, dtype=torch.float64)
+        Ks.append((torch.exp(-12.5 * torch.cdist(x, x) ** 2) + torch.eye(n, dtype=torch.float64)).cuda())
+        ys.append(torch.randn(n, generator=g, dtype=torch.float64).cuda())
+    flat = torch.cat([K.reshape(-1) for K in Ks])
+    cases = [(lambda K: dag.gp_log_marginal_likelihood(K, ys[0]), Ks[0]),
+             (lambda K: dag.gp_log_marginal_likelihood_flat(K, torch.cat(ys), (65, 40)), flat)]
+    for f, K in cases:
+        K = K.clone().requires_grad_(True)
+        v = f(K)
+        w = torch.full_like(v, 2.0).requires_grad_(True)
+        (dK,) = torch.autograd.grad(v, K, w, create_graph=True)
+        (one,) = torch.autograd.grad(f(K), K, torch.ones_like(v))
+        assert torch.allclose(dK, 2.0 * one, rtol=1e-12, atol=1e-12)
+        (dw,) = torch.autograd.grad(dK.sum(), w)
+        assert torch.allclose(dw.sum(), one.sum(), rtol=1e-9)
+        ws = torch.stack([torch.ones_like(v), torch.full_like(v, 3.0)])
+        (both,) = torch.autograd.grad(f(K), K, ws, is_grads_batched=True)
+        assert torch.allclose(both, torch.stack([one, 3.0 * one]), rtol=1e-12, atol=1e-12)
