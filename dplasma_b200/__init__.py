@@ -74,7 +74,7 @@ EXPORTS = (
     "dplasma_b200_sposv_batched", "dplasma_b200_batched_variant", "dplasma_dpotrf_adjoint",
     "dplasma_dtrtri", "dplasma_dlauum", "dplasma_dpotri", "dplasma_dpoinv", "dplasma_dpoinv_sync",
     "dplasma_b200_dpotri_batched", "dplasma_b200_gp_gradient_batched",
-    "pdpotrf_", "dplasma_b200_dpotrf_noalloc", "dplasma_b200_inject_fault",
+    "dplasma_b200_gp_gradient", "pdpotrf_", "dplasma_b200_dpotrf_noalloc", "dplasma_b200_inject_fault",
     "dplasma_b200_set_wait_limits", "dplasma_b200_set_selfcheck", "dplasma_b200_selfcheck", "dplasma_dlange",
     "dplasma_dsymm", "dplasma_b200_dtd_new", "dplasma_b200_dtd_insert", "dplasma_b200_dtd_panel_received",
     "dplasma_b200_dtd_flush", "dplasma_b200_dtd_data_flush_all", "dplasma_b200_dtd_tiles",
@@ -132,6 +132,7 @@ def lib():
     for f in ("dplasma_dlauum", "dplasma_dpotri", "dplasma_dpoinv", "dplasma_dpoinv_sync"):
         getattr(L, f).argtypes = [P, I, pd]
     L.dplasma_b200_dpotri_batched.argtypes = [P, I, P, P, P, P]
+    L.dplasma_b200_gp_gradient.argtypes = [P, pd, I, P, P, P]
     L.dplasma_b200_gp_gradient_batched.argtypes = [P, I, P, P, P, P, P, P, P]
     pi = ctypes.POINTER(I)
     L.pdpotrf_.restype = None

@@ -18,7 +18,7 @@
   (``dplasma_dpotrf`` + ``dplasma_dpotrs``), backward
   ``dK = 1/2 alpha alpha^T - 1/2 K^-1`` with ``K^-1`` -- the Cholesky adjoint
   of the log-determinant (``Lbar = diag(2 / L(i,i))``) -- formed from the
-  factor by ``dplasma_dpotri``, and ``dy = -alpha``.  Gradients with respect to
+  factor by ``dplasma_b200_gp_gradient``, and ``dy = -alpha``.  Gradients with respect to
   parameters of K (a lengthscale, ...) follow by torch's own chain rule.
 
 Matrices cross the C ABI as LAPACK-storage device descriptors: a row-major
@@ -28,6 +28,7 @@ row-major buffer.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -96,17 +97,22 @@ def _plain(g: torch.Tensor) -> bool:
     return True
 
 
-def _inverse_from_factor(Lrow: torch.Tensor) -> torch.Tensor:
-    """K^-1 (symmetric, row-major) from the lower factor L of K."""
-    n = Lrow.shape[0]
-    ctx = context(Lrow.device)
-    buf = Lrow.t().contiguous()              # column-major L
-    torch_ready(buf)
-    rc = ctx.dpotri(Lower, _lapack_desc(buf, n))
+def _gp_gradient(buf: torch.Tensor, rhs: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    """g / 2 (alpha alpha^T - m K^-1) from the factor as _factor leaves it and
+    alpha^T (m x n)."""
+    if not _plain(g):
+        return g * _gp_gradient(buf, rhs, torch.ones((), dtype=buf.dtype, device=buf.device))
+    n = buf.shape[0]
+    ctx = context(buf.device)
+    dK = torch.empty_like(buf)
+    g = g.contiguous()
+    torch_ready(buf, rhs, g, dK)
+    d = _lapack_desc(buf, n)
+    rc = lib().dplasma_b200_gp_gradient(ctx.h, ctypes.byref(d), rhs.shape[0], rhs.data_ptr(), g.data_ptr(),
+                                        dK.data_ptr())
     if rc != 0:
-        raise RuntimeError(f"dplasma_dpotri: {rc} {ctx.last_error()}")
-    up = torch.triu(buf)                     # column-major lower part = row-major upper
-    return up + torch.triu(buf, 1).t()
+        raise RuntimeError(f"dplasma_b200_gp_gradient: {rc} {ctx.last_error()}")
+    return dK
 
 
 class _Cholesky(torch.autograd.Function):
@@ -134,8 +140,7 @@ class _GPLogML(torch.autograd.Function):
         _check_square(K)
         n = K.shape[0]
         Y = y.reshape(n, -1) if y.dim() == 1 else y
-        buf = _factor(K)
-        L = torch.tril(buf.t())
+        buf = _factor(K)                         # column-major lower factor
         ctx = context(K.device)
         # alpha = K^-1 y by dplasma_dpotrs on the factor (column-major rhs)
         # m x n row-major = n x m column-major; a copy (for one column the
@@ -146,20 +151,19 @@ class _GPLogML(torch.autograd.Function):
         if rc != 0:
             raise RuntimeError(f"dplasma_dpotrs: {rc} {ctx.last_error()}")
         alpha = rhs.t()
-        logdet = 2.0 * torch.log(torch.diagonal(L)).sum()
+        logdet = 2.0 * torch.log(torch.diagonal(buf)).sum()
         m = Y.shape[1]
         val = -0.5 * (Y * alpha).sum() - 0.5 * m * logdet - 0.5 * m * n * math.log(2 * math.pi)
-        ctx_.save_for_backward(L, alpha)
+        ctx_.save_for_backward(buf, rhs)
         ctx_.ydim = y.dim()
         return val
 
     @staticmethod
     def backward(ctx_, g):
-        L, alpha = ctx_.saved_tensors
-        m = alpha.shape[1]
-        # K^-1, the adjoint of log det K through the factor, by dplasma_dpotri
-        Kinv = _inverse_from_factor(L)
-        dK = g * (0.5 * alpha @ alpha.t() - 0.5 * m * Kinv)
+        buf, rhs = ctx_.saved_tensors
+        # K^-1 (the adjoint of log det K through the factor) and the rank-m term
+        dK = _gp_gradient(buf, rhs, g)
+        alpha = rhs.t()
         dy = -g * alpha
         if ctx_.ydim == 1:
             dy = dy.reshape(-1)

@@ -42,6 +42,7 @@ constexpr int AG_P = 132;     // shared pitch
 //   LOWER_KGE_I   tiles i >= j                 k in [i, P-1]
 //   LOWER_JKI     tiles i >= j                 k in [j, i]
 //   SYM_KGE_I     tiles i >= j                 k in [i, P-1], A^T B + B^T A
+//   GRAD          as LOWER_KGE_I, its result straight into a GP gradient
 //   LVL_T, LVL_W  one level of the recursive triangular inverse: for every
 //                 diagonal block [o, o+2h) of 2h tiles, with W11 = the inverse
 //                 of its first half and W22 of its second (previous level),
@@ -50,7 +51,7 @@ constexpr int AG_P = 132;     // shared pitch
 //                 (h = rowblk; the last block's second half may be short)
 // Blocks run in order, so every mode starts with its longest K ranges: the last
 // wave is then made of short ones (N = 4096: JKI 1224 us in row order).
-enum : int { AG_LOWER_KGE_I = 1, AG_LOWER_JKI = 2, AG_SYM_KGE_I = 3, AG_LVL_T = 5, AG_LVL_W = 6 };
+enum : int { AG_LOWER_KGE_I = 1, AG_LOWER_JKI = 2, AG_SYM_KGE_I = 3, AG_GRAD = 4, AG_LVL_T = 5, AG_LVL_W = 6 };
 
 struct AgArgs {
     int mode, P, rowblk, nblk;
@@ -61,6 +62,10 @@ struct AgArgs {
     double *C;
     int ldc;
     double alpha, beta;
+    // GRAD: out (n x n, both triangles, ld n) = g / 2 (al al^T - nal * product)
+    const double *al, *g;
+    int nal, n;
+    double *out;
 };
 
 // C(i,j) = alpha * sum_{k in range} op(A)(i,k) B(k,j) + beta * C(i,j), 128x128 tiles
@@ -200,6 +205,26 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             buf ^= 1;
         }
     }
+    if (a.mode == AG_GRAD) {
+        // the tile and its mirror from registers: the inverse, its symmetric copy
+        // and the rank-m term as passes of their own took 1.1 ms of 14 at n = 6001
+        const double hg = 0.5 * *a.g;
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = i * AG_T + wm * 64 + mi * 16 + g + ((q & 2) ? 8 : 0);
+                    const int c = j * AG_T + wn * 32 + ni * 8 + 2 * t + (q & 1);
+                    if (r >= a.n || c >= a.n) continue;
+                    double s = -(double)a.nal * acc[mi][ni][q];
+                    for (int l = 0; l < a.nal; ++l) s = fma(__ldg(a.al + (int64_t)l * a.n + r), __ldg(a.al + (int64_t)l * a.n + c), s);
+                    a.out[(int64_t)c * a.n + r] = hg * s;
+                    if (i != j) a.out[(int64_t)r * a.n + c] = hg * s;
+                }
+        return;
+    }
     // epilogue: loads first, then stores
     double *C = a.C + (int64_t)(j * AG_T) * a.ldc + i * AG_T;
     double old[4][4][4];
@@ -225,10 +250,20 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             }
 }
 
+struct AgGrad {
+    const double *al, *g;
+    int nal, n;
+    double *out;
+};
 static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, int lda, int transA, const double *B,
-                   int ldb, double *C, int ldc, double alpha, double beta)
+                   int ldb, double *C, int ldc, double alpha, double beta, const AgGrad *gr = nullptr)
 {
     AgArgs a;
+    a.al = gr ? gr->al : nullptr;
+    a.g = gr ? gr->g : nullptr;
+    a.nal = gr ? gr->nal : 0;
+    a.n = gr ? gr->n : 0;
+    a.out = gr ? gr->out : nullptr;
     a.mode = mode;
     a.P = P;
     a.rowblk = rowblk;
@@ -381,7 +416,8 @@ __global__ void ag_zero_pivot(const double *L, int ld, int n_valid_rows, const i
 
 // op: 0 trtri (L -> L^-1), 1 lauum (L -> L^T L), 2 potri (L -> (L L^T)^-1);
 // nb/nbi/n describe which padded rows are real (for the INFO of trtri).
-int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int *info)
+// gr (op 2, may be null): the GP gradient is written instead of Lt (whole tiles: nb == nbi).
+static int inverse_or_gradient(Context *ctx, double *Lt, const Geom &g, int op, int unit, int *info, const AgGrad *gr)
 {
     const int Np = g.mt * g.nbi, P = Np / AG_T, ld = Np;
     const size_t nn = (size_t)Np * Np;
@@ -424,6 +460,11 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
         if ((rc = ag_inverse(ctx, L, W, Y, scr, P, ld, unit))) return rc;
         src = W;
     }
+    if (gr) {
+        if ((rc = ag_gemm(ctx, AG_GRAD, P, 0, W, ld, 1, W, ld, Y, ld, 1.0, 0.0, gr))) return rc;
+        CK(cudaStreamSynchronize(st));
+        return 0;
+    }
     double *out = W;
     if (op != 0) {
         // src^T src, lower tiles only (k >= i >= j): the result is symmetric
@@ -435,6 +476,18 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
     ctx->launches++;
     CK(cudaStreamSynchronize(st));
     return 0;
+}
+
+int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int *info)
+{
+    return inverse_or_gradient(ctx, Lt, g, op, unit, info, nullptr);
+}
+
+int gp_gradient_tiles(Context *ctx, double *Lt, const Geom &g, const double *al, int nal, const double *dg, double *out,
+                      int *info)
+{
+    const AgGrad gr = {al, dg, nal, g.n, out};
+    return inverse_or_gradient(ctx, Lt, g, 2, 0, info, &gr);
 }
 
 }  // namespace db2

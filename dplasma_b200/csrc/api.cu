@@ -982,3 +982,25 @@ extern "C" int dplasma_b200_gp_gradient_batched(parsec_context_t *parsec, int ba
     ctx->errmsg[0] = 0;
     return batched_potri(ctx, batch, n, lda, const_cast<double *const *>(L), info, alpha, g, dK);
 }
+
+extern "C" int dplasma_b200_gp_gradient(parsec_context_t *parsec, const parsec_tiled_matrix_t *L, int nrhs,
+                                        const double *alpha, const double *g, double *dK)
+{
+    if (!parsec) return DPLASMA_ERR_NOT_INITIALIZED;
+    int rc;
+    if ((rc = check_square("dplasma_b200_gp_gradient", L))) return rc;
+    if (nrhs < 0 || (L->m > 0 && (!alpha || !g || !dK))) return DPLASMA_ERR_ILLEGAL_VALUE;
+    Context *ctx = &parsec->impl;
+    cudaSetDevice(ctx->device);
+    ctx->launches = 0;
+    ctx->errmsg[0] = 0;
+    if (L->m == 0) return 0;
+    const Geom gc = make_geom(L->m, L->mb), ge = work_geom(L->m, L->mb);
+    if (gc.mt > 65535 || gc.nbi > 512) return DPLASMA_ERR_INTERNAL_LIMIT;
+    double *Lt = (double *)ctx->buffer(BUF_A, ge.elems() * sizeof(double));
+    if (!Lt) return DPLASMA_ERR_OUT_OF_RESOURCES;
+    if ((rc = upload_sym(ctx, L, dplasmaLower, ge, Lt))) return rc;
+    int info = 0;
+    if ((rc = gp_gradient_tiles(ctx, Lt, ge, alpha, nrhs, g, dK, &info))) return rc;
+    return info;
+}

@@ -190,6 +190,9 @@ int symm_tiles(Context *ctx, const double *dA, const Geom &g, const double *in, 
 int potrf_adjoint_tiles(Context *ctx, const double *Lt, double *Lbt, const Geom &g);
 // op 0 trtri, 1 lauum, 2 potri (device tiles, in place); *info as LAPACK dtrtri
 int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int *info);
+// out (n x n, device) = g / 2 (al al^T - nal (L L^T)^-1), al n x nal; *info as above
+int gp_gradient_tiles(Context *ctx, double *Lt, const Geom &g, const double *al, int nal, const double *dg, double *out,
+                      int *info);
 
 // batched.cu
 template <typename T>

@@ -399,6 +399,13 @@ int dplasma_b200_sposv_batched(parsec_context_t *parsec, int batch, const int *n
  * dplasma_dpotri.  All arrays in device memory; one persistent launch. */
 int dplasma_b200_dpotri_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
                                 double *const *A, int *info);
+/* The gradient dK = g / 2 (alpha alpha^T - nrhs K^-1) of g times the
+ * Gaussian-process log marginal likelihood, from the lower factor L of K (any
+ * descriptor, as dplasma_dpotri takes it) and alpha = K^-1 y (n x nrhs, leading
+ * dimension n): n x n, both triangles, leading dimension n.  alpha, g (one
+ * value) and dK in device memory.  Returns INFO > 0 for a zero diagonal entry. */
+int dplasma_b200_gp_gradient(parsec_context_t *ctx, const parsec_tiled_matrix_t *L, int nrhs, const double *alpha,
+                             const double *g, double *dK);
 /* The gradients dK_i = g_i / 2 (alpha_i alpha_i^T - K_i^-1) of g_i times the
  * Gaussian-process log marginal likelihoods of a batch, from the factors L_i as
  * dposv_batched leaves them (column-major lower, leading dimension lda_i; not

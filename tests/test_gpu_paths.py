@@ -4,6 +4,8 @@ edges, re-tiled caller layouts, the one-block-per-CTA sweeps and their column
 groups, the batched kernel's warps per problem, and the Gaussian-process
 gradients.  Each is compared with numpy / torch in 64 bits; tolerances are
 the reference's residual ratio (< 10 in units of N eps) or stated beside."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -149,6 +151,24 @@ def test_batched_pivots_outside_the_fast_range(gpu_ctx, n, scale):
     assert factor_ratio(np.triu(m.cpu().numpy()).T / np.sqrt(scale), A) < 10.0
 
 
+@pytest.mark.parametrize("n,m", [(1, 1), (127, 1), (129, 2), (700, 1), (1500, 3)])
+def test_gp_gradient(n, m):
+    from dplasma_b200 import autograd as dag
+    g = torch.Generator().manual_seed(n)
+    x = torch.rand(n, 3, generator=g, dtype=torch.float64)
+    K = torch.exp(-12.5 * torch.cdist(x, x) ** 2) + torch.eye(n, dtype=torch.float64)
+    y = torch.randn(n, m, generator=g, dtype=torch.float64)
+    Kd, yd = K.cuda().requires_grad_(True), y.cuda().requires_grad_(True)
+    v = dag.gp_log_marginal_likelihood(Kd, yd)
+    dK, dy = torch.autograd.grad(3.0 * v, (Kd, yd))
+    Ki = torch.linalg.inv(K)
+    al = Ki @ y
+    ref = 1.5 * (al @ al.t() - m * Ki)
+    tol = 100 * n * (n + 1) * EPS           # condition <= n + 1 (nugget 1)
+    assert (dK.cpu() - ref).norm() <= tol * ref.norm() and (dy.cpu() + 3.0 * al).norm() <= tol * al.norm() * 3
+    assert torch.equal(dK, dK.t())
+
+
 def test_gp_gradients_differentiate_and_batch_over_the_outer_gradient():
     # the gradients are linear in the incoming one for whoever differentiates
     # (create_graph) or batches it (is_grads_batched) as for the plain kernel call
@@ -174,3 +194,12 @@ def test_gp_gradients_differentiate_and_batch_over_the_outer_gradient():
         ws = torch.stack([torch.ones_like(v), torch.full_like(v, 3.0)])
         (both,) = torch.autograd.grad(f(K), K, ws, is_grads_batched=True)
         assert torch.allclose(both, torch.stack([one, 3.0 * one]), rtol=1e-12, atol=1e-12)
+
+
+def test_gp_gradient_refuses(gpu_ctx):
+    d = db.desc_general(8, 8, 256, 256, storage=db.STORAGE_LAPACK, lda=8)
+    buf = torch.eye(8, dtype=torch.float64, device="cuda")
+    db.attach(d, buf)
+    f = db.lib().dplasma_b200_gp_gradient
+    assert f(None, ctypes.byref(d), 1, None, None, None) == db.ERR_NOT_INITIALIZED
+    assert f(gpu_ctx.h, ctypes.byref(d), 1, None, None, None) == db.ERR_ILLEGAL_VALUE
