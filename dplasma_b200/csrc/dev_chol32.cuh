@@ -1,6 +1,6 @@
-// dev_chol32.cuh -- factorization and inverse of a 32x32 diagonal block by
-// one warp, in steps of four columns (FP64 for the tile Cholesky, FP64 or
-// FP32 for the batched solver).
+// dev_chol32.cuh -- factorization of a 32x32 diagonal block by one warp and
+// substitution with it (FP64 for the tile Cholesky, FP64 or FP32 for the batched
+// solver).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -133,57 +133,9 @@ __device__ __forceinline__ int chol32_blk(T (&d)[32], int lane, T &rdiag, T *Lb)
     return failcol;
 }
 
-// Inverse of the lower 32x32 block L (Lb, from chol32_blk) by one warp, lane
-// c forming column c by a forward sweep in steps of four rows, in the same
-// rotating frame (b[q] = row j + q of the right-hand side at step j):
-// x_j = b_j / L(j,j), then b_i -= L(i,j) x_j below, in the order of the
-// row-by-row sweep.  out(j, c, x) receives Dinv(j, c).
-template <typename T, class Out>
-__device__ __forceinline__ void inv32_blk(const T *Lb, int lane, T rdiag, Out out)
-{
-    T b[32];
-#pragma unroll
-    for (int q = 0; q < 32; ++q) b[q] = (q == lane) ? T(1) : T(0);
-#pragma unroll 1
-    for (int j = 0; j < 32; j += 4) {
-        const T *Lk = Lb + (j >> 2) * 128;
-        const T l10 = Lk[(j + 1) * 4], l20 = Lk[(j + 2) * 4], l21 = Lk[(j + 2) * 4 + 1];
-        const T l30 = Lk[(j + 3) * 4], l31 = Lk[(j + 3) * 4 + 1], l32 = Lk[(j + 3) * 4 + 2];
-        T x[4];
-        x[0] = b[0] * __shfl_sync(0xffffffffu, rdiag, j);
-        b[1] -= l10 * x[0];
-        b[2] -= l20 * x[0];
-        b[3] -= l30 * x[0];
-        x[1] = b[1] * __shfl_sync(0xffffffffu, rdiag, j + 1);
-        b[2] -= l21 * x[1];
-        b[3] -= l31 * x[1];
-        x[2] = b[2] * __shfl_sync(0xffffffffu, rdiag, j + 2);
-        b[3] -= l32 * x[2];
-        x[3] = b[3] * __shfl_sync(0xffffffffu, rdiag, j + 3);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) out(j + r, lane, x[r]);
-#pragma unroll
-        for (int c0 = 4; c0 < 32; c0 += 4) {
-            if (j + c0 < 32) {
-#pragma unroll
-                for (int c = c0; c < c0 + 4; ++c) {
-                    T v[4];
-                    c32_load4(Lk + (j + c) * 4, v);
-                    b[c] -= v[0] * x[0];
-                    b[c] -= v[1] * x[1];
-                    b[c] -= v[2] * x[2];
-                    b[c] -= v[3] * x[3];
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 28; ++q) b[q] = b[q + 4];
-    }
-}
-
 // ---------------------------------------------------------------------------
 // The latency form, column by column: 6,400 cycles for FP64 against 11,400 of
-// chol32_blk, 2,000 for a sweep against 4,900 of inv32_blk.
+// chol32_blk; 2,000 for a sweep against 4,900 of an inverse in steps of four rows.
 // ---------------------------------------------------------------------------
 // the pivots for which the branch-free root is good
 template <typename T>

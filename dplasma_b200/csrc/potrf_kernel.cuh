@@ -2,9 +2,9 @@
 // sm_100a with FP64 tensor cores.
 //
 // The tile DAG of dplasma's src/zpotrf_L.jdf (POTRF(k) -> TRSM(m,k) ->
-// SYRK(k,m) / GEMM(m,n,k)) is executed by one resident CTA per SM.  Each CTA
-// pulls task tickets from a global counter in a precomputed topological order
-// (critical path first, one step of look-ahead), waits on per-tile completion
+// SYRK(k,m) / GEMM(m,n,k)) is executed by one resident CTA per SM, FP64 on
+// 128x128 blocks whatever the tile edge.  Each CTA pulls task tickets from a
+// global counter in a precomputed topological order, waits on per-block completion
 // counters (bounded waits), and runs the task:
 //
 //   warp 8  (producer; warps 9-11 only lend their registers): fetches tickets, waits for the task's dependencies,
@@ -20,10 +20,10 @@
 // unchanged.
 //
 // TRSM(m,k) uses the inverses of the 128x128 diagonal blocks of L(k,k),
-// computed by POTRF(k) into the workspace W: the strip X = A(m,k) L(k,k)^{-T}
-// is solved block-left-looking as GEMM jobs (X_p = (A_p - sum_q X_q L_pq^T)
-// W_pp^T), so all FP64 flops of the path run on the tensor cores except the
-// 32x32 diagonal factorizations.
+// computed by POTRF(k) into the workspace W: L(m,k) = A(m,k) W_k^T; the mixed
+// kernel and the task pools solve the strip of a wider tile block-left-looking
+// (X_p = (A_p - sum_q X_q L_pq^T) W_pp^T), so all FP64 flops of the path run on
+// the tensor cores except POTRF's 32-wide factorizations and substitutions.
 #pragma once
 #include "dev_common.cuh"
 #include "dev_potrf128.cuh"
