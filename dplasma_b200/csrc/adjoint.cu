@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(256) ag_trtri_diag(const double *L, int ld, do
     const double *T = L + (int64_t)(b * AG_T) * ld + b * AG_T;
     double *Wk = scratch + (int64_t)b * AG_T * AG_T;   // 128x128, ld 128
     p128_load(tsm, T, ld, false, tid);
+    cp_async_wait(0);
     __syncthreads();
     p128_invert(tsm, tsm + P128_S + P128_D, unit_diag, Wk, tid >> 5, tid & 31, 1);
     double *Wb = W + (int64_t)(b * AG_T) * ldw + b * AG_T;

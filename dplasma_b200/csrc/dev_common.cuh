@@ -127,6 +127,20 @@ __device__ __forceinline__ void red_release_add(int *p, int v)
 // Order this thread's earlier accesses before its later ones for other SMs
 // (lighter than __threadfence, which is sequentially consistent).
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// 16-byte copy to shared memory through L2 (no register, not the async proxy)
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// at most n of this thread's groups still in flight, n = 0..3
+__device__ __forceinline__ void cp_async_wait(int n)
+{
+    if (n >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (n == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
 // Fire-and-forget FP64 add performed at L2 (no value returned, so the issuing
 // thread never waits for the line).
 __device__ __forceinline__ void red_add_f64(double *p, double v)
@@ -152,7 +166,7 @@ __device__ __forceinline__ bool wait_geq(const int *ctr, int target, const int *
                                          uint64_t limit_ns)
 {
     // the chain's waits are short: poll without pause first
-    for (int i = 0; i < 64; ++i)
+    for (int i = 0; i < 192; ++i)
         if (ld_acquire(ctr) >= target) return true;
     const uint64_t t0 = globaltimer_ns();
     unsigned ns = 32;

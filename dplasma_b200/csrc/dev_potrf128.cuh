@@ -14,7 +14,7 @@
 //     on the chain but the last block's;
 //   - while warp 0 updates and factors the next diagonal block the others update
 //     the rest, assemble the finished rows of the inverse and store what is done.
-// Measured in place: 33 us with load and stores; the form it replaces (block in
+// Measured in place: 35 us with load and stores; the form it replaces (block in
 // L2, inverse on the chain, a panel per barrier) took 123 us where its code was
 // cold and about 75 us warm.
 #pragma once
@@ -149,8 +149,9 @@ static __device__ __noinline__ int p128_diag_general(double *S, const double *T,
 
 // Factor the block in S (column c, row r at S[c * P128_SP + r], lower part)
 // and form W = L^-1, by the 256 threads of barrier `bar` (bar + 1 is used
-// inside); S must be complete (the caller's barrier) and T is the block it was
-// loaded from, leading dimension ld.  The factor's lower triangle goes to T and
+// inside); the first 32 columns of S must be there (the caller's barrier), the
+// threads' copies of the others may be in flight; T is the block it was loaded
+// from, leading dimension ld.  The factor's lower triangle goes to T and
 // W (zero above the diagonal) to the 128x128 block Wb; S keeps the factor, with
 // W's off-diagonal 32x32 blocks transposed in its upper part (W(r, c) at
 // S[r * P128_SP + c]) and the diagonal ones row-major behind it (P128_S).
@@ -244,6 +245,7 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
                 if (u) p128_run_unit(u, S, D, Wb, lane);
             }
         }
+        if (ph == 0) cp_async_wait(0);
         if (put_jj >= 0) p128_put_l(S, put_jj, T, ld, put_w, put_n, lane);
         if (put_d >= 0) p128_put_d(D, put_d, Wb, lane);
         named_bar_sync(bar, 256);
@@ -293,23 +295,17 @@ __device__ __forceinline__ void p128_invert(double *S, double *LB4, int unit, do
 constexpr int P128_INV_DOUBLES = P128_S + P128_D + 4 * P128_LB;
 
 // Load the lower 32-blocks (whole: all) of the 128x128 block at T (leading
-// dimension ld), 256 threads.
+// dimension ld), 256 threads: two groups of asynchronous copies, the first 32
+// columns and the rest, which the caller waits for (through registers, in two
+// rounds, the chain waited 6,400 cycles for the whole block; 38 -> 35 us per
+// POTRF).
 __device__ __forceinline__ void p128_load(double *S, const double *T, int ld, bool whole, int tid)
 {
-    const int r = (tid & 63) * 2, c0 = tid >> 6;
-#pragma unroll 1
-    for (int cc = 0; cc < 128; cc += 64) {
-        double2 v[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int c = cc + c0 + 4 * q;
-            if (whole || r + 2 > (c & ~31)) v[q] = __ldcg(reinterpret_cast<const double2 *>(T + (int64_t)c * ld + r));
-        }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int c = cc + c0 + 4 * q;
-            if (whole || r + 2 > (c & ~31)) *reinterpret_cast<double2 *>(S + c * P128_SP + r) = v[q];
-        }
+    const int r = (tid & 63) * 2;
+#pragma unroll 4
+    for (int c = tid >> 6; c < 128; c += 4) {
+        if (whole || r + 2 > (c & ~31)) cp_async16(S + c * P128_SP + r, T + (int64_t)c * ld + r);
+        if ((c & ~3) == 28 || (c & ~3) == 124) cp_async_commit();
     }
 }
 

@@ -73,10 +73,11 @@ __device__ bool wait_deps(const PotrfArgs &a, uint64_t t)
         return wait_geq(a.upd_done + (int64_t)k * a.mt + k, all_updates<MIXED>(a, k, k), a.abort_flag, a.status,
                         a.dep_limit_ns);
     case T_TRSM:
+        // (a read of a counter takes 0.4 us: the one that is ready last comes last)
         // tensor-core strips also need the split FP16 inverse (second release of POTRF(k))
-        return wait_geq(a.potrf_done + k, tc_strip<MIXED>(a, k, m) ? 2 : 1, a.abort_flag, a.status, a.dep_limit_ns) &&
-               wait_geq(a.upd_done + (int64_t)m * a.mt + k, all_updates<MIXED>(a, m, k), a.abort_flag, a.status,
-                        a.dep_limit_ns);
+        return wait_geq(a.upd_done + (int64_t)m * a.mt + k, all_updates<MIXED>(a, m, k), a.abort_flag, a.status,
+                        a.dep_limit_ns) &&
+               wait_geq(a.potrf_done + k, tc_strip<MIXED>(a, k, m) ? 2 : 1, a.abort_flag, a.status, a.dep_limit_ns);
     case T_GEMM:
         if (MIXED) {
             // chunk k of panels [k*S, min(k*S+S, n)): the last panel's strips
@@ -92,11 +93,12 @@ __device__ bool wait_deps(const PotrfArgs &a, uint64_t t)
             // block order: panels [k, kl]; as above the last panel's strips
             // imply the earlier ones, and a block's updates run in order
             const int kl = k + task_bi(t) - 1;
-            return wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, block_strips(m, kl), a.abort_flag, a.status,
-                            a.dep_limit_ns) &&
-                   wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, block_strips(n, kl), a.abort_flag, a.status, a.dep_limit_ns) &&
-                   wait_geq(a.upd_done + (int64_t)m * a.mt + n, block_update_index(k, n, a.fchunk), a.abort_flag,
-                            a.status, a.dep_limit_ns);
+            return wait_geq(a.upd_done + (int64_t)m * a.mt + n, block_update_index(k, n, a.fchunk), a.abort_flag,
+                            a.status, a.dep_limit_ns) &&
+                   (m == n || wait_geq(a.trsm_done + (int64_t)n * a.mt + kl, block_strips(n, kl), a.abort_flag,
+                                       a.status, a.dep_limit_ns)) &&
+                   wait_geq(a.trsm_done + (int64_t)m * a.mt + kl, block_strips(m, kl), a.abort_flag, a.status,
+                            a.dep_limit_ns);
         }
         return wait_geq(a.trsm_done + (int64_t)m * a.mt + k, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
                wait_geq(a.trsm_done + (int64_t)n * a.mt + k, nbs, a.abort_flag, a.status, a.dep_limit_ns) &&
@@ -230,8 +232,8 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
         task_it++;
         if (end) break;
         const int ty = task_type(t);
-        if (ty == T_POTRF) {
-            // POTRF uses the ring as scratch: wait until the consumers are done
+        if (ty == T_POTRF || (!(MIXED && ty == T_GEMM) && task_slab(a, t) >= 0)) {
+            // POTRF and slabs use the ring as scratch: wait until the consumers are done
             if (!warp_mbar_wait(&ctl->tempty[slot], round & 1, a.pipe_limit_ns)) {
                 if (lane == 0) report(a, ST_MBAR_TIMEOUT, 2, task_it, tk);
                 pipe_ok = false;
@@ -354,10 +356,6 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
             // block order: the operands change with each panel of 128
             const bool panels = !MIXED && a.fchunk && ty == T_GEMM;
             const double *Aop = jb.A, *Bop = jb.B;
-            // a slab: 32 rows of A (and of B, for a diagonal block, what lies below the slab's last column)
-            const int a0 = jb.slab >= 0 ? jb.slab * SLAB_ROWS : 0;
-            const uint32_t arows = jb.slab >= 0 ? SLAB_ROWS : BLK;
-            const uint32_t brows = jb.slab >= 0 && jb.mode == J_SUB_LOWER ? (jb.slab + 1) * SLAB_ROWS : BLK;
             for (int k0 = 0; k0 < jb.K; k0 += BK) {
                 if (panels && (k0 & (BLK - 1)) == 0) {
                     const int j = task_k(t) + k0 / BLK;
@@ -372,14 +370,14 @@ __device__ void producer_warp(const PotrfArgs &a, SmemCtl *ctl, double *ring, co
                 }
                 double *As = ring + s * STAGE_DOUBLES;
                 double *Bs = As + BK * SP;
-                if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], BK * (arows + brows) * (uint32_t)sizeof(double));
+                if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], BK * 2 * BLK * (uint32_t)sizeof(double));
                 __syncwarp();
                 if (lane < BK)
-                    bulk_g2s(As + lane * SP, Aop + (int64_t)(k0 + lane) * jb.lda + a0, arows * sizeof(double),
+                    bulk_g2s(As + lane * SP, Aop + (int64_t)(k0 + lane) * jb.lda, BLK * sizeof(double),
                              &ctl->full[s]);
                 else
                     bulk_g2s(Bs + (lane - BK) * SP, Bop + (int64_t)(k0 + lane - BK) * jb.ldb,
-                             brows * sizeof(double), &ctl->full[s]);
+                             BLK * sizeof(double), &ctl->full[s]);
                 stage_it++;
             }
             prev_signal = jb.signal;
@@ -519,69 +517,101 @@ __device__ __forceinline__ bool consume_job(const PotrfArgs &a, SmemCtl *ctl, co
 
 // ---------------------------------------------------------------------------
 // consumers: a 32-row slab of a 128x128 job (the chain's links), 16 columns per
-// warp.  A link of 32 x 128 x 128 took 7 us where the whole block took 20
-// (strip) and 26 us (update of the diagonal block).
+// warp.  The ring's bulk copies, sixteen columns at a time behind one producer
+// warp, paced a slab at 15 us whatever its product (2.4 to 4.3 us on one SM); the
+// consumers therefore load the operands themselves, everything in flight at once
+// in chunks of 32 columns, with the ring as scratch: 8.5 us a slab, and the
+// factorization of N = 4096 2.45 -> 2.20 ms (N = 12288 with FP16 updates 10.1 ->
+// 9.1).
 // ---------------------------------------------------------------------------
+constexpr int SL_KC = 32;                              // columns per chunk
+constexpr int SL_AP = SLAB_ROWS + 4;                   // pitch of the slab's rows (= 4 mod 16)
+constexpr int SL_CHUNK = SL_KC * (SP + SL_AP);
+constexpr int SL_NCH = 4;                              // chunks in flight
 template <bool MIXED>
-__device__ __forceinline__ bool consume_slab(const PotrfArgs &a, SmemCtl *ctl, const double *ring, const Job &jb,
-                                             uint32_t &stage_it)
+__device__ __forceinline__ void slab_job(const PotrfArgs &a, double *ring, uint64_t t, const Job &jb)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    constexpr uint32_t NST = MIXED ? NSTAGE_MIXED : NSTAGE;
+    const int g = lane >> 2, tq = lane & 3;
     // column group: the two warps of a sub-partition share a triangular load evenly
     const int cg = warp < 4 ? warp : 11 - warp;
+    const int r0 = jb.slab * SLAB_ROWS, nch = jb.K / SL_KC;
+    // a diagonal block's slab is among the rows of B, and B ends with it
     const bool lower = jb.mode == J_SUB_LOWER;
+    const double *A = jb.A, *B = jb.B;
+    if (!MIXED && a.fchunk && task_type(t) == T_GEMM) {
+        A = tile_ptr(a, task_m(t), task_k(t));
+        B = tile_ptr(a, task_n(t), task_k(t));
+    }
+    auto load = [&](int q) {
+        double *Bs = ring + (q % SL_NCH) * SL_CHUNK;
+        const int r = 2 * (tid & 63);
+        // (row c of a triangular B is zero beyond column c)
+        if (r >= (jb.tri ? q * SL_KC : 0) && r < (lower ? r0 + SLAB_ROWS : BLK)) {
+#pragma unroll
+            for (int c = tid >> 6; c < SL_KC; c += 4)
+                cp_async16(Bs + c * SP + r, B + (int64_t)(q * SL_KC + c) * jb.ldb + r);
+        }
+        if (!lower) {
+            double *As = Bs + SL_KC * SP;
+            const int ra = 2 * (tid & 15);
+#pragma unroll
+            for (int c = tid >> 4; c < SL_KC; c += 16)
+                cp_async16(As + c * SL_AP + ra, A + (int64_t)(q * SL_KC + c) * jb.lda + r0 + ra);
+        }
+        cp_async_commit();
+    };
+#pragma unroll 1
+    for (int q = 0; q < SL_NCH && q < nch; ++q) load(q);
     const int klim = jb.tri ? 16 * (cg + 1) : (lower && cg > 2 * jb.slab + 1) ? 0 : jb.K;
+    const int ap = lower ? SP : SL_AP;
     double acc[2][2][4];
     frag_zero(acc);
-    for (int k0 = 0; k0 < jb.K; k0 += BK) {
-        const uint32_t s = stage_it % NST, r = stage_it / NST;
-        if (!warp_mbar_wait(&ctl->full[s], r & 1, a.pipe_limit_ns)) {
-            if (lane == 0) report(a, ST_MBAR_TIMEOUT, 18, stage_it, warp);
-            stage_it += (jb.K - k0) / BK;
-            return false;
-        }
-        if (k0 < klim) {
-            const double *As = ring + s * STAGE_DOUBLES + g;
-            const double *Bs = ring + s * STAGE_DOUBLES + BK * SP + cg * 16 + g;
+#pragma unroll 1
+    for (int q = 0; q < nch; ++q) {
+        cp_async_wait(min(nch - q, SL_NCH) - 1);
+        named_bar_sync(1, NCONS);
+        const double *Bc = ring + (q % SL_NCH) * SL_CHUNK;
+        const double *As = (lower ? Bc + r0 : Bc + SL_KC * SP) + g;
+        const double *Bs = Bc + cg * 16 + g;
+#pragma unroll 1
+        for (int k0 = 0; k0 < SL_KC && q * SL_KC + k0 < klim; k0 += BK) {
 #pragma unroll
             for (int kk = 0; kk < BK; kk += 4) {
-                const int row = (kk + t) * SP;
+                const int col = k0 + kk + tq;
                 double af[2][2], bf[2];
 #pragma unroll
                 for (int mi = 0; mi < 2; ++mi) {
-                    af[mi][0] = As[row + mi * 16];
-                    af[mi][1] = As[row + mi * 16 + 8];
+                    af[mi][0] = As[col * ap + mi * 16];
+                    af[mi][1] = As[col * ap + mi * 16 + 8];
                 }
 #pragma unroll
-                for (int ni = 0; ni < 2; ++ni) bf[ni] = Bs[row + ni * 8];
+                for (int ni = 0; ni < 2; ++ni) bf[ni] = Bs[col * SP + ni * 8];
 #pragma unroll
                 for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
                     for (int ni = 0; ni < 2; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl->empty[s]);
-        stage_it++;
+        if (q + SL_NCH < nch) {
+            named_bar_sync(1, NCONS);
+            load(q + SL_NCH);
+        }
     }
-    const int r0 = jb.slab * SLAB_ROWS;
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = r0 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                const int c = cg * 16 + ni * 8 + 2 * t + (q & 1);
+            for (int e = 0; e < 4; ++e) {
+                const int r = r0 + mi * 16 + g + ((e & 2) ? 8 : 0);
+                const int c = cg * 16 + ni * 8 + 2 * tq + (e & 1);
                 double *p = jb.C + (int64_t)c * jb.ldc + r;
-                if (jb.mode == J_STORE) *p = acc[mi][ni][q];
-                else if (!lower || r >= c) red_add_f64(p, -acc[mi][ni][q]);
-                if (MIXED && jb.p16 && (q & 1)) store_p16<MIXED>(a, jb, acc[mi][ni][q - 1], acc[mi][ni][q], r, c - 1);
+                if (jb.mode == J_STORE) *p = acc[mi][ni][e];
+                else if (!lower || r >= c) red_add_f64(p, -acc[mi][ni][e]);
+                if (MIXED && jb.p16 && (e & 1)) store_p16<MIXED>(a, jb, acc[mi][ni][e - 1], acc[mi][ni][e], r, c - 1);
             }
-    if (jb.signal) fence_acq_rel_gpu();
-    return true;
+    if (jb.signal) fence_acq_rel_gpu();        // read back through L2 by the next job
 }
 
 // ---------------------------------------------------------------------------
@@ -727,6 +757,7 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
     for (int b = 0; b < a.nbs; ++b) {
         double *Tb = T + (int64_t)b * BLK * nbi + b * BLK;
         p128_load(ring, Tb, nbi, false, tid);
+        cp_async_wait(1);                       // the rest lands behind the first diagonal block
         named_bar_sync(1, NCONS);
         const int f = potrf128_smem(ring, &ctl->fail, Tb, nbi, Wk + (int64_t)b * BLK * BLK, warp, lane, 1);
         phase(0);
@@ -752,6 +783,7 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
 #pragma unroll 1
         for (int j = b + 1; j < a.nbs; ++j) {
             p128_load(ring, T + (int64_t)b * BLK * nbi + j * BLK, nbi, true, tid);
+            cp_async_wait(0);
             named_bar_sync(1, NCONS);
 #pragma unroll 1
             for (int i = j; i < a.nbs; ++i)
@@ -1163,17 +1195,25 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             if (MIXED && a.A0 && ty == T_TRSM) {
                 // streamed matrix: the strip's rows = untouched copy + updates,
                 // in place, before the producer loads them
-                const int s = a.crit_slabs ? task_bj(t) - 1 : -1;
+                const int s = task_slab(a, t);
                 stream_add_rows(a, m, k, task_bi(t) * BLK + (s >= 0 ? s * SLAB_ROWS : 0), s >= 0 ? SLAB_ROWS : BLK);
-                fence_proxy_async();
-                __syncwarp();
-                if ((tid & 31) == 0) mbar_arrive(&ctl->prep);
+                if (s >= 0) {
+                    named_bar_sync(1, NCONS);
+                } else {
+                    fence_proxy_async();
+                    __syncwarp();
+                    if ((tid & 31) == 0) mbar_arrive(&ctl->prep);
+                }
             }
             const int nj = task_njobs(a, t);
             for (int j = 0; j < nj; ++j) {
                 const Job jb = task_job(a, t, j);
-                ok = (jb.slab >= 0 ? consume_slab<MIXED>(a, ctl, ring, jb, stage_it)
-                                   : consume_job<MIXED>(a, ctl, ring, jb, stage_it)) && ok;
+                if (jb.slab >= 0) {
+                    slab_job<MIXED>(a, ring, t, jb);
+                    if (j + 1 < nj) named_bar_sync(1, NCONS);   // the next job reads C and takes the ring
+                    continue;
+                }
+                ok = consume_job<MIXED>(a, ctl, ring, jb, stage_it) && ok;
                 if (jb.signal) {
                     fence_proxy_async();
                     if (named_bar_or(1, NCONS, !ok)) {
@@ -1275,6 +1315,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 size_t potrf_smem_bytes(bool mixed)
 {
     const size_t ctl = ((sizeof(SmemCtl) + 127) / 128) * 128;
+    static_assert(SL_NCH * SL_CHUNK <= NSTAGE * STAGE_DOUBLES &&
+                      SL_NCH * SL_CHUNK * 8 <= MX_NST * MX_STAGE_BYTES,
+                  "the ring holds a slab's operands");
     static_assert(NSTAGE * STAGE_DOUBLES >= P128_DOUBLES && MX_NST * MX_STAGE_BYTES >= P128_DOUBLES * 8,
                   "the ring holds POTRF's scratch");
     if (!mixed) return ctl + (size_t)NSTAGE * STAGE_DOUBLES * sizeof(double);
@@ -1446,7 +1489,7 @@ std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, 
 // ---------------------------------------------------------------------------
 // Mixed order: the strips of the next tile row, the chain's link, as SLABS tasks
 // of 32 rows each on as many CTAs (70 us as two 128-row strips of three dependent
-// products, 20 us in slabs).
+// products, 24 us in slabs).
 static void split_critical_strips(std::vector<uint64_t> &v)
 {
     std::vector<uint64_t> out;

@@ -197,7 +197,7 @@ struct Job {
     int lda, ldb, ldc;
     int K;
     int mode;
-    int slab;      // 32-row slab of the block, or -1: all 128 rows
+    int slab;      // 32-row slab of the block, or -1: all 128 rows (task_slab)
     bool tri;      // B is lower triangular (row c is zero beyond column c)
     bool signal;   // the next job of the same task reads this job's output
     // mixed precision, TRSM store jobs: the 16-bit copy of the block is
@@ -206,6 +206,12 @@ struct Job {
     float p16_scale;
 };
 
+// The slab of a strip or an FP64 update, or -1.  Slabs load their operands
+// themselves (slab_job).
+__device__ __forceinline__ int task_slab(const PotrfArgs &a, uint64_t t)
+{
+    return (a.fchunk || a.crit_slabs) && task_type(t) != T_POTRF ? task_bj(t) - 1 : -1;
+}
 // The job sequence of a task (identical on producer and consumer sides).
 __device__ __forceinline__ int task_njobs(const PotrfArgs &a, uint64_t t)
 {
@@ -220,7 +226,7 @@ __device__ __forceinline__ Job task_job(const PotrfArgs &a, uint64_t t, int j)
     const int nbi = a.ld;
     const int k = task_k(t), m = task_m(t), n = task_n(t), bi = task_bi(t), bj = task_bj(t);
     jb.tri = false;
-    jb.slab = (a.fchunk || a.crit_slabs) ? bj - 1 : -1;
+    jb.slab = task_slab(a, t);
     if (task_type(t) == T_GEMM) {
         // C(m,n)[bi,bj] -= A(m,k)[bi,:] * A(n,k)[bj,:]^T     (src/zpotrf_L.jdf:619-623, :453-456)
         jb.A = tile_ptr(a, m, k) + bi * BLK;

@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(256) trtri_diag_kernel(const double *A, double
     const int tid = threadIdx.x;
     const double *T = A + lower_tile_index(k, k, mt) * (int64_t)nbi * nbi + (int64_t)b * 128 * nbi + b * 128;
     p128_load(tsm, T, nbi, false, tid);
+    cp_async_wait(0);
     __syncthreads();
     p128_invert(tsm, tsm + P128_S + P128_D, unit_diag, W + (int64_t)blockIdx.x * 128 * 128, tid >> 5, tid & 31, 1);
 }
