@@ -36,7 +36,9 @@ namespace db2 {
 
 constexpr int AG_T = 128;     // output tile
 constexpr int AG_K = 16;      // K chunk
-constexpr int AG_P = 132;     // shared pitch
+constexpr int AG_P = 132;     // shared pitch of a chunk stored by columns of A (= 4 mod 16)
+constexpr int AG_KP = 20;     // of one stored by rows, K contiguous as in memory (= 4 mod 16)
+constexpr int AG_NST = 4;     // chunks of A and B in shared memory
 
 // Tile sets and K ranges (block indices):
 //   LOWER_KGE_I   tiles i >= j                 k in [i, P-1]
@@ -56,26 +58,33 @@ enum : int { AG_LOWER_KGE_I = 1, AG_LOWER_JKI = 2, AG_SYM_KGE_I = 3, AG_GRAD = 4
 struct AgArgs {
     int mode, P, rowblk, nblk;
     const double *A;
-    int lda, transA;
+    int lda;
     const double *B;
     int ldb;
     double *C;
     int ldc;
-    double alpha, beta;
+    double alpha;
     // GRAD: out (n x n, both triangles, ld n) = g / 2 (al al^T - nal * product)
     const double *al, *g;
     int nal, n;
     double *out;
 };
 
-// C(i,j) = alpha * sum_{k in range} op(A)(i,k) B(k,j) + beta * C(i,j), 128x128 tiles
-constexpr size_t AG_SMEM = 4 * AG_K * AG_P * sizeof(double);   // double-buffered A and B stages
+// C(i,j) = alpha * sum_{k in range} op(A)(i,k) B(k,j), 128x128 tiles; op is the
+// transpose when TA.  Chunks stay as they lie in memory (B, and A when TA, with K
+// contiguous), so they arrive by 16-byte asynchronous copies three ahead and the
+// fragments are read without bank conflicts either way.  Bound: DMMA, and the last
+// wave (N = 4096: L^T Lbar 828 us of 620 at the DMMA peak, Y W 835, W^T Z + Z^T W
+// 1634 of 1240; through registers, stored transposed and two chunks deep, 995, 933
+// and 1963).
+constexpr int AG_OP = 128 * AG_KP;                              // doubles of one operand's chunk
+constexpr size_t AG_SMEM = AG_NST * 2 * AG_OP * sizeof(double);
+static_assert(AG_K * AG_P <= AG_OP, "either form fits");
 
-__global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
+template <bool TA>
+__global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
 {
     extern __shared__ __align__(16) double agsm[];
-    double(*As)[AG_K * AG_P] = reinterpret_cast<double(*)[AG_K * AG_P]>(agsm);
-    double(*Bs)[AG_K * AG_P] = reinterpret_cast<double(*)[AG_K * AG_P]>(agsm + 2 * AG_K * AG_P);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int wm = warp & 1, wn = warp >> 1;
@@ -133,76 +142,58 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
 
     const int kbeg = k0 * AG_T, kend = (k1 + 1) * AG_T;
-    double ra[8], rb[8];
     const double *Aop = a.A, *Bop = a.B;
-    auto load = [&](int kc) {
+    auto load = [&](int slot, int kc) {
+        double *As = agsm + slot * 2 * AG_OP, *Bs = As + AG_OP;
+        // four 16-byte pieces of each operand a thread
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = tid + 256 * q;
-            if (!a.transA) {
-                const int r = e & 127, kk = e >> 7;
-                ra[q] = Aop[(int64_t)(ako * AG_T + kc + kk) * a.lda + i * AG_T + r];
-            } else {
-                const int kk = e & 15, r = e >> 4;
-                ra[q] = Aop[(int64_t)(i * AG_T + r) * a.lda + ako * AG_T + kc + kk];
+        for (int q = 0; q < 4; ++q) {
+            if (!TA) {
+                const int r = 2 * (tid & 63), kk = (tid >> 6) + 4 * q;
+                cp_async16(As + kk * AG_P + r, Aop + (int64_t)(ako * AG_T + kc + kk) * a.lda + i * AG_T + r);
             }
-            const int kk = e & 15, c = e >> 4;
-            rb[q] = Bop[(int64_t)(j * AG_T + c) * a.ldb + bko * AG_T + kc + kk];
-        }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int e = tid + 256 * q;
-            if (!a.transA) {
-                const int r = e & 127, kk = e >> 7;
-                As[buf][kk * AG_P + r] = ra[q];
-            } else {
-                const int kk = e & 15, r = e >> 4;
-                As[buf][kk * AG_P + r] = ra[q];
-            }
-            const int kk = e & 15, c = e >> 4;
-            Bs[buf][kk * AG_P + c] = rb[q];
+            const int kk = 2 * (tid & 7), r = (tid >> 3) + 32 * q;
+            if (TA) cp_async16(As + r * AG_KP + kk, Aop + (int64_t)(i * AG_T + r) * a.lda + ako * AG_T + kc + kk);
+            cp_async16(Bs + r * AG_KP + kk, Bop + (int64_t)(j * AG_T + r) * a.ldb + bko * AG_T + kc + kk);
         }
     };
     // one pass over K, or two with the operands exchanged (SYM)
-    const int len = kend - kbeg, total = a.mode == AG_SYM_KGE_I ? 2 * len : len;
-    auto stage = [&](int at) {
-        if (at >= len) {
-            Aop = a.B;
-            Bop = a.A;
-        }
-        load(kbeg + (at >= len ? at - len : at));
-    };
-    if (total > 0) {
-        stage(0);
-        store(0);
-        __syncthreads();
-        int buf = 0;
-        for (int at = 0; at < total; at += AG_K) {
-            const bool more = at + AG_K < total;
-            if (more) stage(at + AG_K);
-            const double *Ab = As[buf] + wm * 64 + g;
-            const double *Bb = Bs[buf] + wn * 32 + g;
-#pragma unroll
-            for (int kk = 0; kk < AG_K; kk += 4) {
-                double af[4][2], bf[4];
-                const int row = (kk + t) * AG_P;
-#pragma unroll
-                for (int mi = 0; mi < 4; ++mi) {
-                    af[mi][0] = Ab[row + mi * 16];
-                    af[mi][1] = Ab[row + mi * 16 + 8];
-                }
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) bf[ni] = Bb[row + ni * 8];
-#pragma unroll
-                for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
+    const int len = kend - kbeg, nch = (a.mode == AG_SYM_KGE_I ? 2 * len : len) / AG_K;
+    auto stage = [&](int ch) {
+        if (ch < nch) {
+            const int at = ch * AG_K;
+            if (at >= len) {
+                Aop = a.B;
+                Bop = a.A;
             }
-            if (more) store(buf ^ 1);
-            __syncthreads();
-            buf ^= 1;
+            load(ch % AG_NST, kbeg + (at >= len ? at - len : at));
+        }
+        cp_async_commit();                     // (empty at the end: the count of groups stays even)
+    };
+    constexpr int ar = TA ? AG_KP : 1, ak = TA ? 1 : AG_P;      // strides of a chunk of A
+#pragma unroll 1
+    for (int ch = 0; ch < AG_NST - 1; ++ch) stage(ch);
+#pragma unroll 1
+    for (int ch = 0; ch < nch; ++ch) {
+        cp_async_wait(AG_NST - 2);
+        __syncthreads();                       // chunk ch is there, chunk ch - 1 is free
+        stage(ch + AG_NST - 1);
+        const double *Ab = agsm + (ch % AG_NST) * 2 * AG_OP + (wm * 64 + g) * ar + t * ak;
+        const double *Bb = agsm + (ch % AG_NST) * 2 * AG_OP + AG_OP + (wn * 32 + g) * AG_KP + t;
+#pragma unroll
+        for (int kk = 0; kk < AG_K; kk += 4) {
+            double af[4][2], bf[4];
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi) {
+                af[mi][0] = Ab[kk * ak + mi * 16 * ar];
+                af[mi][1] = Ab[kk * ak + (mi * 16 + 8) * ar];
+            }
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni) bf[ni] = Bb[kk + ni * 8 * AG_KP];
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
         }
     }
     if (a.mode == AG_GRAD) {
@@ -225,9 +216,7 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
                 }
         return;
     }
-    // epilogue: loads first, then stores
     double *C = a.C + (int64_t)(j * AG_T) * a.ldc + i * AG_T;
-    double old[4][4][4];
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
@@ -236,17 +225,7 @@ __global__ void __launch_bounds__(256) ag_gemm_kernel(AgArgs a)
             for (int q = 0; q < 4; ++q) {
                 const int r = wm * 64 + mi * 16 + g + ((q & 2) ? 8 : 0);
                 const int c = wn * 32 + ni * 8 + 2 * t + (q & 1);
-                old[mi][ni][q] = a.beta != 0.0 ? C[(int64_t)c * a.ldc + r] : 0.0;
-            }
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = wm * 64 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                const int c = wn * 32 + ni * 8 + 2 * t + (q & 1);
-                C[(int64_t)c * a.ldc + r] = a.alpha * acc[mi][ni][q] + a.beta * old[mi][ni][q];
+                C[(int64_t)c * a.ldc + r] = a.alpha * acc[mi][ni][q];
             }
 }
 
@@ -256,7 +235,7 @@ struct AgGrad {
     double *out;
 };
 static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, int lda, int transA, const double *B,
-                   int ldb, double *C, int ldc, double alpha, double beta, const AgGrad *gr = nullptr)
+                   int ldb, double *C, int ldc, double alpha, const AgGrad *gr = nullptr)
 {
     AgArgs a;
     a.al = gr ? gr->al : nullptr;
@@ -270,19 +249,18 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
     a.nblk = rowblk > 0 ? (P + 2 * rowblk - 1) / (2 * rowblk) : 0;
     a.A = A;
     a.lda = lda;
-    a.transA = transA;
     a.B = B;
     a.ldb = ldb;
     a.C = C;
     a.ldc = ldc;
     a.alpha = alpha;
-    a.beta = beta;
     int ntile;
     if (mode == AG_LVL_T || mode == AG_LVL_W) ntile = a.nblk * rowblk * rowblk;
     else ntile = P * (P + 1) / 2;
     if (ntile <= 0) return 0;
-    CK(cudaFuncSetAttribute(ag_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AG_SMEM));
-    ag_gemm_kernel<<<ntile, 256, AG_SMEM, ctx->stream>>>(a);
+    auto fn = transA ? ag_gemm_kernel<true> : ag_gemm_kernel<false>;
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AG_SMEM));
+    fn<<<ntile, 256, AG_SMEM, ctx->stream>>>(a);
     CK(cudaGetLastError());
     ctx->launches++;
     return 0;
@@ -361,8 +339,8 @@ static int ag_inverse(Context *ctx, const double *L, double *W, double *Y, doubl
     CK(cudaGetLastError());
     ctx->launches++;
     for (int h = 1; h < P; h *= 2) {
-        if ((rc = ag_gemm(ctx, AG_LVL_T, P, h, L, ld, 0, W, ld, Y, ld, 1.0, 0.0))) return rc;
-        if ((rc = ag_gemm(ctx, AG_LVL_W, P, h, W, ld, 0, Y, ld, W, ld, -1.0, 0.0))) return rc;
+        if ((rc = ag_gemm(ctx, AG_LVL_T, P, h, L, ld, 0, W, ld, Y, ld, 1.0))) return rc;
+        if ((rc = ag_gemm(ctx, AG_LVL_W, P, h, W, ld, 0, Y, ld, W, ld, -1.0))) return rc;
     }
     return 0;
 }
@@ -388,14 +366,14 @@ int potrf_adjoint_tiles(Context *ctx, const double *Lt, double *Lbt, const Geom 
     // W = L^-1
     if ((rc = ag_inverse(ctx, L, W, Y, scr, P, ld, 0))) return rc;
     // Y = Phi(L^T Lbar), lower tiles, k >= i
-    if ((rc = ag_gemm(ctx, AG_LOWER_KGE_I, P, 0, L, ld, 1, Z, ld, Y, ld, 1.0, 0.0))) return rc;
+    if ((rc = ag_gemm(ctx, AG_LOWER_KGE_I, P, 0, L, ld, 1, Z, ld, Y, ld, 1.0))) return rc;
     ag_phi<<<P, 256, 0, st>>>(Y, ld, P);
     CK(cudaGetLastError());
     ctx->launches++;
     // Z = Y W, lower tiles, j <= k <= i
-    if ((rc = ag_gemm(ctx, AG_LOWER_JKI, P, 0, Y, ld, 0, W, ld, Z, ld, 1.0, 0.0))) return rc;
+    if ((rc = ag_gemm(ctx, AG_LOWER_JKI, P, 0, Y, ld, 0, W, ld, Z, ld, 1.0))) return rc;
     // Abar = sym(W^T Z), lower tiles
-    if ((rc = ag_gemm(ctx, AG_SYM_KGE_I, P, 0, W, ld, 1, Z, ld, Y, ld, 0.5, 0.0))) return rc;
+    if ((rc = ag_gemm(ctx, AG_SYM_KGE_I, P, 0, W, ld, 1, Z, ld, Y, ld, 0.5))) return rc;
     ag_move<false><<<tg, 256, 0, st>>>(Lbt, g.mt, g.nbi, Y, ld);
     CK(cudaGetLastError());
     ctx->launches++;
@@ -462,14 +440,14 @@ static int inverse_or_gradient(Context *ctx, double *Lt, const Geom &g, int op, 
         src = W;
     }
     if (gr) {
-        if ((rc = ag_gemm(ctx, AG_GRAD, P, 0, W, ld, 1, W, ld, Y, ld, 1.0, 0.0, gr))) return rc;
+        if ((rc = ag_gemm(ctx, AG_GRAD, P, 0, W, ld, 1, W, ld, Y, ld, 1.0, gr))) return rc;
         CK(cudaStreamSynchronize(st));
         return 0;
     }
     double *out = W;
     if (op != 0) {
         // src^T src, lower tiles only (k >= i >= j): the result is symmetric
-        if ((rc = ag_gemm(ctx, AG_LOWER_KGE_I, P, 0, src, ld, 1, src, ld, Y, ld, 1.0, 0.0))) return rc;
+        if ((rc = ag_gemm(ctx, AG_LOWER_KGE_I, P, 0, src, ld, 1, src, ld, Y, ld, 1.0))) return rc;
         out = Y;
     }
     ag_move<false><<<tg, 256, 0, st>>>(Lt, g.mt, g.nbi, out, ld);
