@@ -1543,14 +1543,15 @@ static int prepare_tasks(Context *ctx, PotrfArgs &a, int mt, int nbs, int chunk)
 // Panels per FP64 update task on a grid of P blocks.  Every task pays one pass of
 // L2 reductions over its block (about 10 us beside 17 us of products per
 // panel), so the large grids take many (N = 32768, P = 256: 4 panels 391 ms, 8
-// 367, 12 362.6, 15 360.6; P = 128: 8 48.6, 12 48.4, 15 48.8); on a small grid
-// the open chunk of the next column would take longer than a step of the chain
-// it runs beside (P = 64: 4 8.30 ms, 6 8.19, 8 8.31; P = 32: 2 2.744, 4 2.741, 6
-// 2.864, 8 3.038).
+// 367, 12 362.6, 15 360.6; P = 128: 8 48.6, 12 48.4, 15 48.8; P = 96: 4 21.9, 6
+// 21.2, 8 21.0; P = 64: 4 7.48, 6 7.47, 8 7.62); on a small grid the open chunk of
+// the next column would take longer than a step of the chain it runs beside (P = 56:
+// 3 5.54 ms, 4 5.46, 6 5.62; P = 40: 1 3.00, 2 2.74, 3 2.79, 4 2.84; P = 32: 1 2.00,
+// 2 1.92, 4 2.08; P = 8: 2 0.434, 4 0.469).
 static int f64_panels(const Context *ctx, int P)
 {
     if (ctx->f64_chunk > 0) return ctx->f64_chunk;
-    return P <= 48 ? 4 : P <= 96 ? 6 : P <= 192 ? 12 : 15;
+    return P <= 44 ? 2 : P <= 60 ? 4 : P <= 96 ? 6 : P <= 192 ? 12 : 15;
 }
 
 // The counters of a launch in one zeroed array: 16 words (ticket, INFO, abort,
