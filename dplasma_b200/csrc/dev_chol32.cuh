@@ -28,6 +28,14 @@ __device__ __forceinline__ void c32_load4(const float *p, float (&v)[4])
     v[2] = a.z;
     v[3] = a.w;
 }
+// 16 bytes
+__device__ __forceinline__ void c32_loadv(const double *p, double (&v)[2])
+{
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    v[0] = a.x;
+    v[1] = a.y;
+}
+__device__ __forceinline__ void c32_loadv(const float *p, float (&v)[4]) { c32_load4(p, v); }
 __device__ __forceinline__ void c32_store4(double *p, const double (&v)[4])
 {
     reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
@@ -134,8 +142,9 @@ __device__ __forceinline__ int chol32_blk(T (&d)[32], int lane, T &rdiag, T *Lb)
 }
 
 // ---------------------------------------------------------------------------
-// The latency form, column by column: 6,400 cycles for FP64 against 11,400 of
-// chol32_blk; 2,000 for a sweep against 4,900 of an inverse in steps of four rows.
+// The latency form, column by column: 5,400 cycles for FP64 against 11,400 of
+// chol32_blk (6,400 with a load per value of the last column); 2,000 for a sweep
+// against 4,900 of an inverse in steps of four rows.
 // ---------------------------------------------------------------------------
 // the pivots for which the branch-free root is good
 template <typename T>
@@ -148,13 +157,13 @@ template <>
 struct c32_range<float> {
     static constexpr float lo = 1e-30f, hi = 1e30f;
 };
-// Columns per unrolled body: 16 is the fastest alone (5,200 cycles) but its code
-// is four times as long, and every caller runs it between other code: the
-// factorizations are alike for 4, 8 and 16 and the batched solver is 5 to 15 %
-// faster with 4 (6,400 cycles).
+// Columns per unrolled body: 16 is the fastest alone but its code is four times as
+// long, and every caller runs it between other code: the factorizations are alike
+// for 4, 8 and 16 and the batched solver is 5 to 15 % faster with 4.
 constexpr int C32_U = 4;
-constexpr int C32_LB = 1024 + 64;   // the blocked copy and what the unrolled loop may read past it
 constexpr int C32_RD = 1024;        // 1 / diagonal, 32 values behind the blocked copy
+constexpr int C32_CB = 1024 + 32;   // the last two columns, 48 values each (rows past the block are read)
+constexpr int C32_LB = C32_CB + 96;
 // 1 / sqrt(x) without a branch, x within the range the caller checks: the
 // hardware's approximation and two Newton steps y += y (1/2 - x/2 y^2).
 __device__ __forceinline__ float rsqrt_newton(float x) { return rsqrtf(x); }
@@ -170,13 +179,18 @@ __device__ __forceinline__ double rsqrt_newton(double x)
 
 // Columns J0 .. J0+15 of the 32x32 factorization (frame: d[k] = A(i, j + k) at
 // column j); LIVE columns of the frame are kept up to date.
-template <typename T, int LIVE>
+template <typename T, int LIVE, bool VEC>
 __device__ __forceinline__ void chol32_half(T (&d)[32], int J0, int lane, T &dg, T &lp, T &piv, T &rdiag, bool &ok,
                                             T *Sd, int sp, T *Lb)
 {
-#pragma unroll C32_U
-    for (int jj = 0; jj < 16; ++jj) {
-        const int j = J0 + jj;
+    T *Cb = Lb + C32_CB;
+    constexpr int V = 16 / sizeof(T);
+    static_assert(C32_U == 4, "column j0 + u starts at the vector boundary u & (V - 1)");
+#pragma unroll 1
+    for (int j0 = J0; j0 < J0 + 16; j0 += C32_U)
+#pragma unroll
+    for (int u = 0; u < C32_U; ++u) {
+        const int j = j0 + u;
         // what the next pivot needs from lane j + 1, before the pivot's root is known
         const T dn = __shfl_sync(0xffffffffu, dg, j + 1);       // its diagonal entry
         const T an = __shfl_sync(0xffffffffu, d[0], j + 1);     // A(j+1, j)
@@ -185,9 +199,22 @@ __device__ __forceinline__ void chol32_half(T (&d)[32], int J0, int lane, T &dg,
         // column j - 1 applied to the columns beyond j
         if (j > 0) {
             // (rows past the block, k >= 32 - j, feed columns that are never used)
-            const T *Lp = Lb + ((j - 1) >> 2) * 128 + j * 4 + ((j - 1) & 3);
+            if (VEC) {
+                // from its contiguous copy, 16 bytes a load
+                const T *Lp = Cb + ((u + 1) & 1) * 48 + j0;
 #pragma unroll
-            for (int k = 1; k < LIVE; ++k) d[k] = fma(-lp, Lp[4 * k], d[k]);
+                for (int r = (u + 1) / V * V; r < u + LIVE; r += V) {
+                    T v[V];
+                    c32_loadv(Lp + r, v);
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (r + e > u && r + e < u + LIVE) d[r + e - u] = fma(-lp, v[e], d[r + e - u]);
+                }
+            } else {
+                const T *Lp = Lb + ((j - 1) >> 2) * 128 + j * 4 + ((j - 1) & 3);
+#pragma unroll
+                for (int k = 1; k < LIVE; ++k) d[k] = fma(-lp, Lp[4 * k], d[k]);
+            }
         }
         const T ln = an * r;                                     // L(j+1, j)
         const T pn = fma(-ln, ln, dn);
@@ -200,6 +227,7 @@ __device__ __forceinline__ void chol32_half(T (&d)[32], int J0, int lane, T &dg,
             rdiag = r;
         }
         if (Sd && lane >= j) Sd[j * sp + lane] = l;
+        if (VEC) Cb[(u & 1) * 48 + lane] = l;
         Lb[(j >> 2) * 128 + lane * 4 + (j & 3)] = lane >= j ? l : T(0);
         __syncwarp();
         lp = l;
@@ -216,7 +244,10 @@ __device__ __forceinline__ void chol32_half(T (&d)[32], int J0, int lane, T &dg,
 // is null, the lower triangle at Sd (column c, row r at c * sp + r).  Returns
 // false when a pivot leaves the range in which the branch-free root is good (or
 // is not positive): the results are then useless.
-template <typename T>
+// VEC: 5,400 cycles (FP64) against 6,400; the FP64 scheduler kernel goes without, as
+// the loads' registers made it spill 196 bytes instead of 20 (a POTRF 36.7 us
+// against 34.5).
+template <typename T, bool VEC = true>
 __device__ __forceinline__ bool chol32_col(T (&d)[32], int lane, T *Sd, int sp, T *Lb, T *rd)
 {
     T dg = T(0), lp = T(0), rdiag = T(0);
@@ -225,8 +256,8 @@ __device__ __forceinline__ bool chol32_col(T (&d)[32], int lane, T *Sd, int sp, 
         if (lane == c) dg = d[c];
     T piv = __shfl_sync(0xffffffffu, dg, 0);
     bool ok = true;
-    chol32_half<T, 32>(d, 0, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
-    chol32_half<T, 16>(d, 16, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
+    chol32_half<T, 32, VEC>(d, 0, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
+    chol32_half<T, 16, VEC>(d, 16, lane, dg, lp, piv, rdiag, ok, Sd, sp, Lb);
     rd[lane] = rdiag;
     __syncwarp();
     return ok;
@@ -253,8 +284,6 @@ __device__ __forceinline__ void sweep32_half(const T *Lb, const T *rd, T (&b)[32
         b[3] -= l31 * x[1];
         x[3] = (b[3] - l32 * x[2]) * r4[3];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) out(j + r, x[r]);
-#pragma unroll
         for (int c = 4; c < LIVE; ++c) {
             T v[4];
             c32_load4(Lk + c * 4, v);
@@ -264,6 +293,9 @@ __device__ __forceinline__ void sweep32_half(const T *Lb, const T *rd, T (&b)[32
             y -= v[2] * x[2];
             b[c - 4] = y - v[3] * x[3];
         }
+        // (after the loads of this step, which could not pass the stores)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) out(j + r, x[r]);
     }
 }
 // Solve L x = b for one right-hand side per lane (b[c], c = 0..31), L in the

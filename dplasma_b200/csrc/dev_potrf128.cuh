@@ -14,7 +14,7 @@
 //     on the chain but the last block's;
 //   - while warp 0 updates and factors the next diagonal block the others update
 //     the rest, assemble the finished rows of the inverse and store what is done.
-// Measured in place: 35 us with load and stores; the form it replaces (block in
+// Measured in place: 34 us with load and stores; the form it replaces (block in
 // L2, inverse on the chain, a panel per barrier) took 123 us where its code was
 // cold and about 75 us warm.
 #pragma once
@@ -156,7 +156,8 @@ static __device__ __noinline__ int p128_diag_general(double *S, const double *T,
 // W's off-diagonal 32x32 blocks transposed in its upper part (W(r, c) at
 // S[r * P128_SP + c]) and the diagonal ones row-major behind it (P128_S).
 // Returns the failing column, the same in every thread, or -1; *fail is a
-// shared word.
+// shared word.  VEC: as chol32_col.
+template <bool VEC>
 __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, int ld, double *Wb, int warp, int lane,
                                              int bar)
 {
@@ -200,7 +201,7 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
 #pragma unroll
                 for (int c = 0; c < 32; ++c) d[c] = (c <= lane) ? Sd[c * SP + lane] : 0.0;
                 int f = -1;
-                if (!chol32_col(d, lane, Sd, SP, Lb, rd)) f = p128_diag_general(S, T, ld, j, Lb, rd, lane);
+                if (!chol32_col<double, VEC>(d, lane, Sd, SP, Lb, rd)) f = p128_diag_general(S, T, ld, j, Lb, rd, lane);
                 if (lane == 0) *fail = f >= 0 ? p0 + f : -1;
             } else if (helper && j > 0) {
                 // trailing blocks (bi, bk), j <= bk <= bi, but (j, j)

@@ -759,7 +759,7 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
         p128_load(ring, Tb, nbi, false, tid);
         cp_async_wait(1);                       // the rest lands behind the first diagonal block
         named_bar_sync(1, NCONS);
-        const int f = potrf128_smem(ring, &ctl->fail, Tb, nbi, Wk + (int64_t)b * BLK * BLK, warp, lane, 1);
+        const int f = potrf128_smem<MIXED>(ring, &ctl->fail, Tb, nbi, Wk + (int64_t)b * BLK * BLK, warp, lane, 1);
         phase(0);
         if (f >= 0) {
             if (tid == 0) {
