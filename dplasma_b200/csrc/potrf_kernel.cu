@@ -1182,7 +1182,11 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
         int *release = nullptr;
         bool ok = true;
         if (ty == T_POTRF) {
-            if (MIXED && a.A0) stream_add_rows(a, k, k, 0, a.nbi);   // potrf_task's first barrier orders it
+            if (MIXED && a.A0) {
+                // streamed matrix: potrf_task's copies read what other threads add here
+                stream_add_rows(a, k, k, 0, a.nbi);
+                named_bar_sync(1, NCONS);
+            }
             potrf_task<MIXED>(a, ctl, ring, k);
             if (ctl->fail < 0) release = a.potrf_done + k;
         } else if (ty == T_TRSM && tc_strip<MIXED>(a, k, m)) {

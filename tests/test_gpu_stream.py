@@ -20,7 +20,7 @@ import dplasma_b200 as db
 pytestmark = pytest.mark.gpu
 
 
-def _solve(ctx, A0, B0, NB, fmt, pinned):
+def _solve(ctx, A0, B0, NB, fmt, pinned, **opts):
     N, NRHS = B0.shape
     dA, dB, dX = db.desc_sym(N, NB, db.Lower), db.desc_general(N, NRHS, NB, NB), db.desc_general(N, NRHS, NB, NB)
     bufs = []
@@ -33,7 +33,7 @@ def _solve(ctx, A0, B0, NB, fmt, pinned):
             bufs.append(t)
         db.attach(d, host)
         bufs.append(host)
-    rc, st = ctx.dsposv(db.Lower, dA, dB, dX, fmt=fmt)
+    rc, st = ctx.dsposv(db.Lower, dA, dB, dX, fmt=fmt, **opts)
     assert rc == 0, ctx.last_error()
     X = db.unpack(bufs[-1], dX)
     Aafter = db.unpack(bufs[-5] if pinned else bufs[0], dA)
@@ -65,6 +65,26 @@ def test_streamed_solve_matches_uploaded(N, fmt, cb):
     assert np.array_equal(As[keep], A0[keep])          # A unchanged
     assert abs(sts["anorm"] - stu["anorm"]) <= 1e-13 * stu["anorm"]
     assert oracle.check_daxmb(oracle.LOWER, A0, B0, np.asfortranarray(Xs)) < 10.0
+
+
+@pytest.mark.parametrize("N,fmt,u", [(1024, db.FP16_SPLIT, 2.0 ** -21), (4096, db.FP16_SPLIT, 2.0 ** -21),
+                                     (4096, db.FP16, 2.0 ** -11), (4096, db.BF16, 2.0 ** -8)])
+def test_streamed_factor_without_refinement(N, fmt, u):
+    """The solution of the factor alone (the stopping test accepts any residual,
+    so no refinement hides an inaccurate factor): streamed and uploaded agree to
+    the rounding u of the 16-bit panels.  With A = N I + E, ||E||_2 < N / 2, a
+    relative error of 2u + u^2 in each panel product changes the solution by at
+    most 2u ||A^-1|| ||E|| < 2u for either form (a diagonal block without A's
+    entries changes it by O(1), or is not positive definite)."""
+    NB, NRHS = 256, 4
+    A0 = oracle.dplgsy(N, NB, 3872)
+    B0 = oracle.dplrnt(N, NRHS, NB, NB, 3873)
+    with db.Context(0) as ctx:
+        Xs, sts, _ = _solve(ctx, A0, B0, NB, fmt, pinned=True, bwdmax=1e30)
+        Xu, stu, _ = _solve(ctx, A0, B0, NB, fmt, pinned=False, bwdmax=1e30)
+    for st in (sts, stu):
+        assert st["iter"] == 0 and st["fallback"] == 0 and st["fmt_used"] == fmt, (sts, stu)
+    assert np.abs(Xs - Xu).max() <= 4 * u * np.abs(Xu).max()
 
 
 def test_streamed_not_positive_definite():
