@@ -105,7 +105,14 @@ static int check_general(const char *func, const parsec_tiled_matrix_t *B)
 static bool in_place_ok(const parsec_tiled_matrix_t *A, dplasma_enum_t uplo, const Geom &g)
 {
     return A->location == DPLASMA_B200_DEVICE && A->storage == PARSEC_MATRIX_TILE && A->uplo == dplasmaLower &&
-           uplo == dplasmaLower && g.nbi == g.nb && g.nb == A->mb && (g.n % g.nb) == 0 && A->lmt == g.mt;
+           uplo == dplasmaLower && g.nbi == g.nb && g.nb == A->mb && (g.n % g.nb) == 0 && A->lmt == g.mt &&
+           aligned16(A->mat);
+}
+// test hook (not part of the public header): whether a factorization or solve
+// works on the caller's storage, or on a copy
+extern "C" int dplasma_b200_debug_in_place(dplasma_enum_t uplo, const parsec_tiled_matrix_t *A)
+{
+    return in_place_ok(A, uplo, work_geom(A->m, A->mb)) ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------

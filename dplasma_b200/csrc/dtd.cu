@@ -83,8 +83,8 @@ void dtd_free(dplasma_b200_dtd_t *tp)
 
 // The tile layout the scheduler needs (lower triangle of tiles packed by
 // columns, nb a multiple of 128) is the caller's when the descriptor is a
-// device-resident lower TILE descriptor with 128 | nb and nb | n; otherwise a
-// device copy is made here and written back by dplasma_b200_dtd_data_flush_all.
+// device-resident lower TILE descriptor with 128 | nb and nb | n whose storage
+// is 16-byte aligned; otherwise a device copy is made here and written back by dplasma_b200_dtd_data_flush_all.
 extern "C" dplasma_b200_dtd_t *dplasma_b200_dtd_new(parsec_context_t *parsec, dplasma_enum_t uplo,
                                                     parsec_tiled_matrix_t *A)
 {
@@ -111,7 +111,8 @@ extern "C" dplasma_b200_dtd_t *dplasma_b200_dtd_new(parsec_context_t *parsec, dp
         return nullptr;
     }
     const bool inplace = A->location == DPLASMA_B200_DEVICE && A->storage == PARSEC_MATRIX_TILE &&
-                         A->uplo == dplasmaLower && g.nbi == g.nb && (g.n % g.nb) == 0 && A->lmt == g.mt;
+                         A->uplo == dplasmaLower && g.nbi == g.nb && (g.n % g.nb) == 0 && A->lmt == g.mt &&
+                         aligned16(A->mat);
     const int mt = g.mt > 0 ? g.mt : 1;
     tp->ins_potrf.assign(mt, 0);
     tp->ins_trsm.assign((size_t)mt * mt, 0);

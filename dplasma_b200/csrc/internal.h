@@ -132,6 +132,9 @@ struct Geom {
     size_t elems() const { return ntiles() * tile_elems(); }
 };
 Geom make_geom(int n, int nb);
+// a caller's matrix the kernels may work on where it lies: their bulk copies,
+// asynchronous copies and tensor maps take 16-byte aligned addresses only
+inline bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 Geom work_geom(int n, int nb);
 
 // potrf_kernel.cu

@@ -15,7 +15,8 @@
 //   * the matrix: device-resident, TILE storage of the lower triangle of
 //     tiles (dplasma_b200_sym_desc_init with dplasmaLower), nb a multiple of
 //     128 and at most 512, n a multiple of nb, and at most
-//     NOALLOC_MAX_BLOCK_ROWS row blocks of 128 (n <= 8192);
+//     NOALLOC_MAX_BLOCK_ROWS row blocks of 128 (n <= 8192), 16-byte aligned
+//     (a matrix of one tile may lie anywhere: it goes through the array);
 //   * the array is sized for that maximum (about 8.4 MiB) and stays allocated
 //     on every GPU that loads the library until the process exits;
 //   * every call uses the same array and finds the previous call's contents:
@@ -130,6 +131,12 @@ extern "C" int dplasma_b200_dpotrf_noalloc(void *stream, dplasma_enum_t uplo, pa
         fprintf(stderr, "[dplasma_b200_dpotrf_noalloc] cannot run under stream capture\n");
         return DPLASMA_ERR_NOT_SUPPORTED;
     }
+    // the kernel's copies take 16-byte addresses; one tile fits the scratch
+    const bool through_scratch = !aligned16(A->mat);
+    if (through_scratch && mt > 1) {
+        fprintf(stderr, "[dplasma_b200_dpotrf_noalloc] more than one tile needs 16-byte aligned storage\n");
+        return DPLASMA_ERR_NOT_SUPPORTED;
+    }
     const char *lim = getenv("DPLASMA_B200_WAIT_LIMIT_MS");
     const long lim_ms = lim ? atol(lim) : 4000;
     const uint64_t limit_ns = (uint64_t)(lim_ms > 0 ? lim_ms : 4000) * 1000000ull;
@@ -168,10 +175,26 @@ extern "C" int dplasma_b200_dpotrf_noalloc(void *stream, dplasma_enum_t uplo, pa
         cudaGetLastError();
         return DPLASMA_ERR_UNEXPECTED;
     }
+    double *dA = (double *)A->mat;
+    const size_t tile = (size_t)nb * nb * sizeof(double);
+    static_assert((size_t)4 * 128 * 128 * sizeof(double) + (size_t)512 * 512 * sizeof(double) <= W_BYTES,
+                  "behind the inverses of one tile there is room for the tile");
+    if (through_scratch) {
+        dA = W + 4 * 128 * 128;
+        if (cudaMemcpyAsync(dA, A->mat, tile, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+            cudaGetLastError();
+            return DPLASMA_ERR_UNEXPECTED;
+        }
+    }
     int info = 0, status = 0, diag[4] = {0, 0, 0, 0};
-    const int rc = potrf_launch_prealloc(st, (double *)A->mat, mt, nb, nb, n, W, tasks, (int)ntasks, ctr, grid,
-                                         limit_ns, &info, &status, diag);
+    const int rc = potrf_launch_prealloc(st, dA, mt, nb, nb, n, W, tasks, (int)ntasks, ctr, grid, limit_ns, &info,
+                                         &status, diag);
     if (rc) return rc;
+    if (through_scratch && (cudaMemcpyAsync(A->mat, dA, tile, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
+                            cudaStreamSynchronize(st) != cudaSuccess)) {
+        cudaGetLastError();
+        return DPLASMA_ERR_UNEXPECTED;
+    }
     if (status != 0) {
         fprintf(stderr, "[dplasma_b200_dpotrf_noalloc] scheduler status %d (site %d)\n", status, diag[0]);
         return DPLASMA_ERR_UNEXPECTED;

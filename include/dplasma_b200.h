@@ -255,7 +255,7 @@ int dplasma_dsymm(parsec_context_t *parsec, dplasma_enum_t side, dplasma_enum_t 
 /* dplasma_b200_dpotrf_noalloc: no counterpart in the reference.  The lower
  * tile Cholesky of a device-resident matrix (TILE storage of the lower
  * triangle of tiles, nb a multiple of 128 and at most 512, n a multiple of nb,
- * n <= 8192) for callers that cannot allocate device memory, e.g. code that
+ * n <= 8192; 16-byte aligned unless it is one tile) for callers that cannot allocate device memory, e.g. code that
  * hands the library memory from its own pool and may not let the device heap
  * grow.  It allocates nothing: its scratch is one fixed array of about
  * 8.4 MiB in the library's device image, held on every GPU that loads the
