@@ -996,7 +996,7 @@ extern "C" int dplasma_b200_gp_gradient(parsec_context_t *parsec, const parsec_t
     if (!parsec) return DPLASMA_ERR_NOT_INITIALIZED;
     int rc;
     if ((rc = check_square("dplasma_b200_gp_gradient", L))) return rc;
-    if (nrhs < 0 || (L->m > 0 && (!alpha || !g || !dK))) return DPLASMA_ERR_ILLEGAL_VALUE;
+    if (nrhs < 0 || (L->m > 0 && ((nrhs > 0 && !alpha) || !g || !dK))) return DPLASMA_ERR_ILLEGAL_VALUE;
     Context *ctx = &parsec->impl;
     cudaSetDevice(ctx->device);
     ctx->launches = 0;

@@ -403,7 +403,7 @@ int dplasma_b200_dpotri_batched(parsec_context_t *parsec, int batch, const int *
  * Gaussian-process log marginal likelihood, from the lower factor L of K (any
  * descriptor, as dplasma_dpotri takes it) and alpha = K^-1 y (n x nrhs, leading
  * dimension n): n x n, both triangles, leading dimension n.  alpha, g (one
- * value) and dK in device memory.  Returns INFO > 0 for a zero diagonal entry. */
+ * value) and dK in device memory; alpha may be NULL for nrhs = 0.  Returns INFO > 0 for a zero diagonal entry. */
 int dplasma_b200_gp_gradient(parsec_context_t *ctx, const parsec_tiled_matrix_t *L, int nrhs, const double *alpha,
                              const double *g, double *dK);
 /* The gradients dK_i = g_i / 2 (alpha_i alpha_i^T - K_i^-1) of g_i times the

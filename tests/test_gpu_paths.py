@@ -196,6 +196,17 @@ def test_gp_gradients_differentiate_and_batch_over_the_outer_gradient():
         assert torch.allclose(both, torch.stack([one, 3.0 * one]), rtol=1e-12, atol=1e-12)
 
 
+def test_gp_without_targets():
+    # no columns: value and gradient are zero
+    from dplasma_b200 import autograd as dag
+    n = 200
+    K = (torch.eye(n, dtype=torch.float64) * 2.0).cuda().requires_grad_(True)
+    y = torch.empty(n, 0, dtype=torch.float64, device="cuda", requires_grad=True)
+    v = dag.gp_log_marginal_likelihood(K, y)
+    dK, dy = torch.autograd.grad(v, (K, y))
+    assert float(v.detach()) == 0.0 and dy.shape == (n, 0) and bool((dK == 0).all())
+
+
 def test_gp_gradient_refuses(gpu_ctx):
     d = db.desc_general(8, 8, 256, 256, storage=db.STORAGE_LAPACK, lda=8)
     buf = torch.eye(8, dtype=torch.float64, device="cuda")
@@ -203,3 +214,7 @@ def test_gp_gradient_refuses(gpu_ctx):
     f = db.lib().dplasma_b200_gp_gradient
     assert f(None, ctypes.byref(d), 1, None, None, None) == db.ERR_NOT_INITIALIZED
     assert f(gpu_ctx.h, ctypes.byref(d), 1, None, None, None) == db.ERR_ILLEGAL_VALUE
+    g, out = torch.ones((), dtype=torch.float64, device="cuda"), torch.empty_like(buf)
+    torch.cuda.synchronize()
+    assert f(gpu_ctx.h, ctypes.byref(d), 1, None, g.data_ptr(), out.data_ptr()) == db.ERR_ILLEGAL_VALUE
+    assert f(gpu_ctx.h, ctypes.byref(d), 0, None, None, out.data_ptr()) == db.ERR_ILLEGAL_VALUE
