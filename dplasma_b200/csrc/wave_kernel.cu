@@ -76,6 +76,7 @@ struct WaveArgs {
     // opt-in trace: per CTA WV_TR_SLOTS ns counters, then the publish time of every block
     unsigned long long *trace;
 };
+constexpr size_t WV_EXCH_MAX = 64u << 20;   // exchange buffer of launches cleared together, bytes
 constexpr int WV_TR_SLOTS = 8;   // flag wait, Y staging, M + publish, deferred, L(nnq) + Z, rest, positions, -
 
 struct __align__(16) WaveCtl {
@@ -943,11 +944,13 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
     // status, then one flag per block and group, for each launch
     const size_t per = 4 + (size_t)nblk * sh.groups;
     int *ctr = (int *)ctx->buffer(BUF_SOLVE_CTR, per * nlaunch * sizeof(int));
+    // the exchange buffer of several launches is cleared at a time; the launches
+    // run one after the other, so many columns take turns in a bounded one
     const size_t xbytes = (size_t)nblk * 128 * per_launch * sizeof(double);
-    double *X = (double *)ctx->buffer(BUF_WX_EXCH, xbytes * nlaunch);
+    const int nx = (int)std::min<size_t>(nlaunch, std::max<size_t>(1, WV_EXCH_MAX / xbytes));
+    double *X = (double *)ctx->buffer(BUF_WX_EXCH, xbytes * nx);
     if (!ctr || !X) return DPLASMA_ERR_OUT_OF_RESOURCES;
     CK(cudaMemsetAsync(ctr, 0, per * nlaunch * sizeof(int), ctx->stream));
-    CK(cudaMemsetAsync(X, 0xff, xbytes * nlaunch, ctx->stream));      // WV_EMPTY
     // L: rows of the tiles contiguous (nbi), one line per tile column;
     // W: 128x128 column-major blocks.  Boxes of 16 doubles (128 bytes, the
     // swizzle span) by 32 (forward: k columns) or 128 (backward: columns).
@@ -975,6 +978,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
                             128 * sizeof(double), 16, box1, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc0) return rc0;
     for (int ch = 0; ch < nlaunch; ++ch) {
+        if (ch % nx == 0) CK(cudaMemsetAsync(X, 0xff, xbytes * std::min(nx, nlaunch - ch), ctx->stream));   // WV_EMPTY
         WaveArgs a;
         a.A = dA;
         a.W = W;
@@ -986,7 +990,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
         a.nblk = nblk;
         a.c0 = ch * per_launch;
         a.gsub = sh.gsub;
-        a.X = X + (size_t)ch * (xbytes / sizeof(double));
+        a.X = X + (size_t)(ch % nx) * (xbytes / sizeof(double));
         a.alpha = alpha;
         a.status = ctr + per * ch;
         a.flags = ctr + per * ch + 4;

@@ -96,6 +96,34 @@ def test_sweep_shapes(gpu_ctx, n, nrhs, uplo):
     assert r / ((np.abs(A).sum(1).max() * np.abs(X).sum(1).max() + np.abs(B).sum(1).max()) * n * EPS) < 10.0
 
 
+def test_sweep_exchange_buffer_is_bounded():
+    # many columns go through the sweep in turns: the workspace is the padded
+    # right-hand sides and a bounded exchange buffer, not a second copy of them;
+    # the columns repeat, so every turn gives the first one's results
+    n, nrhs, period = 512, 49152, 64
+    A = spd(n, n)
+    with db.Context(0) as ctx:
+        d, buf = dev_desc(A, 256, db.Lower, True)
+        assert ctx.dpotrf(db.Lower, d) == 0, ctx.last_error()
+        b = torch.rand(period, n, dtype=torch.float64, device="cuda").sub_(0.5)
+        B = b.repeat(nrhs // period, 1).contiguous()
+        torch.cuda.synchronize()
+
+        def solve(cols, t):
+            e = db.attach(db.desc_general(n, cols, 256, 256, storage=db.STORAGE_LAPACK, lda=n), t)
+            assert ctx.dpotrs(db.Lower, d, e) == 0, ctx.last_error()
+
+        solve(period, b)
+        free = torch.cuda.mem_get_info()[0]
+        solve(nrhs, B)
+        grown = free - torch.cuda.mem_get_info()[0]
+    assert grown < 1.5 * 8 * n * nrhs, grown
+    X, first = B.view(-1, period, n), b.cpu().numpy()
+    assert bool((X == X[0]).all())
+    r = np.abs(A @ first.T - A @ X[0].cpu().numpy().T).max()
+    assert r <= n * EPS * np.abs(A).sum(1).max() * np.abs(first).max()
+
+
 def test_sweep_passes_nans_on(gpu_ctx):
     # every NaN payload travels through the sweep's exchange buffer, the one
     # that marks an empty word included
