@@ -1399,7 +1399,7 @@ static void block_share(std::vector<uint64_t> &v, int bw, int bh)
     v.swap(out);
 }
 
-std::vector<uint64_t> build_potrf_tasks_mixed(int mt, int nbs, int delay, int S, int bw = 0, int bh = 0)
+static std::vector<uint64_t> build_potrf_tasks_mixed(int mt, int nbs, int delay, int S, int bw, int bh)
 {
     std::vector<uint64_t> v;
     auto push_trsm = [&](int k) {
@@ -1447,7 +1447,6 @@ std::vector<uint64_t> build_potrf_tasks_mixed(int mt, int nbs, int delay, int S,
 // on column k+1, POTRF(k+1), the open chunk up to panel k on column k+2 (it
 // runs beside POTRF(k+1)), `delay` tasks of the step's share, TRSM(*,k+1), the
 // rest of the share.
-static void block_share(std::vector<uint64_t> &v, int bw, int bh);
 std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, int bh)
 {
     std::vector<uint64_t> v;
@@ -1488,14 +1487,12 @@ std::vector<uint64_t> build_potrf_tasks_blocks(int P, int S, int delay, int bw, 
     return v;
 }
 
-// ---------------------------------------------------------------------------
-// host: run one factorization of the device tiles
-// ---------------------------------------------------------------------------
-// Mixed order: the strips of the next tile row, the chain's link, as SLABS tasks
-// of 32 rows each on as many CTAs (70 us as two 128-row strips of three dependent
-// products, 24 us in slabs).
-static void split_critical_strips(std::vector<uint64_t> &v)
+// The mixed order as it is launched: the strips of the next tile row, the chain's
+// link, as SLABS tasks of 32 rows each on as many CTAs (70 us as two 128-row strips
+// of three dependent products, 24 us in slabs).
+static std::vector<uint64_t> build_potrf_tasks_mixed_slabs(int mt, int nbs, int delay, int S, int bw, int bh)
 {
+    const std::vector<uint64_t> v = build_potrf_tasks_mixed(mt, nbs, delay, S, bw, bh);
     std::vector<uint64_t> out;
     out.reserve(v.size() + v.size() / 8);
     for (uint64_t t : v) {
@@ -1506,9 +1503,12 @@ static void split_critical_strips(std::vector<uint64_t> &v)
         for (int s = 0; s < SLABS; ++s)
             out.push_back(make_task(T_TRSM, task_k(t), task_m(t), task_n(t), task_bi(t), 1 + s));
     }
-    v.swap(out);
+    return out;
 }
 
+// ---------------------------------------------------------------------------
+// host: run one factorization of the device tiles
+// ---------------------------------------------------------------------------
 // The ticket order of a shape on the device (kept until another shape is
 // factored), with the tickets of the POTRFs behind it.  chunk > 0: mixed, this
 // many panels per update task; chunk < 0: FP64 on blocks, -chunk panels.
@@ -1517,10 +1517,9 @@ static int prepare_tasks(Context *ctx, PotrfArgs &a, int mt, int nbs, int chunk)
     const bool mixed = chunk > 0;
     const int delay = mixed ? ctx->mx_delay : ctx->potrf_delay;
     if (ctx->task_mt != mt || ctx->task_nbs != nbs || ctx->task_delay != delay || ctx->task_mixed != chunk) {
-        std::vector<uint64_t> tasks =
-            mixed ? build_potrf_tasks_mixed(mt, nbs, delay, chunk, ctx->mx_block_w, ctx->mx_block_h)
+        const std::vector<uint64_t> tasks =
+            mixed ? build_potrf_tasks_mixed_slabs(mt, nbs, delay, chunk, ctx->mx_block_w, ctx->mx_block_h)
                   : build_potrf_tasks_blocks(mt * nbs, -chunk, delay, ctx->f64_block, ctx->f64_block);
-        if (mixed) split_critical_strips(tasks);
         const size_t nt = tasks.size();
         int np = 0;
         std::vector<int> pos;
@@ -2227,7 +2226,7 @@ int potrf_launch_prealloc(cudaStream_t st, double *dA, int mt, int nbi, int nb_u
 extern "C" int dplasma_b200_debug_task_list_blocked(int mixed_chunk, int mt, int nbs, int delay, int bw, int bh,
                                                     unsigned long long *out, int cap)
 {
-    const std::vector<uint64_t> v = db2::build_potrf_tasks_mixed(mt, nbs, delay, mixed_chunk, bw, bh);
+    const std::vector<uint64_t> v = db2::build_potrf_tasks_mixed_slabs(mt, nbs, delay, mixed_chunk, bw, bh);
     for (size_t i = 0; i < v.size() && (int)i < cap; ++i) out[i] = v[i];
     return (int)v.size();
 }
@@ -2244,8 +2243,9 @@ extern "C" int dplasma_b200_debug_task_list_blocks(int P, int S, int delay, int 
 extern "C" int dplasma_b200_debug_task_list(int mixed_chunk, int mt, int nbs, int delay, unsigned long long *out,
                                             int cap)
 {
-    const std::vector<uint64_t> v = mixed_chunk > 0 ? db2::build_potrf_tasks_mixed(mt, nbs, delay, mixed_chunk)
-                                                    : db2::build_potrf_tasks(mt, nbs, delay);
+    const std::vector<uint64_t> v =
+        mixed_chunk > 0 ? db2::build_potrf_tasks_mixed_slabs(mt, nbs, delay, mixed_chunk, 0, 0)
+                        : db2::build_potrf_tasks(mt, nbs, delay);
     for (size_t i = 0; i < v.size() && (int)i < cap; ++i) out[i] = v[i];
     return (int)v.size();
 }

@@ -4,9 +4,10 @@ CTAs take tickets in order and a task starts once its dependencies are met,
 so the factorization makes progress without any co-residency assumption iff
 every task's dependencies are produced by tasks earlier in the order.  The
 rules replayed here are the ones the kernel waits on (the dataflow of
-src/zpotrf_L.jdf as per-tile completion counts), for the FP64 list (one task
-per 128x128 block and panel) and the mixed-precision list (one task per
-tile and chunk of S panels)."""
+src/zpotrf_L.jdf as per-tile completion counts), for the tile order (one task
+per 128x128 block and panel) and the mixed-precision order as it is launched
+(one update task per tile and chunk of S panels, the strips of the next tile row
+in four slabs each)."""
 import ctypes
 
 import numpy as np
@@ -15,6 +16,7 @@ import pytest
 import dplasma_b200 as db
 
 T_POTRF, T_TRSM, T_GEMM = 1, 2, 3
+SLABS = 4           # 32-row tasks per 128-row strip of the next tile row (mixed order)
 
 
 def tasks(chunk, mt, nbs, delay):
@@ -33,6 +35,12 @@ def replay(tl, mt, nbs, S):
     trsm = np.zeros((mt, mt), int)
     upd = np.zeros((mt, mt), int)
 
+    slabs = set()
+
+    def strips(m, k):
+        # tasks that complete the strips of tile (m, k)
+        return nbs * SLABS if S and m == k + 1 else nbs
+
     def all_updates(m, n):
         if S:
             return -(-n // S)
@@ -44,14 +52,19 @@ def replay(tl, mt, nbs, S):
             potrf[k] += 1
         elif ty == T_TRSM:
             assert potrf[k] == 1 and upd[m, k] == all_updates(m, k), (i, ty, k, m)
+            if S and m == k + 1:
+                assert 1 <= bj <= SLABS and bi < nbs and (k, bi, bj) not in slabs, (i, k, bi, bj)
+                slabs.add((k, bi, bj))
+            else:
+                assert bj == 0, (i, k, m)
             trsm[m, k] += 1
         else:
             assert ty == T_GEMM
             if S:
                 kl = min(k * S + S, n) - 1
-                assert trsm[m, kl] == nbs and trsm[n, kl] == nbs and upd[m, n] >= k, (i, k, m, n)
+                assert trsm[m, kl] == strips(m, kl) and trsm[n, kl] == strips(n, kl) and upd[m, n] >= k, (i, k, m, n)
             else:
-                assert trsm[m, k] == nbs and trsm[n, k] == nbs, (i, k, m, n)
+                assert trsm[m, k] == strips(m, k) and trsm[n, k] == strips(n, k), (i, k, m, n)
                 step = nbs * (nbs + 1) // 2 if m == n else nbs * nbs
                 assert upd[m, n] >= k * step, (i, k, m, n)
             upd[m, n] += 1
@@ -59,7 +72,7 @@ def replay(tl, mt, nbs, S):
     assert (potrf == 1).all()
     for m in range(mt):
         for k in range(m):
-            assert trsm[m, k] == nbs
+            assert trsm[m, k] == strips(m, k)
         for n in range(m + 1):
             assert upd[m, n] == all_updates(m, n)
 
