@@ -104,8 +104,9 @@ def _gp_gradient(buf: torch.Tensor, rhs: torch.Tensor, g: torch.Tensor) -> torch
         return g * _gp_gradient(buf, rhs, torch.ones((), dtype=buf.dtype, device=buf.device))
     n = buf.shape[0]
     ctx = context(buf.device)
+    # saved tensors come back from a hook with any strides
+    buf, rhs, g = buf.contiguous(), rhs.contiguous(), g.contiguous()
     dK = torch.empty_like(buf)
-    g = g.contiguous()
     torch_ready(buf, rhs, g, dK)
     d = _lapack_desc(buf, n)
     rc = lib().dplasma_b200_gp_gradient(ctx.h, ctypes.byref(d), rhs.shape[0], rhs.data_ptr(), g.data_ptr(),
@@ -262,7 +263,7 @@ def _gp_flat_backward(Lflat, alpha, g, lay):
         n2 = lay["n32"].long() ** 2
         return (g.index_select(0, torch.repeat_interleave(torch.arange(B, device=dev), n2)) * dK,
                 -g.index_select(0, lay["pid"]) * alpha)
-    g = g.contiguous()
+    Lflat, alpha, g = Lflat.contiguous(), alpha.contiguous(), g.contiguous()
     dK = torch.empty_like(Lflat)
     pL = Lflat.data_ptr() + 8 * lay["moff"]
     pal = alpha.data_ptr() + 8 * lay["voff"]

@@ -224,6 +224,34 @@ def test_gp_gradients_differentiate_and_batch_over_the_outer_gradient():
         assert torch.allclose(both, torch.stack([one, 3.0 * one]), rtol=1e-12, atol=1e-12)
 
 
+def test_gp_gradients_through_saved_tensor_hooks():
+    # a hook may give the saved factor and solution back with other strides
+    from dplasma_b200 import autograd as dag
+    g = torch.Generator().manual_seed(6)
+    Ks, ys = [], []
+    for n in (70, 33):
+        x = torch.rand(n, 3, generator=g, dtype=torch.float64)
+        Ks.append((torch.exp(-12.5 * torch.cdist(x, x) ** 2) + torch.eye(n, dtype=torch.float64)).cuda())
+        ys.append(torch.randn(n, generator=g, dtype=torch.float64).cuda())
+    y2 = torch.stack([ys[0], 2 * ys[0] + 1], 1)
+    cases = [(dag.gp_log_marginal_likelihood, (Ks[0], ys[0])), (dag.gp_log_marginal_likelihood, (Ks[0], y2)),
+             (lambda K, y: dag.gp_log_marginal_likelihood_flat(K, y, (70, 33)).sum(),
+              (torch.cat([K.reshape(-1) for K in Ks]), torch.cat(ys))),
+             (lambda *t: dag.gp_log_marginal_likelihood_batched(t[:2], t[2:]).sum(), (*Ks, *ys))]
+
+    def spread(t):
+        # the same values, no two of them side by side
+        return torch.stack([t, torch.full_like(t, 7.0)], -1)[..., 0]
+
+    for f, args in cases:
+        args = [a.clone().requires_grad_(True) for a in args]
+        plain = torch.autograd.grad(f(*args), args)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, spread):
+            v = f(*args)
+        for a, b in zip(torch.autograd.grad(v, args), plain):
+            assert torch.equal(a, b)
+
+
 def test_gp_without_targets():
     # no columns: value and gradient are zero
     from dplasma_b200 import autograd as dag
