@@ -102,24 +102,28 @@ __device__ __forceinline__ int bt_diag(T *A, int lda, int j0, int jb, bool in_sm
 
 // The next diagonal block (tile (0,0) of the trailing matrix) before it is
 // factored, C -= P P^T in lower 16x16 quarters q = 0 (top), 1 (below), 2: to the
-// matrix and to shared memory at Sd (pitch BT_DP).
+// matrix and to shared memory at Sd (pitch BT_DP).  The products are summed by
+// themselves and subtracted once, here and in bt_tile: accumulated onto C, every
+// product is rounded at the size of C (factors of 256 diagonally dominant FP64
+// columns 2.5e-16 off instead of 1.0e-16, FP32 1.4e-7 instead of 5.4e-8).
 __device__ __forceinline__ void bt_quarter(double *C, int lda, int m, const double *Pr, int sr, double *Sd, int q,
                                            int lane)
 {
     const int g = lane >> 2, t = lane & 3;
     const int qr = q == 0 ? 0 : 16, qc = q == 2 ? 16 : 0;
-    double acc[2][4];
+    double old[2][4], acc[2][4];
 #pragma unroll
     for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = qr + g + ((e & 2) ? 8 : 0), c = qc + ni * 8 + 2 * t + (e & 1);
-            acc[ni][e] = (r < m && c <= r) ? C[(int64_t)c * lda + r] : 0.0;
+            old[ni][e] = (r < m && c <= r) ? C[(int64_t)c * lda + r] : 0.0;
+            acc[ni][e] = 0.0;
         }
 #pragma unroll
     for (int kk = 0; kk < 32; kk += 4) {
         const double *pk = Pr + (int64_t)(kk + t) * sr + g;
-        const double a0 = qr + g < m ? -pk[qr] : 0.0, a1 = qr + g + 8 < m ? -pk[qr + 8] : 0.0;
+        const double a0 = qr + g < m ? pk[qr] : 0.0, a1 = qr + g + 8 < m ? pk[qr + 8] : 0.0;
 #pragma unroll
         for (int ni = 0; ni < 2; ++ni)
             dmma_16x8x4(acc[ni], a0, a1, qc + ni * 8 + g < m ? pk[qc + ni * 8] : 0.0);
@@ -129,119 +133,135 @@ __device__ __forceinline__ void bt_quarter(double *C, int lda, int m, const doub
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = qr + g + ((e & 2) ? 8 : 0), c = qc + ni * 8 + 2 * t + (e & 1);
-            Sd[c * BT_DP + r] = acc[ni][e];
-            if (r < m && c <= r) C[(int64_t)c * lda + r] = acc[ni][e];
+            const double v = old[ni][e] - acc[ni][e];
+            Sd[c * BT_DP + r] = v;
+            if (r < m && c <= r) C[(int64_t)c * lda + r] = v;
         }
 }
 __device__ __forceinline__ void bt_quarter(float *C, int lda, int m, const float *Pr, int sr, float *Sd, int q, int lane)
 {
     // half the columns of a row per lane: quarter q has rows qr + (lane / 2), eight columns each
     const int qr = q == 0 ? 0 : 16, qc = (q == 2 ? 16 : 0) + 8 * (lane & 1), r = qr + (lane >> 1);
-    float acc[8];
+    float old[8], acc[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = (r < m && qc + j <= r) ? C[(int64_t)(qc + j) * lda + r] : 0.f;
+    for (int j = 0; j < 8; ++j) {
+        old[j] = (r < m && qc + j <= r) ? C[(int64_t)(qc + j) * lda + r] : 0.f;
+        acc[j] = 0.f;
+    }
 #pragma unroll 8
     for (int k = 0; k < 32; ++k) {
-        const float pr = -Pr[k * sr + r];
+        const float pr = Pr[k * sr + r];
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[j] = fmaf(pr, Pr[k * sr + qc + j], acc[j]);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        Sd[(qc + j) * BT_DP + r] = acc[j];
-        if (r < m && qc + j <= r) C[(int64_t)(qc + j) * lda + r] = acc[j];
+        const float v = old[j] - acc[j];
+        Sd[(qc + j) * BT_DP + r] = v;
+        if (r < m && qc + j <= r) C[(int64_t)(qc + j) * lda + r] = v;
     }
 }
 
 // One 32x32 tile (rb, cb), rb >= cb, of the trailing update C -= P P^T by one
 // warp; C is the trailing matrix (origin at A(o, o)), m its order, P the panel
-// (rows beyond m zero) with k stride RP.  The C values are the accumulators'
-// start.
-// FULL: all 32 x 32 elements exist (below the diagonal block, inside m).
-template <bool FULL>
+// (rows beyond m zero) with k stride RP.  The C values are on their way while the
+// products are formed.
+// FULL: all 32 x 32 elements exist (below the diagonal block, inside m).  NI: 8-column
+// groups of the tile formed at a time (two where the registers are limited).
+template <bool FULL, int NI>
 __device__ __forceinline__ void bt_tile_f64(double *A, int lda, int o, int m, const double *P, int RP, int rb, int cb,
                                             int lane)
 {
     const int g = lane >> 2, t = lane & 3;
-    double *C = A + (int64_t)(o + cb * 32 + 2 * t) * lda + o + rb * 32 + g;
-    const int mr = m - rb * 32 - g, mc = m - cb * 32 - 2 * t, dd = rb == cb ? g - 2 * t : 1 << 20;
-    // element (row 16 mi + 8 h, column 8 ni + e) of this thread
-    auto in = [&](int r, int c) { return FULL || (r < mr && c < mc && r - c + dd >= 0); };
-    double acc[2][4][4];
+#pragma unroll 1
+    for (int n0 = 0; n0 < 32; n0 += 8 * NI) {
+        double *C = A + (int64_t)(o + cb * 32 + n0 + 2 * t) * lda + o + rb * 32 + g;
+        const int mr = m - rb * 32 - g, mc = m - cb * 32 - n0 - 2 * t, dd = rb == cb ? g - n0 - 2 * t : 1 << 20;
+        // element (row 16 mi + 8 h, column 8 ni + e) of this thread
+        auto in = [&](int r, int c) { return FULL || (r < mr && c < mc && r - c + dd >= 0); };
+        double old[2][NI][4], acc[2][NI][4];
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-        const double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
+        for (int ni = 0; ni < NI; ++ni) {
+            const double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
+            for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
-                acc[mi][ni][q] = in(r, c) ? ((q & 1) ? p1 : p0)[r] : 0.0;
+                for (int q = 0; q < 4; ++q) {
+                    const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
+                    old[mi][ni][q] = in(r, c) ? ((q & 1) ? p1 : p0)[r] : 0.0;
+                    acc[mi][ni][q] = 0.0;
+                }
+        }
+        const double *a0 = P + t * RP + rb * 32 + g, *b0 = P + t * RP + cb * 32 + n0 + g;
+#pragma unroll
+        for (int kk = 0; kk < 32; kk += 4) {
+            double af[2][2], bf[NI];
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi) {
+                af[mi][0] = a0[mi * 16];
+                af[mi][1] = a0[mi * 16 + 8];
             }
-    }
-    const double *a0 = P + t * RP + rb * 32 + g, *b0 = P + t * RP + cb * 32 + g;
 #pragma unroll
-    for (int kk = 0; kk < 32; kk += 4) {
-        double af[2][2], bf[4];
+            for (int ni = 0; ni < NI; ++ni) bf[ni] = b0[ni * 8];
+            a0 += 4 * RP;
+            b0 += 4 * RP;
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
-            af[mi][0] = -a0[mi * 16];
-            af[mi][1] = -a0[mi * 16 + 8];
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < NI; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
         }
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) bf[ni] = b0[ni * 8];
-        a0 += 4 * RP;
-        b0 += 4 * RP;
+        for (int ni = 0; ni < NI; ++ni) {
+            double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
+            for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
-    }
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-        double *p0 = C + (int64_t)(ni * 8) * lda, *p1 = p0 + lda;
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
-                if (in(r, c)) ((q & 1) ? p1 : p0)[r] = acc[mi][ni][q];
-            }
+                for (int q = 0; q < 4; ++q) {
+                    const int r = mi * 16 + ((q & 2) ? 8 : 0), c = ni * 8 + (q & 1);
+                    if (in(r, c)) ((q & 1) ? p1 : p0)[r] = old[mi][ni][q] - acc[mi][ni][q];
+                }
+        }
     }
 }
+template <int NI>
 __device__ __forceinline__ void bt_tile(double *A, int lda, int o, int m, const double *P, int RP, int rb, int cb,
                                         int lane)
 {
-    if (rb > cb && rb * 32 + 32 <= m) bt_tile_f64<true>(A, lda, o, m, P, RP, rb, cb, lane);
-    else bt_tile_f64<false>(A, lda, o, m, P, RP, rb, cb, lane);
+    if (rb > cb && rb * 32 + 32 <= m) bt_tile_f64<true, NI>(A, lda, o, m, P, RP, rb, cb, lane);
+    else bt_tile_f64<false, NI>(A, lda, o, m, P, RP, rb, cb, lane);
 }
-// FP32: lane = row of the tile, 32 columns per lane (the panel values of the
-// columns are broadcasts)
+// FP32: lane = row of the tile, 8 NI columns per lane at a time (the panel values
+// of the columns are broadcasts)
+template <int NI>
 __device__ __forceinline__ void bt_tile(float *A, int lda, int o, int m, const float *P, int RP, int rb, int cb,
                                         int lane)
 {
     const int r = rb * 32 + lane;
-    float acc[32];
+#pragma unroll 1
+    for (int c0 = cb * 32; c0 < cb * 32 + 32; c0 += 8 * NI) {
+        float old[8 * NI], acc[8 * NI];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        const int c = cb * 32 + j;
-        acc[j] = (r < m && c < m && r >= c) ? A[(int64_t)(o + c) * lda + o + r] : 0.f;
-    }
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-        const float pr = -P[k * RP + r];
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            float v[4];
-            c32_load4(P + k * RP + cb * 32 + j, v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j + e] = fmaf(pr, v[e], acc[j + e]);
+        for (int j = 0; j < 8 * NI; ++j) {
+            const int c = c0 + j;
+            old[j] = (r < m && c < m && r >= c) ? A[(int64_t)(o + c) * lda + o + r] : 0.f;
+            acc[j] = 0.f;
         }
-    }
+#pragma unroll 4
+        for (int k = 0; k < 32; ++k) {
+            const float pr = P[k * RP + r];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        const int c = cb * 32 + j;
-        if (r < m && c < m && r >= c) A[(int64_t)(o + c) * lda + o + r] = acc[j];
+            for (int j = 0; j < 8 * NI; j += 4) {
+                float v[4];
+                c32_load4(P + k * RP + c0 + j, v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j + e] = fmaf(pr, v[e], acc[j + e]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8 * NI; ++j) {
+            const int c = c0 + j;
+            if (r < m && c < m && r >= c) A[(int64_t)(o + c) * lda + o + r] = old[j] - acc[j];
+        }
     }
 }
 
@@ -249,7 +269,7 @@ __device__ __forceinline__ void bt_tile(float *A, int lda, int o, int m, const f
 // look-ahead: after the panel, three warps update the next diagonal block; then
 // warp 0 factors it while the other warps update the rest of the trailing matrix.
 // P: the panel, RP its k stride.  Returns INFO (0 or the 1-based failing column).
-template <typename T, int NT>
+template <typename T, int NT, int NI>
 __device__ int bt_factor(T *A, int n, int lda, T *Lb, T *P, int RP, int *sflag, double *logdet_out,
                          T *B, int nrhs, T *dscr, T *ybuf)
 {
@@ -341,7 +361,7 @@ __device__ int bt_factor(T *A, int n, int lda, T *Lb, T *P, int RP, int *sflag, 
                     ++cb;
                 }
                 const int rb = cb + rem;
-                bt_tile(A, lda, o, m, P, RP, rb, cb, lane);
+                bt_tile<NI>(A, lda, o, m, P, RP, rb, cb, lane);
             }
             if (B) {
 #pragma unroll 1
@@ -458,7 +478,7 @@ __global__ void __launch_bounds__(NT, OCC) batched_posv_kernel(BatchArgs<T> a)
         int info = 0;
         if (n > 0) {
             T *Bi = (a.B && a.nrhs > 0) ? a.B[i] : nullptr;
-            info = bt_factor<T, NT>(a.A[i], n, lda, Lb, P, a.prow + 4, sflag,
+            info = bt_factor<T, NT, NT * OCC <= 256 ? 4 : 2>(a.A[i], n, lda, Lb, P, a.prow + 4, sflag,
                                     a.logdet ? a.logdet + i : nullptr, Bi, a.nrhs, dscr, ybuf);
             if (info == 0 && Bi) bt_backward<T, NT>(a.A[i], n, lda, Bi, a.nrhs, dscr, Lb, P);
         } else if (threadIdx.x == 0 && a.logdet) {

@@ -287,11 +287,11 @@ __device__ __forceinline__ void sweep32_half(const T *Lb, const T *rd, T (&b)[32
         for (int c = 4; c < LIVE; ++c) {
             T v[4];
             c32_load4(Lk + c * 4, v);
-            T y = b[c];
-            y -= v[0] * x[0];
-            y -= v[1] * x[1];
-            y -= v[2] * x[2];
-            b[c - 4] = y - v[3] * x[3];
+            T s = v[0] * x[0];
+            s += v[1] * x[1];
+            s += v[2] * x[2];
+            s += v[3] * x[3];
+            b[c - 4] = b[c] - s;                     // one rounding at the size of b per four columns
         }
         // (after the loads of this step, which could not pass the stores)
 #pragma unroll

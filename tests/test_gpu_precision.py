@@ -1,0 +1,58 @@
+"""GPU tests of the accuracy of the factors, against the factor in extended
+precision (80-bit on the host).
+
+For a diagonally dominant matrix (entries uniform in [-0.5, 0.5], n added to the
+diagonal) the error of the factor is that of its diagonal: every subtraction from
+a(i,i) ~ n rounds by at most u n, all else is smaller by a factor of n.  With m
+such roundings of variance at most u^2 / 3 (relative, independent), l(i,i) =
+sqrt(a(i,i)) has half their error and one rounding of its own, so the factor is
+off by at most about u / sqrt(3) sqrt(m / 4 + 1).  The products of a panel of 32
+columns are summed by themselves and subtracted once; inside a 32-wide diagonal
+block the columns are subtracted one after the other (15.5 on average).  Were
+every product rounded at the size of a(i,i), m would be n / 2."""
+import numpy as np
+import pytest
+
+import dplasma_b200 as db
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def dominant(n, seed, dtype=np.float64):
+    g = np.random.default_rng(seed)
+    a = g.uniform(-0.5, 0.5, (n, n))
+    a = np.tril(a) + np.tril(a, -1).T
+    a[np.diag_indices(n)] += n
+    return np.ascontiguousarray(a.astype(dtype))
+
+
+def factor_extended(A):
+    A = A.astype(np.longdouble)
+    n = A.shape[0]
+    L = np.zeros_like(A)
+    for j in range(n):
+        c = A[j:, j] / np.sqrt(A[j, j])
+        L[j:, j] = c
+        A[j + 1:, j + 1:] -= np.multiply.outer(c[1:], c[1:])
+    return L
+
+
+def relative_error(F, L):
+    return float(np.linalg.norm((F.astype(np.longdouble) - L).astype(np.float64)) / np.linalg.norm(L.astype(np.float64)))
+
+
+def bound(u, m):
+    return u / np.sqrt(3.0) * np.sqrt(m / 4 + 1)
+
+
+@pytest.mark.parametrize("dtype,u", [(np.float64, 2.0 ** -53), (np.float32, 2.0 ** -24)])
+@pytest.mark.parametrize("n,count", [(96, 400), (200, 400), (256, 40), (512, 3)])      # the shapes of the batched kernel
+def test_batched_factor(gpu_ctx, n, count, dtype, u):
+    mats = [dominant(n, s, dtype) for s in range(2)]
+    dev = [torch.from_numpy(mats[i % 2].copy()).cuda() for i in range(count)]
+    info, _ = gpu_ctx.posv_batched(dev)
+    assert int(info.abs().max()) == 0
+    for A, F in zip(mats, dev[:2]):
+        err = relative_error(np.triu(F.cpu().numpy()).T, factor_extended(A))
+        assert err <= bound(u, 15.5 + n / 64), err / u
