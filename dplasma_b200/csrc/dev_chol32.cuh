@@ -291,7 +291,7 @@ __device__ __forceinline__ void sweep32_half(const T *Lb, const T *rd, T (&b)[32
             s += v[1] * x[1];
             s += v[2] * x[2];
             s += v[3] * x[3];
-            b[c - 4] = b[c] - s;                     // one rounding at the size of b per four columns
+            b[c - 4] = b[c] - s;               // one rounding at the size of b per four columns
         }
         // (after the loads of this step, which could not pass the stores)
 #pragma unroll
@@ -307,6 +307,53 @@ __device__ __forceinline__ void sweep32(const T *Lb, const T *rd, T (&b)[32], Ou
 {
     sweep32_half<T, 32>(Lb, rd, b, 0, out);
     sweep32_half<T, 16>(Lb, rd, b, 16, out);
+}
+
+// The same for right-hand sides that lie in shared memory (in(c) = b_c, read when
+// column c is reached): the frame holds the sums s_c = sum_k L(c,k) x_k from zero,
+// x_c = b_c / L(c,c) - s_c / L(c,c), so no product is rounded at the size of b and
+// nothing is added to the chain.
+template <typename T, int LIVE, class In, class Out>
+__device__ __forceinline__ void sweep32_sums_half(const T *Lb, const T *rd, T (&s)[32], int J0, In &in, Out &out)
+{
+#pragma unroll 1
+    for (int j = J0; j < J0 + 16; j += 4) {
+        const T *Lk = Lb + (j >> 2) * 128 + j * 4;
+        T r4[4], br[4];
+        c32_load4(rd + j, r4);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) br[r] = in(j + r) * r4[r];
+        const T l10 = Lk[4], l20 = Lk[8], l21 = Lk[9], l30 = Lk[12], l31 = Lk[13], l32 = Lk[14];
+        T x[4];
+        x[0] = fma(-s[0], r4[0], br[0]);
+        x[1] = fma(-fma(l10, x[0], s[1]), r4[1], br[1]);
+        s[2] = fma(l20, x[0], s[2]);
+        s[3] = fma(l30, x[0], s[3]);
+        x[2] = fma(-fma(l21, x[1], s[2]), r4[2], br[2]);
+        s[3] = fma(l31, x[1], s[3]);
+        x[3] = fma(-fma(l32, x[2], s[3]), r4[3], br[3]);
+#pragma unroll
+        for (int c = 4; c < LIVE; ++c) {
+            T v[4];
+            c32_load4(Lk + c * 4, v);
+            T y = s[c];
+            y = fma(v[0], x[0], y);
+            y = fma(v[1], x[1], y);
+            y = fma(v[2], x[2], y);
+            s[c - 4] = fma(v[3], x[3], y);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) out(j + r, x[r]);
+    }
+}
+template <typename T, class In, class Out>
+__device__ __forceinline__ void sweep32_sums(const T *Lb, const T *rd, In in, Out out)
+{
+    T s[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) s[c] = T(0);
+    sweep32_sums_half<T, 32>(Lb, rd, s, 0, in, out);
+    sweep32_sums_half<T, 16>(Lb, rd, s, 16, in, out);
 }
 
 }  // namespace db2

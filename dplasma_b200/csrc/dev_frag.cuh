@@ -58,6 +58,26 @@ __device__ __forceinline__ void frag_store(const double (&acc)[MI][NI][4], doubl
             for (int q = 0; q < 4; ++q)
                 p[(mi * 16 + g + ((q & 2) ? 8 : 0)) * rs + (ni * 8 + 2 * t + (q & 1)) * cs] = acc[mi][ni][q];
 }
+// element (r, c) at p[r * rs + c * cs] -= acc
+template <int MI, int NI>
+__device__ __forceinline__ void frag_sub(const double (&acc)[MI][NI][4], double *p, int rs, int cs, int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int mi = 0; mi < MI; ++mi) {
+        double old[NI][4];             // the loads may not pass the stores
+#pragma unroll
+        for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                old[ni][q] = p[(mi * 16 + g + ((q & 2) ? 8 : 0)) * rs + (ni * 8 + 2 * t + (q & 1)) * cs];
+#pragma unroll
+        for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                p[(mi * 16 + g + ((q & 2) ? 8 : 0)) * rs + (ni * 8 + 2 * t + (q & 1)) * cs] = old[ni][q] - acc[mi][ni][q];
+    }
+}
 template <int MI, int NI>
 __device__ __forceinline__ void frag_zero(double (&acc)[MI][NI][4])
 {

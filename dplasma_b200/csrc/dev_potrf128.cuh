@@ -12,6 +12,9 @@
 //     which needs the factor only.  The inverse of the diagonal block is the
 //     same sweep on the unit vectors, beside it on another warp, so no inverse is
 //     on the chain but the last block's;
+//   - every panel's products are summed by themselves and subtracted once:
+//     accumulated onto the block, each would be rounded at the block's size (a
+//     factor of 256 columns 2.1e-16 off instead of 1.2e-16, diagonally dominant);
 //   - while warp 0 updates and factors the next diagonal block the others update
 //     the rest, assemble the finished rows of the inverse and store what is done.
 // Measured in place: 34 us with load and stores; the form it replaces (block in
@@ -127,11 +130,16 @@ static __device__ __noinline__ int p128_diag_general(double *S, const double *T,
     const int p0 = 32 * j;
     double *Sd = S + p0 * SP + p0;
     {
+        // panel by panel, as the updates of potrf128_smem
         double acc[2][4][4];
         frag_load(acc, T + (int64_t)p0 * ld + p0, 1, ld, lane);
-        for (int l = 0; l < j; ++l) mma32(acc, S + l * 32 * SP + p0, SP, 1, S + l * 32 * SP + p0, SP, 1, true, lane);
         __syncwarp();
         frag_store(acc, Sd, 1, SP, lane);
+        for (int l = 0; l < j; ++l) {
+            frag_zero(acc);
+            mma32(acc, S + l * 32 * SP + p0, SP, 1, S + l * 32 * SP + p0, SP, 1, false, lane);
+            frag_sub(acc, Sd, 1, SP, lane);
+        }
         __syncwarp();
     }
     double d[32];
@@ -174,25 +182,26 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
             const int nrow = 3 - j;
             if (warp <= nrow) {
                 const bool inv = warp == nrow;
-                double b[32];
-                double *Xp = S + p0 * SP + (j + 1 + warp) * 32 + lane;
-#pragma unroll
-                for (int c = 0; c < 32; ++c) b[c] = inv ? (c == lane ? 1.0 : 0.0) : Xp[c * SP];
+                double *Xp = S + p0 * SP + (inv ? 0 : (j + 1 + warp) * 32) + lane;
                 double *o = inv ? D + j * 32 * DP + lane : Xp;
                 const int os = inv ? DP : SP;
-                sweep32(Lb, rd, b, [&](int c, double x) { o[c * os] = x; });
+                sweep32_sums<double>(Lb, rd, [&](int c) { return inv ? (c == lane ? 1.0 : 0.0) : Xp[c * SP]; },
+                                     [&](int c, double x) { o[c * os] = x; });
             }
         } else if (j < 4) {
             double *Sd = S + p0 * SP + p0;
             if (j > 0 && warp < 3) {
                 // the next diagonal block, one lower 16x16 quarter per warp
                 const int qr = warp == 0 ? 0 : 16, qc = warp == 2 ? 16 : 0;
-                double acc[1][2][4];
+                double old[1][2][4], acc[1][2][4];
                 double *C = Sd + qc * SP + qr;
-                frag_load(acc, C, 1, SP, lane);
+                frag_load(old, C, 1, SP, lane);
                 const double *X = S + (p0 - 32) * SP + p0;
-                mma32(acc, X + qr, SP, 1, X + qc, SP, 1, true, lane);
-                frag_store(acc, C, 1, SP, lane);
+                frag_zero(acc);
+                mma32(acc, X + qr, SP, 1, X + qc, SP, 1, false, lane);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) old[0][e >> 2][e & 3] -= acc[0][e >> 2][e & 3];
+                frag_store(old, C, 1, SP, lane);
                 if (warp > 0) named_bar_arrive(bar + 1, 96);
             }
             if (warp == 0) {
@@ -217,10 +226,9 @@ __device__ __forceinline__ int potrf128_smem(double *S, int *fail, double *T, in
                     const int bi = j + bk + rem;
                     bk += j;
                     double acc[2][4][4];
-                    double *C = S + bk * 32 * SP + bi * 32;
-                    frag_load(acc, C, 1, SP, lane);
-                    mma32(acc, X + bi * 32, SP, 1, X + bk * 32, SP, 1, true, lane);
-                    frag_store(acc, C, 1, SP, lane);
+                    frag_zero(acc);
+                    mma32(acc, X + bi * 32, SP, 1, X + bk * 32, SP, 1, false, lane);
+                    frag_sub(acc, S + bk * 32 * SP + bi * 32, 1, SP, lane);
                 }
                 put_jj = j - 1;
                 put_w = 5 - w;
@@ -271,11 +279,9 @@ __device__ __forceinline__ void p128_invert(double *S, double *LB4, int unit, do
         for (int c = 0; c < 32; ++c) Lb[(c >> 2) * 128 + lane * 4 + (c & 3)] = c <= lane ? Sd[c * SP] : 0.0;
         rd[lane] = unit ? 1.0 : 1.0 / Sd[lane * SP];
         __syncwarp();
-        double b[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) b[c] = c == lane ? 1.0 : 0.0;
         double *o = D + warp * 32 * DP + lane;
-        sweep32(Lb, rd, b, [&](int c, double x) { o[c * DP] = x; });
+        sweep32_sums<double>(Lb, rd, [&](int c) { return c == lane ? 1.0 : 0.0; },
+                             [&](int c, double x) { o[c * DP] = x; });
     } else {
         // W is zero above its diagonal blocks
 #pragma unroll 1

@@ -56,3 +56,16 @@ def test_batched_factor(gpu_ctx, n, count, dtype, u):
     for A, F in zip(mats, dev[:2]):
         err = relative_error(np.triu(F.cpu().numpy()).T, factor_extended(A))
         assert err <= bound(u, 15.5 + n / 64), err / u
+
+
+@pytest.mark.parametrize("n,nb", [(100, 256), (128, 128), (300, 256), (512, 128)])
+def test_dense_factor(gpu_ctx, n, nb):
+    # 128-wide blocks: 1.5 panels of 32 on average before an entry inside its block,
+    # and one subtraction per block column to the left of it
+    A = dominant(n, n)
+    buf = torch.from_numpy(A.copy()).cuda()
+    torch.cuda.synchronize()
+    d = db.attach(db.desc_general(n, n, nb, nb, storage=db.STORAGE_LAPACK, lda=n), buf)
+    assert gpu_ctx.dpotrf(db.Lower, d) == 0, gpu_ctx.last_error()
+    err = relative_error(np.triu(buf.cpu().numpy()).T, factor_extended(A))
+    assert err <= bound(2.0 ** -53, 15.5 + 1.5 + n / 256), err * 2.0 ** 53
