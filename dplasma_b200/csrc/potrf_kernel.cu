@@ -615,6 +615,84 @@ __device__ __forceinline__ void slab_job(const PotrfArgs &a, double *ring, uint6
 }
 
 // ---------------------------------------------------------------------------
+// consumers: a 32-row slab of the FP64 link L(k+1,k) = A(k+1,k) L(k,k)^-T, by
+// substitution over the four 32-column blocks of L(k,k),
+//     X_p = (A_p - sum_{q<p} X_q L_pq^T) D_p^T,   D_p = L_pp^-1 (diagonal blocks of W).
+// A product with W, the inverse of the whole block, takes as many operations, but
+// its error grows with the condition of 128 columns instead of 32 (the factor of
+// 256 columns of a squared-exponential kernel with nugget 1e-2: 6.0e-15 off, by
+// blocks 4.3e-15; N = 4096: 1.862 and 1.875 ms).  Everything is in flight at once, one group of copies per
+// block; a warp forms 16 x 8 of each 32 x 32 block.
+// ---------------------------------------------------------------------------
+constexpr int SLAB_STRIP_DOUBLES = BLK * SP + BLK * SL_AP + 32 * SL_AP;
+__device__ __forceinline__ void slab_strip(const PotrfArgs &a, double *ring, uint64_t t, const Job &jb)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tq = lane & 3;
+    const int r0 = jb.slab * SLAB_ROWS;
+    const double *L = tile_ptr(a, task_k(t), task_k(t));
+    double *Bs = ring;                    // L below its 32-wide diagonal blocks, D in them (column c at c * SP)
+    double *Xs = Bs + BLK * SP;           // A, then X (column c at c * SL_AP)
+    double *Ss = Xs + BLK * SL_AP;        // one block's right-hand sides
+    const int rb = 2 * (tid & 63), ra = 2 * (tid & 15);
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        if (rb >= 32 * q) {
+            const bool d = rb < 32 * q + 32;
+            const double *src = d ? jb.B : L;
+            const int ld = d ? jb.ldb : a.ld;
+#pragma unroll
+            for (int c = 32 * q + (tid >> 6); c < 32 * q + 32; c += 4)
+                cp_async16(Bs + c * SP + rb, src + (int64_t)c * ld + rb);
+        }
+#pragma unroll
+        for (int c = 32 * q + (tid >> 4); c < 32 * q + 32; c += 16)
+            cp_async16(Xs + c * SL_AP + ra, jb.A + (int64_t)c * jb.lda + r0 + ra);
+        cp_async_commit();
+    }
+    const int rw = (warp & 1) * 16 + g, n0 = (warp >> 1) * 8;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+        cp_async_wait(3 - p);
+        named_bar_sync(1, NCONS);         // block p's operands, and X of the blocks before
+        double *Xp = Xs + 32 * p * SL_AP;
+        double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+        const double *Ax = Xs + tq * SL_AP + rw, *Bl = Bs + tq * SP + 32 * p + n0 + g;
+#pragma unroll 4
+        for (int kk = 0; kk < 32 * p; kk += 8)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = kk + 4 * h;
+                dmma_16x8x4(acc[h], Ax[k * SL_AP], Ax[k * SL_AP + 8], Bl[k * SP]);
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = (n0 + 2 * tq + (e & 1)) * SL_AP + rw + ((e & 2) ? 8 : 0);
+            Ss[i] = Xp[i] - (acc[0][e] + acc[1][e]);
+            acc[0][e] = acc[1][e] = 0.0;
+        }
+        named_bar_sync(1, NCONS);
+        const double *As = Ss + tq * SL_AP + rw, *Bd = Bs + (32 * p + tq) * SP + 32 * p + n0 + g;
+#pragma unroll
+        for (int kk = 0; kk < 32; kk += 8)
+            if (kk <= n0) {               // D is lower triangular
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = kk + 4 * h;
+                    dmma_16x8x4(acc[h], As[k * SL_AP], As[k * SL_AP + 8], Bd[k * SP]);
+                }
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = n0 + 2 * tq + (e & 1), r = rw + ((e & 2) ? 8 : 0);
+            const double x = acc[0][e] + acc[1][e];
+            Xp[c * SL_AP + r] = x;
+            jb.C[(int64_t)(32 * p + c) * jb.ldc + r0 + r] = x;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // mixed precision, tensor-core TRSM: the whole inverse of L(k,k),
 //     Linv = [W0 0; Linv10 W1]   (W0, W1 the 128-block inverses, Linv10 = -W1 L10 W0),
 // as the B operand of the strips' products, B[n][q] = Linv(n, q) / t_q * s_b in
@@ -1213,7 +1291,8 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
             for (int j = 0; j < nj; ++j) {
                 const Job jb = task_job(a, t, j);
                 if (jb.slab >= 0) {
-                    slab_job<MIXED>(a, ring, t, jb);
+                    if (!MIXED && a.fchunk && ty == T_TRSM) slab_strip(a, ring, t, jb);
+                    else slab_job<MIXED>(a, ring, t, jb);
                     if (j + 1 < nj) named_bar_sync(1, NCONS);   // the next job reads C and takes the ring
                     continue;
                 }
@@ -1322,6 +1401,7 @@ size_t potrf_smem_bytes(bool mixed)
     static_assert(SL_NCH * SL_CHUNK <= NSTAGE * STAGE_DOUBLES &&
                       SL_NCH * SL_CHUNK * 8 <= MX_NST * MX_STAGE_BYTES,
                   "the ring holds a slab's operands");
+    static_assert(SLAB_STRIP_DOUBLES <= NSTAGE * STAGE_DOUBLES, "and a strip slab's");
     static_assert(NSTAGE * STAGE_DOUBLES >= P128_DOUBLES && MX_NST * MX_STAGE_BYTES >= P128_DOUBLES * 8,
                   "the ring holds POTRF's scratch");
     if (!mixed) return ctl + (size_t)NSTAGE * STAGE_DOUBLES * sizeof(double);

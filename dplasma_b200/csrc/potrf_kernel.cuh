@@ -20,7 +20,8 @@
 // unchanged.
 //
 // TRSM(m,k) uses the inverses of the 128x128 diagonal blocks of L(k,k),
-// computed by POTRF(k) into the workspace W: L(m,k) = A(m,k) W_k^T; the mixed
+// computed by POTRF(k) into the workspace W: L(m,k) = A(m,k) W_k^T, but the link
+// L(k+1,k), which is solved by 32-wide blocks (slab_strip); the mixed
 // kernel and the task pools solve the strip of a wider tile block-left-looking
 // (X_p = (A_p - sum_q X_q L_pq^T) W_pp^T), so all FP64 flops of the path run on
 // the tensor cores except POTRF's 32-wide factorizations and substitutions.

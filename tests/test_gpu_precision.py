@@ -69,3 +69,27 @@ def test_dense_factor(gpu_ctx, n, nb):
     assert gpu_ctx.dpotrf(db.Lower, d) == 0, gpu_ctx.last_error()
     err = relative_error(np.triu(buf.cpu().numpy()).T, factor_extended(A))
     assert err <= bound(2.0 ** -53, 15.5 + 1.5 + n / 256), err * 2.0 ** 53
+
+
+@pytest.mark.parametrize("n", [160, 256])
+def test_dense_link_residual(gpu_ctx, n):
+    # L11 bidiagonal with 1 and -1.25: the inverse of its 128 columns grows to
+    # 1.25^128 = 3e12, those of its 32-wide diagonal blocks to 5 * 1.25^32 = 6e3.  All
+    # entries are dyadic, so A is exact.  A solve of the rows below by 32-wide blocks
+    # leaves a residual of at most 32 u |D| |L| <= 32 u 2.25 * 6.4e3 times the rows; a
+    # product with the inverse of the whole block one about 3e12 u.
+    g = np.random.default_rng(n)
+    L = np.zeros((n, n))
+    i = np.arange(128)
+    L[i, i] = 1.0
+    L[i[1:], i[:-1]] = -1.25
+    L[128:, :128] = g.integers(-8, 9, (n - 128, 128)) / 8.0
+    L[128:, 128:] = 4.0 * np.eye(n - 128)
+    A = L @ L.T
+    buf = torch.from_numpy(A.copy()).cuda()
+    torch.cuda.synchronize()
+    d = db.attach(db.desc_general(n, n, 256, 256, storage=db.STORAGE_LAPACK, lda=n), buf)
+    assert gpu_ctx.dpotrf(db.Lower, d) == 0, gpu_ctx.last_error()
+    F = np.triu(buf.cpu().numpy()).T.astype(np.longdouble)
+    R = (A[128:, :128] - F[128:, :128] @ F[:128, :128].T).astype(np.float64)
+    assert np.linalg.norm(R) <= 32 * 2.0 ** -53 * 2.25 * 6.4e3 * np.linalg.norm(F[128:, :128].astype(np.float64))
