@@ -64,10 +64,14 @@ struct AgArgs {
     double *C;
     int ldc;
     double alpha;
-    // GRAD: out (n x n, both triangles, ld n) = g / 2 (al al^T - nal * product)
+    // GRAD: out (n x n, both triangles, ld n) = g / 2 (al al^T - nal * product);
+    // alt (null: al al^T in the epilogue): al^T, K contiguous, padded with zeros to
+    // nk = 16 ceil(nal / 16) by whole tiles, for al al^T as a product of its own
     const double *al, *g;
     int nal, n;
     double *out;
+    const double *alt;
+    int nk;
 };
 
 // C(i,j) = alpha * sum_{k in range} op(A)(i,k) B(k,j), 128x128 tiles; op is the
@@ -81,7 +85,8 @@ constexpr int AG_OP = 128 * AG_KP;                              // doubles of on
 constexpr size_t AG_SMEM = AG_NST * 2 * AG_OP * sizeof(double);
 static_assert(AG_K * AG_P <= AG_OP, "either form fits");
 
-template <bool TA>
+// COLS: GRAD with alt (al al^T first).
+template <bool TA, bool COLS>
 __global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
 {
     extern __shared__ __align__(16) double agsm[];
@@ -143,6 +148,7 @@ __global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
 
     const int kbeg = k0 * AG_T, kend = (k1 + 1) * AG_T;
     const double *Aop = a.A, *Bop = a.B;
+    int lda = a.lda, ldb = a.ldb;
     auto load = [&](int slot, int kc) {
         double *As = agsm + slot * 2 * AG_OP, *Bs = As + AG_OP;
         // four 16-byte pieces of each operand a thread
@@ -150,18 +156,30 @@ __global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
         for (int q = 0; q < 4; ++q) {
             if (!TA) {
                 const int r = 2 * (tid & 63), kk = (tid >> 6) + 4 * q;
-                cp_async16(As + kk * AG_P + r, Aop + (int64_t)(ako * AG_T + kc + kk) * a.lda + i * AG_T + r);
+                cp_async16(As + kk * AG_P + r, Aop + (int64_t)(ako * AG_T + kc + kk) * lda + i * AG_T + r);
             }
             const int kk = 2 * (tid & 7), r = (tid >> 3) + 32 * q;
-            if (TA) cp_async16(As + r * AG_KP + kk, Aop + (int64_t)(i * AG_T + r) * a.lda + ako * AG_T + kc + kk);
-            cp_async16(Bs + r * AG_KP + kk, Bop + (int64_t)(j * AG_T + r) * a.ldb + bko * AG_T + kc + kk);
+            if (TA) cp_async16(As + r * AG_KP + kk, Aop + (int64_t)(i * AG_T + r) * lda + ako * AG_T + kc + kk);
+            cp_async16(Bs + r * AG_KP + kk, Bop + (int64_t)(j * AG_T + r) * ldb + bko * AG_T + kc + kk);
         }
     };
-    // one pass over K, or two with the operands exchanged (SYM)
-    const int len = kend - kbeg, nch = (a.mode == AG_SYM_KGE_I ? 2 * len : len) / AG_K;
+    // one pass over K, or two with the operands exchanged (SYM), after nal chunks of
+    // al^T (GRAD with many columns)
+    const int len = kend - kbeg, nal = COLS ? a.nk / AG_K : 0;
+    const int nch = nal + (a.mode == AG_SYM_KGE_I ? 2 * len : len) / AG_K;
     auto stage = [&](int ch) {
-        if (ch < nch) {
-            const int at = ch * AG_K;
+        if (COLS && ch < nal) {
+            Aop = Bop = a.alt;
+            lda = ldb = a.nk;
+            load(ch % AG_NST, ch * AG_K);
+        } else if (ch < nch) {
+            const int at = (ch - nal) * AG_K;
+            if (COLS && at == 0) {
+                Aop = a.A;
+                Bop = a.B;
+                lda = a.lda;
+                ldb = a.ldb;
+            }
             if (at >= len) {
                 Aop = a.B;
                 Bop = a.A;
@@ -173,10 +191,27 @@ __global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
     constexpr int ar = TA ? AG_KP : 1, ak = TA ? 1 : AG_P;      // strides of a chunk of A
 #pragma unroll 1
     for (int ch = 0; ch < AG_NST - 1; ++ch) stage(ch);
+    // element (mi, ni, q) of this thread in the result
+    auto row = [&](int mi, int q) { return i * AG_T + wm * 64 + mi * 16 + g + ((q & 2) ? 8 : 0); };
+    auto col = [&](int ni, int q) { return j * AG_T + wn * 32 + ni * 8 + 2 * t + (q & 1); };
 #pragma unroll 1
     for (int ch = 0; ch < nch; ++ch) {
         cp_async_wait(AG_NST - 2);
         __syncthreads();                       // chunk ch is there, chunk ch - 1 is free
+        if (COLS && ch == nal) {
+            // al al^T is complete: it waits in the result's place (read back below by
+            // the thread that wrote it)
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int r = row(mi, q), c = col(ni, q);
+                        if (r < a.n && c < a.n) a.out[(int64_t)c * a.n + r] = acc[mi][ni][q];
+                        acc[mi][ni][q] = 0.0;
+                    }
+        }
         stage(ch + AG_NST - 1);
         const double *Ab = agsm + (ch % AG_NST) * 2 * AG_OP + (wm * 64 + g) * ar + t * ak;
         const double *Bb = agsm + (ch % AG_NST) * 2 * AG_OP + AG_OP + (wn * 32 + g) * AG_KP + t;
@@ -201,19 +236,30 @@ __global__ void __launch_bounds__(256, 1) ag_gemm_kernel(AgArgs a)
         // and the rank-m term as passes of their own took 1.1 ms of 14 at n = 6001
         const double hg = 0.5 * *a.g;
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
+        for (int mi = 0; mi < 4; ++mi) {
+            // (the stores below may not be passed by loads: those of 16 values first)
+            double s[4][4];
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int r = i * AG_T + wm * 64 + mi * 16 + g + ((q & 2) ? 8 : 0);
-                    const int c = j * AG_T + wn * 32 + ni * 8 + 2 * t + (q & 1);
-                    if (r >= a.n || c >= a.n) continue;
-                    double s = -(double)a.nal * acc[mi][ni][q];
-                    for (int l = 0; l < a.nal; ++l) s = fma(__ldg(a.al + (int64_t)l * a.n + r), __ldg(a.al + (int64_t)l * a.n + c), s);
-                    a.out[(int64_t)c * a.n + r] = hg * s;
-                    if (i != j) a.out[(int64_t)r * a.n + c] = hg * s;
+                    const int r = row(mi, q), c = col(ni, q);
+                    s[ni][q] = COLS && r < a.n && c < a.n ? a.out[(int64_t)c * a.n + r] : 0.0;
                 }
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = row(mi, q), c = col(ni, q);
+                    if (r >= a.n || c >= a.n) continue;
+                    double v = fma(-(double)a.nal, acc[mi][ni][q], s[ni][q]);
+                    if (!COLS)
+                        for (int l = 0; l < a.nal; ++l)
+                            v = fma(__ldg(a.al + (int64_t)l * a.n + r), __ldg(a.al + (int64_t)l * a.n + c), v);
+                    a.out[(int64_t)c * a.n + r] = hg * v;
+                    if (i != j) a.out[(int64_t)r * a.n + c] = hg * v;
+                }
+        }
         return;
     }
     double *C = a.C + (int64_t)(j * AG_T) * a.ldc + i * AG_T;
@@ -233,6 +279,8 @@ struct AgGrad {
     const double *al, *g;
     int nal, n;
     double *out;
+    const double *alt;
+    int nk;
 };
 static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, int lda, int transA, const double *B,
                    int ldb, double *C, int ldc, double alpha, const AgGrad *gr = nullptr)
@@ -243,6 +291,8 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
     a.nal = gr ? gr->nal : 0;
     a.n = gr ? gr->n : 0;
     a.out = gr ? gr->out : nullptr;
+    a.alt = gr ? gr->alt : nullptr;
+    a.nk = gr ? gr->nk : 0;
     a.mode = mode;
     a.P = P;
     a.rowblk = rowblk;
@@ -258,7 +308,8 @@ static int ag_gemm(Context *ctx, int mode, int P, int rowblk, const double *A, i
     if (mode == AG_LVL_T || mode == AG_LVL_W) ntile = a.nblk * rowblk * rowblk;
     else ntile = P * (P + 1) / 2;
     if (ntile <= 0) return 0;
-    auto fn = transA ? ag_gemm_kernel<true> : ag_gemm_kernel<false>;
+    auto fn = !transA ? ag_gemm_kernel<false, false>
+                      : a.alt ? ag_gemm_kernel<true, true> : ag_gemm_kernel<true, false>;
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AG_SMEM));
     fn<<<ntile, 256, AG_SMEM, ctx->stream>>>(a);
     CK(cudaGetLastError());
@@ -462,10 +513,38 @@ int inverse_tiles(Context *ctx, double *Lt, const Geom &g, int op, int unit, int
     return inverse_or_gradient(ctx, Lt, g, op, unit, info, nullptr);
 }
 
+// al^T (row l of alt's K is column l of al), zero beyond n rows and nal columns
+__global__ void __launch_bounds__(256) ag_transpose_pad(const double *al, int n, int nal, double *alt, int nk, int np)
+{
+    __shared__ double sm[32][33];
+    const int r0 = blockIdx.x * 32, l0 = blockIdx.y * 32, x = threadIdx.x & 31;
+    for (int y = threadIdx.x >> 5; y < 32; y += 8)
+        sm[y][x] = r0 + x < n && l0 + y < nal ? al[(int64_t)(l0 + y) * n + r0 + x] : 0.0;
+    __syncthreads();
+    for (int y = threadIdx.x >> 5; y < 32; y += 8)
+        if (r0 + y < np && l0 + x < nk) alt[(int64_t)(r0 + y) * nk + l0 + x] = sm[x][y];
+}
+
+// Columns of al from which al al^T is a product of its own.  In the epilogue each
+// column costs two loads and a multiply-add per element outside the tensor cores;
+// gradient of n = 4096 with 1 / 4 / 64 / 1024 columns, ms: in the epilogue 2.42 /
+// 2.66 / 2.84 / 8.04, as a product 2.45 / 2.41 / 2.50 / 3.04 (n = 1000: 0.68 / 0.73 /
+// 0.83 / 2.07 and 0.68 / 0.68 / 0.69 / 0.83).
+constexpr int AG_GRAD_COLS = 4;
 int gp_gradient_tiles(Context *ctx, double *Lt, const Geom &g, const double *al, int nal, const double *dg, double *out,
                       int *info)
 {
-    const AgGrad gr = {al, dg, nal, g.n, out};
+    AgGrad gr = {al, dg, nal, g.n, out, nullptr, 0};
+    if (nal >= AG_GRAD_COLS) {
+        const int np = g.mt * g.nbi;
+        gr.nk = (nal + AG_K - 1) / AG_K * AG_K;
+        double *alt = (double *)ctx->buffer(BUF_B, (size_t)np * gr.nk * sizeof(double));
+        if (!alt) return DPLASMA_ERR_OUT_OF_RESOURCES;
+        ag_transpose_pad<<<dim3(np / 32, (gr.nk + 31) / 32), 256, 0, ctx->stream>>>(al, g.n, nal, alt, gr.nk, np);
+        CK(cudaGetLastError());
+        ctx->launches++;
+        gr.alt = alt;
+    }
     return inverse_or_gradient(ctx, Lt, g, 2, 0, info, &gr);
 }
 

@@ -179,7 +179,8 @@ def test_batched_pivots_outside_the_fast_range(gpu_ctx, n, scale):
     assert factor_ratio(np.triu(m.cpu().numpy()).T / np.sqrt(scale), A) < 10.0
 
 
-@pytest.mark.parametrize("n,m", [(1, 1), (127, 1), (129, 2), (700, 1), (1500, 3)])
+@pytest.mark.parametrize("n,m", [(1, 1), (127, 1), (129, 2), (700, 1), (1500, 3), (1, 4), (130, 4), (130, 16),
+                                 (255, 17), (300, 700)])
 def test_gp_gradient(n, m):
     from dplasma_b200 import autograd as dag
     g = torch.Generator().manual_seed(n)
