@@ -835,8 +835,7 @@ extern "C" int dplasma_b200_sposv_batched(parsec_context_t *parsec, int batch, c
 extern "C" const char *dplasma_b200_batched_variant(const parsec_context_t *parsec)
 {
     if (!parsec) return "";
-    const Context *ctx = &parsec->impl;
-    return batched_variant_name(1, ctx->bt_last_variant);
+    return parsec->impl.bt_last_variant;
 }
 
 // ---------------------------------------------------------------------------

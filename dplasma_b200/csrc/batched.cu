@@ -18,12 +18,13 @@
 //      the FMA pipes), the next diagonal block first so that warp 0 factors
 //      it while the others finish the update.
 // What bounds a problem is the latency of these steps, so several problems
-// share an SM (bt_variants).  The solve ends with the backward sweep on the
+// share an SM where there are enough of them (bt_choose).  The solve ends with the backward sweep on the
 // factor in 32-row blocks; the log-determinant is 2 * sum log L(i,i).
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include <algorithm>
+#include <functional>
 #include <numeric>
 #include <vector>
 
@@ -525,36 +526,98 @@ struct BtVariant {
     const char *name;
     BtLaunch<T> fn;
 };
+// FP64 has the first three
 template <typename T>
-static const BtVariant<T> *bt_variants(int &count)
+static const BtVariant<T> *bt_variants();
+template <>
+const BtVariant<double> *bt_variants<double>()
 {
-    static const BtVariant<T> v[] = {
-        {"1 warp per problem", bt_launch<T, 32, 8>},
-        {"4 warps per problem", bt_launch<T, 128, 3>},
-        {"8 warps per problem", bt_launch<T, 256, 1>},
-        {"8 warps per problem, two per SM", bt_launch<T, 256, 2>},
-    };
-    count = (int)(sizeof(v) / sizeof(v[0]));
+    static const BtVariant<double> v[] = {{"1 warp per problem", bt_launch<double, 32, 8>},
+                                          {"4 warps per problem", bt_launch<double, 128, 3>},
+                                          {"8 warps per problem", bt_launch<double, 256, 1>}};
+    return v;
+}
+template <>
+const BtVariant<float> *bt_variants<float>()
+{
+    static const BtVariant<float> v[] = {{"1 warp per problem", bt_launch<float, 32, 8>},
+                                         {"4 warps per problem", bt_launch<float, 128, 3>},
+                                         {"8 warps per problem", bt_launch<float, 256, 1>},
+                                         {"8 warps per problem, two per SM", bt_launch<float, 256, 2>}};
     return v;
 }
 
-// Warps per problem: a problem's latency falls with its warps (large problems, and
-// batches that leave SMs idle), the work in flight on an SM rises with the
-// problems that share it (small ones).  Kernel times in ms on 148 SMs with 1 / 4 /
-// 8 / 8 warps two per SM:
-//   FP32, 8192 problems of 8 to 96:     0.338 / 0.432 / 0.955 / 0.570
-//   FP64, 1024 problems of 64 to 256:   0.614 / 0.391 / 0.482 / 0.520
-//   FP64, 4096 problems of 32 to 512:   22.4  / 9.6   / 5.45  / 7.7
-//   FP32, 2000 problems of 64 to 512:     -   / 2.60  / 2.60  / 2.26
-//   FP64, 2000 problems of 8 to 64:     0.081 / 0.130
-// (before, with the inverse of each diagonal block on the chain and the shapes timed
-// on the caller's batch: 0.78, 0.54, 7.6 for the first three).
-static int bt_choose(bool fp64, int batch, int nmax, int sms)
+// Warps per problem: a problem's latency falls with its warps, the work in flight on
+// an SM rises with the problems that share it.  The launch ends with whichever is
+// later, its largest problem or the last of its work:
+//   largest: `one` when it has the SM to itself, `full` when `per` like it share the
+//            SM, in between by the problems per SM of the batch;
+//   work:    sum of full / per over the problems, shared by the SMs.
+// The table holds kernel times in us of 148 problems of order 32, 64, 128, .. on 148
+// SMs and of per x 148.  On 419 batches (one order or uniform up to one, 1 to 4096
+// problems, many small ones with a few large) the choice costs 0.5 % on average and
+// 19 % at most over the best shape of each, where a rule by the largest order alone
+// cost up to 2.5 times (FP64, 500 of order 64 and 20 of 256: 294 us with four warps,
+// 115 with eight; FP32, 297 of 8 to 768: 2.97 ms with eight warps two per SM, 1.57
+// one per SM; FP32, 8192 of 8 to 96: 0.31 ms with one warp, 0.96 with eight).
+struct BtTimes {
+    int per;
+    float one[6], full[6];
+};
+constexpr float BT_LAUNCH = 6.f;              // of each time, once per launch
+static const BtTimes BT_TIMES_F64[] = {
+    {8, {24.4f, 44.f, 109.f, 394.f, 2370.f}, {33.9f, 64.8f, 241.f, 1390.f, 18800.f}},
+    {3, {24.2f, 41.6f, 77.5f, 207.f, 1080.f}, {26.3f, 45.2f, 97.9f, 342.f, 3210.f}},
+    {1, {18.1f, 28.4f, 49.3f, 115.f, 571.f}, {18.1f, 28.4f, 49.3f, 115.f, 571.f}}};
+static const BtTimes BT_TIMES_F32[] = {
+    {8, {20.f, 37.3f, 92.3f, 386.f, 2240.f, 16200.f}, {24.5f, 48.6f, 131.f, 854.f, 7280.f, 130000.f}},
+    {3, {16.6f, 24.2f, 42.9f, 136.f, 764.f, 5520.f}, {18.f, 28.1f, 59.5f, 231.f, 1410.f, 16500.f}},
+    {1, {16.2f, 22.5f, 38.8f, 106.f, 520.f, 3590.f}, {16.2f, 22.5f, 38.8f, 106.f, 520.f, 3590.f}},
+    {2, {16.4f, 24.f, 43.f, 144.f, 742.f, 5260.f}, {17.9f, 26.2f, 51.1f, 181.f, 983.f, 10500.f}}};
+
+// a row of the table at an order of b 32-wide blocks, by powers between its points
+static double bt_time(const float *y, int points, int b)
 {
-    if (batch <= 2 * sms) return 2;
-    if (nmax <= 96) return 0;
-    if (nmax <= 256) return 1;
-    return fp64 ? 2 : 3;
+    const double x = log2((double)std::max(b, 1));
+    const int i = std::min((int)x, points - 2);
+    return y[i] * pow((double)y[i + 1] / y[i], x - i);
+}
+
+// order(i): the i-th largest order
+template <class Order>
+static int bt_choose(bool fp64, int batch, int sms, Order order)
+{
+    const BtTimes *t = fp64 ? BT_TIMES_F64 : BT_TIMES_F32;
+    const int nv = fp64 ? 3 : 4, points = fp64 ? 5 : 6;
+    // problems by their 32-wide blocks
+    int count[BT_NMAX / BT_NB + 1] = {0};
+    const int top = batch > 0 ? (order(0) + BT_NB - 1) / BT_NB : 0;
+    for (int b = top, from = 0; b >= 0; --b) {
+        int lo = from, hi = batch;                 // the first beyond those of b blocks
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (order(mid) > (b - 1) * BT_NB) lo = mid + 1;
+            else hi = mid;
+        }
+        count[b] = lo - from;
+        from = lo;
+    }
+    int best = 0;
+    double best_us = 0.0;
+    for (int v = 0; v < nv; ++v) {
+        const double share = std::min((double)t[v].per, std::max(1.0, (double)batch / sms));
+        const double one = bt_time(t[v].one, points, top), full = bt_time(t[v].full, points, top);
+        const double largest = t[v].per > 1 ? one + (full - one) * (share - 1.0) / (t[v].per - 1) : one;
+        double work = 0.0;
+        for (int b = 0; b <= top; ++b)
+            if (count[b]) work += count[b] * (bt_time(t[v].full, points, b) - BT_LAUNCH);
+        const double us = std::max(largest, BT_LAUNCH + work / ((double)sms * t[v].per));
+        if (v == 0 || us < best_us) {
+            best = v;
+            best_us = us;
+        }
+    }
+    return best;
 }
 
 template <typename T>
@@ -601,30 +664,18 @@ int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *c
     a.info = d_info;
     a.order = dord;
     a.ticket = dord + batch + 32;
-    int nv = 0;
-    const BtVariant<T> *vars = bt_variants<T>(nv);
-    const int choice = bt_choose(sizeof(T) == 8, batch, nmax, ctx->sms);
+    const int choice = bt_choose(sizeof(T) == 8, batch, ctx->sms, [&](int i) { return hn[order[i]]; });
+    const BtVariant<T> &shape = bt_variants<T>()[choice];
     CK(cudaEventRecord(ctx->ev0, st));
-    const int rc = vars[choice].fn(ctx, a, nmax);
+    const int rc = shape.fn(ctx, a, nmax);
     if (rc) return rc;
-    ctx->bt_last_variant = choice;
+    ctx->bt_last_variant = shape.name;
     CK(cudaEventRecord(ctx->ev1, st));
     CK(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     ctx->last_factor_ms = ms;
     return 0;
-}
-
-const char *batched_variant_name(int fp64, int v)
-{
-    int nv = 0;
-    if (fp64) {
-        const BtVariant<double> *vs = bt_variants<double>(nv);
-        return (v >= 0 && v < nv) ? vs[v].name : "";
-    }
-    const BtVariant<float> *vs = bt_variants<float>(nv);
-    return (v >= 0 && v < nv) ? vs[v].name : "";
 }
 
 // ---------------------------------------------------------------------------
@@ -915,3 +966,11 @@ template int batched_posv<float>(Context *, int, const int *, const int *, float
                                  double *, int *);
 
 }  // namespace db2
+
+// Test hook (not part of the public header): the launch shape of a batch of orders n
+extern "C" int dplasma_b200_debug_batched_choice(int fp64, int sms, int batch, const int *n)
+{
+    std::vector<int> sorted(n, n + batch);
+    std::sort(sorted.begin(), sorted.end(), std::greater<int>());
+    return db2::bt_choose(fp64 != 0, batch, sms, [&](int i) { return sorted[i]; });
+}

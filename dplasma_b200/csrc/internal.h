@@ -82,7 +82,7 @@ struct Context {
     long long last_tasks_executed = 0;
     long long last_tickets = 0, last_tickets_bad = 0;   // self check of the last factorization
     int inject_kind = 0, inject_arg = -1;                // one-shot fault injection of the next factorization
-    int bt_last_variant = -1;
+    const char *bt_last_variant = "";        // name of the last batched launch's shape
     char errmsg[512] = {0};
     char trace_path[512] = {0};   // DPLASMA_B200_TRACE: per-task timestamps of the scheduler
     char wave_trace_path[512] = {0};   // DPLASMA_B200_WAVE_TRACE: per-sweep summary of the triangular sweeps
@@ -201,7 +201,6 @@ int gp_gradient_tiles(Context *ctx, double *Lt, const Geom &g, const double *al,
 template <typename T>
 int batched_posv(Context *ctx, int batch, const int *d_n, const int *d_lda, T *const *d_A, T *const *d_B, int nrhs,
                  double *d_logdet, int *d_info);
-const char *batched_variant_name(int fp64, int v);
 // d_alpha (may be null), d_g, d_out: the GP gradient instead of the inverse
 int batched_potri(Context *ctx, int batch, const int *d_n, const int *d_lda, double *const *d_A, int *d_info,
                   const double *const *d_alpha = nullptr, const double *d_g = nullptr, double *const *d_out = nullptr);

@@ -387,7 +387,7 @@ int dplasma_dpotrf_adjoint(parsec_context_t *parsec, dplasma_enum_t uplo, const 
  * n[i], overwritten by X_i; B itself or B[i] may be NULL to factor only);
  * logdet (double[batch], 2 sum log L_i(j,j); NaN when INFO > 0; may be
  * NULL); info (int[batch], LAPACK INFO of each problem).  The warps per
- * problem follow from the largest order and the batch.  Returns 0 or a
+ * problem follow from the orders and the batch.  Returns 0 or a
  * negative code. */
 int dplasma_b200_dposv_batched(parsec_context_t *parsec, int batch, const int *n, const int *lda,
                                double *const *A, double *const *B, int nrhs, double *logdet, int *info);

@@ -141,11 +141,12 @@ def test_sweep_passes_nans_on(gpu_ctx):
     assert np.isnan(X[0]).all() and np.isnan(X[1]).all() and (X[2] == 0).all()
 
 
-@pytest.mark.parametrize("count,lo,hi,dtype,nrhs", [
-    (700, 1, 96, "f64", 1), (700, 90, 96, "f32", 3), (600, 97, 256, "f64", 2), (600, 97, 256, "f32", 16),
-    (320, 257, 300, "f64", 1), (320, 257, 300, "f32", 1), (3, 500, 512, "f64", 1), (3, 1000, 1024, "f32", 1),
-    (40, 1, 70, "f64", 4)])
-def test_batched_shapes(gpu_ctx, count, lo, hi, dtype, nrhs):
+@pytest.mark.parametrize("count,lo,hi,dtype,nrhs,shape", [
+    (1200, 90, 96, "f64", 1, "1 warp"), (1300, 80, 96, "f32", 3, "1 warp"), (700, 1, 96, "f64", 1, "4 warps"),
+    (700, 90, 96, "f32", 3, "4 warps"), (600, 97, 256, "f64", 2, "8 warps"), (600, 97, 256, "f32", 16, "two per SM"),
+    (320, 257, 300, "f64", 1, "8 warps"), (320, 257, 300, "f32", 1, "two per SM"), (3, 500, 512, "f64", 1, "8 warps"),
+    (3, 1000, 1024, "f32", 1, "8 warps"), (40, 1, 70, "f64", 4, "8 warps")])
+def test_batched_shapes(gpu_ctx, count, lo, hi, dtype, nrhs, shape):
     # kernels with nugget 1: condition <= n + 1, so solutions agree to about n eps times that
     dt = torch.float64 if dtype == "f64" else torch.float32
     g = torch.Generator().manual_seed(count + hi)
@@ -160,6 +161,7 @@ def test_batched_shapes(gpu_ctx, count, lo, hi, dtype, nrhs):
     rhs = [y.to(dt).cuda() for y in ys]
     info, logdet = gpu_ctx.posv_batched(mats, rhs)
     assert (info == 0).all()
+    assert shape in gpu_ctx.batched_variant()          # every kernel of bt_variants is among these
     u = EPS if dtype == "f64" else 2.0 ** -24
     for n, K, y, m, r, ld in zip(sizes, Ks, ys, mats, rhs, logdet):
         L = torch.linalg.cholesky(K)

@@ -47,7 +47,7 @@ def bound(u, m):
 
 
 @pytest.mark.parametrize("dtype,u", [(np.float64, 2.0 ** -53), (np.float32, 2.0 ** -24)])
-@pytest.mark.parametrize("n,count", [(96, 400), (200, 400), (256, 40), (512, 3)])      # the shapes of the batched kernel
+@pytest.mark.parametrize("n,count", [(96, 1400), (96, 400), (200, 700), (300, 290), (512, 3)])   # every shape
 def test_batched_factor(gpu_ctx, n, count, dtype, u):
     mats = [dominant(n, s, dtype) for s in range(2)]
     dev = [torch.from_numpy(mats[i % 2].copy()).cuda() for i in range(count)]
