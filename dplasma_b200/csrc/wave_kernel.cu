@@ -860,6 +860,7 @@ __global__ void __launch_bounds__(WV_THREADS, 1)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             wv_send(Xp + (ni * 8 + 2 * t + (e & 1)) * 128 + ((e & 2) ? rb : ra), acc[ni][e]);
+    if (a.trace && group == 0 && tid == 0) a.trace[(int64_t)P * WV_TR_SLOTS + p] = globaltimer_ns();
 #pragma unroll
     for (int ni = 0; ni < NT; ++ni)
 #pragma unroll
@@ -956,7 +957,7 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
     // swizzle span) by 32 (forward: k columns) or 128 (backward: columns).
     // the critical path's products W_b L_{b,b-1} (or L_{b+1,b} W_b)
     // (one block per CTA: also W_b L_{b,b-2})
-    const bool chain = sh.gsub == nblk && !ctx->wave_trace_path[0];
+    const bool chain = sh.gsub == nblk;
     const int nd = chain ? 2 : 1;
     double *M = (double *)ctx->buffer(BUF_WM, (size_t)nd * nblk * 128 * 128 * sizeof(double));
     if (!M) return DPLASMA_ERR_OUT_OF_RESOURCES;
@@ -1021,8 +1022,8 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
                             : launch_wave<32, false>(ctx, a, cta, chain, lmap, wmap, mmap);
         if (rc) return rc;
         if (a.trace) {
-            // one line per sweep: CTA-summed ns per part, and the mean step of
-            // the wavefront (ns between consecutive publishes) per eighth of the blocks
+            // one line per sweep: CTA-summed ns per part (trsm_wave_kernel), and the mean
+            // step of the wavefront (ns between consecutive publishes) per eighth of the blocks
             std::vector<unsigned long long> h((size_t)sh.gsub * WV_TR_SLOTS + nblk);
             CK(cudaMemcpyAsync(h.data(), a.trace, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                                ctx->stream));
@@ -1031,15 +1032,14 @@ int trsm_wave(Context *ctx, const double *dA, const double *W, const Geom &g, do
             for (int b = 0; b < sh.gsub; ++b)
                 for (int k = 0; k < WV_TR_SLOTS; ++k) sum[k] += h[(size_t)b * WV_TR_SLOTS + k];
             if (FILE *f = fopen(ctx->wave_trace_path, "a")) {
-                fprintf(f, "sweep trans %d nblk %d nc %d cta_ns wait %llu stage %llu crit %llu deferred %llu znext %llu "
+                fprintf(f, "sweep %s trans %d nblk %d nc %d cta_ns wait %llu stage %llu crit %llu deferred %llu znext %llu "
                            "rest %llu positions %llu steps_ns",
-                        transposed, nblk, nc, sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6]);
+                        chain ? "chain" : "wave", transposed, nblk, nc, sum[0], sum[1], sum[2], sum[3], sum[4], sum[5], sum[6]);
                 const unsigned long long *pt = h.data() + (size_t)sh.gsub * WV_TR_SLOTS;
                 for (int e = 0; e < 8; ++e) {
                     const int q0 = e * nblk / 8, q1 = (e + 1) * nblk / 8;
                     const int b0 = transposed ? nblk - 1 - q0 : q0, b1 = transposed ? nblk - q1 : q1 - 1;
-                    const long long d = (long long)pt[b1] - (long long)pt[b0];
-                    fprintf(f, " %lld", q1 - 1 > q0 ? d / (q1 - 1 - q0) : 0);
+                    fprintf(f, " %lld", q1 - 1 > q0 ? ((long long)pt[b1] - (long long)pt[b0]) / (q1 - 1 - q0) : 0ll);
                 }
                 fprintf(f, "\n");
                 fclose(f);

@@ -96,6 +96,29 @@ def test_sweep_shapes(gpu_ctx, n, nrhs, uplo):
     assert r / ((np.abs(A).sum(1).max() * np.abs(X).sum(1).max() + np.abs(B).sum(1).max()) * n * EPS) < 10.0
 
 
+def test_sweep_trace_is_of_the_sweep_that_runs(tmp_path, monkeypatch):
+    # one block per CTA: the traced sweep is the chain, and gives the untraced results
+    n, nrhs = 4096, 8
+    A = spd(n, n)
+    B = np.random.default_rng(2).uniform(-0.5, 0.5, (nrhs, n))
+    out = []
+    for path in ("", str(tmp_path / "wave")):
+        monkeypatch.setenv("DPLASMA_B200_WAVE_TRACE", path)
+        with db.Context(0) as ctx:
+            d, buf = dev_desc(A, 256, db.Lower, True)
+            b = torch.from_numpy(B.copy()).cuda()
+            torch.cuda.synchronize()
+            e = db.attach(db.desc_general(n, nrhs, 256, 256, storage=db.STORAGE_LAPACK, lda=n), b)
+            assert ctx.dposv(db.Lower, d, e) == 0, ctx.last_error()
+            out.append(b)
+    assert torch.equal(out[0], out[1])
+    lines = (tmp_path / "wave").read_text().splitlines()
+    assert [l.split()[:4] for l in lines] == [["sweep", "chain", "trans", "0"], ["sweep", "chain", "trans", "1"]]
+    for l in lines:
+        steps = [int(v) for v in l.split("steps_ns")[1].split()]
+        assert len(steps) == 8 and all(0 < s < 1000000 for s in steps)
+
+
 def test_sweep_exchange_buffer_is_bounded():
     # many columns go through the sweep in turns: the workspace is the padded
     # right-hand sides and a bounded exchange buffer, not a second copy of them;
