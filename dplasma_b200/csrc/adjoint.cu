@@ -25,9 +25,6 @@
 // x = A^-1 b gives Abar = -A^-1 xbar x^T (symmetrized) and bbar = A^-1 xbar.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <vector>
-
 #include "dev_common.cuh"
 #include "dev_potrf128.cuh"
 #include "internal.h"
@@ -436,17 +433,15 @@ int potrf_adjoint_tiles(Context *ctx, const double *Lt, double *Lbt, const Geom 
 // inverses: trtri, lauum, potri on the device tiles (lower, padded), in place
 // ---------------------------------------------------------------------------
 // first zero pivot of the diagonal (1-based, 0 if none): LAPACK dtrtri INFO
-__global__ void ag_zero_pivot(const double *L, int ld, int n_valid_rows, const int *rowmap, int *info)
+__global__ void ag_zero_pivot(const double *L, int ld, int n, int *info)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_valid_rows; i += gridDim.x * blockDim.x) {
-        const int ip = rowmap ? rowmap[i] : i;
-        if (L[(int64_t)ip * ld + ip] == 0.0) atomicMin(info, i + 1);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        if (L[(int64_t)i * ld + i] == 0.0) atomicMin(info, i + 1);
 }
 
-// op: 0 trtri (L -> L^-1), 1 lauum (L -> L^T L), 2 potri (L -> (L L^T)^-1);
-// nb/nbi/n describe which padded rows are real (for the INFO of trtri).
-// gr (op 2, may be null): the GP gradient is written instead of Lt (whole tiles: nb == nbi).
+// op: 0 trtri (L -> L^-1), 1 lauum (L -> L^T L), 2 potri (L -> (L L^T)^-1), on whole
+// tiles (work_geom: nb == nbi, row i of the caller is row i of the tiles).
+// gr (op 2, may be null): the GP gradient is written instead of Lt.
 static int inverse_or_gradient(Context *ctx, double *Lt, const Geom &g, int op, int unit, int *info, const AgGrad *gr)
 {
     const int Np = g.mt * g.nbi, P = Np / AG_T, ld = Np;
@@ -462,19 +457,10 @@ static int inverse_or_gradient(Context *ctx, double *Lt, const Geom &g, int op, 
     ctx->launches++;
     *info = 0;
     if (op != 1 && !unit) {
-        // zero pivots (real rows only: row i of the caller is padded row (i/nb)*nbi + i%nb)
         int *dinfo = (int *)(scr);
         const int big = 0x7fffffff;
         CK(cudaMemcpyAsync(dinfo, &big, sizeof(int), cudaMemcpyHostToDevice, st));
-        // a row map is only needed when nb < nbi; build it on the host
-        int *dmap = nullptr;
-        if (g.nb != g.nbi) {
-            std::vector<int> map(g.n);
-            for (int i = 0; i < g.n; ++i) map[i] = (i / g.nb) * g.nbi + i % g.nb;
-            dmap = dinfo + 32;
-            CK(cudaMemcpyAsync(dmap, map.data(), g.n * sizeof(int), cudaMemcpyHostToDevice, st));
-        }
-        ag_zero_pivot<<<ctx->sms, 256, 0, st>>>(L, ld, g.n, dmap, dinfo);
+        ag_zero_pivot<<<ctx->sms, 256, 0, st>>>(L, ld, g.n, dinfo);
         CK(cudaGetLastError());
         int h = big;
         CK(cudaMemcpyAsync(&h, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
