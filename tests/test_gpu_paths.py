@@ -41,7 +41,8 @@ def factor_ratio(L, A):
     (1, 1, "L", False), (31, 32, "L", False), (33, 128, "U", True), (127, 128, "L", True), (129, 93, "U", False),
     (256, 200, "L", False),            # as many tiles of 128 as of 200: still two layouts
     (257, 256, "L", True), (640, 128, "L", False), (1000, 320, "U", True), (1536, 512, "L", False),
-    (6400, 128, "L", False)])          # 50 blocks: six panels per update task
+    (6400, 128, "L", False),           # 50 blocks: four panels per update task
+    (7937, 256, "L", True)])           # 63 blocks, the last one a single row: six panels
 def test_factor_shapes(gpu_ctx, n, nb, uplo, lapack):
     A = spd(n, n)
     up = db.Lower if uplo == "L" else db.Upper
@@ -54,6 +55,18 @@ def test_factor_shapes(gpu_ctx, n, nb, uplo, lapack):
     # the other triangle of what is stored is not touched
     other = np.triu if uplo == "L" else np.tril
     assert np.array_equal(other(out, 1 if uplo == "L" else -1), other(before, 1 if uplo == "L" else -1))
+
+
+@pytest.mark.parametrize("panels", [1, 3, 6, 12, 15])
+def test_factor_panels_per_update(panels, monkeypatch):
+    # the counts that large orders take, and others, on one of 18 blocks (the last chunk
+    # of a column is open)
+    monkeypatch.setenv("DPLASMA_B200_F64_CHUNK", str(panels))
+    A = spd(2200, panels)
+    with db.Context(0) as ctx:
+        d, buf = dev_desc(A, 256, db.Lower, True)
+        assert ctx.dpotrf(db.Lower, d) == 0, ctx.last_error()
+    assert factor_ratio(np.tril(db.unpack(buf.cpu().numpy(), d)), A) < 10.0
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -990, 2.0 ** 990])
