@@ -300,14 +300,14 @@ def bench_adjoint(torch):
     batch = {"problems": 1024, "n": "uniform integer in [64, 256], seed 13", "forward_ms": tb_f,
              "forward_backward_ms": tb_fb, "dlengthscale": float(lsb.grad),
              "note": "wall clock including the kernel-matrix construction (se_kernel_batched, flat form) and the gradient "
-                     "assembly; library part: one dplasma_b200_dposv_batched and one dplasma_b200_dpotri_batched "
-                     "launch"}
+                     "assembly; library part: one dplasma_b200_dposv_batched and one "
+                     "dplasma_b200_gp_gradient_batched launch"}
     return {"n": n, "forward_ms": t_f, "forward_backward_ms": t_fb, "backward_over_forward": t_fb / t_f - 1.0,
             "batch": batch,
             "forward_tflops": flops_f / (t_f * 1e-3) / 1e12, "value": float(v), "dlengthscale": float(ls.grad),
             "cholesky_adjoint_ms": t_adj,
-            "note": "GP backward = dplasma_dpotri for K^-1 (the log-det adjoint; 2/3 N^3 FP64 tensor-core flops) "
-                    "and rank-1 terms; forward = dplasma_dpotrf + dplasma_dpotrs; cholesky_adjoint_ms = "
+            "note": "GP backward = dplasma_b200_gp_gradient: K^-1 from the factor (the log-det adjoint; 2/3 N^3 FP64 "
+                    "tensor-core flops), its last product written as the gradient; forward = dplasma_dpotrf + dplasma_dpotrs; cholesky_adjoint_ms = "
                     "dplasma_dpotrf_adjoint for a dense lower Lbar (autograd.cholesky backward, about 1.3 N^3 flops)"}
 
 

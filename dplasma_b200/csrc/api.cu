@@ -253,8 +253,8 @@ extern "C" double dplasma_b200_fp64_peak_tflops(parsec_context_t *p)
 static int potrf_impl(Context *ctx, dplasma_enum_t uplo, parsec_tiled_matrix_t *A, double **factor_out, Geom *gout,
                       int nb_tasks = 0)
 {
-    // nb_tasks: tile edge of the task DAG when it differs from the caller's
-    // tiles (the recursive variant's sub-tiles); 0 = the caller's
+    // nb_tasks: tile edge to factor on when it differs from the caller's tiles
+    // (the recursive variant's sub-tiles); 0 = the caller's
     const int nbt = nb_tasks > 0 ? nb_tasks : A->mb;
     const Geom gc = make_geom(A->m, nbt);
     Geom g = work_geom(A->m, nbt);
@@ -333,9 +333,10 @@ extern "C" int dplasma_b200_taskpool_run(parsec_context_t *parsec, parsec_taskpo
 // src/zpotrf_wrapper.c:425-451.  The reference splits each task on an NB tile
 // into a sub-DAG on hmb x hmb sub-tiles (src/zpotrf_L.jdf:168-192, the
 // RECURSIVE bodies); the sub-tiles of every task together are the flat tile
-// algorithm with tile edge hmb, which is what runs here: the device
-// scheduler's tasks are built on hmb tiles (copied from and back to the
-// caller's NB tiles).  hmb <= 0 or hmb >= NB factors on the NB tiles.
+// algorithm with tile edge hmb, which is what runs here, on a copy in hmb tiles (128
+// where hmb is no multiple of it).  The scheduler's tasks are 128x128 blocks whatever
+// the edge, so hmb changes the layout and the INFO checks, not the schedule.
+// hmb <= 0 or hmb >= NB factors on the NB tiles.
 extern "C" int dplasma_dpotrf_rec(parsec_context_t *parsec, dplasma_enum_t uplo, parsec_tiled_matrix_t *A, int hmb)
 {
     if (uplo != dplasmaUpper && uplo != dplasmaLower) {

@@ -791,14 +791,6 @@ __device__ void linv16_task(const PotrfArgs &a, int k, const double *Wk, const d
     named_bar_sync(1, NCONS);
 }
 
-// ---------------------------------------------------------------------------
-// consumers: POTRF(k) of one diagonal tile + inverses of its 128x128 diagonal
-// blocks (src/zpotrf_L.jdf:194-206 computes the factor with
-// LAPACKE_dpotrf_work; the inverses feed the TRSM jobs).
-// Blocked right-looking with 32-column panels: one warp factors the 32x32
-// diagonal block in shared memory and inverts it, the panel solve and the
-// trailing update run on the FP64 tensor cores.
-// ---------------------------------------------------------------------------
 // Streamed matrix: the updates accumulated in A (from zero); the consumer
 // threads add the untouched copy of `rows` rows from row r0 of tile (m, k)
 // (all its columns) before the task that factors or solves it reads them.
@@ -816,6 +808,15 @@ __device__ __forceinline__ void stream_add_rows(const PotrfArgs &a, int m, int k
     }
 }
 
+// ---------------------------------------------------------------------------
+// consumers: POTRF(k) of one diagonal tile + inverses of its 128x128 diagonal
+// blocks (src/zpotrf_L.jdf:194-206 computes the factor with
+// LAPACKE_dpotrf_work; the inverses feed the TRSM jobs).
+// Block by block: the 128x128 factor and its inverse in shared memory
+// (potrf128_smem: 32-wide panels, rows solved by substitution), then, in a wider
+// tile, the strips below as products with that inverse and the update of the
+// blocks to the right.  The FP64 order has 128-wide tiles only.
+// ---------------------------------------------------------------------------
 template <bool MIXED>
 __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k)
 {

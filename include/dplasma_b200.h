@@ -149,11 +149,11 @@ void dplasma_dpotrf_Destruct(parsec_taskpool_t *tp);
 int dplasma_b200_taskpool_run(parsec_context_t *parsec, parsec_taskpool_t *tp);
 
 /* dplasma_dpotrf_rec / _setrecursive: src/zpotrf_wrapper.c:425-451
- * (dplasma_z.h:83, 273).  With 0 < hmb < NB the tasks of the factorization
- * run on hmb x hmb sub-tiles (the reference's recursive bodies split each NB
+ * (dplasma_z.h:83, 273).  With 0 < hmb < NB the factorization runs on a copy
+ * in hmb x hmb sub-tiles (the reference's recursive bodies split each NB
  * tile task into a sub-DAG on hmb tiles, src/zpotrf_L.jdf:168-192; together
- * they are the tile algorithm with tile edge hmb); the caller's NB tiles are
- * copied to and from that layout.  Otherwise the same as dplasma_dpotrf.
+ * they are the tile algorithm with tile edge hmb), 128 wide where hmb is no
+ * multiple of 128; the tasks are 128x128 blocks whatever the edge.  Otherwise the same as dplasma_dpotrf.
  * _setrecursive sets hmb for a taskpool made by dplasma_dpotrf_New. */
 int dplasma_dpotrf_rec(parsec_context_t *parsec, dplasma_enum_t uplo, parsec_tiled_matrix_t *A, int hmb);
 void dplasma_dpotrf_setrecursive(parsec_taskpool_t *tp, int hmb);
