@@ -316,6 +316,69 @@ __device__ __forceinline__ void p128_load(double *S, const double *T, int ld, bo
     }
 }
 
+// A = A L^-T in place for 128 rows beside a factored block, 16 rows per warp, by
+// substitution over the four 32-wide blocks of L as potrf128_smem left it in S (X_p =
+// (A_p - sum_{q<p} X_q L_pq^T) D_p^T).  A product with the 128-wide inverse is faster
+// (p128_rows; a 256-wide tile takes 142 us against 132), but its error grows with the condition of 128 columns;
+// the FP64 tiles of the task pools and the allocation-free entry take this one.  X
+// goes through L2 between the steps; only this warp touches its rows.
+__device__ __forceinline__ void p128_solve_rows(const double *S, double *A, int ld, int warp, int lane)
+{
+    constexpr int SP = P128_SP, DP = P128_DP;
+    const int g = lane >> 2, t = lane & 3;
+    double *Ar = A + warp * 16 + g;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+        double acc[4][4], a[8][2];
+        double *Ap = Ar + (int64_t)(32 * p) * ld;
+        auto at = [&](int n4, int e) { return Ap + (int64_t)(8 * n4 + 2 * t + (e & 1)) * ld + ((e & 2) ? 8 : 0); };
+        auto operand = [&](int b) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) a[q][h] = __ldcg(Ar + (int64_t)(32 * b + 4 * q + t) * ld + 8 * h);
+        };
+#pragma unroll
+        for (int n4 = 0; n4 < 4; ++n4)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n4][e] = 0.0;
+#pragma unroll 1
+        for (int b = 0; b < p; ++b) {
+            operand(b);
+            const double *Bl = S + (32 * b + t) * SP + 32 * p + g;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int n4 = 0; n4 < 4; ++n4) dmma_16x8x4(acc[n4], a[q][0], a[q][1], Bl[4 * q * SP + 8 * n4]);
+        }
+        if (p > 0) {
+#pragma unroll
+            for (int n4 = 0; n4 < 4; ++n4)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n4][e] = __ldcg(at(n4, e)) - acc[n4][e];
+#pragma unroll
+            for (int n4 = 0; n4 < 4; ++n4)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) *at(n4, e) = acc[n4][e];
+            __syncwarp();
+        }
+        operand(p);
+        __syncwarp();
+        const double *Dl = S + P128_S + (32 * p + g) * DP + t;
+#pragma unroll
+        for (int n4 = 0; n4 < 4; ++n4) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n4][e] = 0.0;
+#pragma unroll
+            for (int q = 0; q < 2 * n4 + 2; ++q)             // D is lower triangular
+                dmma_16x8x4(acc[n4], a[q][0], a[q][1], Dl[8 * n4 * DP + 4 * q]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) *at(n4, e) = acc[n4][e];
+        }
+        __syncwarp();
+    }
+}
+
 // One 128x128x128 product inside a diagonal tile, 16 rows per warp, all 128
 // columns (64 accumulators a thread), A from L2 and B from S:
 //   strip   C = A W^T with the inverse as potrf128_smem left it in S (K block

@@ -814,10 +814,10 @@ __device__ __forceinline__ void stream_add_rows(const PotrfArgs &a, int m, int k
 // LAPACKE_dpotrf_work; the inverses feed the TRSM jobs).
 // Block by block: the 128x128 factor and its inverse in shared memory
 // (potrf128_smem: 32-wide panels, rows solved by substitution), then, in a wider
-// tile, the strips below as products with that inverse and the update of the
-// blocks to the right.  The FP64 order has 128-wide tiles only.
+// tile, the strips below (mixed: products with that inverse; SUBST: substitution)
+// and the update of the blocks to the right.  The FP64 order has 128-wide tiles only.
 // ---------------------------------------------------------------------------
-template <bool MIXED>
+template <bool MIXED, bool SUBST>
 __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -850,12 +850,13 @@ __device__ void potrf_task(const PotrfArgs &a, SmemCtl *ctl, double *ring, int k
             return;
         }
         if (b + 1 == a.nbs) break;
-        // the rest of the tile: strips X_i = A_ib W_b^T, then C_ij -= X_i X_j^T
+        // the rest of the tile: strips X_i = A_ib L_bb^-T, then C_ij -= X_i X_j^T
         // with X_j in shared memory
 #pragma unroll 1
         for (int i = b + 1; i < a.nbs; ++i) {
             double *Ai = T + (int64_t)b * BLK * nbi + i * BLK;
-            p128_rows(true, false, ring, Ai, Ai, nbi, warp, lane);
+            if (SUBST) p128_solve_rows(ring, Ai, nbi, warp, lane);
+            else p128_rows(true, false, ring, Ai, Ai, nbi, warp, lane);
         }
         named_bar_sync(1, NCONS);
         phase(1);
@@ -1234,7 +1235,7 @@ __device__ bool tc_trsm(const PotrfArgs &a, SmemCtl *ctl, unsigned char *ring16,
 // that ORs the failure flags of all consumer warps, so no warp is ever left
 // waiting alone at a named barrier.
 // ---------------------------------------------------------------------------
-template <bool MIXED>
+template <bool MIXED, bool SUBST>
 __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
 {
     const int tid = threadIdx.x;
@@ -1266,7 +1267,7 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
                 stream_add_rows(a, k, k, 0, a.nbi);
                 named_bar_sync(1, NCONS);
             }
-            potrf_task<MIXED>(a, ctl, ring, k);
+            potrf_task<MIXED, SUBST>(a, ctl, ring, k);
             if (ctl->fail < 0) release = a.potrf_done + k;
         } else if (ty == T_TRSM && tc_strip<MIXED>(a, k, m)) {
             ok = tc_trsm(a, ctl, ring16, t, st16, mx_it, tcuse);
@@ -1338,8 +1339,13 @@ __device__ void consumer_warps(const PotrfArgs &a, SmemCtl *ctl, double *ring)
 // (setmaxnreg.inc to CONSUMER_REGS): 4*32*48 + 8*32*224 = 63488 <= 384*168, and
 // per sub-partition 1*32*48 + 2*32*224 = 15872 <= 16384.
 // MIXED: the trailing updates run on the 16-bit tensor cores (tmap describes
-// the 16-bit panel copies); the FP64 instantiation ignores tmap.
-template <bool MIXED>
+// the 16-bit panel copies); the FP64 instantiations ignore tmap.
+// SUBST: the strips inside a diagonal tile of several 128x128 blocks by substitution
+// (FP64 tiles of the task pools and the allocation-free entry).  The block order has
+// one block per tile; its instantiation keeps the loop over them all the same, as
+// without it the compiler lays the kernel out so that N = 4096 takes 1.91 ms instead
+// of 1.87.
+template <bool MIXED, bool SUBST>
 __global__ void __launch_bounds__(NTHREADS, 1)
     potrf_persistent_kernel(PotrfArgs a, const __grid_constant__ CUtensorMap tmap,
                             const __grid_constant__ CUtensorMap lmap)
@@ -1383,7 +1389,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(CONSUMER_REGS));
         if (MIXED) tc_fence_after();
-        consumer_warps<MIXED>(a, ctl, ring);
+        consumer_warps<MIXED, SUBST>(a, ctl, ring);
         if (MIXED) {
             // every consumer warp leaves the loop at the same point
             tc_fence_before();
@@ -1903,11 +1909,11 @@ int potrf_run(Context *ctx, double *dA, int mt, int nbi, int nb_user, int n_user
         p16_scale_kernel<<<mt, nbi, 0, st>>>(dA, mt, nbi, a.p16_target, a.scl);
         CK(cudaGetLastError());
         ctx->launches += 1;
-        CK(cudaFuncSetAttribute(potrf_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        potrf_persistent_kernel<true><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
+        CK(cudaFuncSetAttribute(potrf_persistent_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        potrf_persistent_kernel<true, false><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
     } else {
-        CK(cudaFuncSetAttribute(potrf_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        potrf_persistent_kernel<false><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
+        CK(cudaFuncSetAttribute(potrf_persistent_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        potrf_persistent_kernel<false, false><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, st));
@@ -2070,7 +2076,7 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     memset(&lmap, 0, sizeof(lmap));
     if (tc && (e = setup_tc_trsm(ctx, a, &lmap, mt)) != 0) return e;
     const size_t smem = potrf_smem_bytes(true);
-    CK(cudaFuncSetAttribute(potrf_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(potrf_persistent_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
     struct Evs {
         std::vector<cudaEvent_t> v;
@@ -2120,7 +2126,7 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
     // One launch in the ordinary ticket order: the updates never wait for
     // data, POTRF(k) and the strips of column k wait for column k's phase.
     // The columns of phase p are one contiguous run of tiles.
-    potrf_persistent_kernel<true><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
+    potrf_persistent_kernel<true, false><<<grid, NTHREADS, smem, st>>>(a, tmap, lmap);
     CK(cudaGetLastError());
     ctx->launches += 1;
     auto tile_of_col = [&](int c) { return c < mt ? (size_t)lower_tile_index(c, c, mt) : ntl; };
@@ -2160,20 +2166,22 @@ int potrf_run_streamed(Context *ctx, const double *hA, double *A0, double *L, in
 }  // namespace db2
 
 namespace db2 {
-template <bool MIXED>
+template <bool MIXED, bool SUBST>
 static int max_blocks_per_sm()
 {
     const size_t smem = potrf_smem_bytes(MIXED);
-    if (cudaFuncSetAttribute(potrf_persistent_kernel<MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return 0;
+    const auto fn = potrf_persistent_kernel<MIXED, SUBST>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, potrf_persistent_kernel<MIXED>, NTHREADS, smem) != cudaSuccess)
-        return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, NTHREADS, smem) != cudaSuccess) return 0;
     return n;
 }
-int potrf_max_blocks_per_sm(bool mixed) { return mixed ? max_blocks_per_sm<true>() : max_blocks_per_sm<false>(); }
-int potrf_max_blocks_per_sm() { return max_blocks_per_sm<false>(); }
+int potrf_max_blocks_per_sm(bool mixed)
+{
+    return mixed ? max_blocks_per_sm<true, false>()
+                 : std::min(max_blocks_per_sm<false, false>(), max_blocks_per_sm<false, true>());
+}
+int potrf_max_blocks_per_sm() { return potrf_max_blocks_per_sm(false); }
 }  // namespace db2
 
 // ---------------------------------------------------------------------------
@@ -2283,10 +2291,10 @@ int potrf_launch_prealloc(cudaStream_t st, double *dA, int mt, int nbi, int nb_u
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));
     const size_t smem = potrf_smem_bytes(false);
-    if (cudaFuncSetAttribute(potrf_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(potrf_persistent_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
         return DPLASMA_ERR_UNEXPECTED;
-    potrf_persistent_kernel<false><<<grid, NTHREADS, smem, st>>>(a, tmap, tmap);
+    potrf_persistent_kernel<false, true><<<grid, NTHREADS, smem, st>>>(a, tmap, tmap);
     if (cudaGetLastError() != cudaSuccess) return DPLASMA_ERR_UNEXPECTED;
     int hs[8];
     if (cudaMemcpyAsync(hs, ctr, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess) return DPLASMA_ERR_UNEXPECTED;

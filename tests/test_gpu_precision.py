@@ -10,6 +10,8 @@ off by at most about u / sqrt(3) sqrt(m / 4 + 1).  The products of a panel of 32
 columns are summed by themselves and subtracted once; inside a 32-wide diagonal
 block the columns are subtracted one after the other (15.5 on average).  Were
 every product rounded at the size of a(i,i), m would be n / 2."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -71,13 +73,10 @@ def test_dense_factor(gpu_ctx, n, nb):
     assert err <= bound(2.0 ** -53, 15.5 + 1.5 + n / 256), err * 2.0 ** 53
 
 
-@pytest.mark.parametrize("n", [160, 256])
-def test_dense_link_residual(gpu_ctx, n):
-    # L11 bidiagonal with 1 and -1.25: the inverse of its 128 columns grows to
-    # 1.25^128 = 3e12, those of its 32-wide diagonal blocks to 5 * 1.25^32 = 6e3.  All
-    # entries are dyadic, so A is exact.  A solve of the rows below by 32-wide blocks
-    # leaves a residual of at most 32 u |D| |L| <= 32 u 2.25 * 6.4e3 times the rows; a
-    # product with the inverse of the whole block one about 3e12 u.
+def growing(n):
+    """A = L L^T, exact (all entries dyadic), with L bidiagonal (1 and -1.25) in its
+    first 128 columns: the inverse of those grows to 1.25^128 = 3e12, the inverses of
+    their 32-wide diagonal blocks to 5 * 1.25^32 = 6e3."""
     g = np.random.default_rng(n)
     L = np.zeros((n, n))
     i = np.arange(128)
@@ -85,11 +84,28 @@ def test_dense_link_residual(gpu_ctx, n):
     L[i[1:], i[:-1]] = -1.25
     L[128:, :128] = g.integers(-8, 9, (n - 128, 128)) / 8.0
     L[128:, 128:] = 4.0 * np.eye(n - 128)
-    A = L @ L.T
-    buf = torch.from_numpy(A.copy()).cuda()
+    return L @ L.T
+
+
+@pytest.mark.parametrize("entry,n,nb", [("potrf", 160, 256), ("potrf", 256, 256), ("dtd", 256, 256), ("noalloc", 256, 256),
+                                        ("noalloc", 512, 512)])
+def test_rows_below_an_ill_conditioned_block(gpu_ctx, entry, n, nb):
+    # A solve of the rows below by 32-wide blocks leaves a residual of at most
+    # 32 u |D| |L| <= 32 u 2.25 * 6.4e3 times the rows; a product with the inverse of
+    # the 128 columns one of about 3e12 u.
+    A = growing(n)
+    if entry == "potrf":
+        d = db.desc_general(n, n, nb, nb, storage=db.STORAGE_LAPACK, lda=n)
+    else:
+        d = db.desc_sym(n, nb, db.Lower)
+    buf = torch.from_numpy(db.pack(np.asfortranarray(A), d)).cuda()
     torch.cuda.synchronize()
-    d = db.attach(db.desc_general(n, n, 256, 256, storage=db.STORAGE_LAPACK, lda=n), buf)
-    assert gpu_ctx.dpotrf(db.Lower, d) == 0, gpu_ctx.last_error()
-    F = np.triu(buf.cpu().numpy()).T.astype(np.longdouble)
+    db.attach(d, buf)
+    if entry == "noalloc":
+        rc = db.lib().dplasma_b200_dpotrf_noalloc(None, db.Lower, ctypes.byref(d))
+    else:
+        rc = (gpu_ctx.dpotrf if entry == "potrf" else gpu_ctx.dpotrf_dtd)(db.Lower, d)
+    assert rc == 0, gpu_ctx.last_error()
+    F = np.tril(db.unpack(buf.cpu().numpy(), d)).astype(np.longdouble)
     R = (A[128:, :128] - F[128:, :128] @ F[:128, :128].T).astype(np.float64)
     assert np.linalg.norm(R) <= 32 * 2.0 ** -53 * 2.25 * 6.4e3 * np.linalg.norm(F[128:, :128].astype(np.float64))
