@@ -319,9 +319,10 @@ __device__ __forceinline__ void p128_load(double *S, const double *T, int ld, bo
 // A = A L^-T in place for 128 rows beside a factored block, 16 rows per warp, by
 // substitution over the four 32-wide blocks of L as potrf128_smem left it in S (X_p =
 // (A_p - sum_{q<p} X_q L_pq^T) D_p^T).  A product with the 128-wide inverse is faster
-// (p128_rows; a 256-wide tile takes 142 us against 132), but its error grows with the condition of 128 columns;
-// the FP64 tiles of the task pools and the allocation-free entry take this one.  X
-// goes through L2 between the steps; only this warp touches its rows.
+// (p128_rows; a 256-wide tile takes 132 us with it, 142 with this), but its error grows
+// with the condition of 128 columns; the FP64 tiles of the task pools and the
+// allocation-free entry take this one.  X goes through L2 between the steps; only this
+// warp touches its rows.
 __device__ __forceinline__ void p128_solve_rows(const double *S, double *A, int ld, int warp, int lane)
 {
     constexpr int SP = P128_SP, DP = P128_DP;

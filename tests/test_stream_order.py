@@ -51,7 +51,7 @@ def test_barrier_between_the_addition_and_potrf():
     start = src.index("void consumer_warps(")
     body = src[start:src.index("__launch_bounds__", start)]
     add = body.index("stream_add_rows(a, k, k")
-    between = body[add:body.index("potrf_task<MIXED>(", add)]
+    between = body[add:body.index("potrf_task<MIXED", add)]
     assert "named_bar_sync(1, NCONS)" in between
     # the strips' additions end in a barrier (slabs) or in the producer's mbarrier
     strip = body[body.index("stream_add_rows(a, m, k"):]
