@@ -17,7 +17,7 @@
 //     factor of 256 columns 2.1e-16 off instead of 1.2e-16, diagonally dominant);
 //   - while warp 0 updates and factors the next diagonal block the others update
 //     the rest, assemble the finished rows of the inverse and store what is done.
-// Measured in place: 34 us with load and stores; the form it replaces (block in
+// Measured in place: 35 us with load and stores; the form it replaces (block in
 // L2, inverse on the chain, a panel per barrier) took 123 us where its code was
 // cold and about 75 us warm.
 #pragma once
